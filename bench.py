@@ -148,7 +148,7 @@ def algorithmic_bytes(kernel, model_cfg, n_atoms, n_bonds, slots):
             return (16.0 + 4.0 + 12.0 + 4.0 * 4 * CR) * n_bonds + (4.0 * nq * CR + 4.0 * 4 * CR + 48.0 + 16.0) * n_atoms
     if kernel == "nl_compact":            # list entry (j, S) and positions in, record + slot out
         return (8.0 + 16.0 + 4.0) * slots + 24.0 * n_atoms
-    if kernel == "force_gather_kernel":   # bond force and reverse index in, force out
+    if kernel == "finish_kernel":   # bond force and reverse index in, force out
         return (12.0 + 4.0 + 12.0) * slots + 24.0 * n_atoms
     return None
 

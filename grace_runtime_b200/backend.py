@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import sys
 
 import numpy as np
 
@@ -121,15 +122,15 @@ def _check(rc):
 
 
 def _ptr(a):
-    return None if a is None else a.ctypes.data_as(C.c_void_p)
+    return None if a is None else a.__array_interface__["data"][0]
 
 
 def _len_of(a, name):
+    if hasattr(a, "shape"):
+        return int(a.shape[0])
     cai = getattr(a, "__cuda_array_interface__", None)
     if cai is not None:
         return int(cai["shape"][0])
-    if hasattr(a, "shape"):
-        return int(a.shape[0])
     raise ValueError(f"{name}: the atom count must be given with raw device addresses")
 
 
@@ -353,6 +354,18 @@ def _dev_ptr(a, name, dtype, shape, optional=False):
         if int(a) == 0 and optional:
             return None
         return C.c_void_p(int(a))
+    torch = sys.modules.get("torch")
+    if torch is not None and isinstance(a, torch.Tensor) and a.is_cuda and not a.requires_grad:
+        # the same checks on the tensor itself: its __cuda_array_interface__ is a dictionary built anew at 5 us per argument
+        if a.dtype is not (torch.float64 if dtype is np.float64 else torch.int32):
+            raise ValueError(f"{name} must have dtype {np.dtype(dtype).name} (no conversion is made)")
+        if a.shape != shape:
+            raise ValueError(f"{name}: wrong shape {tuple(a.shape)}, expected {tuple(shape)}")
+        if not a.is_contiguous():
+            raise ValueError(f"{name} must be C-contiguous")
+        if a.get_device() != device():
+            raise ValueError(f"{name} must be on the module's GPU (cuda:{device()})")
+        return C.c_void_p(a.data_ptr())
     cai = getattr(a, "__cuda_array_interface__", None)
     if cai is not None:
         if cai.get("typestr") != _TYPESTR[np.dtype(dtype)]:
@@ -503,12 +516,12 @@ class System:
         n = len(types)
         positions = _as(positions, np.float64, (n, 3))
         cell = _as(cell, np.float64, (3, 3))
-        pbc = _as(np.asarray(pbc).astype(bool), np.uint8, (3,))
+        pbc = _as(np.asarray(pbc).astype(bool).view(np.uint8), np.uint8, (3,))
         flags = (FLAG_ENERGIES if energies else 0) | (FLAG_ENERGY_ONLY if energy_only else 0) | (FLAG_UQ if uq else 0)
         e = np.zeros(1)
         v = np.zeros(6)
-        f = None if energy_only else np.zeros((n, 3))
-        ea = np.zeros(n) if energies else None
+        f = None if energy_only else np.empty((n, 3))
+        ea = np.empty(n) if energies else None
         if uq:
             g, sg, cl = np.zeros(n), np.zeros(n), np.zeros(n)
             _check(_lib.grace_system_set_uq_outputs(self._h, _ptr(g), _ptr(sg), _ptr(cl)))
@@ -537,7 +550,7 @@ class System:
             n = _len_of(types, "types")
         n = int(n)
         cell = _as(cell, np.float64, (3, 3))
-        pbc = _as(np.asarray(pbc).astype(bool), np.uint8, (3,))
+        pbc = _as(np.asarray(pbc).astype(bool).view(np.uint8), np.uint8, (3,))
         e = _dev_ptr(energy, "energy", np.float64, (1,))
         f = _dev_ptr(forces, "forces", np.float64, (n, 3), optional=True)
         v = _dev_ptr(virial, "virial", np.float64, (6,), optional=True)
@@ -680,8 +693,8 @@ class Batch:
         flags = (FLAG_ENERGIES if energies else 0) | (FLAG_ENERGY_ONLY if energy_only else 0) | (FLAG_UQ if uq else 0)
         e = np.zeros(nsys)
         v = np.zeros((nsys, 6))
-        f = None if energy_only else np.zeros((ntot, 3))
-        ea = np.zeros(ntot) if energies else None
+        f = None if energy_only else np.empty((ntot, 3))
+        ea = np.empty(ntot) if energies else None
         if uq:
             g, sg, cl = np.zeros(ntot), np.zeros(ntot), np.zeros(ntot)
             _check(_lib.grace_batch_set_uq_outputs(self._h, _ptr(g), _ptr(sg), _ptr(cl)))

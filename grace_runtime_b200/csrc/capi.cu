@@ -122,6 +122,7 @@ int grace_finalize(void)
       if (e->e) e->e->release();
     comm_finalize();
     cudaStreamSynchronize(d.stream);
+    device_pool_trim();
     cudaStreamDestroy(d.stream);
     d.stream = nullptr;
     d.initialized = false;
@@ -281,6 +282,7 @@ void grace_model_free(grace_model *m)
 {
   std::lock_guard<std::recursive_mutex> lk(g_device_mu);
   delete m;
+  device_pool_trim();
 }
 
 int grace_system_create(const grace_model *m, const char *const *species, int n_species, double skin, int spline,
@@ -390,13 +392,13 @@ int grace_system_release_buffers(grace_system *s)
   return guarded([&] {
     if (!s) throw InvalidArgument("system must be given");
     s->s->release();
+    device_pool_trim();
   });
 }
 int grace_system_stage_ms(const grace_system *s, double *ms5)
 {
   if (!s || !ms5) return GRACE_INVALID_ARGUMENT;
-  for (int k = 0; k < 5; k++) ms5[k] = s->s->stage_ms[k];
-  return GRACE_OK;
+  return guarded([&] { const_cast<grace_system *>(s)->s->stage_ms(ms5); });
 }
 void grace_system_free(grace_system *s)
 {
@@ -498,6 +500,7 @@ int grace_batch_release_buffers(grace_batch *b)
   return guarded([&] {
     if (!b) throw InvalidArgument("batch must be given");
     b->b->release();
+    device_pool_trim();
   });
 }
 void grace_batch_free(grace_batch *b)

@@ -622,39 +622,6 @@ void launch_chunk_from_rows_f64(float *t, const double *rows, int nf, int C, int
             C, NA, na, a0, ilist);
 }
 
-// ---- forces: gather of the bond forces of an atom and of their reverse bonds, no atomics ------------------------
-// one warp per atom: F_i = sum_q fv[q] - fv[rev[q]] over the slots q of atom i (fp64 sum of the fp32 bond forces)
-__global__ void __launch_bounds__(128) force_gather_kernel(const long long *__restrict__ off,
-                                                           const int *__restrict__ rev, const float *__restrict__ fv,
-                                                           const int *__restrict__ perm, double *forces, int n)
-{
-  const int i = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-  const int lane = threadIdx.x & 31;
-  if (i >= n) return;    // whole warps leave together
-  double f0 = 0.0, f1 = 0.0, f2 = 0.0;
-  for (long long q = off[i] + lane; q < off[i + 1]; q += 32) {
-    const long long p = rev[q];
-    f0 += (double) fv[3 * q] - (double) fv[3 * p];
-    f1 += (double) fv[3 * q + 1] - (double) fv[3 * p + 1];
-    f2 += (double) fv[3 * q + 2] - (double) fv[3 * p + 2];
-  }
-  for (int s = 16; s > 0; s >>= 1) {
-    f0 += __shfl_xor_sync(0xffffffffu, f0, s);
-    f1 += __shfl_xor_sync(0xffffffffu, f1, s);
-    f2 += __shfl_xor_sync(0xffffffffu, f2, s);
-  }
-  if (lane == 0) {
-    double *o = forces + 3 * (size_t) perm[i];
-    o[0] = f0; o[1] = f1; o[2] = f2;
-  }
-}
-
-void launch_force_gather(const long long *off, const int *rev, const float *fv, const int *perm, double *forces, int n)
-{
-  if (n == 0) return;
-  GB_LAUNCH(force_gather_kernel, (n + 3) / 4, 128, 0, off, rev, fv, perm, forces, n);
-}
-
 // one warp per atom j: lanes over the `width` floats of a row, the atom's bonds one after the other
 __global__ void __launch_bounds__(128) msg_grad_gather_kernel(BondsDev b, const int *__restrict__ rev,
                                                               const float *__restrict__ gslot, float *gmsg, int width,
@@ -760,23 +727,6 @@ void launch_add_f64(const double *v, double *out, long long n)
 }
 
 // ---- per-structure sums (deterministic: fixed tree per segment) ------------------------------------------------
-// one block per (segment, component)
-__global__ void __launch_bounds__(256) segment_sum_kernel(const double *__restrict__ v, int K,
-                                                          const int *__restrict__ seg, double *out)
-{
-  __shared__ double sh[256];
-  const int s = blockIdx.x, k = blockIdx.y;
-  double acc = 0.0;
-  for (int i = seg[s] + threadIdx.x; i < seg[s + 1]; i += blockDim.x) acc += v[(size_t) i * K + k];
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  for (int st = 128; st > 0; st >>= 1) {
-    if ((int) threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[(size_t) s * K + k] = sh[0];
-}
-
 // few long segments (one large structure): NB blocks per (segment, component) write partial sums over equal slices
 // of the segment, a second launch adds them in slice order - still a fixed tree
 __global__ void __launch_bounds__(256) segment_partial_kernel(const double *__restrict__ v, int K,
@@ -809,25 +759,73 @@ __global__ void __launch_bounds__(32) segment_final_kernel(const double *__restr
 void launch_segment_sum(const double *v, int K, const int *seg, int nseg, double *out, double *scratch, int nb)
 {
   if (nseg == 0) return;
-  if (scratch && nb > 1) {
-    GB_LAUNCH(segment_partial_kernel, dim3(nseg, K, nb), 256, 0, v, K, seg, scratch);
-    GB_LAUNCH(segment_final_kernel, nseg * K, 32, 0, scratch, nb, out);
+  GB_LAUNCH(segment_partial_kernel, dim3(nseg, K, nb), 256, 0, v, K, seg, scratch);
+  GB_LAUNCH(segment_final_kernel, nseg * K, 32, 0, scratch, nb, out);
+}
+
+// What leaves an evaluation, in one launch: blocks [0, nsum) add the per-atom energies and virial rows of a structure
+// each (seven columns at once, by a fixed tree), the others give a warp per atom that gathers its
+// force in list order and moves its per-atom values to the caller's order; the error words of the call are
+// collected beside the sums so that one copy brings everything to the host.  Bound by launch latency for small
+// structures, where this was up to nine launches and copies of 2 - 7 us each.
+__global__ void __launch_bounds__(256) finish_kernel(FinishDev F, int nsum)
+{
+  const int t = threadIdx.x;
+  if ((int) blockIdx.x < nsum) {
+    __shared__ double sh[7][256];
+    const int s = blockIdx.x, lo = F.seg[s], hi = F.seg[s + 1];
+    double acc[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int i = lo + t; i < hi; i += 256) {
+      acc[0] += F.e_atom[i];
+      if (F.virial) {
+#pragma unroll
+        for (int k = 0; k < 6; k++) acc[1 + k] += F.vir_atom[6 * (size_t) i + k];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 7; k++) sh[k][t] = acc[k];
+    __syncthreads();
+    for (int st = 128; st > 0; st >>= 1) {
+      if (t < st)
+#pragma unroll
+        for (int k = 0; k < 7; k++) sh[k][t] += sh[k][t + st];
+      __syncthreads();
+    }
+    if (t == 0 && F.energy) F.energy[s] = sh[0][0];
+    if (t < 6 && F.virial) F.virial[6 * (size_t) s + t] = sh[1 + t][0];
     return;
   }
-  GB_LAUNCH(segment_sum_kernel, dim3(nseg, K), 256, 0, v, K, seg, out);
+  const int b = (int) blockIdx.x - nsum, i = b * 8 + (t >> 5), lane = t & 31;
+  if (b == 0 && t == 0 && F.status) {
+    const int f = F.nl_flag[0] | F.nl_flag[1], e = F.tc_flag ? *F.tc_flag : 0;
+    F.status[0] = F.first ? f : F.status[0] | f;
+    F.status[1] = F.first ? e : F.status[1] | e;
+  }
+  if (i >= F.n) return;
+  const size_t at = F.perm[i];
+  if (F.forces) {
+    double f0 = 0.0, f1 = 0.0, f2 = 0.0;
+    for (long long q = F.off[i] + lane; q < F.off[i + 1]; q += 32) {
+      const long long p = F.rev[q];
+      f0 += (double) F.fv[3 * q] - (double) F.fv[3 * p];
+      f1 += (double) F.fv[3 * q + 1] - (double) F.fv[3 * p + 1];
+      f2 += (double) F.fv[3 * q + 2] - (double) F.fv[3 * p + 2];
+    }
+    for (int s = 16; s > 0; s >>= 1) {
+      f0 += __shfl_xor_sync(0xffffffffu, f0, s);
+      f1 += __shfl_xor_sync(0xffffffffu, f1, s);
+      f2 += __shfl_xor_sync(0xffffffffu, f2, s);
+    }
+    if (lane < 3) F.forces[3 * at + lane] = lane == 0 ? f0 : lane == 1 ? f1 : f2;
+  }
+  if (lane == 0 && F.energies) F.energies[at] = F.e_atom[i];
+  if (F.uq && lane < 3) (lane == 0 ? F.gamma : lane == 1 ? F.sigma : F.cluster)[at] = F.uq[(size_t) lane * F.n + i];
 }
 
-__global__ void __launch_bounds__(256) scatter_f64_kernel(const double *__restrict__ v, const int *__restrict__ perm,
-                                                          double *out, int n)
+void launch_finish(const FinishDev &F, int nsum)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[perm[i]] = v[i];
-}
-
-void launch_scatter_f64(const double *v, const int *perm, double *out, int n)
-{
-  if (n == 0) return;
-  GB_LAUNCH(scatter_f64_kernel, (n + 255) / 256, 256, 0, v, perm, out, n);
+  const int atom_blocks = F.forces || F.energies || F.uq ? (F.n + 7) / 8 : 1;
+  GB_LAUNCH(finish_kernel, nsum + atom_blocks, 256, 0, F, nsum);
 }
 
 }    // namespace gb

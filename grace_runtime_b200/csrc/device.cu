@@ -116,17 +116,76 @@ void after_launch(const char *name)
   if (e != cudaSuccess) cuda_check(e, name);
 }
 
+namespace {
+constexpr size_t POOL_BLOCK = (size_t) 256 << 20, POOL_TOTAL = (size_t) 1 << 30;
+std::mutex g_pool_mu;
+std::multimap<size_t, void *> g_pool;    // free blocks by size
+std::map<void *, size_t> g_block;        // size of every block that came from the driver
+size_t g_pool_bytes = 0;
+
+// a pooled block of at least `bytes` that wastes at most as much again (small ones: 64 KB), or null
+void *pool_take(size_t bytes)
+{
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  auto it = g_pool.lower_bound(bytes);
+  if (it == g_pool.end() || it->first > 2 * bytes + ((size_t) 64 << 10)) return nullptr;
+  void *p = it->second;
+  g_pool_bytes -= it->first;
+  g_pool.erase(it);
+  return p;
+}
+
+void driver_free(void *p)
+{
+  if (g_dev.initialized) cudaFree(p);
+}
+
+void pool_give(void *p)
+{
+  {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    auto it = g_block.find(p);
+    if (it != g_block.end() && it->second <= POOL_BLOCK && g_pool_bytes + it->second <= POOL_TOTAL && g_dev.initialized) {
+      g_pool.emplace(it->second, p);
+      g_pool_bytes += it->second;
+      return;
+    }
+    if (it != g_block.end()) g_block.erase(it);
+  }
+  driver_free(p);
+}
+}    // namespace
+
+void device_pool_trim()
+{
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  for (auto &kv : g_pool) {
+    g_block.erase(kv.second);
+    driver_free(kv.second);
+  }
+  g_pool.clear();
+  g_pool_bytes = 0;
+}
+
 void *device_alloc(size_t bytes, const char *label)
 {
   require_initialized();
   if (bytes == 0) bytes = 16;
-  void *p = nullptr;
-  GB_CUDA(cudaMalloc(&p, bytes));
+  void *p = pool_take(bytes);
+  if (!p) {
+    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+      (void) cudaGetLastError();
+      device_pool_trim();
+      GB_CUDA(cudaMalloc(&p, bytes));
+    }
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    g_block[p] = bytes;
+  }
   // the injected failure comes after the allocation, as the reference's hook does (kk_core.cpp:128-141): the buffer is
-  // returned to the device before the error is raised
+  // returned before the error is raised
   if (g_dev.fail_alloc_nth > 0 && label && std::strstr(label, g_dev.fail_label.c_str()) != nullptr &&
       --g_dev.fail_alloc_nth == 0) {
-    cudaFree(p);
+    pool_give(p);
     throw OutOfMemory(std::string("out of device memory (injected) allocating '") + label + "'");
   }
   g_live[p] = bytes;
@@ -152,7 +211,29 @@ void device_free(void *p)
     g_tracked_bytes -= tr->second.second;
     g_tracked.erase(tr);
   }
-  if (g_dev.initialized) cudaFree(p);
+  pool_give(p);
+}
+
+char *PinnedBuf::ensure(size_t bytes)
+{
+  if (bytes <= cap_) return p_;
+  release();
+  const size_t want = bytes + bytes / 2 + 4096;
+  void *p = nullptr;
+  if (cudaMallocHost(&p, want) != cudaSuccess) {
+    (void) cudaGetLastError();
+    return nullptr;
+  }
+  p_ = static_cast<char *>(p);
+  cap_ = want;
+  return p_;
+}
+
+void PinnedBuf::release()
+{
+  if (p_ && g_dev.initialized) cudaFreeHost(p_);
+  p_ = nullptr;
+  cap_ = 0;
 }
 
 size_t device_bytes_live() { return g_live_bytes; }
@@ -163,47 +244,47 @@ StageTimer::~StageTimer()
   for (auto e : pool_) cudaEventDestroy(e);
 }
 
-cudaEvent_t StageTimer::take()
+int StageTimer::mark()
 {
+  if (used_ > 0 && at_launch_ == g_dev.launches) return (int) used_ - 1;    // nothing launched since the last event
   if (used_ == pool_.size()) {
     cudaEvent_t e;
     GB_CUDA(cudaEventCreate(&e));
     pool_.push_back(e);
   }
-  return pool_[used_++];
+  GB_CUDA(cudaEventRecord(pool_[used_], g_dev.stream));
+  at_launch_ = g_dev.launches;
+  return (int) used_++;
 }
 
 void StageTimer::reset()
 {
   spans_.clear();
   used_ = 0;
+  at_launch_ = ~0ull;
   for (int s = 0; s < NSTAGE; s++) open_[s] = -1;
 }
 
 void StageTimer::begin(int stage)
 {
-  Span sp{stage, take(), take()};
-  GB_CUDA(cudaEventRecord(sp.a, g_dev.stream));
   open_[stage] = (int) spans_.size();
-  spans_.push_back(sp);
+  spans_.push_back(Span{stage, mark(), -1});
 }
 
 void StageTimer::end(int stage)
 {
   if (open_[stage] < 0) return;
-  GB_CUDA(cudaEventRecord(spans_[open_[stage]].b, g_dev.stream));
+  spans_[open_[stage]].b = mark();
   open_[stage] = -1;
 }
 
 void StageTimer::collect(double *ms)
 {
   for (int s = 0; s < NSTAGE; s++) ms[s] = 0.0;
-  for (size_t q = 0; q < spans_.size(); q++) {
-    bool closed = true;
-    for (int s = 0; s < NSTAGE; s++) closed = closed && open_[s] != (int) q;
-    if (!closed) continue;
+  for (const Span &sp : spans_) {
+    if (sp.b <= sp.a) continue;    // not closed, or nothing was launched inside
     float t = 0.0f;
-    if (cudaEventElapsedTime(&t, spans_[q].a, spans_[q].b) == cudaSuccess) ms[spans_[q].stage] += t;
+    if (cudaEventElapsedTime(&t, pool_[sp.a], pool_[sp.b]) == cudaSuccess) ms[sp.stage] += t;
   }
 }
 

@@ -66,8 +66,15 @@ std::string profile_report();
     ::gb::after_launch(#kernel);                                                    \
   } while (0)
 
+// Device memory of the library.  Freed blocks of up to 256 MB stay in a pool of at most 1 GB and serve later requests
+// of about their size: a Batch that gives its buffers back after every call (the default of the interface) otherwise
+// pays the driver's allocation and release, which synchronise the device, for every buffer of every call (24 structures
+// of GRACE-2L: 7.8 ms per call for 2.8 ms of kernels).  All work on the blocks runs on the library's one stream, so a
+// reused block is ordered behind its last use.  device_pool_trim() returns the pool to the driver; release_buffers,
+// freeing a model, grace_finalize and an allocation that fails do so.
 void *device_alloc(size_t bytes, const char *label);
 void device_free(void *p);
+void device_pool_trim();
 
 // a device array that grows on demand (contents are not kept across a grow)
 template<class T> class DBuf {
@@ -119,6 +126,33 @@ template<class T> class DBuf {
   const char *label_ = "buffer";
 };
 
+// Page-locked host memory for the small transfers of a call: copies from it are one asynchronous DMA each, where a copy
+// from pageable memory goes through the driver's staging and blocks the caller.  get() is null when the memory cannot be
+// had (the caller then copies from and to the user's arrays directly).
+class PinnedBuf {
+ public:
+  PinnedBuf() = default;
+  PinnedBuf(const PinnedBuf &) = delete;
+  PinnedBuf &operator=(const PinnedBuf &) = delete;
+  PinnedBuf(PinnedBuf &&o) noexcept { *this = std::move(o); }
+  PinnedBuf &operator=(PinnedBuf &&o) noexcept
+  {
+    if (this != &o) {
+      release();
+      p_ = o.p_; cap_ = o.cap_;
+      o.p_ = nullptr; o.cap_ = 0;
+    }
+    return *this;
+  }
+  ~PinnedBuf() { release(); }
+  char *ensure(size_t bytes);
+  void release();
+
+ private:
+  char *p_ = nullptr;
+  size_t cap_ = 0;
+};
+
 // bytes currently allocated through device_alloc (diagnostics)
 size_t device_bytes_live();
 // allocation tracking of the reference's test interface (python/kk/kk_core.cpp:143-184): from track_alloc(true) on,
@@ -127,8 +161,8 @@ void track_alloc(bool on);
 size_t tracked_peak_bytes();
 std::vector<std::pair<std::string, size_t>> tracked_live();
 
-// device time per stage of one compute call: pairs of CUDA events on the launch stream, summed per stage after the
-// call's synchronize (a stage may be entered once per chunk)
+// device time per stage of one compute call: pairs of CUDA events on the launch stream, summed per stage when they are
+// asked for (a stage may be entered once per chunk).  A stage that begins where another ended shares its event.
 class StageTimer {
  public:
   enum { NL = 0, GEOM, FWD, BWD, TOTAL, NSTAGE };
@@ -139,15 +173,16 @@ class StageTimer {
   void reset();
   void begin(int stage);
   void end(int stage);
-  void collect(double *ms);    // after a stream synchronize
+  void collect(double *ms);    // times of the spans since reset(), after a stream synchronize
 
  private:
-  struct Span { int stage; cudaEvent_t a, b; };
+  struct Span { int stage; int a, b; };    // events (indices into pool_); b < 0: not closed
   std::vector<Span> spans_;
   std::vector<cudaEvent_t> pool_;
   size_t used_ = 0;
+  uint64_t at_launch_ = ~0ull;    // launch count when the last event was recorded
   int open_[NSTAGE] = {-1, -1, -1, -1, -1};
-  cudaEvent_t take();
+  int mark();
 };
 
 }    // namespace gb

@@ -61,11 +61,21 @@ __global__ void __launch_bounds__(256) types_to_mu(const int *__restrict__ types
   }
 }
 
-__global__ void __launch_bounds__(256) types_differ(const int *__restrict__ a, const int *__restrict__ b, int *flag,
-                                                    long long n)
+// The checks of a call on its list, in one pass: types in range (bit 1; elements written), types as when the list was
+// built (2) and no atom further than sqrt(lim2) from where it was then (4; NaN counts as moved).
+__global__ void __launch_bounds__(256) list_check(const int *__restrict__ types, const int *__restrict__ t2m, int ns, int *mu,
+                                                  const int *__restrict__ types_prev, const double *__restrict__ pos,
+                                                  const double *__restrict__ xbuild, double lim2, int *flag, long long n)
 {
   const long long i = (long long) blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && a[i] != b[i]) atomicOr(flag, 2);
+  if (i >= n) return;
+  const int t = types[i];
+  const bool ok = t >= 1 && t <= ns;
+  mu[i] = ok ? t2m[t - 1] : 0;
+  int f = (ok ? 0 : 1) | (t != types_prev[i] ? 2 : 0);
+  const double dx = pos[3 * i] - xbuild[3 * i], dy = pos[3 * i + 1] - xbuild[3 * i + 1], dz = pos[3 * i + 2] - xbuild[3 * i + 2];
+  if (!(dx * dx + dy * dy + dz * dz <= lim2)) f |= 4;
+  if (f) atomicOr(flag, f);
 }
 
 unsigned nblocks(long long n, int per) { return (unsigned) ((n + per - 1) / per); }
@@ -358,14 +368,15 @@ double Engine::per_atom_bytes(int64_t n_eval) const
 int Engine::auto_chunk(int64_t n) const
 {
   if (plan_.layers == 3) return (int) std::max<int64_t>(n, 1);    // one pass
+  // per-operation passes: large enough that the atom tiles of a pass fill the GPU, small enough to bound the work memory
+  const int64_t most = std::min<int64_t>(std::max<int64_t>(n, 1), use_fused(n) ? ((int64_t) 1 << 22) : (use_tc(n) ? 524288 : 32768));
+  const double held = 4.0 * (double) arena_.capacity(), per = per_atom_bytes(n);
+  // what the work buffer already holds needs no look at the free memory (a driver call of 10 us and more per evaluation)
+  if ((double) most * per <= held) return (int) most;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = (size_t) 8 << 30;
-  const double budget = 0.35 * (double) free_b + 4.0 * (double) arena_.capacity();
-  int64_t c = (int64_t) (budget / per_atom_bytes(n));
-  // per-operation passes: large enough that the atom tiles of a pass fill the GPU, small enough to bound the work memory
-  c = std::min<int64_t>(c, use_fused(n) ? ((int64_t) 1 << 22) : (use_tc(n) ? 524288 : 32768));
-  c = std::max<int64_t>(c, 512);
-  return (int) std::min<int64_t>(c, std::max<int64_t>(n, 1));
+  const int64_t c = (int64_t) ((0.35 * (double) free_b + held) / per);
+  return (int) std::min<int64_t>(std::max<int64_t>(n, 1), std::max<int64_t>(std::min(c, most), 512));
 }
 
 void Engine::release_work()
@@ -692,7 +703,7 @@ void Engine::evaluate_fused(NeighborList &nl, bool energy_only, int NA, StageTim
   BondsDev b0 = nl.bonds(), b1 = nl.bonds();
   b0.ilist = R.list0;
   b1.ilist = R.list1;
-  const int64_t n0 = R.list0 ? R.n0 : n, n1 = R.list1 ? R.n1 : n;
+  const int64_t n0 = R.list0 ? R.n0 : R.hi0, n1 = R.list1 ? R.n1 : R.hi1;    // without lists the ranges start at 0
   if (P.layers == 1) {
     const LayerDev L = layer_dev(L1_);
     const float *gQ = arena_.get() + (size_t) L1_.q_floats * NA;
@@ -790,8 +801,9 @@ void Engine::evaluate_chunked(NeighborList &nl, bool energy_only, int NA, StageT
     const int64_t w1 = (s1.hi - s1.lo + 3) / 4 * 4;
     size_t free_b = 0, total_b = 0;
     const size_t need = (size_t) L1_.per_atom * (size_t) w1 * sizeof(float);
-    if (w1 < ((int64_t) 1 << 30) && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
-        need <= (size_t) (0.45 * (double) free_b) + arena1_.capacity() * sizeof(float)) {
+    const size_t held = arena1_.capacity() * sizeof(float);
+    if (w1 < ((int64_t) 1 << 30) &&
+        (need <= held || (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && need <= (size_t) (0.45 * (double) free_b) + held))) {
       try {
         base1 = arena1_.ensure((size_t) L1_.per_atom * (size_t) w1);
         NA1 = (int) w1;
@@ -914,6 +926,11 @@ ActiveRanges Engine::active_ranges(NeighborList &nl, int nlocal, int ninner, DBu
   R.hi0 = R.hi1 = R.n0 = R.n1 = n;
   if (nlocal < 0 || n == 0) return R;
   R.nlocal = nlocal;
+  if (nl.external()) {    // a caller's own list keeps the caller's order, local atoms first: the ranges are exact
+    R.hi0 = R.n0 = std::min<int64_t>(nlocal, n);
+    R.hi1 = R.n1 = ninner < 0 ? n : std::min<int64_t>(std::max(ninner, nlocal), n);
+    return R;
+  }
   // once per list build: the order of the list on the host, the two sets in that order back to the device
   std::vector<int> perm((size_t) n), l0, l1;
   cudaStream_t st = dev().stream;
@@ -965,6 +982,7 @@ void Engine::evaluate(NeighborList &nl, bool energy_only, const OutputsDev &out,
   if (n == 0) {
     if (out.energy) GB_CUDA(cudaMemsetAsync(out.energy, 0, sizeof(double) * nsys, st));
     if (out.virial && !energy_only) GB_CUDA(cudaMemsetAsync(out.virial, 0, sizeof(double) * 6 * nsys, st));
+    if (out.status && out.first) GB_CUDA(cudaMemsetAsync(out.status, 0, 2 * sizeof(int), st));
     return;
   }
   if (plan_.layers == 3) {
@@ -1033,15 +1051,6 @@ void Engine::evaluate(NeighborList &nl, bool energy_only, const OutputsDev &out,
   }
   if (fused_now) evaluate_fused(nl, energy_only, NA, tm, R);
   else evaluate_chunked(nl, energy_only, NA, tm, R);
-  if (tc_now_) {
-    int e = 0;
-    GB_CUDA(cudaMemcpyAsync(&e, tc_error_.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
-    GB_CUDA(cudaStreamSynchronize(st));
-    if (e) {
-      GB_CUDA(cudaMemsetAsync(tc_error_.get(), 0, sizeof(int), st));
-      throw DeviceError("the tensor-core FC kernel gave up waiting for its matrix instructions");
-    }
-  }
   if (exact_) {
     rad1_.check();
     if (plan_.layers == 2) rad2_.check();
@@ -1054,24 +1063,49 @@ void Engine::write_outputs(NeighborList &nl, bool energy_only, const OutputsDev 
 {
   const int64_t n = nl.n();
   const int nsys = nl.nsys();
-  float *fv = fv_.get();
-  // one or a few large structures: partial sums by 64 blocks per structure and component
-  const int nb = (nsys <= 8 && n > 16384) ? 64 : 1;
-  double *scr = nb > 1 ? sum_scratch_.ensure((size_t) nsys * 6 * nb) : nullptr;
-  if (out.energy) launch_segment_sum(e_atom_.get(), 1, nl.seg(), nsys, out.energy, scr, nb);
-  if (out.energies) launch_scatter_f64(e_atom_.get(), nl.perm(), out.energies, (int) n);
+  FinishDev F{};
+  F.n = (int) n;
+  F.seg = nl.seg();
+  F.e_atom = e_atom_.get();
+  F.vir_atom = energy_only ? nullptr : vir_atom_.get();
+  F.perm = nl.perm();
+  F.energies = out.energies;
   if (uq_now_) {
-    launch_scatter_f64(uq_out_.get(), nl.perm(), out.gamma, (int) n);
-    launch_scatter_f64(uq_out_.get() + n, nl.perm(), out.sigma, (int) n);
-    launch_scatter_f64(uq_out_.get() + 2 * n, nl.perm(), out.cluster, (int) n);
+    F.uq = uq_out_.get();
+    F.gamma = out.gamma; F.sigma = out.sigma; F.cluster = out.cluster;
   }
-  if (!energy_only) {
-    if (out.virial) launch_segment_sum(vir_atom_.get(), 6, nl.seg(), nsys, out.virial, scr, nb);
-    if (out.forces) {
-      if (nl.external()) launch_force_scatter(nl.bonds(), fv, out.forces, (long long) n);    // accumulates
-      else launch_force_gather(nl.off(), nl.rev(), fv, nl.perm(), out.forces, (int) n);
+  if (!energy_only && out.forces) {
+    if (nl.external()) launch_force_scatter(nl.bonds(), fv_.get(), out.forces, (long long) n);    // accumulates
+    else {
+      F.off = nl.off(); F.rev = nl.rev(); F.fv = fv_.get();
+      F.forces = out.forces;
     }
   }
+  F.nl_flag = nl.flag();
+  F.tc_flag = tc_now_ ? tc_error_.get() : nullptr;
+  F.status = out.status;
+  F.first = out.first ? 1 : 0;
+  double *virial = energy_only ? nullptr : out.virial;
+  // one or a few large structures: partial sums by 64 blocks per structure and component
+  if (nsys <= 8 && n > 16384) {
+    const int nb = 64;
+    double *scr = sum_scratch_.ensure((size_t) nsys * 6 * nb);
+    if (out.energy) launch_segment_sum(e_atom_.get(), 1, nl.seg(), nsys, out.energy, scr, nb);
+    if (virial) launch_segment_sum(vir_atom_.get(), 6, nl.seg(), nsys, virial, scr, nb);
+    launch_finish(F, 0);
+  } else {
+    F.energy = out.energy;
+    F.virial = virial;
+    launch_finish(F, F.energy || F.virial ? nsys : 0);
+  }
+}
+
+void Engine::check_status(const int *status)
+{
+  if (status[0] & 4) throw DeviceError("neighbour list: a bond without its reverse bond");
+  if (!status[1]) return;
+  GB_CUDA(cudaMemsetAsync(tc_error_.get(), 0, sizeof(int), dev().stream));
+  throw DeviceError("the tensor-core FC kernel gave up waiting for its matrix instructions");
 }
 
 // ---- model -----------------------------------------------------------------------------------------------------
@@ -1112,11 +1146,82 @@ namespace {
 
 void label_ws(Workspace &w)
 {
-  w.pos.set_label("system:positions"); w.energy.set_label("system:energy"); w.virial.set_label("system:virial");
-  w.forces.set_label("system:forces"); w.energies.set_label("system:energies"); w.types.set_label("system:types");
   w.mu.set_label("system:elements"); w.t2m.set_label("system:type_map"); w.flag.set_label("system:flag");
-  w.types_prev.set_label("system:types");
+  w.types_prev.set_label("system:types"); w.in.set_label("system:positions"); w.out.set_label("system:results");
 }
+
+// The inputs and results of a call of up to this many bytes go through one page-locked block each: two transfers per call
+// instead of one per array, none of which blocks the caller.  Larger ones are bound by the copy itself and use the
+// caller's arrays directly.
+constexpr size_t STAGE_BYTES = (size_t) 4 << 20;
+// Host inputs of up to this many atoms are checked against the list on the CPU (2 ns per atom): on the device the check is a
+// launch and a read-back, 25 us before anything else of the call can start.
+constexpr int HOST_CHECK_ATOMS = 16384;
+
+// head of the result block: energy, virial [6], the two status words
+constexpr size_t HEAD = 8;
+
+struct Staged {
+  const int *types;
+  const double *pos;
+};
+
+// types and positions of a call from the host to the device
+Staged stage_inputs(Workspace &w, int64_t n, const int *types, const double *pos)
+{
+  cudaStream_t st = dev().stream;
+  const size_t pb = sizeof(double) * 3 * (size_t) n, tb = sizeof(int) * (size_t) n;
+  char *d = w.in.ensure(pb + tb);
+  char *h = pb + tb <= STAGE_BYTES ? w.h_in.ensure(pb + tb) : nullptr;
+  if (h) {
+    std::memcpy(h, pos, pb);
+    std::memcpy(h + pb, types, tb);
+    GB_CUDA(cudaMemcpyAsync(d, h, pb + tb, cudaMemcpyHostToDevice, st));
+  } else {
+    GB_CUDA(cudaMemcpyAsync(d, pos, pb, cudaMemcpyHostToDevice, st));
+    GB_CUDA(cudaMemcpyAsync(d + pb, types, tb, cudaMemcpyHostToDevice, st));
+  }
+  return Staged{reinterpret_cast<const int *>(d + pb), reinterpret_cast<const double *>(d)};
+}
+
+// Device block of a call's results: the head, then `parts` arrays of doubles.  fetch() brings all of it to the caller's
+// arrays (null: skipped) and waits for the call's work; head [HEAD] gets the head.
+struct ResultBlock {
+  double *d;
+  std::vector<std::pair<double *, size_t>> parts;    // caller's array, doubles
+  size_t total = HEAD;
+  double *add(double *host, size_t count)    // offset of the part in the block, as a pointer once `d` is set
+  {
+    double *at = d + total;
+    parts.emplace_back(host, count);
+    total += count;
+    return at;
+  }
+  void fetch(Workspace &w, double *head)
+  {
+    cudaStream_t st = dev().stream;
+    const size_t bytes = total * sizeof(double);
+    char *h = w.h_out.ensure(bytes <= STAGE_BYTES ? bytes : HEAD * sizeof(double));
+    const bool whole = h && bytes <= STAGE_BYTES;
+    if (!whole) {
+      size_t at = HEAD;
+      for (auto &p : parts) {
+        if (p.first && p.second) GB_CUDA(cudaMemcpyAsync(p.first, d + at, p.second * sizeof(double), cudaMemcpyDeviceToHost, st));
+        at += p.second;
+      }
+    }
+    GB_CUDA(cudaMemcpyAsync(h ? (void *) h : (void *) head, d, whole ? bytes : HEAD * sizeof(double), cudaMemcpyDeviceToHost, st));
+    GB_CUDA(cudaStreamSynchronize(st));
+    if (h) std::memcpy(head, h, HEAD * sizeof(double));
+    if (whole) {
+      const double *q = reinterpret_cast<const double *>(h) + HEAD;
+      for (auto &p : parts) {
+        if (p.first && p.second) std::memcpy(p.first, q, p.second * sizeof(double));
+        q += p.second;
+      }
+    }
+  }
+};
 
 int read_int(const int *d)
 {
@@ -1160,6 +1265,12 @@ void SystemObj::release()
   label_ws(ws_);
   have_list_ = false;
   engine_->release_work();
+}
+
+void SystemObj::stage_ms(double *ms5)
+{
+  require_initialized();
+  timer_.collect(ms5);
 }
 
 void SystemObj::set_owned(int nlocal_, int ninner_)
@@ -1221,38 +1332,52 @@ void SystemObj::compute_once(int n, const int *types, const double *pos, bool de
 {
   cudaStream_t st = dev().stream;
   const bool eonly = flags & 2, want_e = flags & 1, want_uq = flags & 4;
-  timer_.reset();
-  timer_.begin(StageTimer::TOTAL);
   const int ns = (int) t2m_.size();
-  const int *d_types = types;
-  const double *d_pos = pos;
-  ws_.flag.ensure(1);
-  GB_CUDA(cudaMemsetAsync(ws_.flag.get(), 0, sizeof(int), st));
-  if (n > 0) {
-    if (!device_in) {
-      ws_.types.ensure(n);
-      ws_.pos.ensure(3 * (size_t) n);
-      GB_CUDA(cudaMemcpyAsync(ws_.types.get(), types, sizeof(int) * n, cudaMemcpyHostToDevice, st));
-      GB_CUDA(cudaMemcpyAsync(ws_.pos.get(), pos, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st));
-      d_types = ws_.types.get();
-      d_pos = ws_.pos.get();
-    }
-    ws_.mu.ensure(n);
-    ws_.t2m.upload(t2m_);
-    GB_LAUNCH(types_to_mu, nblocks(n, 256), 256, 0, d_types, ws_.t2m.get(), ns, ws_.mu.get(), ws_.flag.get(), (long long) n);
-  }
-  // rebuild when the atoms, cell or pbc changed or an atom moved more than half the skin (kk_core.cpp:691-708); the
-  // three device-side checks (types in range, types unchanged, displacements) set bits of one flag, read back once
+  const bool on_host = !device_in && n > 0 && n <= HOST_CHECK_ATOMS;
+  // rebuild when the atoms, cell or pbc changed or an atom moved more than half the skin (kk_core.cpp:691-708)
   bool need = !have_list_ || list_n_ != n || ws_.h_cell.size() != 9 || std::memcmp(ws_.h_cell.data(), cell, 72) != 0 ||
               std::memcmp(ws_.h_pbc.data(), pbc, 3) != 0;
-  if (n > 0) {
-    if (!need) {
-      GB_LAUNCH(types_differ, nblocks(n, 256), 256, 0, d_types, ws_.types_prev.get(), ws_.flag.get(), (long long) n);
-      nl_.moved_launch(d_pos, 0.5 * skin_, ws_.flag.get(), 4);
+  bool checked = n == 0;
+  if (on_host) {
+    for (int i = 0; i < n; i++)
+      if (types[i] < 1 || types[i] > ns) throw InvalidArgument("types must be 1 .. len(species)");
+    if (!need && (int64_t) ws_.h_types.size() == n) {    // the list was built from host arrays
+      need = std::memcmp(ws_.h_types.data(), types, sizeof(int) * (size_t) n) != 0;
+      const double lim2 = 0.25 * skin_ * skin_, *x0 = ws_.h_xbuild.data();
+      for (int i = 0; i < n && !need; i++) {
+        const double dx = pos[3 * (size_t) i] - x0[3 * (size_t) i], dy = pos[3 * (size_t) i + 1] - x0[3 * (size_t) i + 1],
+                     dz = pos[3 * (size_t) i + 2] - x0[3 * (size_t) i + 2];
+        need = !(dx * dx + dy * dy + dz * dz <= lim2);    // NaN counts as moved
+      }
+      checked = true;
+    } else if (need) {
+      checked = true;
     }
-    const int fl = read_int(ws_.flag.get());
-    if (fl & 1) throw InvalidArgument("types must be 1 .. len(species)");
-    if (fl & 6) need = true;
+  }
+  timer_.reset();
+  timer_.begin(StageTimer::TOTAL);
+  const int *d_types = types;
+  const double *d_pos = pos;
+  if (n > 0 && !device_in) {
+    const Staged in = stage_inputs(ws_, n, types, pos);
+    d_types = in.types;
+    d_pos = in.pos;
+  }
+  if (n > 0 && (need || !checked)) {
+    if (!ws_.t2m.get()) ws_.t2m.upload(t2m_);
+    ws_.mu.ensure(n);
+    ws_.flag.ensure(1);
+    if (!checked) GB_CUDA(cudaMemsetAsync(ws_.flag.get(), 0, sizeof(int), st));
+    if (need)
+      GB_LAUNCH(types_to_mu, nblocks(n, 256), 256, 0, d_types, ws_.t2m.get(), ns, ws_.mu.get(), ws_.flag.get(), (long long) n);
+    else
+      GB_LAUNCH(list_check, nblocks(n, 256), 256, 0, d_types, ws_.t2m.get(), ns, ws_.mu.get(), ws_.types_prev.get(), d_pos,
+                nl_.build_positions(), 0.25 * skin_ * skin_, ws_.flag.get(), (long long) n);
+    if (!checked) {
+      const int fl = read_int(ws_.flag.get());
+      if (fl & 1) throw InvalidArgument("types must be 1 .. len(species)");
+      if (fl & 6) need = true;
+    }
   }
   if (need) {
     timer_.begin(StageTimer::NL);
@@ -1264,6 +1389,12 @@ void SystemObj::compute_once(int n, const int *types, const double *pos, bool de
       ws_.types_prev.ensure(n);
       GB_CUDA(cudaMemcpyAsync(ws_.types_prev.get(), d_types, sizeof(int) * n, cudaMemcpyDeviceToDevice, st));
     }
+    if (on_host) {
+      ws_.h_types.assign(types, types + n);
+      ws_.h_xbuild.assign(pos, pos + 3 * (size_t) n);
+    } else {
+      ws_.h_types.clear();
+    }
     list_n_ = n;
     have_list_ = true;
     rebuilds++;
@@ -1274,7 +1405,11 @@ void SystemObj::compute_once(int n, const int *types, const double *pos, bool de
   float *fv = engine_->bond_forces(nl_.nslots());
   nl_.prepare(d_pos, engine_->rcsq(), model_->model.n_elements, fv);
   timer_.end(StageTimer::GEOM);
+  ResultBlock res;
+  const size_t m = (size_t) n;
+  res.d = ws_.out.ensure(HEAD + (device_out ? 0 : m * ((eonly || !forces ? 0 : 3) + (want_e && energies ? 1 : 0) + (want_uq ? 3 : 0))));
   OutputsDev o;
+  o.status = reinterpret_cast<int *>(res.d + 7);
   if (device_out) {
     o.energy = energy;
     o.virial = eonly ? nullptr : virial;
@@ -1282,14 +1417,14 @@ void SystemObj::compute_once(int n, const int *types, const double *pos, bool de
     o.energies = want_e ? energies : nullptr;
     if (want_uq) { o.gamma = uq_out.gamma; o.sigma = uq_out.sigma; o.cluster = uq_out.cluster; }
   } else {
-    o.energy = ws_.energy.ensure(1);
-    if (!eonly && virial) o.virial = ws_.virial.ensure(6);
-    if (!eonly && forces) o.forces = ws_.forces.ensure(3 * (size_t) std::max(n, 1));
-    if (want_e && energies) o.energies = ws_.energies.ensure(std::max(n, 1));
+    o.energy = res.d;
+    if (!eonly && virial) o.virial = res.d + 1;
+    if (!eonly && forces) o.forces = res.add(forces, 3 * m);
+    if (want_e && energies) o.energies = res.add(energies, m);
     if (want_uq) {
-      o.gamma = ws_.uq.ensure(3 * (size_t) std::max(n, 1));
-      o.sigma = o.gamma + n;
-      o.cluster = o.gamma + 2 * (size_t) n;
+      o.gamma = res.add(uq_out.gamma, m);
+      o.sigma = res.add(uq_out.sigma, m);
+      o.cluster = res.add(uq_out.cluster, m);
     }
   }
   engine_->evaluate(nl_, eonly, o, chunk, &timer_, nlocal >= 0 ? &ranges : nullptr);
@@ -1297,24 +1432,18 @@ void SystemObj::compute_once(int n, const int *types, const double *pos, bool de
     if (n != exchange.n()) throw InvalidArgument("the atom count differs from the one the exchange plan was made for");
     exchange.run(eonly ? nullptr : o.forces, o.energy, eonly ? nullptr : o.virial);
   }
-  if (!device_out) {
-    if (energy) GB_CUDA(cudaMemcpyAsync(energy, o.energy, sizeof(double), cudaMemcpyDeviceToHost, st));
-    if (o.virial) GB_CUDA(cudaMemcpyAsync(virial, o.virial, sizeof(double) * 6, cudaMemcpyDeviceToHost, st));
-    if (o.forces && n > 0) GB_CUDA(cudaMemcpyAsync(forces, o.forces, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, st));
-    if (o.energies && n > 0) GB_CUDA(cudaMemcpyAsync(energies, o.energies, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
-    if (want_uq && n > 0) {
-      GB_CUDA(cudaMemcpyAsync(uq_out.gamma, o.gamma, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
-      GB_CUDA(cudaMemcpyAsync(uq_out.sigma, o.sigma, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
-      GB_CUDA(cudaMemcpyAsync(uq_out.cluster, o.cluster, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
-    }
-  }
   timer_.end(StageTimer::TOTAL);
-  const int fl = n > 0 ? nl_.take_flag() : 0;    // synchronises the stream
-  GB_CUDA(cudaStreamSynchronize(st));
-  timer_.collect(stage_ms);
-  if (fl & 2) {
-    have_list_ = false;
+  double head[HEAD];
+  res.fetch(ws_, head);
+  const int *status = reinterpret_cast<const int *>(head + 7);
+  if (status[0]) have_list_ = false;
+  engine_->check_status(status);
+  if (status[0] & 2) {
     throw InvalidArgument("two atoms at the same position (a bond of length 0): not a physical structure");
+  }
+  if (!device_out) {
+    if (energy) *energy = head[0];
+    if (o.virial) std::memcpy(virial, head + 1, 6 * sizeof(double));
   }
 }
 
@@ -1357,20 +1486,21 @@ void EngineRunObj::run(int nlocal, int nall, const int *d_type, const double *d_
   std::lock_guard<std::mutex> lk(engine_->mu);
   cudaStream_t st = dev().stream;
   const int n = nall, ns = (int) t2m_.size();
-  ws_.flag.ensure(1);
-  GB_CUDA(cudaMemsetAsync(ws_.flag.get(), 0, sizeof(int), st));
-  ws_.energy.ensure(1);
-  ws_.virial.ensure(6);
+  ResultBlock res;
+  res.d = ws_.out.ensure(HEAD + (d_eatom ? std::max(n, 1) : 0));
   OutputsDev o;
-  o.energy = ws_.energy.get();
+  o.status = reinterpret_cast<int *>(res.d + 7);
+  o.energy = res.d;
   if (!eonly) {
-    o.virial = ws_.virial.get();
+    o.virial = res.d + 1;
     o.forces = d_f;
   }
-  if (d_eatom) o.energies = ws_.energies.ensure(std::max(n, 1));
+  if (d_eatom) o.energies = res.d + HEAD;
   if (n > 0) {
+    ws_.flag.ensure(1);
+    GB_CUDA(cudaMemsetAsync(ws_.flag.get(), 0, sizeof(int), st));
     ws_.mu.ensure(n);
-    ws_.t2m.upload(t2m_);
+    if (!ws_.t2m.get()) ws_.t2m.upload(t2m_);
     GB_LAUNCH(types_to_mu, nblocks(n, 256), 256, 0, d_type, ws_.t2m.get(), ns, ws_.mu.get(), ws_.flag.get(), (long long) n);
     if (read_int(ws_.flag.get()) & 1) throw InvalidArgument("types must be 1 .. len(species)");
   }
@@ -1381,11 +1511,13 @@ void EngineRunObj::run(int nlocal, int nall, const int *d_type, const double *d_
   const int chunk = chunk_req_ < 0 ? engine_->auto_chunk(std::max(nlocal, 1)) : chunk_req_;
   engine_->evaluate(nl_, eonly, o, chunk, nullptr, &ranges, &hooks);
   if (d_eatom && nlocal > 0) launch_add_f64(o.energies, d_eatom, nlocal);
-  if (energy) GB_CUDA(cudaMemcpyAsync(energy, o.energy, sizeof(double), cudaMemcpyDeviceToHost, st));
-  if (virial6 && !eonly) GB_CUDA(cudaMemcpyAsync(virial6, o.virial, sizeof(double) * 6, cudaMemcpyDeviceToHost, st));
-  const int fl = n > 0 ? nl_.take_flag() : 0;    // synchronises the stream
-  GB_CUDA(cudaStreamSynchronize(st));
-  if (fl & 2) throw InvalidArgument("two atoms at the same position (a bond of length 0): not a physical structure");
+  double head[HEAD];
+  res.fetch(ws_, head);
+  const int *status = reinterpret_cast<const int *>(head + 7);
+  engine_->check_status(status);
+  if (status[0] & 2) throw InvalidArgument("two atoms at the same position (a bond of length 0): not a physical structure");
+  if (energy) *energy = head[0];
+  if (virial6 && !eonly) std::memcpy(virial6, head + 1, 6 * sizeof(double));
 }
 
 // ---- batch -----------------------------------------------------------------------------------------------------
@@ -1463,22 +1595,25 @@ void BatchObj::compute_once(int nsys, const int *natoms, int64_t ntot, const int
   host_seconds = 0.0;
   const int *d_types = types;
   const double *d_pos = pos;
-  ws_.flag.ensure(1);
-  GB_CUDA(cudaMemsetAsync(ws_.flag.get(), 0, sizeof(int), st));
   if (ntot > 0) {
-    if (!device_io) {
-      ws_.types.ensure(ntot);
-      ws_.pos.ensure(3 * (size_t) ntot);
-      GB_CUDA(cudaMemcpyAsync(ws_.types.get(), types, sizeof(int) * ntot, cudaMemcpyHostToDevice, st));
-      GB_CUDA(cudaMemcpyAsync(ws_.pos.get(), pos, sizeof(double) * 3 * ntot, cudaMemcpyHostToDevice, st));
-      d_types = ws_.types.get();
-      d_pos = ws_.pos.get();
+    ws_.flag.ensure(1);
+    if (!device_io) {    // host types are checked here: no read-back before the passes can start
+      for (int64_t i = 0; i < ntot; i++)
+        if (types[i] < 1 || types[i] > ns) throw InvalidArgument("types must be 1 .. len(species)");
+      const Staged in = stage_inputs(ws_, ntot, types, pos);
+      d_types = in.types;
+      d_pos = in.pos;
+    } else {
+      GB_CUDA(cudaMemsetAsync(ws_.flag.get(), 0, sizeof(int), st));
     }
     ws_.mu.ensure(ntot);
-    ws_.t2m.upload(t2m_);
+    if (!ws_.t2m.get()) ws_.t2m.upload(t2m_);
     GB_LAUNCH(types_to_mu, nblocks(ntot, 256), 256, 0, d_types, ws_.t2m.get(), ns, ws_.mu.get(), ws_.flag.get(), (long long) ntot);
-    if (read_int(ws_.flag.get()) & 1) throw InvalidArgument("types must be 1 .. len(species)");
+    if (device_io && (read_int(ws_.flag.get()) & 1)) throw InvalidArgument("types must be 1 .. len(species)");
   }
+  ResultBlock res;
+  const size_t mt = (size_t) ntot, msys = (size_t) nsys;
+  res.d = ws_.out.ensure(HEAD + (device_io ? 0 : msys * 7 + mt * ((eonly || !forces ? 0 : 3) + (want_e && energies ? 1 : 0) + (want_uq ? 3 : 0))));
   OutputsDev all;
   if (device_io) {
     all.energy = energy;
@@ -1487,21 +1622,19 @@ void BatchObj::compute_once(int nsys, const int *natoms, int64_t ntot, const int
     all.energies = want_e ? energies : nullptr;
     if (want_uq) { all.gamma = uq_out.gamma; all.sigma = uq_out.sigma; all.cluster = uq_out.cluster; }
   } else {
-    all.energy = ws_.energy.ensure(std::max(nsys, 1));
-    if (!eonly && virial) all.virial = ws_.virial.ensure(6 * (size_t) std::max(nsys, 1));
-    if (!eonly && forces) all.forces = ws_.forces.ensure(3 * (size_t) std::max<int64_t>(ntot, 1));
-    if (want_e && energies) all.energies = ws_.energies.ensure(std::max<int64_t>(ntot, 1));
+    all.energy = res.add(energy, msys);
+    if (!eonly && virial) all.virial = res.add(virial, 6 * msys);
+    if (!eonly && forces) all.forces = res.add(forces, 3 * mt);
+    if (want_e && energies) all.energies = res.add(energies, mt);
     if (want_uq) {
-      const size_t m = (size_t) std::max<int64_t>(ntot, 1);
-      all.gamma = ws_.uq.ensure(3 * m);
-      all.sigma = all.gamma + m;
-      all.cluster = all.gamma + 2 * m;
+      all.gamma = res.add(uq_out.gamma, mt);
+      all.sigma = res.add(uq_out.sigma, mt);
+      all.cluster = res.add(uq_out.cluster, mt);
     }
   }
   // passes of whole structures with at most max_nall atoms (a single larger structure gets a pass of its own)
   int s0 = 0;
   int64_t a0 = 0;
-  bool zero_bond = false;
   while (s0 < nsys) {
     int s1 = s0;
     int64_t na = 0;
@@ -1511,7 +1644,6 @@ void BatchObj::compute_once(int nsys, const int *natoms, int64_t ntot, const int
               cutoff_);
     float *fv = engine_->bond_forces(nl_.nslots());
     nl_.prepare(d_pos + 3 * a0, engine_->rcsq(), model_->model.n_elements, fv);
-    GB_CUDA(cudaStreamSynchronize(st));
     host_seconds += std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     OutputsDev o;
     o.energy = all.energy ? all.energy + s0 : nullptr;
@@ -1519,25 +1651,19 @@ void BatchObj::compute_once(int nsys, const int *natoms, int64_t ntot, const int
     o.forces = all.forces ? all.forces + 3 * a0 : nullptr;
     o.energies = all.energies ? all.energies + a0 : nullptr;
     if (want_uq) { o.gamma = all.gamma + a0; o.sigma = all.sigma + a0; o.cluster = all.cluster + a0; }
+    o.status = reinterpret_cast<int *>(res.d + 7);
+    o.first = passes == 0;
     engine_->evaluate(nl_, eonly, o, chunk, nullptr);
-    if (na > 0 && (nl_.take_flag() & 2)) zero_bond = true;
     passes++;
     s0 = s1;
     a0 += na;
   }
-  if (!device_io) {
-    if (energy && nsys > 0) GB_CUDA(cudaMemcpyAsync(energy, all.energy, sizeof(double) * nsys, cudaMemcpyDeviceToHost, st));
-    if (all.virial && nsys > 0) GB_CUDA(cudaMemcpyAsync(virial, all.virial, sizeof(double) * 6 * nsys, cudaMemcpyDeviceToHost, st));
-    if (all.forces && ntot > 0) GB_CUDA(cudaMemcpyAsync(forces, all.forces, sizeof(double) * 3 * ntot, cudaMemcpyDeviceToHost, st));
-    if (all.energies && ntot > 0) GB_CUDA(cudaMemcpyAsync(energies, all.energies, sizeof(double) * ntot, cudaMemcpyDeviceToHost, st));
-    if (want_uq && ntot > 0) {
-      GB_CUDA(cudaMemcpyAsync(uq_out.gamma, all.gamma, sizeof(double) * ntot, cudaMemcpyDeviceToHost, st));
-      GB_CUDA(cudaMemcpyAsync(uq_out.sigma, all.sigma, sizeof(double) * ntot, cudaMemcpyDeviceToHost, st));
-      GB_CUDA(cudaMemcpyAsync(uq_out.cluster, all.cluster, sizeof(double) * ntot, cudaMemcpyDeviceToHost, st));
-    }
-  }
-  GB_CUDA(cudaStreamSynchronize(st));
-  if (zero_bond) throw InvalidArgument("two atoms at the same position (a bond of length 0): not a physical structure");
+  double head[HEAD] = {};
+  if (passes == 0) GB_CUDA(cudaMemsetAsync(res.d + 7, 0, sizeof(double), st));
+  res.fetch(ws_, head);
+  const int *status = reinterpret_cast<const int *>(head + 7);
+  engine_->check_status(status);
+  if (status[0] & 2) throw InvalidArgument("two atoms at the same position (a bond of length 0): not a physical structure");
 }
 
 }    // namespace gb

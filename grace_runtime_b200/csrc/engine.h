@@ -82,6 +82,10 @@ struct OutputsDev {
   double *energies = nullptr;    // [n] caller's order
   // UQ (all three or none): extrapolation grade, Mahalanobis distance and cluster per atom, [n] caller's order
   double *gamma = nullptr, *sigma = nullptr, *cluster = nullptr;
+  // error words of the call, [0] the list's (2: two atoms at one position), [1] the tensor-core kernels' (check_status);
+  // `first`: the first pass of the call, which writes them (later passes or theirs in)
+  int *status = nullptr;
+  bool first = true;
 };
 
 class Engine {
@@ -99,6 +103,8 @@ class Engine {
   // act (optional): owned atoms and active ranges of a domain-decomposed caller
   void evaluate(NeighborList &nl, bool energy_only, const OutputsDev &out, int chunk, StageTimer *tm,
                 const ActiveRanges *act = nullptr, const ExchangeHooks *hooks = nullptr);
+  // throws when the status words an evaluation left (host copy) report a failure of the tensor-core kernels
+  void check_status(const int *status);
   // ranges of the list order that hold the atoms with caller index < nlocal / < ninner (reads back 4 integers)
   ActiveRanges active_ranges(NeighborList &nl, int nlocal, int ninner, DBuf<int> &list0, DBuf<int> &list1);
   // bond-force slots [3 * nslots] the list zeroes for bonds outside the cutoff (grown here)
@@ -198,11 +204,13 @@ struct UqOutputs {
 };
 
 struct Workspace {
-  DBuf<double> pos, energy, virial, forces, energies, uq;
-  DBuf<int> types, mu, t2m, flag, types_prev;
-  std::vector<double> h_cell;
+  DBuf<char> in;                        // positions and types of a host call
+  DBuf<double> out;                     // results of a call (host calls: all of them; device calls: the status words)
+  DBuf<int> mu, t2m, flag, types_prev;
+  PinnedBuf h_in, h_out;
+  std::vector<double> h_cell, h_xbuild;    // h_types, h_xbuild: what the list was built from, when that came from the host
+  std::vector<int> h_types;
   std::vector<unsigned char> h_pbc;
-  std::vector<int> h_natoms;
 };
 
 class SystemObj {
@@ -224,7 +232,7 @@ class SystemObj {
   void set_exchange(int n, int nlocal_, int ninner_, const int32_t *send_counts, const int32_t *send_index,
                     const int32_t *recv_counts, const int32_t *recv_index);
   Exchange exchange;
-  double stage_ms[StageTimer::NSTAGE] = {0, 0, 0, 0, 0};
+  void stage_ms(double *ms5);    // device time per stage of the last call
   void release();
   std::mutex mu;
   const NeighborList &neighbor_list() const { return nl_; }

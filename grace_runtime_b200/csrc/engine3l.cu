@@ -691,7 +691,8 @@ struct State3L {
   int npairs = 0;
   DBuf<float> rho_sum, drho;
   DBuf<double> eW0, eW1;
-  int NA = 0;
+  const float *bound[3] = {nullptr, nullptr, nullptr};    // arena and atom stride the tensor tables point into
+  int bound_NC[3] = {0, 0, 0};
 };
 
 void Engine::setup_3l()
@@ -768,16 +769,6 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
   const int nt = 128, nblk = (n + nt - 1) / nt;
   // large evaluations: the projections, reduces and FCs with 16 / 32 / 64 channels as tensor-core grouped GEMMs (mv_tc.cu)
   tc_now_ = dense_ == Dense::Tc || (n >= tc_min_atoms_ && dense_ == Dense::Auto);
-  auto check_tc = [&]() {
-    if (!tc_now_) return;
-    int e = 0;
-    GB_CUDA(cudaMemcpyAsync(&e, tc_error_.get(), sizeof(int), cudaMemcpyDeviceToHost, dev().stream));
-    GB_CUDA(cudaStreamSynchronize(dev().stream));
-    if (e) {
-      GB_CUDA(cudaMemsetAsync(tc_error_.get(), 0, sizeof(int), dev().stream));
-      throw DeviceError("the tensor-core FC kernel gave up waiting for its matrix instructions");
-    }
-  };
   // every bond needs the radial table of its element pair: the species of every System / Batch of this engine were
   // prepared when it was created (prepare_species); a bond of a pair without a table is left out by the kernels
   if (tm) tm->begin(StageTimer::FWD);
@@ -849,10 +840,15 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
     per_all += S.E[k].per_atom;
     per_max = std::max(per_max, S.E[k].per_atom);
   }
-  size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = (size_t) 8 << 30;
-  double budget = 0.7 * (double) free_b;
+  bool held = true;    // the arenas hold all layers already: no look at the free memory
+  for (int k = 0; k < 3; k++) held = held && (double) S.E[k].per_atom * NA <= (double) S.arena[k].capacity();
+  double budget = 0.0;
   for (int k = 0; k < 3; k++) budget += 4.0 * (double) S.arena[k].capacity();
+  if (!held) {
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = (size_t) 8 << 30;
+    budget += 0.7 * (double) free_b;
+  }
   if (const char *env = getenv("GRACE_B200_3L_CHUNK")) budget = std::min(budget, 4.0 * per_all * std::max(4, atoi(env)) - 1.0);
   const bool keep = 4.0 * (double) per_all * NA <= budget;
   int NC = NA;    // atoms per pass (a multiple of 4: the atom stride of the arena)
@@ -878,7 +874,11 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
     LayerEngine &E = S.E[k];
     DBuf<float> &ar = S.arena[keep ? k : 0];
     float *base = ar.ensure((size_t) (keep ? E.per_atom : per_max) * NC);
-    bind_arena(E, base, NC);
+    if (S.bound[k] != base || S.bound_NC[k] != NC) {    // the tensor table on the device moves with the arena only
+      bind_arena(E, base, NC);
+      S.bound[k] = base;
+      S.bound_NC[k] = NC;
+    }
     return base;
   };
   // forward operations of layer k for the atoms [a0, a0 + na); outputs: the message rows and the density sums
@@ -926,10 +926,7 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
   const Readout3Dev ro{S.eW0.get(), S.eW1.get(), shift_.get(), Q.en0, Q.en1, plan_.out_scale, Q.e_nin, Q.e_nh, Q.e_act};
   GB_LAUNCH(readout3_kernel, nblk, nt, 0, ro, S.rho_sum.get(), mu, e_atom_.get(), S.drho.get(), energy_only ? 0 : 1, n);
   if (tm) tm->end(StageTimer::FWD);
-  if (energy_only) {
-    check_tc();
-    return;
-  }
+  if (energy_only) return;
   if (tm) tm->begin(StageTimer::BWD);
   // the reverse bond kernels add their shares (three layers, channel slices) to the bond forces and the virial
   launch_fill_zero(fv_.get(), sizeof(float) * 3 * (size_t) std::max<int64_t>(nl.nslots(), 1));
@@ -948,7 +945,6 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
     }
   }
   if (tm) tm->end(StageTimer::BWD);
-  check_tc();
 }
 
 }    // namespace gb

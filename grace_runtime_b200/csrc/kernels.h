@@ -186,9 +186,6 @@ void launch_gather_int(const int *v, const int *list, int *out, long long n);
 // bonds whose other atom is a ghost (perm[i] >= nlocal) are left out - its layer was not evaluated, its slots hold nothing
 void launch_msg_grad_gather(const BondsDev &b, const int *rev, const float *gslot, float *gmsg, int width, const int *ilist,
                             long long n, const int *perm, int nlocal);
-// F_i = sum over the slots q of atom i of fv[q] - fv[rev[q]], written at the caller's index of atom i
-void launch_force_gather(const long long *off, const int *rev, const float *fv, const int *perm, double *forces,
-                         int n);
 // lists without a reverse-bond index (a caller's own list with ghost atoms): forces[i] += sum of the atom's bond forces,
 // forces[j] -= each bond force, with fp64 atomic adds (forces is accumulated into, indexed like the list's atoms)
 void launch_force_scatter(const BondsDev &b, const float *fv, double *forces, long long n);
@@ -202,11 +199,26 @@ void launch_add_f64(const double *v, double *out, long long n);
 void static_sum(const double *d_values, long long n, int K, double *d_out);
 long long static_sum_max_rows();
 int static_sum_max_cols();
-// scratch (nseg * K * nb doubles) with nb > 1: two launches with nb partial sums per (segment, component), for few long
-// segments
-void launch_segment_sum(const double *v, int K, const int *seg, int nseg, double *out, double *scratch = nullptr,
-                        int nb = 1);
-// out[perm[i]] = v[i]
-void launch_scatter_f64(const double *v, const int *perm, double *out, int n);
+// scratch: nseg * K * nb doubles; two launches with nb partial sums per (segment, component), for few long segments
+void launch_segment_sum(const double *v, int K, const int *seg, int nseg, double *out, double *scratch, int nb);
+// What leaves an evaluation (null pointers: not wanted).  F_i = sum over the slots q of atom i of fv[q] - fv[rev[q]];
+// per-atom values go to perm[i]
+struct FinishDev {
+  int n;
+  const int *seg;                     // [structures + 1]
+  const double *e_atom, *vir_atom;    // [n], [n][6]
+  double *energy, *virial;            // per structure (blocks 0 .. nsum)
+  const int *perm;
+  const long long *off;
+  const int *rev;
+  const float *fv;
+  double *forces, *energies;
+  const double *uq;                   // [3][n]
+  double *gamma, *sigma, *cluster;
+  const int *nl_flag, *tc_flag;       // error words of the list and (null: not used) of the tensor-core kernels
+  int *status;                        // [2] where they go: written by the first pass of a call, or-ed by later ones
+  int first;
+};
+void launch_finish(const FinishDev &F, int nsum);
 
 }    // namespace gb

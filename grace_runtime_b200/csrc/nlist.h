@@ -34,10 +34,6 @@ class NeighborList {
   // atomic adds and to add the neighbours' message gradients atomically, as the reference's engines do.
   void adopt(int nlocal, int nall, const int *d_mu, const int *d_numneigh, const int *d_neighbors, int maxneigh);
   bool external() const { return external_; }
-  // true when an atom moved more than half the skin since the build (device max-reduce, one int read back)
-  bool moved_beyond(const double *d_pos, double half_skin);
-  // the same check without the read-back: sets `bit` of the caller's device flag
-  void moved_launch(const double *d_pos, double half_skin, int *d_flag, int bit);
   // positions of this call into list order (wrapped with the images of the build) and the bonds inside the pair
   // cutoffs rcsq [n_elements][n_elements]: records compacted to the front of each atom's slots; bond forces of the
   // slots left out are zeroed in fv
@@ -52,8 +48,9 @@ class NeighborList {
   const int *rev() const { return rev_.get(); }
   const long long *off() const { return off_.get(); }
   const int *seg() const { return seg_.get(); }            // [nsys + 1] atom ranges of the structures in list order
-  // error bits raised by prepare() since it was called (2: a bond of length 0); synchronises the stream
-  int take_flag();
+  // device: two error words, [0] raised by prepare() (2: a bond of length 0), [1] by the build (4: no reverse bond)
+  const int *flag() const { return flag_.get(); }
+  const double *build_positions() const { return xbuild_.get(); }    // device: the caller's positions of the last build
   void release();
   size_t bytes() const;
   // diagnostics: the list of the last build (radius cutoff + skin) on the host, in the caller's atom order and frame:
@@ -67,7 +64,7 @@ class NeighborList {
   std::vector<NLStructHost> st_;
   DBuf<NLStructHost> d_st_;
   DBuf<double> frac_, xs_, xbuild_, lohi_;
-  DBuf<int> img_, img_s_, sid_, sid_s_, binid_, b3_s_, count_, fill_, members_, perm_, mu_s_, cnt_full_, cnt_, nbr_j_,
+  DBuf<int> img_, img_s_, sid_, sid_s_, binid_, b3_s_, count_, members_, perm_, mu_s_, cnt_full_, cnt_, nbr_j_,
       nbr_S_, rev_, cslot_, seg_, flag_;
   DBuf<long long> start_, off_, scan_tmp_;
   DBuf<float4> rec_;

@@ -1,5 +1,5 @@
 // Column sums of a device matrix of doubles (per-atom energies or virial rows -> totals) without any device
-// allocation: the two-level variant of segment_sum_kernel (chain.cu) whose per-block partial sums live in a
+// allocation: the two-level variant of segment_partial_kernel (chain.cu) whose per-block partial sums live in a
 // file-scope device array instead of a buffer obtained from the allocator.  No counterpart in the reference.
 //
 // The array is one per device and shared by every call: the first 256 bytes hold the arrival counter of the blocks
