@@ -522,112 +522,128 @@ struct EqNormDev {
   double eps;
 };
 
-// EquivariantRMSNorm of one atom per thread (libgrace/include/grace/fused_3l_cpu.h:346-370): x [f][NA][C] -> y rows [i][f][C]
-__global__ void eqnorm_fwd_kernel(EqNormDev E, const float *__restrict__ x, float *__restrict__ y, int NA, int n, int a0)
+// The norms and the readout: a CTA (norms of the messages) or a warp (densities, readout) per atom, lanes along the channels.
+// A thread per atom, which read 1600 values of its row one after the other, left all but a few SMs idle at hundreds of atoms
+// (250 atoms: 2.0 ms for the two reverse norms, 0.8 ms forward).
+constexpr int EQ_WARPS = 8;
+
+__device__ __forceinline__ double warp_sum(double v)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  y += (size_t) a0 * E.nf * E.C;    // rows of the atoms of the pass
-  double S = 0.0;
-  for (int f = 0; f < E.nf; f++) {
-    const float *xf = x + ((size_t) f * NA + i) * E.C;
+  for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+  return v;
+}
+__device__ __forceinline__ double block_sum(double v, double *sh)    // v: the same on all lanes of a warp
+{
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double s = 0.0;
+  for (int w = 0; w < EQ_WARPS; w++) s += sh[w];
+  return s;
+}
+
+// EquivariantRMSNorm (libgrace/include/grace/fused_3l_cpu.h:346-370): x [f][NA][C] -> y rows [i][f][C]
+__global__ void __launch_bounds__(32 * EQ_WARPS) eqnorm_fwd_kernel(EqNormDev E, const float *__restrict__ x, float *__restrict__ y, int NA,
+                                                                   int a0)
+{
+  __shared__ double sh[EQ_WARPS];
+  const int i = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto mean = [&](int f) {
+    if (!E.center || E.mask[f] == 0.0f) return 0.0;
     double m = 0.0;
-    if (E.center && E.mask[f] != 0.0f) {
-      for (int c = 0; c < E.C; c++) m += xf[c];
-      m = m / E.C * E.mask[f];
-    }
+    for (int c = lane; c < E.C; c += 32) m += x[((size_t) f * NA + i) * E.C + c];
+    return warp_sum(m) / E.C * E.mask[f];
+  };
+  double S = 0.0;
+  for (int f = warp; f < E.nf; f += EQ_WARPS) {
+    const double m = mean(f);
     double s2 = 0.0;
-    for (int c = 0; c < E.C; c++) {
-      const float v = (float) (xf[c] - m);
+    for (int c = lane; c < E.C; c += 32) {
+      const float v = (float) (x[((size_t) f * NA + i) * E.C + c] - m);
       s2 += (double) v * v;
     }
     S += E.dw[f] * s2;
   }
-  const double r = 1.0 / sqrt(S / E.C + E.eps);
-  for (int f = 0; f < E.nf; f++) {
-    const float *xf = x + ((size_t) f * NA + i) * E.C, *a = E.aff + (size_t) E.e[f] * E.C;
-    float *yf = y + ((size_t) i * E.nf + f) * E.C;
-    double m = 0.0;
-    if (E.center && E.mask[f] != 0.0f) {
-      for (int c = 0; c < E.C; c++) m += xf[c];
-      m = m / E.C * E.mask[f];
-    }
-    for (int c = 0; c < E.C; c++) yf[c] = (float) ((float) (xf[c] - m) * r) * a[c];
+  const double r = 1.0 / sqrt(block_sum(warp_sum(S), sh) / E.C + E.eps);
+  for (int f = warp; f < E.nf; f += EQ_WARPS) {
+    const double m = mean(f);
+    for (int c = lane; c < E.C; c += 32)
+      y[((size_t) (a0 + i) * E.nf + f) * E.C + c] =
+          (float) ((float) (x[((size_t) f * NA + i) * E.C + c] - m) * r) * E.aff[(size_t) E.e[f] * E.C + c];
   }
 }
 
 // gx [f][NA][C] = adjoint of the above for dy rows [i][f][C] (:373-415)
-__global__ void eqnorm_bwd_kernel(EqNormDev E, const float *__restrict__ x, const float *__restrict__ dy, float *__restrict__ gx, int NA,
-                                  int n, int a0)
+__global__ void __launch_bounds__(32 * EQ_WARPS) eqnorm_bwd_kernel(EqNormDev E, const float *__restrict__ x, const float *__restrict__ dy,
+                                                                   float *__restrict__ gx, int NA, int a0)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  dy += (size_t) a0 * E.nf * E.C;
-  double S = 0.0, dot = 0.0;
-  for (int f = 0; f < E.nf; f++) {
-    const float *xf = x + ((size_t) f * NA + i) * E.C, *a = E.aff + (size_t) E.e[f] * E.C, *d = dy + ((size_t) i * E.nf + f) * E.C;
+  __shared__ double sh[EQ_WARPS];
+  const int i = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto mean = [&](int f) {
+    if (!E.center || E.mask[f] == 0.0f) return 0.0;
     double m = 0.0;
-    if (E.center && E.mask[f] != 0.0f) {
-      for (int c = 0; c < E.C; c++) m += xf[c];
-      m = m / E.C * E.mask[f];
-    }
+    for (int c = lane; c < E.C; c += 32) m += x[((size_t) f * NA + i) * E.C + c];
+    return warp_sum(m) / E.C * E.mask[f];
+  };
+  double S = 0.0, dot = 0.0;
+  for (int f = warp; f < E.nf; f += EQ_WARPS) {
+    const float *xf = x + ((size_t) f * NA + i) * E.C, *a = E.aff + (size_t) E.e[f] * E.C, *d = dy + ((size_t) (a0 + i) * E.nf + f) * E.C;
+    const double m = mean(f);
     double s2 = 0.0;
-    for (int c = 0; c < E.C; c++) {
+    for (int c = lane; c < E.C; c += 32) {
       const float v = (float) (xf[c] - m);
       s2 += (double) v * v;
       dot += (double) d[c] * a[c] * v;
     }
     S += E.dw[f] * s2;
   }
+  S = block_sum(warp_sum(S), sh);
+  dot = block_sum(warp_sum(dot), sh);
   const double r = 1.0 / sqrt(S / E.C + E.eps), k3 = r * r * r * dot / E.C;
-  for (int f = 0; f < E.nf; f++) {
-    const float *xf = x + ((size_t) f * NA + i) * E.C, *a = E.aff + (size_t) E.e[f] * E.C, *d = dy + ((size_t) i * E.nf + f) * E.C;
+  for (int f = warp; f < E.nf; f += EQ_WARPS) {
+    const float *xf = x + ((size_t) f * NA + i) * E.C, *a = E.aff + (size_t) E.e[f] * E.C, *d = dy + ((size_t) (a0 + i) * E.nf + f) * E.C;
     float *o = gx + ((size_t) f * NA + i) * E.C;
-    const bool centred = E.center && E.mask[f] != 0.0f;
-    double m = 0.0;
-    if (centred) {
-      for (int c = 0; c < E.C; c++) m += xf[c];
-      m = m / E.C * E.mask[f];
+    const double m = mean(f), kf = k3 * E.dw[f];
+    double gm = 0.0;
+    if (E.center && E.mask[f] != 0.0f) {
+      for (int c = lane; c < E.C; c += 32) gm += (float) (r * d[c] * a[c] - kf * (float) (xf[c] - m));
+      gm = warp_sum(gm) / E.C * E.mask[f];
     }
-    const double kf = k3 * E.dw[f];
-    double mean = 0.0;
-    for (int c = 0; c < E.C; c++) mean += (float) (r * d[c] * a[c] - kf * (float) (xf[c] - m));
-    mean = centred ? mean / E.C * E.mask[f] : 0.0;
-    for (int c = 0; c < E.C; c++) o[c] = (float) ((float) (r * d[c] * a[c] - kf * (float) (xf[c] - m)) - mean);
+    for (int c = lane; c < E.C; c += 32) o[c] = (float) ((float) (r * d[c] * a[c] - kf * (float) (xf[c] - m)) - gm);
   }
 }
 
 // RMSNorm of the density (:416-425): x [NA][wr] (one function) -> y rows [i][wr]; sum rows += y
-__global__ void rmsnorm_fwd_kernel(const float *__restrict__ x, const float *__restrict__ scale, int n0, int wr, float *__restrict__ sum,
-                                   int first, int n, int a0)
+__global__ void __launch_bounds__(128) rmsnorm_fwd_kernel(const float *__restrict__ x, const float *__restrict__ scale, int n0, int wr,
+                                                          float *__restrict__ sum, int first, int n, int a0)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= n) return;
   const float *xi = x + (size_t) i * wr;
   float *s = sum + (size_t) (a0 + i) * wr;
   double q = 0.0;
-  for (int c = n0; c < wr; c++) q += (double) xi[c] * xi[c];
-  const double r = 1.0 / sqrt(q / (wr - n0) + 1e-10);
-  for (int c = 0; c < wr; c++) {
+  for (int c = n0 + lane; c < wr; c += 32) q += (double) xi[c] * xi[c];
+  const double r = 1.0 / sqrt(warp_sum(q) / (wr - n0) + 1e-10);
+  for (int c = lane; c < wr; c += 32) {
     const float y = c < n0 ? xi[c] : (float) (xi[c] * r) * scale[c - n0];
     s[c] = first ? y : s[c] + y;
   }
 }
 
-__global__ void rmsnorm_bwd_kernel(const float *__restrict__ x, const float *__restrict__ scale, int n0, int wr,
-                                   const float *__restrict__ dy, float *__restrict__ gx, int n, int a0)
+__global__ void __launch_bounds__(128) rmsnorm_bwd_kernel(const float *__restrict__ x, const float *__restrict__ scale, int n0, int wr,
+                                                          const float *__restrict__ dy, float *__restrict__ gx, int n, int a0)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= n) return;
   const float *xi = x + (size_t) i * wr, *d = dy + (size_t) (a0 + i) * wr;
   float *o = gx + (size_t) i * wr;
   double q = 0.0, g = 0.0;
-  for (int c = n0; c < wr; c++) {
+  for (int c = n0 + lane; c < wr; c += 32) {
     q += (double) xi[c] * xi[c];
     g += (double) d[c] * scale[c - n0] * xi[c];
   }
-  const double r = 1.0 / sqrt(q / (wr - n0) + 1e-10), k = r * r * r * g / (wr - n0);
-  for (int c = 0; c < wr; c++) o[c] = c < n0 ? d[c] : (float) (r * d[c] * scale[c - n0] - k * xi[c]);
+  const double r = 1.0 / sqrt(warp_sum(q) / (wr - n0) + 1e-10), k = r * r * r * warp_sum(g) / (wr - n0);
+  for (int c = lane; c < wr; c += 32) o[c] = c < n0 ? d[c] : (float) (r * d[c] * scale[c - n0] - k * xi[c]);
 }
 
 struct Readout3Dev {
@@ -637,23 +653,22 @@ struct Readout3Dev {
 };
 
 // E_i = (MLP(sum[1:]) + sum[0]) scale + shift (fp64, :1334-1374); d: dE/d(sum) rows [i][1 + nin]
-__global__ void readout3_kernel(Readout3Dev R, const float *__restrict__ sum, const int *__restrict__ mu, double *__restrict__ e_atom,
-                                float *__restrict__ d, int want_grad, int n)
+__global__ void __launch_bounds__(128) readout3_kernel(Readout3Dev R, const float *__restrict__ sum, const int *__restrict__ mu,
+                                                       double *__restrict__ e_atom, float *__restrict__ d, int want_grad, int n)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ double s_ds[4][128];
+  __shared__ float s_h[4][128];
+  const int w = threadIdx.x >> 5, i = blockIdx.x * 4 + w, lane = threadIdx.x & 31;
   if (i >= n) return;
   const int wr = R.nin + 1;
   const float *h = sum + (size_t) i * wr;
-  double e = 0.0;
   float *di = d + (size_t) i * wr;
-  if (want_grad)
-    for (int c = 0; c < wr; c++) di[c] = c == 0 ? (float) R.oscale : 0.0f;
-  double acc_d[128];
-  if (want_grad)
-    for (int c = 0; c < R.nin; c++) acc_d[c] = 0.0;
-  for (int j = 0; j < R.nh; j++) {
+  for (int c = lane; c < R.nin; c += 32) s_h[w][c] = h[c + 1];
+  __syncwarp();
+  double e = 0.0;
+  for (int j = lane; j < R.nh; j += 32) {    // a lane per hidden unit
     double s = 0.0;
-    for (int c = 0; c < R.nin; c++) s += (double) h[c + 1] * R.W0[(size_t) c * R.nh + j];
+    for (int c = 0; c < R.nin; c++) s += (double) s_h[w][c] * R.W0[(size_t) c * R.nh + j];
     s *= R.n0;
     double act, dact;
     if (R.act == 1) {
@@ -665,15 +680,18 @@ __global__ void readout3_kernel(Readout3Dev R, const float *__restrict__ sum, co
       dact = sg * (1.0 + s * (1.0 - sg));
     }
     e += R.W1[j] * act;
-    if (want_grad) {
-      const double ds = R.oscale * R.n1 * R.W1[j] * dact * R.n0;
-      for (int c = 0; c < R.nin; c++) acc_d[c] += R.W0[(size_t) c * R.nh + j] * ds;
-    }
+    s_ds[w][j] = R.oscale * R.n1 * R.W1[j] * dact * R.n0;
   }
-  e *= R.n1;
-  e_atom[i] = (e + (double) h[0]) * R.oscale + R.shift[mu[i]];
-  if (want_grad)
-    for (int c = 0; c < R.nin; c++) di[c + 1] = (float) acc_d[c];
+  e = warp_sum(e) * R.n1;
+  __syncwarp();
+  if (lane == 0) e_atom[i] = (e + (double) h[0]) * R.oscale + R.shift[mu[i]];
+  if (!want_grad) return;
+  if (lane == 0) di[0] = (float) R.oscale;
+  for (int c = lane; c < R.nin; c += 32) {    // a lane per input
+    double g = 0.0;
+    for (int j = 0; j < R.nh; j++) g += R.W0[(size_t) c * R.nh + j] * s_ds[w][j];
+    di[c + 1] = (float) g;
+  }
 }
 
 }    // namespace
@@ -766,7 +784,6 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
   const BondsDev bonds = nl.bonds();
   const int *mu = bonds.mu;
   const SHTable sht = sh_table_host();
-  const int nt = 128, nblk = (n + nt - 1) / nt;
   // large evaluations: the projections, reduces and FCs with 16 / 32 / 64 channels as tensor-core grouped GEMMs (mv_tc.cu)
   tc_now_ = dense_ == Dense::Tc || (n >= tc_min_atoms_ && dense_ == Dense::Auto);
   // every bond needs the radial table of its element pair: the species of every System / Batch of this engine were
@@ -887,7 +904,6 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
     const Shape sh = shape(L);
     LayerEngine &E = S.E[k];
     const std::vector<TensorDev> &T = E.tensors_host;
-    const int nbk = (na + nt - 1) / nt;
     if (!simt_only && plan_.nlm <= 32 && L.nlmi <= 32 && L.C % S3M_CH == 0)
       GB_LAUNCH(spbf3_fwd_mma_kernel, dim3(na, L.C / S3M_CH), 32 * S3M_CH, smem_mma, bonds, spbf(k), sht, T[L.tA].p, NC, a0);
     else
@@ -896,9 +912,9 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
     if (!outputs) return;
     if (k < 2) {
       const EqNormDev e{S.eq_dw[k].get(), S.eq_mask[k].get(), S.eq_aff[k].get(), S.eq_e[k].get(), L.nfEQ, L.cEQ, L.eq_center, L.eq_eps};
-      GB_LAUNCH(eqnorm_fwd_kernel, nbk, nt, 0, e, T[L.tEQ].p, S.msg[k].get(), NC, na, a0);
+      GB_LAUNCH(eqnorm_fwd_kernel, na, 32 * EQ_WARPS, 0, e, T[L.tEQ].p, S.msg[k].get(), NC, a0);
     }
-    GB_LAUNCH(rmsnorm_fwd_kernel, nbk, nt, 0, T[L.tRHO].p, S.rho_scale[k].get(), L.rho_n0, wr, S.rho_sum.get(), k == 0 ? 1 : 0, na, a0);
+    GB_LAUNCH(rmsnorm_fwd_kernel, (na + 3) / 4, 128, 0, T[L.tRHO].p, S.rho_scale[k].get(), L.rho_n0, wr, S.rho_sum.get(), k == 0 ? 1 : 0, na, a0);
   };
   // reverse operations of layer k for the atoms [a0, a0 + na), whose forward tensors are in the bound arena
   auto reverse = [&](int k, int a0, int na, float *base) {
@@ -906,13 +922,12 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
     const Shape sh = shape(L);
     LayerEngine &E = S.E[k];
     const std::vector<TensorDev> &T = E.tensors_host;
-    const int nbk = (na + nt - 1) / nt;
     if (L.dense.zero_grads)
       launch_fill_zero(base + (size_t) E.grad_begin * NC, sizeof(float) * (size_t) (E.grad_end - E.grad_begin) * NC);
-    GB_LAUNCH(rmsnorm_bwd_kernel, nbk, nt, 0, T[L.tRHO].p, S.rho_scale[k].get(), L.rho_n0, wr, S.drho.get(), T[L.tGRHO].p, na, a0);
+    GB_LAUNCH(rmsnorm_bwd_kernel, (na + 3) / 4, 128, 0, T[L.tRHO].p, S.rho_scale[k].get(), L.rho_n0, wr, S.drho.get(), T[L.tGRHO].p, na, a0);
     if (k < 2) {
       const EqNormDev e{S.eq_dw[k].get(), S.eq_mask[k].get(), S.eq_aff[k].get(), S.eq_e[k].get(), L.nfEQ, L.cEQ, L.eq_center, L.eq_eps};
-      GB_LAUNCH(eqnorm_bwd_kernel, nbk, nt, 0, e, T[L.tEQ].p, S.gmsg[k].get(), T[L.tGEQ].p, NC, na, a0);
+      GB_LAUNCH(eqnorm_bwd_kernel, na, 32 * EQ_WARPS, 0, e, T[L.tEQ].p, S.gmsg[k].get(), T[L.tGEQ].p, NC, a0);
     }
     run(E, L.dense.bwd, mu + a0, na, NC);
     GB_LAUNCH(spbf3_bwd_kernel, dim3(na, sh.slices), sh.threads, sh.smem_bwd, bonds, spbf(k), sht, T[L.tGA].p, NC, fv_.get(), vir_atom_.get(),
@@ -924,7 +939,7 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
     for (int a0 = 0; a0 < n; a0 += NC) forward(k, a0, std::min(NC, n - a0), true);
   }
   const Readout3Dev ro{S.eW0.get(), S.eW1.get(), shift_.get(), Q.en0, Q.en1, plan_.out_scale, Q.e_nin, Q.e_nh, Q.e_act};
-  GB_LAUNCH(readout3_kernel, nblk, nt, 0, ro, S.rho_sum.get(), mu, e_atom_.get(), S.drho.get(), energy_only ? 0 : 1, n);
+  GB_LAUNCH(readout3_kernel, (n + 3) / 4, 128, 0, ro, S.rho_sum.get(), mu, e_atom_.get(), S.drho.get(), energy_only ? 0 : 1, n);
   if (tm) tm->end(StageTimer::FWD);
   if (energy_only) return;
   if (tm) tm->begin(StageTimer::BWD);
