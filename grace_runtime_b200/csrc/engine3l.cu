@@ -5,13 +5,15 @@
 // of the density; the readout on the sum of the three densities; then everything in reverse.  While they fit, the
 // tensors of the three layers of all atoms are kept for the reverse pass; larger structures run every layer in passes
 // over atom chunks and recompute a chunk's forward tensors when it is reversed.  A first form of the path, checked
-// against the reference's CPU engine; its bond kernels are bound by instruction issue and not tuned.
+// against the reference's CPU engine.
 #include "engine.h"
 
 #include "bond_common.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
+#include <cstring>
 
 namespace gb {
 
@@ -26,35 +28,17 @@ struct Spbf3Dev {
   float *gmsg;               // [n][nlmi][C] its gradient, added to atomically (null: layer 1)
   const float *zproj;        // [n_elements][C]
   const float *l0mask;       // [nlmi]
-  const int *lt;             // [nlm]
-  const int *cg_off, *cg_p, *cgt_off, *cgt_f;
-  const float *cg_v, *cgt_v;
+  const int *cg_off, *cgt_off;    // the couple by output function, and by (harmonic, message function) pair
+  const int2 *cg;            // (harmonic << 16 | message function, coefficient bits)
+  const int2 *cgt;           // (output function, coefficient bits)
   int N, C, nl, nlm, nlmi, nfA, nel;
 };
 
 
-// Y (and its gradient) of one bond by one thread; lm < nlm are kept
-__device__ void stage_harmonics(const SHTable &sht, float ux, float uy, float uz, int nlm, float *Y, float *G)
-{
-  sph_harm<4, true>(sht, ux, uy, uz, [&](int lm, float v, float gx, float gy, float gz) {
-    if (lm < nlm) {
-      Y[lm] = v;
-      if (G) {
-        G[3 * lm] = gx;
-        G[3 * lm + 1] = gy;
-        G[3 * lm + 2] = gz;
-      }
-    }
-  });
-}
-
-constexpr int S3_BB = 64;    // bonds whose harmonics are staged at once
-constexpr int S3_T = 5;      // a thread keeps a tile of S3_T x S3_T (Y lm, message function) pairs of one channel in registers
-
-// Thread layout of both kernels.  A CTA works on one atom and a slice of CC = 2^cshift channels (blockIdx.y); thread
-// tid has the channel c = tid % CC of the slice and the tile g = tid / CC of the (ly, li) plane: ly in [5 tl, 5 tl + 5),
-// li in [5 ti, 5 ti + 5) with tl = g / nTI, ti = g % nTI.  The 25 products of a tile and a bond need 5 + 5 shared-memory
-// reads, and the bond sums P (or their gradients) never leave the registers.
+constexpr int S3_BB = 64;     // bonds whose harmonics and geometry are staged at once
+constexpr int S3_NBS = 8;     // bonds whose radial functions are evaluated together
+constexpr int S3_LIT = 5;     // message functions of a thread
+constexpr int S3_WARPS = 5;   // most warps of a CTA
 
 __device__ __forceinline__ void s3_cp16(void *dst_smem, const void *src)
 {
@@ -63,456 +47,362 @@ __device__ __forceinline__ void s3_cp16(void *dst_smem, const void *src)
 __device__ __forceinline__ void s3_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void s3_cp_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// geometry of a bond: neighbour, its element, table of the element pair, table row and offset, distance and cutoff.
-// Worked out once per batch of bonds by one thread per bond (a chain of dependent global loads: record -> element of the
-// neighbour -> table of the pair) and kept in shared memory, 8 words per bond.
-struct S3Bond {
-  int j, muj, slot, k0;
+// Geometry of a bond, worked out once per batch of bonds by one thread per bond (a chain of dependent global loads: record
+// -> element of the neighbour -> table of the pair) and kept in shared memory.
+struct __align__(16) S3Bond {
+  int j, muj;
+  long long tab;    // offset of the bond's table row in floats, < 0: no table for this element pair, the bond is left out
   float t, r, rc;
+  int pad;
 };
-__device__ __forceinline__ void s3_bond_store(const BondsDev &b, const Spbf3Dev &L, long long at, int mui, float *meta)
-{
-  const float4 rec = b.rec[at];
-  const int j = __float_as_int(rec.w), muj = b.mu[j];
-  const float r = sqrtf(rec.x * rec.x + rec.y * rec.y + rec.z * rec.z), rc = L.rc[mui * L.nel + muj];
-  int k0;
-  float t;
-  spline_locate(r / rc, L.N, k0, t);
-  meta[0] = __int_as_float(j);
-  meta[1] = __int_as_float(muj);
-  meta[2] = __int_as_float(L.pair_slot[mui * L.nel + muj]);    // < 0: no table for this element pair, the bond is left out
-  meta[3] = __int_as_float(k0);
-  meta[4] = t;
-  meta[5] = r;
-  meta[6] = rc;
-}
-__device__ __forceinline__ S3Bond s3_bond(const float *meta)
+__device__ __forceinline__ S3Bond s3_bond(const BondsDev &b, const Spbf3Dev &L, const float4 &rec, int mui)
 {
   S3Bond o;
-  o.j = __float_as_int(meta[0]);
-  o.muj = __float_as_int(meta[1]);
-  o.slot = __float_as_int(meta[2]);
-  o.k0 = __float_as_int(meta[3]);
-  o.t = meta[4];
-  o.r = meta[5];
-  o.rc = meta[6];
+  o.j = __float_as_int(rec.w);
+  o.muj = b.mu[o.j];
+  o.r = sqrtf(rec.x * rec.x + rec.y * rec.y + rec.z * rec.z);
+  o.rc = L.rc[mui * L.nel + o.muj];
+  int k0;
+  spline_locate(o.r / o.rc, L.N, k0, o.t);
+  const int slot = L.pair_slot[mui * L.nel + o.muj];
+  o.tab = slot < 0 ? -1 : (long long) slot * L.tab_stride + (long long) k0 * L.nl * L.C * 4;
+  o.pad = 0;
   return o;
 }
 
-// asynchronous copies of what the bonds [at, at + ns) of an atom read from global memory, for the channel slice c0 ..
-// c0 + CC: the table rows [nl][CC] float4 of each bond to craw, the message rows [nlmi][CC] of its neighbour to mraw,
-// the chemical weights [CC] of the neighbour's element to zraw
-__device__ __forceinline__ void s3_issue(const Spbf3Dev &L, const float *meta, int ns, int c0, int cshift, float4 *craw, float *mraw,
-                                         float *zraw, int tid, int nth)
+// Bond sums of GRACE-3L and their reverse.  With U[ly] = Y_ly R_l(ly)[c] and I[li] = msg_j[li][c] + mask[li] zproj[mu_j][c] a
+// channel c of an atom is a small outer-product sum over the bonds j,
+//     P[ly][li] = sum_j U[ly] I[li]         (forward),
+//     W[ly] = sum_li gP[ly][li] I[li],  dE/dmsg_j[li] = sum_ly gP[ly][li] U[ly]      (reverse, per bond),
+// 625 multiply-adds per bond and channel at lmax 4 (three times that in reverse).  A CTA works on one atom and 32 channels,
+// lane = channel; a warp owns 5 message functions and ALL harmonics of them, so that a thread keeps 25 x 5 sums (or their
+// gradient) in registers and one bond costs it 5 message loads, 5 radial values and the harmonics (16-byte broadcast reads)
+// for 125 multiply-adds (250 in reverse), where tiles of 5 x 5 over 25 warps needed 10 shared-memory reads for 25 and staged
+// U and I through shared memory.  The message rows go straight from global memory to the registers of the one warp that
+// needs them, a bond ahead.  Bound by instruction issue: about 190 (forward) and 450 (reverse) instructions per bond and
+// warp.  31,250 atoms, lmax 4, 64 channels, both message layers: see the table of measurements at spbf3_bwd_kernel.
+// A layer without messages has one function: the warps share the bonds instead (LIT = 1).
+
+// radial functions (and derivatives) of the bonds of a group: thread e of the CTA owns the values e, e + nth, ... of
+// [bond][l][channel]; the coefficients travel to its own piece of `raw` by asynchronous copies issued a group ahead
+__device__ __forceinline__ void s3_issue(const Spbf3Dev &L, const S3Bond *meta, int ns, int c0, float4 *raw, int tid, int nth)
 {
-  const int CC = 1 << cshift, nT = L.nl * CC, nM4 = L.nlmi * CC / 4;
-  for (int s = 0; s < ns; s++) {
-    const S3Bond B = s3_bond(meta + 8 * s);
-    if (tid < CC / 4) s3_cp16(zraw + s * CC + 4 * tid, L.zproj + (size_t) B.muj * L.C + c0 + 4 * tid);
-    const float4 *tab = reinterpret_cast<const float4 *>(L.tab + (size_t) max(B.slot, 0) * L.tab_stride) + (size_t) B.k0 * L.nl * L.C + c0;
-    for (int e = tid; e < nT; e += nth) s3_cp16(craw + s * nT + e, tab + (e >> cshift) * L.C + (e & (CC - 1)));
-    if (L.msg) {
-      const float *m = L.msg + (size_t) B.j * L.nlmi * L.C + c0;
-      for (int e = tid; e < nM4; e += nth) {
-        const int li = (4 * e) >> cshift, cc = (4 * e) & (CC - 1);
-        s3_cp16(mraw + s * L.nlmi * CC + 4 * e, m + (size_t) li * L.C + cc);
-      }
-    }
+  for (int e = tid; e < ns * L.nl * 32; e += nth) {
+    const int c = e & 31, sl = e >> 5, s = sl / L.nl, l = sl - s * L.nl;
+    const long long at = meta[s].tab;
+    if (at >= 0 && c0 + c < L.C) s3_cp16(raw + e, L.tab + at + 4 * ((long long) l * L.C + c0 + c));
   }
   s3_cp_commit();
 }
-
-// ---- forward bond sums on the tensor cores --------------------------------------------------------------------------
-// For one atom and one channel c the bond sums are a small matrix product over the bonds j:
-//     P[ly][li] = sum_j U[j][ly] Ic[j][li],   U[j][ly] = Y_ly(j) R_l(ly)(j)[c],  Ic[j][li] = msg_j[li][c] + mask[li] z[mu_j][c]
-// with M = (lmax + 1)^2 <= 32 rows, N = message functions <= 32 columns, K = bonds.  A warp owns a channel and keeps the
-// 32 x 32 accumulators in registers (mma.sync m16n8k8 tf32, 2 x 4 tiles); every product is three instructions on hi / lo
-// splits (a_lo b_hi + a_hi b_lo + a_hi b_hi), which keeps fp32-level accuracy.  A CTA works on one atom and a slice of
-// 16 channels; the operands of 16 bonds at a time are staged in shared memory with a row stride of 40 floats, which
-// makes the fragment reads of a warp conflict-free.
-constexpr int S3M_CH = 16, S3M_GB = 16, S3M_LD = 40, S3M_CS = S3M_GB * S3M_LD + 1;    // CS: floats per channel block (odd: the
-                                                                                        // channel-major stores of the staging spread over the banks)
-
-__device__ __forceinline__ void s3_split(float x, unsigned &hi, unsigned &lo)
+template<bool GRAD>
+__device__ __forceinline__ void s3_radial(const Spbf3Dev &L, const S3Bond *meta, int ns, int c0, const float4 *raw, float *R, float *dR,
+                                          int tid, int nth)
 {
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
-  const float r = x - __uint_as_float(hi);
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(r));
-}
-__device__ __forceinline__ void s3_mma(float (&d)[4], const unsigned (&a)[4], const unsigned (&b)[2])
-{
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+  for (int e = tid; e < ns * L.nl * 32; e += nth) {
+    const int c = e & 31, s = (e >> 5) / L.nl;
+    float v = 0.0f, d = 0.0f;
+    if (meta[s].tab >= 0 && c0 + c < L.C) {
+      const float4 cf = raw[e];
+      const float t = meta[s].t;
+      v = cf.x + t * (cf.y + t * (cf.z + t * cf.w));
+      if (GRAD) d = (cf.y + t * (2.0f * cf.z + t * 3.0f * cf.w)) * (float) L.N;
+    }
+    R[e] = v;
+    if (GRAD) dR[e] = d;
+  }
 }
 
-__global__ void __launch_bounds__(32 * S3M_CH) spbf3_fwd_mma_kernel(BondsDev b, Spbf3Dev L, SHTable sht, float *__restrict__ A, int NA, int a0)
+// message functions li0 .. li0 + LIT of the neighbour of a bond, channel c
+template<int LIT>
+__device__ __forceinline__ void s3_message(const Spbf3Dev &L, const S3Bond &B, int li0, int c, bool in, unsigned masked, const float *mask,
+                                           float (&ic)[LIT])
 {
+#pragma unroll
+  for (int q = 0; q < LIT; q++)
+    ic[q] = L.msg && in && li0 + q < L.nlmi ? __ldg(L.msg + ((size_t) B.j * L.nlmi + li0 + q) * L.C + c) : 0.0f;
+  if (masked) {
+    const float z = in ? __ldg(L.zproj + (size_t) B.muj * L.C + c) : 0.0f;
+#pragma unroll
+    for (int q = 0; q < LIT; q++) ic[q] = fmaf(mask[q], z, ic[q]);
+  }
+}
+
+template<int LMAX> struct S3 {
+  static constexpr int NLM = (LMAX + 1) * (LMAX + 1), NL = LMAX + 1, YLD = (NLM + 3) / 4 * 4;
+};
+
+// A[f][a][c] = sum_q cg[q, f] P[q][c], q = ly nlmi + li
+template<int LMAX, int LIT>
+__global__ void __launch_bounds__(32 * S3_WARPS, 2) spbf3_fwd_kernel(BondsDev b, Spbf3Dev L, SHTable sht, float *__restrict__ A, int NA,
+                                                                     int a0)
+{
+  constexpr int NLM = S3<LMAX>::NLM, NL = S3<LMAX>::NL, YLD = S3<LMAX>::YLD;
   extern __shared__ __align__(16) float sm[];
-  const int C = L.C, nlm = L.nlm, nlmi = L.nlmi, nth = blockDim.x;
-  float *Us = sm, *Is = Us + S3M_CH * S3M_CS, *meta = Is + S3M_CH * S3M_CS + 3, *Ys = meta + 8 * S3_BB;
-  float *mask = Ys + S3_BB * nlm;
-  int *lts = reinterpret_cast<int *>(mask + 32);
-  const int a = blockIdx.x, i = a0 + a, c0 = blockIdx.y * S3M_CH, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int g = lane >> 2, t = lane & 3;
+  float *Ps = sm;                                                  // [nlm nlmi][32], after the bond loop; below: during it
+  float4 *raw = reinterpret_cast<float4 *>(sm);                    // [NBS][nl][32]
+  float *Rs = sm + 4 * S3_NBS * NL * 32;                           // [2][NBS][nl][32]
+  float *Ys = Rs + 2 * S3_NBS * NL * 32;                           // [BB][YLD]
+  S3Bond *meta = reinterpret_cast<S3Bond *>(Ys + S3_BB * YLD);     // [BB]
+  const int nth = blockDim.x, nw = nth >> 5, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ap = blockIdx.y, i = a0 + ap, c0 = blockIdx.x * 32, c = c0 + lane;
+  const bool in = c < L.C;
   const long long base = b.off[i];
   const int nb = b.cnt[i], mui = b.mu[i];
-  float acc[2][4][4];
+  const int ntile = LIT == 1 ? 1 : (L.nlmi + LIT - 1) / LIT, nround = LIT == 1 ? 1 : (ntile + nw - 1) / nw;
+  float acc[NLM][LIT];
+  for (int round = 0; round < nround; round++) {
+    const int li0 = LIT == 1 ? 0 : (round * nw + warp) * LIT;
+    float mask[LIT];
+    unsigned masked = 0;
 #pragma unroll
-  for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-    for (int nt = 0; nt < 4; nt++)
-#pragma unroll
-      for (int r = 0; r < 4; r++) acc[mt][nt][r] = 0.0f;
-  for (int e = tid; e < nlm; e += nth) lts[e] = L.lt[e];
-  for (int e = tid; e < 32; e += nth) mask[e] = e < nlmi ? L.l0mask[e] : 0.0f;
-  for (int q0 = 0; q0 < nb; q0 += S3_BB) {
-    const int nq = min(S3_BB, nb - q0);
-    __syncthreads();    // harmonics and geometry of the previous batch are no longer read
-    for (int e = tid; e < nq; e += nth) {
-      const float4 rec = b.rec[base + q0 + e];
-      const float ir = rsqrtf(rec.x * rec.x + rec.y * rec.y + rec.z * rec.z);
-      stage_harmonics(sht, rec.x * ir, rec.y * ir, rec.z * ir, nlm, Ys + e * nlm, nullptr);
-      s3_bond_store(b, L, base + q0 + e, mui, meta + 8 * e);
+    for (int q = 0; q < LIT; q++) {
+      mask[q] = li0 + q < L.nlmi ? L.l0mask[li0 + q] : 0.0f;
+      masked |= mask[q] != 0.0f;
     }
-    for (int q = 0; q < nq; q += S3M_GB) {
-      const int ns = min(S3M_GB, nq - q);
-      __syncthreads();    // the operands of the previous group are no longer read; harmonics and geometry are staged
-      // operands of the group: rows (channel, bond), the function index runs along the lanes; rows of bonds beyond the
-      // group and functions beyond the model's are zero
-      for (int e = tid; e < S3M_CH * S3M_GB * 32; e += nth) {    // U: a warp per (channel, bond) row, the lanes along ly
-        const int f = e & 31, row = e >> 5, s = row % S3M_GB, ch = row / S3M_GB;
-        float u = 0.0f;
-        if (s < ns && f < nlm) {
-          const S3Bond B = s3_bond(meta + 8 * (q + s));
-          if (B.slot >= 0) {
-            const float4 cf = reinterpret_cast<const float4 *>(L.tab + (size_t) B.slot * L.tab_stride)[((size_t) B.k0 * L.nl + lts[f]) * C + c0 + ch];
-            u = Ys[(q + s) * nlm + f] * (cf.x + B.t * (cf.y + B.t * (cf.z + B.t * cf.w)));
-          }
-        }
-        Us[ch * S3M_CS + s * S3M_LD + f] = u;
-      }
-      for (int e = tid; e < S3M_GB * 32 * S3M_CH; e += nth) {    // Ic: the lanes along the channels (whole 64-byte pieces of a row)
-        const int ch = e % S3M_CH, f = (e / S3M_CH) & 31, s = e / (S3M_CH * 32);
-        float ic = 0.0f;
-        if (s < ns && f < nlmi) {
-          const S3Bond B = s3_bond(meta + 8 * (q + s));
-          ic = (L.msg ? L.msg[((size_t) B.j * nlmi + f) * C + c0 + ch] : 0.0f) + mask[f] * L.zproj[(size_t) B.muj * C + c0 + ch];
-        }
-        Is[ch * S3M_CS + s * S3M_LD + f] = ic;
+#pragma unroll
+    for (int a = 0; a < NLM; a++)
+#pragma unroll
+      for (int q = 0; q < LIT; q++) acc[a][q] = 0.0f;
+    for (int q0 = 0; q0 < nb; q0 += S3_BB) {
+      const int nq = min(S3_BB, nb - q0);
+      __syncthreads();    // what the batch before (the sums of the round before) left is no longer read
+      for (int e = tid; e < nq; e += nth) {
+        const float4 rec = b.rec[base + q0 + e];
+        const float ir = rsqrtf(rec.x * rec.x + rec.y * rec.y + rec.z * rec.z);
+        sph_harm<LMAX, false>(sht, rec.x * ir, rec.y * ir, rec.z * ir, [&](int lm, float v, float, float, float) { Ys[e * YLD + lm] = v; });
+        meta[e] = s3_bond(b, L, rec, mui);
       }
       __syncthreads();
-      const float *Uw = Us + warp * S3M_CS, *Iw = Is + warp * S3M_CS;
+      s3_issue(L, meta, min(S3_NBS, nq), c0, raw, tid, nth);
+      float nxt[LIT];
+      if (LIT > 1) s3_message<LIT>(L, meta[0], li0, c, in, masked, mask, nxt);
+      for (int q = 0, k = 0; q < nq; q += S3_NBS, k ^= 1) {
+        const int ns = min(S3_NBS, nq - q);
+        float *R = Rs + k * S3_NBS * NL * 32;
+        s3_cp_wait();
+        s3_radial<false>(L, meta + q, ns, c0, raw, R, nullptr, tid, nth);
+        if (q + S3_NBS < nq) s3_issue(L, meta + q + S3_NBS, min(S3_NBS, nq - q - S3_NBS), c0, raw, tid, nth);
+        __syncthreads();    // R of this group is complete; the other half was last read before the barrier of the group before
+        for (int s = LIT == 1 ? warp : 0; s < ns; s += LIT == 1 ? nw : 1) {
+          float ic[LIT];
+          if (LIT == 1) s3_message<LIT>(L, meta[q + s], li0, c, in, masked, mask, ic);
+          else {
 #pragma unroll
-      for (int k8 = 0; k8 < S3M_GB; k8 += 8) {
-        if (k8 >= ns) break;
-        // A[m = ly][k = bond] = U[bond][ly], B[k = bond][n = li] = Ic[bond][li]
-        unsigned ah[2][4], al[2][4], bh[4][2], bl[4][2];
-#pragma unroll
-        for (int mt = 0; mt < 2; mt++) {
-          s3_split(Uw[(k8 + t) * S3M_LD + 16 * mt + g], ah[mt][0], al[mt][0]);
-          s3_split(Uw[(k8 + t) * S3M_LD + 16 * mt + g + 8], ah[mt][1], al[mt][1]);
-          s3_split(Uw[(k8 + t + 4) * S3M_LD + 16 * mt + g], ah[mt][2], al[mt][2]);
-          s3_split(Uw[(k8 + t + 4) * S3M_LD + 16 * mt + g + 8], ah[mt][3], al[mt][3]);
-        }
-#pragma unroll
-        for (int nt = 0; nt < 4; nt++) {
-          s3_split(Iw[(k8 + t) * S3M_LD + 8 * nt + g], bh[nt][0], bl[nt][0]);
-          s3_split(Iw[(k8 + t + 4) * S3M_LD + 8 * nt + g], bh[nt][1], bl[nt][1]);
-        }
-#pragma unroll
-        for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-          for (int nt = 0; nt < 4; nt++) {
-            s3_mma(acc[mt][nt], al[mt], bh[nt]);
-            s3_mma(acc[mt][nt], ah[mt], bl[nt]);
-            s3_mma(acc[mt][nt], ah[mt], bh[nt]);
+            for (int x = 0; x < LIT; x++) ic[x] = nxt[x];
+            if (q + s + 1 < nq) s3_message<LIT>(L, meta[q + s + 1], li0, c, in, masked, mask, nxt);
           }
+          const float4 *Y4 = reinterpret_cast<const float4 *>(Ys + (q + s) * YLD);
+          float Rl[NL];
+#pragma unroll
+          for (int l = 0; l < NL; l++) Rl[l] = R[(s * NL + l) * 32 + lane];
+          constexpr int L_OF[25] = {0, 1, 1, 1, 2, 2, 2, 2, 2, 3, 3, 3, 3, 3, 3, 3, 4, 4, 4, 4, 4, 4, 4, 4, 4};
+#pragma unroll
+          for (int y = 0; y < YLD / 4; y++) {
+            const float4 yv = Y4[y];
+            const float ya[4] = {yv.x, yv.y, yv.z, yv.w};
+#pragma unroll
+            for (int x = 0; x < 4; x++) {
+              const int ly = 4 * y + x;
+              if (ly >= NLM) continue;
+              const float u = ya[x] * Rl[L_OF[ly]];
+#pragma unroll
+              for (int z = 0; z < LIT; z++) acc[ly][z] = fmaf(u, ic[z], acc[ly][z]);
+            }
+          }
+        }
       }
     }
-  }
-  // P of the 16 channels to shared memory [channel][ly][li] (32 x 33), then the couple: one thread per (function, channel)
-  __syncthreads();
-  float *Ps = sm;
-  {
-    float *Pw = Ps + warp * 32 * 33;
-#pragma unroll
-    for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-      for (int nt = 0; nt < 4; nt++) {
-        Pw[(16 * mt + g) * 33 + 8 * nt + 2 * t] = acc[mt][nt][0];
-        Pw[(16 * mt + g) * 33 + 8 * nt + 2 * t + 1] = acc[mt][nt][1];
-        Pw[(16 * mt + g + 8) * 33 + 8 * nt + 2 * t] = acc[mt][nt][2];
-        Pw[(16 * mt + g + 8) * 33 + 8 * nt + 2 * t + 1] = acc[mt][nt][3];
-      }
-  }
-  __syncthreads();
-  for (int e = tid; e < L.nfA * S3M_CH; e += nth) {
-    const int f = e / S3M_CH, ch = e - f * S3M_CH;
-    const float *Pc = Ps + ch * 32 * 33;
-    float v = 0.0f;
-    for (int k = L.cg_off[f]; k < L.cg_off[f + 1]; k++) {
-      const int q = L.cg_p[k], ly = q / nlmi, li = q - ly * nlmi;
-      v = fmaf(L.cg_v[k], Pc[ly * 33 + li], v);
-    }
-    A[((size_t) f * NA + a) * C + c0 + ch] = v;
-  }
-}
-
-constexpr int S3_NBS = 4;    // bonds staged and worked on together: one pair of barriers and one round of global loads for all
-
-// A[f][a][c] = sum_q cg[q, f] P[q][c],  P[(ly, li)][c] = sum_bonds Y_ly R[l(ly)][c] (msg_j[li][c] + mask[li] zproj[mu_j][c])
-__global__ void __launch_bounds__(832) spbf3_fwd_kernel(BondsDev b, Spbf3Dev L, SHTable sht, float *__restrict__ A, int NA, int cshift,
-                                                        int nTI, int a0)
-{
-  extern __shared__ __align__(16) float sm[];
-  const int C = L.C, nlm = L.nlm, nlmi = L.nlmi, CC = 1 << cshift, nth = blockDim.x;
-  const int nU = nlm * CC, nI = nlmi * CC;
-  const int nT = L.nl * CC;
-  float4 *craw = reinterpret_cast<float4 *>(sm);                      // [2][NBS][nl][CC] table rows
-  float *mraw = reinterpret_cast<float *>(craw + 2 * S3_NBS * nT);    // [2][NBS][nlmi][CC] message rows
-  float *zraw = mraw + 2 * (size_t) S3_NBS * nI;                      // [2][NBS][CC] chemical weights of the neighbours' elements
-  float *meta = zraw + 2 * S3_NBS * CC, *Ys = meta + 8 * S3_BB, *U = Ys + S3_BB * nlm, *Ic = U + (size_t) S3_NBS * nU,
-        *As = Ic + (size_t) S3_NBS * nI, *mask = As + (size_t) L.nfA * CC;
-  int *lts = reinterpret_cast<int *>(mask + nlmi);                    // l of each lm, and the mask of the message functions above
-  const int ap = blockIdx.x, i = a0 + ap, c0 = blockIdx.y * CC, tid = threadIdx.x;
-  const int c = tid & (CC - 1), g = tid >> cshift, tl = g / nTI, ti = g - tl * nTI, ly0 = S3_T * tl, li0 = S3_T * ti;
-  const long long base = b.off[i];
-  const int nb = b.cnt[i], mui = b.mu[i];
-  float acc[S3_T][S3_T];
-#pragma unroll
-  for (int a = 0; a < S3_T; a++)
-#pragma unroll
-    for (int q = 0; q < S3_T; q++) acc[a][q] = 0.0f;
-  for (int e = tid; e < nlm; e += nth) lts[e] = L.lt[e];
-  for (int e = tid; e < nlmi; e += nth) mask[e] = L.l0mask[e];
-  for (int q0 = 0; q0 < nb; q0 += S3_BB) {
-    const int nq = min(S3_BB, nb - q0);
-    __syncthreads();    // the harmonics of the previous batch are no longer read
-    for (int e = tid; e < nq; e += nth) {
-      const float4 rec = b.rec[base + q0 + e];
-      const float ir = rsqrtf(rec.x * rec.x + rec.y * rec.y + rec.z * rec.z);
-      stage_harmonics(sht, rec.x * ir, rec.y * ir, rec.z * ir, nlm, Ys + e * nlm, nullptr);
-      s3_bond_store(b, L, base + q0 + e, mui, meta + 8 * e);
-    }
+    // the couple: the sums of this round go to shared memory, and each function collects the pairs it is made of (a function
+    // is added up by one thread per channel, across the rounds in global memory)
     __syncthreads();
-    s3_issue(L, meta, min(S3_NBS, nq), c0, cshift, craw, mraw, zraw, tid, nth);    // the first group of the batch
-    for (int q = 0, k = 0; q < nq; q += S3_NBS, k ^= 1) {
-      const int ns = min(S3_NBS, nq - q);
-      s3_cp_wait();
-      __syncthreads();    // this group's rows have arrived; U and Ic of the previous group are no longer read
-      if (q + S3_NBS < nq)    // the next group's rows travel while this group is worked on
-        s3_issue(L, meta + 8 * (q + S3_NBS), min(S3_NBS, nq - q - S3_NBS), c0, cshift, craw + (k ^ 1) * S3_NBS * nT,
-                 mraw + (size_t) (k ^ 1) * S3_NBS * nI, zraw + (k ^ 1) * S3_NBS * CC, tid, nth);
-      for (int s = 0; s < ns; s++) {
-        const S3Bond B = s3_bond(meta + 8 * (q + s));
-        const float4 *cr = craw + (k * S3_NBS + s) * nT;
-        const float *mr = mraw + (size_t) (k * S3_NBS + s) * nI, *Y = Ys + (q + s) * nlm;
-        const float t = B.t;
-        for (int e = tid; e < nU; e += nth) {    // U[ly][c] = Y_ly R_l(ly)[c]
-          const int ly = e >> cshift, cc = e & (CC - 1);
-          const float4 cf = cr[lts[ly] * CC + cc];
-          U[s * nU + e] = B.slot < 0 ? 0.0f : Y[ly] * (cf.x + t * (cf.y + t * (cf.z + t * cf.w)));
-        }
-        for (int e = tid; e < nI; e += nth) {
-          const int li = e >> cshift, cc = e & (CC - 1);
-          Ic[s * nI + e] = (L.msg ? mr[e] : 0.0f) + mask[li] * zraw[(k * S3_NBS + s) * CC + cc];
-        }
-      }
-      __syncthreads();
-      for (int s = 0; s < ns; s++) {
-        float u[S3_T], ic[S3_T];
+    const int pitch = LIT == 1 ? 1 : nw * LIT;
 #pragma unroll
-        for (int a = 0; a < S3_T; a++) u[a] = ly0 + a < nlm ? U[s * nU + (ly0 + a) * CC + c] : 0.0f;
+    for (int a = 0; a < NLM; a++)
 #pragma unroll
-        for (int q2 = 0; q2 < S3_T; q2++) ic[q2] = li0 + q2 < nlmi ? Ic[s * nI + (li0 + q2) * CC + c] : 0.0f;
-#pragma unroll
-        for (int a = 0; a < S3_T; a++)
-#pragma unroll
-          for (int q2 = 0; q2 < S3_T; q2++) acc[a][q2] = fmaf(u[a], ic[q2], acc[a][q2]);
-      }
-    }
-  }
-  // the couple: every pair's sum goes to the functions it feeds (shared-memory adds), then the slice is written
-  __syncthreads();
-  for (int e = tid; e < L.nfA * CC; e += nth) As[e] = 0.0f;
-  __syncthreads();
-#pragma unroll
-  for (int a = 0; a < S3_T; a++)
-#pragma unroll
-    for (int q2 = 0; q2 < S3_T; q2++) {
-      if (ly0 + a >= nlm || li0 + q2 >= nlmi) continue;
-      const int q = (ly0 + a) * nlmi + li0 + q2;
-      for (int t = L.cgt_off[q]; t < L.cgt_off[q + 1]; t++) atomicAdd(&As[L.cgt_f[t] * CC + c], L.cgt_v[t] * acc[a][q2]);
-    }
-  __syncthreads();
-  for (int e = tid; e < L.nfA * CC; e += nth) {
-    const int f = e >> cshift, cc = e & (CC - 1);
-    A[((size_t) f * NA + ap) * C + c0 + cc] = As[e];
-  }
-}
-
-// Reverse of the above from gA: bond forces and per-atom virial (added: the caller clears them before the first layer
-// is reversed), dE/dmsg of the neighbours.  The thread's tile of gP[(ly, li)][c] = sum_f cg[q, f] gA[f][c] stays in
-// registers; per bond
-//   W[ly][c] = sum_li gP Ic[li][c],   dE/dmsg_j[li][c] += sum_ly gP Y_ly R_l[c]      (tiles add their shares in shared memory)
-//   gY[ly] = sum_c W R_l[c] (a warp per ly),  dE/dx = sum_{ly, c} W Y_ly dR_l[c]
-// and the bond force is linear in (gY, dE/dx), so every channel slice adds its own share.
-__global__ void __launch_bounds__(832) spbf3_bwd_kernel(BondsDev b, Spbf3Dev L, SHTable sht, const float *__restrict__ gA, int NA,
-                                                        float *__restrict__ fv, double *__restrict__ vir_atom, int cshift, int nTI,
-                                                        int a0)
-{
-  extern __shared__ __align__(16) float sm[];
-  const int C = L.C, nlm = L.nlm, nlmi = L.nlmi, CC = 1 << cshift, nth = blockDim.x;
-  const int nU = nlm * CC, nI = nlmi * CC;
-  const int nT = L.nl * CC;
-  float4 *craw = reinterpret_cast<float4 *>(sm);                      // [2][NBS][nl][CC] table rows
-  float *mraw = reinterpret_cast<float *>(craw + 2 * S3_NBS * nT);    // [2][NBS][nlmi][CC] message rows
-  float *zraw = mraw + 2 * (size_t) S3_NBS * nI;                      // [2][NBS][CC] chemical weights of the neighbours' elements
-  float *meta = zraw + 2 * S3_NBS * CC, *Ys = meta + 8 * S3_BB, *Gs = Ys + S3_BB * nlm, *Rl = Gs + 3 * S3_BB * nlm, *dRl = Rl + (size_t) S3_NBS * nU,
-        *W = dRl + (size_t) S3_NBS * nU;
-  float *Ic = W + (size_t) S3_NBS * nU, *gI = Ic + (size_t) S3_NBS * nI, *gY = gI + (size_t) S3_NBS * nI, *dedx = gY + S3_NBS * nlm;
-  float *mask = dedx + 8;
-  int *lts = reinterpret_cast<int *>(mask + nlmi);
-  const int ap = blockIdx.x, i = a0 + ap, c0 = blockIdx.y * CC, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int c = tid & (CC - 1), g = tid >> cshift, tl = g / nTI, ti = g - tl * nTI, ly0 = S3_T * tl, li0 = S3_T * ti;
-  const long long base = b.off[i];
-  const int nb = b.cnt[i], mui = b.mu[i];
-  double vir[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  float gp[S3_T][S3_T];
-#pragma unroll
-  for (int a = 0; a < S3_T; a++)
-#pragma unroll
-    for (int q2 = 0; q2 < S3_T; q2++) {
+      for (int q = 0; q < LIT; q++) Ps[(LIT == 1 ? warp * NLM + a : a * pitch + warp * LIT + q) * 32 + lane] = acc[a][q];
+    __syncthreads();
+    for (int f = warp; f < L.nfA; f += nw) {
       float v = 0.0f;
-      if (ly0 + a < nlm && li0 + q2 < nlmi) {
-        const int q = (ly0 + a) * nlmi + li0 + q2;
-        for (int t = L.cgt_off[q]; t < L.cgt_off[q + 1]; t++) v = fmaf(L.cgt_v[t], gA[((size_t) L.cgt_f[t] * NA + ap) * C + c0 + c], v);
+      const int k1 = L.cg_off[f + 1];
+#pragma unroll 4
+      for (int k = L.cg_off[f]; k < k1; k++) {
+        const int2 t = __ldg(L.cg + k);    // (harmonic, message function), coefficient
+        const int ly = t.x >> 16, li = (t.x & 0xffff) - round * pitch;
+        if (LIT == 1) {
+          float p = 0.0f;
+          for (int w = 0; w < nw; w++) p += Ps[(w * NLM + ly) * 32 + lane];
+          v = fmaf(__int_as_float(t.y), p, v);
+        } else if (li >= 0 && li < pitch) {
+          v = fmaf(__int_as_float(t.y), Ps[(ly * pitch + li) * 32 + lane], v);
+        }
       }
-      gp[a][q2] = v;
+      float *o = A + ((size_t) f * NA + ap) * L.C + c;
+      if (in) *o = round > 0 ? *o + v : v;
     }
-  for (int e = tid; e < nlm; e += nth) lts[e] = L.lt[e];
-  for (int e = tid; e < nlmi; e += nth) mask[e] = L.l0mask[e];
-  for (int q0 = 0; q0 < nb; q0 += S3_BB) {
-    const int nq = min(S3_BB, nb - q0);
-    __syncthreads();    // the harmonics of the previous batch are no longer read
-    for (int e = tid; e < nq; e += nth) {
-      const float4 rec = b.rec[base + q0 + e];
-      const float ir = rsqrtf(rec.x * rec.x + rec.y * rec.y + rec.z * rec.z);
-      stage_harmonics(sht, rec.x * ir, rec.y * ir, rec.z * ir, nlm, Ys + e * nlm, Gs + 3 * e * nlm);
-      s3_bond_store(b, L, base + q0 + e, mui, meta + 8 * e);
+  }
+}
+
+// Reverse of the above from gA: bond forces and per-atom virial (added: the caller clears them before the first layer is
+// reversed), dE/dmsg of the neighbours.  Per bond a thread needs, beside W and dE/dmsg, its share of
+//     sum_ly,c W R_l dY_ly/du   and   dE/dx = sum_ly,c W Y_ly dR_l/dx,
+// both summed over the functions of its warp as they come (the radial values are taken out of the sums over m), so that
+// only four numbers per bond and warp are added over the lanes and none of W leaves the registers.
+template<int LMAX, int LIT>
+__global__ void __launch_bounds__(32 * S3_WARPS, 2) spbf3_bwd_kernel(BondsDev b, Spbf3Dev L, SHTable sht, const float *__restrict__ gA,
+                                                                     int NA, float *__restrict__ fv, double *__restrict__ vir_atom,
+                                                                     int a0)
+{
+  constexpr int NLM = S3<LMAX>::NLM, NL = S3<LMAX>::NL;
+  extern __shared__ __align__(16) float sm[];
+  float4 *G4 = reinterpret_cast<float4 *>(sm);                       // [BB][NLM] gradient of the harmonic, its value
+  float4 *raw = G4 + S3_BB * NLM;                                    // [NBS][nl][32]
+  float *Rs = reinterpret_cast<float *>(raw + S3_NBS * NL * 32);     // [2][NBS][nl][32], then the derivatives
+  float *dRs = Rs + 2 * S3_NBS * NL * 32;
+  S3Bond *meta = reinterpret_cast<S3Bond *>(dRs + 2 * S3_NBS * NL * 32);    // [BB]
+  float *red = reinterpret_cast<float *>(meta + S3_BB);              // [2][NBS][4]
+  double *vir = reinterpret_cast<double *>(red + 2 * S3_NBS * 4);    // [NBS][6]
+  float *gAs = reinterpret_cast<float *>(vir + S3_NBS * 6);          // [nfA][32]
+  const int nth = blockDim.x, nw = nth >> 5, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ap = blockIdx.y, i = a0 + ap, c0 = blockIdx.x * 32, c = c0 + lane;
+  const bool in = c < L.C;
+  const long long base = b.off[i];
+  const int nb = b.cnt[i], mui = b.mu[i];
+  const int ntile = LIT == 1 ? 1 : (L.nlmi + LIT - 1) / LIT, nround = LIT == 1 ? 1 : (ntile + nw - 1) / nw;
+  for (int f = warp; f < L.nfA; f += nw) gAs[f * 32 + lane] = in ? __ldg(gA + ((size_t) f * NA + ap) * L.C + c) : 0.0f;
+  for (int e = tid; e < S3_NBS * 6; e += nth) vir[e] = 0.0;
+  for (int e = tid; e < 2 * S3_NBS * 4; e += nth) red[e] = 0.0f;
+  __syncthreads();
+  // force and virial share of the bond `tid` of a group from the four sums of its warps
+  auto finish = [&](int at, int ns, float *r4) {
+    if (tid >= ns) return;
+    const S3Bond B = meta[at + tid];
+    const float gx = r4[4 * tid], gy = r4[4 * tid + 1], gz = r4[4 * tid + 2], dedx = r4[4 * tid + 3];
+    r4[4 * tid] = r4[4 * tid + 1] = r4[4 * tid + 2] = r4[4 * tid + 3] = 0.0f;
+    const long long slot = base + B.pad;
+    const float4 rec = b.rec[slot];
+    const float r = B.r, ir = 1.0f / r, ux = rec.x * ir, uy = rec.y * ir, uz = rec.z * ir;
+    const float dEdr = dedx / B.rc, gr = gx * ux + gy * uy + gz * uz;
+    const float f0 = dEdr * ux + (gx - gr * ux) * ir, f1 = dEdr * uy + (gy - gr * uy) * ir, f2 = dEdr * uz + (gz - gr * uz) * ir;
+    float *o = fv + 3 * (size_t) b.cslot[slot];
+    atomicAdd(o, f0);
+    atomicAdd(o + 1, f1);
+    atomicAdd(o + 2, f2);
+    const double dx = -(double) ux * r, dy = -(double) uy * r, dz = -(double) uz * r;
+    double *v = vir + 6 * tid;
+    v[0] += dx * f0; v[1] += dy * f1; v[2] += dz * f2;
+    v[3] += dx * f1; v[4] += dx * f2; v[5] += dy * f2;
+  };
+  for (int round = 0; round < nround; round++) {
+    const int li0 = LIT == 1 ? 0 : (round * nw + warp) * LIT;
+    float mask[LIT], gp[NLM][LIT];
+    unsigned masked = 0;
+#pragma unroll
+    for (int q = 0; q < LIT; q++) {
+      mask[q] = li0 + q < L.nlmi ? L.l0mask[li0 + q] : 0.0f;
+      masked |= mask[q] != 0.0f;
     }
-    __syncthreads();
-    s3_issue(L, meta, min(S3_NBS, nq), c0, cshift, craw, mraw, zraw, tid, nth);    // the first group of the batch
-    for (int q = 0, k = 0; q < nq; q += S3_NBS, k ^= 1) {
-      const int ns = min(S3_NBS, nq - q);
-      s3_cp_wait();
-      __syncthreads();    // this group's rows have arrived; the buffers of the previous group are no longer read
-      if (q + S3_NBS < nq)    // the next group's rows travel while this group is worked on
-        s3_issue(L, meta + 8 * (q + S3_NBS), min(S3_NBS, nq - q - S3_NBS), c0, cshift, craw + (k ^ 1) * S3_NBS * nT,
-                 mraw + (size_t) (k ^ 1) * S3_NBS * nI, zraw + (k ^ 1) * S3_NBS * CC, tid, nth);
-      if (tid < S3_NBS) dedx[tid] = 0.0f;
-      for (int s = 0; s < ns; s++) {
-        const S3Bond B = s3_bond(meta + 8 * (q + s));
-        const float4 *cr = craw + (k * S3_NBS + s) * nT;
-        const float *mr = mraw + (size_t) (k * S3_NBS + s) * nI;
-        const float t = B.t;
-        for (int e = tid; e < nU; e += nth) {
-          const int ly = e >> cshift, cc = e & (CC - 1);
-          const float4 cf = cr[lts[ly] * CC + cc];
-          Rl[s * nU + e] = B.slot < 0 ? 0.0f : cf.x + t * (cf.y + t * (cf.z + t * cf.w));
-          dRl[s * nU + e] = B.slot < 0 ? 0.0f : (cf.y + t * (2.0f * cf.z + t * 3.0f * cf.w)) * (float) L.N;
-          W[s * nU + e] = 0.0f;
-        }
-        for (int e = tid; e < nI; e += nth) {
-          const int li = e >> cshift, cc = e & (CC - 1);
-          Ic[s * nI + e] = (L.msg ? mr[e] : 0.0f) + mask[li] * zraw[(k * S3_NBS + s) * CC + cc];
-          gI[s * nI + e] = 0.0f;
-        }
-      }
-      __syncthreads();
 #pragma unroll
-      for (int s = 0; s < S3_NBS; s++) {    // unrolled: the bonds of the group are independent work for the scheduler
-        if (s >= ns) break;
-        const float *Y = Ys + (q + s) * nlm;
-        float u[S3_T], ic[S3_T];
+    for (int a = 0; a < NLM; a++)
 #pragma unroll
-        for (int a = 0; a < S3_T; a++) u[a] = ly0 + a < nlm ? Y[ly0 + a] * Rl[s * nU + (ly0 + a) * CC + c] : 0.0f;
-#pragma unroll
-        for (int q2 = 0; q2 < S3_T; q2++) ic[q2] = li0 + q2 < nlmi ? Ic[s * nI + (li0 + q2) * CC + c] : 0.0f;
-        float w[S3_T], v[S3_T];
-#pragma unroll
-        for (int a = 0; a < S3_T; a++) w[a] = 0.0f;
-#pragma unroll
-        for (int q2 = 0; q2 < S3_T; q2++) v[q2] = 0.0f;
-#pragma unroll
-        for (int a = 0; a < S3_T; a++)
-#pragma unroll
-          for (int q2 = 0; q2 < S3_T; q2++) {
-            w[a] = fmaf(gp[a][q2], ic[q2], w[a]);
-            v[q2] = fmaf(gp[a][q2], u[a], v[q2]);
-          }
-#pragma unroll
-        for (int a = 0; a < S3_T; a++)
-          if (ly0 + a < nlm) atomicAdd(&W[s * nU + (ly0 + a) * CC + c], w[a]);
-        if (L.gmsg) {
-#pragma unroll
-          for (int q2 = 0; q2 < S3_T; q2++)
-            if (li0 + q2 < nlmi) atomicAdd(&gI[s * nI + (li0 + q2) * CC + c], v[q2]);
-        }
-      }
-      __syncthreads();
-      for (int s = 0; s < ns; s++) {
-        const float *Y = Ys + (q + s) * nlm;
-        float part = 0.0f;    // this thread's share of dE/dx
-        for (int e = tid; e < nU; e += nth) part = fmaf(W[s * nU + e] * Y[e >> cshift], dRl[s * nU + e], part);
-        for (int sh = 16; sh > 0; sh >>= 1) part += __shfl_xor_sync(0xffffffffu, part, sh);
-        if (lane == 0 && part != 0.0f) atomicAdd(&dedx[s], part);
-        if (L.gmsg) {
-          const int j = __float_as_int(meta[8 * (q + s)]);
-          for (int e = tid; e < nI / 4; e += nth) {    // four channels per atomic (16-byte vector add)
-            const int li = (4 * e) >> cshift, cc = (4 * e) & (CC - 1);
-            atomicAdd(reinterpret_cast<float4 *>(L.gmsg + ((size_t) j * nlmi + li) * C + c0 + cc),
-                      *reinterpret_cast<const float4 *>(gI + s * nI + 4 * e));
+      for (int q = 0; q < LIT; q++) {
+        float v = 0.0f;
+        if (li0 + q < L.nlmi) {
+          const int p = a * L.nlmi + li0 + q, k1 = __ldg(L.cgt_off + p + 1);
+          for (int k = __ldg(L.cgt_off + p); k < k1; k++) {
+            const int2 t = __ldg(L.cgt + k);    // function, coefficient
+            v = fmaf(__int_as_float(t.y), gAs[t.x * 32 + lane], v);
           }
         }
-        for (int ly = warp; ly < nlm; ly += nth / 32) {    // a warp per ly: the sum over the channels of the slice
-          float v = 0.0f;
-          for (int cc = lane; cc < CC; cc += 32) v = fmaf(W[s * nU + ly * CC + cc], Rl[s * nU + ly * CC + cc], v);
-          for (int sh = 16; sh > 0; sh >>= 1) v += __shfl_xor_sync(0xffffffffu, v, sh);
-          if (lane == 0) gY[s * nlm + ly] = v;
+        gp[a][q] = v;
+      }
+    for (int q0 = 0; q0 < nb; q0 += S3_BB) {
+      const int nq = min(S3_BB, nb - q0);
+      __syncthreads();    // what the batch before left is no longer read
+      for (int e = tid; e < nq; e += nth) {
+        const float4 rec = b.rec[base + q0 + e];
+        const float ir = rsqrtf(rec.x * rec.x + rec.y * rec.y + rec.z * rec.z);
+        sph_harm<LMAX, true>(sht, rec.x * ir, rec.y * ir, rec.z * ir, [&](int lm, float v, float gx, float gy, float gz) {
+          G4[e * NLM + lm] = make_float4(gx, gy, gz, v);
+        });
+        S3Bond B = s3_bond(b, L, rec, mui);
+        B.pad = q0 + e;    // where its record is
+        meta[e] = B;
+      }
+      __syncthreads();
+      s3_issue(L, meta, min(S3_NBS, nq), c0, raw, tid, nth);
+      float nxt[LIT];
+      if (LIT > 1) s3_message<LIT>(L, meta[0], li0, c, in, masked, mask, nxt);
+      int k = 0;
+      for (int q = 0; q < nq; q += S3_NBS, k ^= 1) {
+        const int ns = min(S3_NBS, nq - q);
+        float *R = Rs + k * S3_NBS * NL * 32, *dR = dRs + k * S3_NBS * NL * 32;
+        s3_cp_wait();
+        s3_radial<true>(L, meta + q, ns, c0, raw, R, dR, tid, nth);
+        if (q + S3_NBS < nq) s3_issue(L, meta + q + S3_NBS, min(S3_NBS, nq - q - S3_NBS), c0, raw, tid, nth);
+        __syncthreads();    // R of this group is complete, and so are the sums of the group before
+        if (q > 0) finish(q - S3_NBS, S3_NBS, red + (k ^ 1) * S3_NBS * 4);
+        for (int s = LIT == 1 ? warp : 0; s < ns; s += LIT == 1 ? nw : 1) {
+          float ic[LIT], v[LIT];
+          const int j = meta[q + s].j;
+          if (LIT == 1) s3_message<LIT>(L, meta[q + s], li0, c, in, masked, mask, ic);
+          else {
+#pragma unroll
+            for (int x = 0; x < LIT; x++) ic[x] = nxt[x];
+            if (q + s + 1 < nq) s3_message<LIT>(L, meta[q + s + 1], li0, c, in, masked, mask, nxt);
+          }
+          const float4 *G = G4 + (q + s) * NLM;
+#pragma unroll
+          for (int x = 0; x < LIT; x++) v[x] = 0.0f;
+          float gx = 0.0f, gy = 0.0f, gz = 0.0f, dx = 0.0f;
+#pragma unroll
+          for (int l = 0; l < NL; l++) {
+            const float Rl = R[(s * NL + l) * 32 + lane], dRl = dR[(s * NL + l) * 32 + lane];
+            float lx = 0.0f, ly = 0.0f, lz = 0.0f, lr = 0.0f;
+#pragma unroll
+            for (int m = l * l; m < (l + 1) * (l + 1); m++) {
+              const float4 g = G[m];
+              const float u = g.w * Rl;
+              float w = 0.0f;
+#pragma unroll
+              for (int x = 0; x < LIT; x++) {
+                w = fmaf(gp[m][x], ic[x], w);
+                v[x] = fmaf(gp[m][x], u, v[x]);
+              }
+              lx = fmaf(w, g.x, lx);
+              ly = fmaf(w, g.y, ly);
+              lz = fmaf(w, g.z, lz);
+              lr = fmaf(w, g.w, lr);
+            }
+            gx = fmaf(Rl, lx, gx);
+            gy = fmaf(Rl, ly, gy);
+            gz = fmaf(Rl, lz, gz);
+            dx = fmaf(dRl, lr, dx);
+          }
+          if (L.gmsg && in) {
+#pragma unroll
+            for (int x = 0; x < LIT; x++)
+              if (li0 + x < L.nlmi) atomicAdd(L.gmsg + ((size_t) j * L.nlmi + li0 + x) * L.C + c, v[x]);
+          }
+          // the four sums over the lanes by one tree: two exchanges leave each lane one of them, three more add it up
+          {
+            const bool h = lane & 16, g = lane & 8;
+            const float a0_ = (h ? gz : gx) + __shfl_xor_sync(0xffffffffu, h ? gx : gz, 16);
+            const float a1_ = (h ? dx : gy) + __shfl_xor_sync(0xffffffffu, h ? gy : dx, 16);
+            float t = (g ? a1_ : a0_) + __shfl_xor_sync(0xffffffffu, g ? a0_ : a1_, 8);
+            t += __shfl_xor_sync(0xffffffffu, t, 4);
+            t += __shfl_xor_sync(0xffffffffu, t, 2);
+            t += __shfl_xor_sync(0xffffffffu, t, 1);
+            if ((lane & 7) == 0) atomicAdd(red + (k * S3_NBS + s) * 4 + (h ? 2 : 0) + (g ? 1 : 0), t);
+          }
         }
       }
       __syncthreads();
-      if (tid < ns) {    // one thread per bond of the group
-        const int s = tid;
-        const float4 rec = b.rec[base + q0 + q + s];
-        const S3Bond B = s3_bond(meta + 8 * (q + s));
-        const float r = B.r, ir = 1.0f / r, rc = B.rc;
-        const float ux = rec.x * ir, uy = rec.y * ir, uz = rec.z * ir;
-        const float *Gq = Gs + 3 * (q + s) * nlm;
-        float gx = 0.0f, gy = 0.0f, gz = 0.0f;
-        for (int lm = 0; lm < nlm; lm++) {
-          const float w = gY[s * nlm + lm];
-          gx = fmaf(w, Gq[3 * lm], gx);
-          gy = fmaf(w, Gq[3 * lm + 1], gy);
-          gz = fmaf(w, Gq[3 * lm + 2], gz);
-        }
-        const float dEdr = dedx[s] / rc, gr = gx * ux + gy * uy + gz * uz;
-        const float f0 = dEdr * ux + (gx - gr * ux) * ir, f1 = dEdr * uy + (gy - gr * uy) * ir, f2 = dEdr * uz + (gz - gr * uz) * ir;
-        float *o = fv + 3 * (size_t) b.cslot[base + q0 + q + s];
-        atomicAdd(o, f0);
-        atomicAdd(o + 1, f1);
-        atomicAdd(o + 2, f2);
-        const double dx = -(double) ux * r, dy = -(double) uy * r, dz = -(double) uz * r;
-        vir[0] += dx * f0; vir[1] += dy * f1; vir[2] += dz * f2;
-        vir[3] += dx * f1; vir[4] += dx * f2; vir[5] += dy * f2;
-      }
+      if (nq > 0) finish((nq - 1) / S3_NBS * S3_NBS, nq - (nq - 1) / S3_NBS * S3_NBS, red + (k ^ 1) * S3_NBS * 4);
     }
   }
   if (tid < S3_NBS)
     for (int k = 0; k < 6; k++)
-      if (vir[k] != 0.0) atomicAdd(vir_atom + 6 * (size_t) i + k, vir[k]);
+      if (vir[6 * tid + k] != 0.0) atomicAdd(vir_atom + 6 * (size_t) i + k, vir[6 * tid + k]);
 }
 
 struct EqNormDev {
@@ -699,8 +589,9 @@ __global__ void __launch_bounds__(128) readout3_kernel(Readout3Dev R, const floa
 // device state of the three layers
 struct State3L {
   LayerEngine E[3];
-  DBuf<float> arena[3], tab[3], zproj[3], l0mask[3], cg_v[3], cgt_v[3], rho_scale[3];
-  DBuf<int> lt[3], cg_off[3], cg_p[3], cgt_off[3], cgt_f[3];
+  DBuf<float> arena[3], tab[3], zproj[3], l0mask[3], rho_scale[3];
+  DBuf<int> cg_off[3], cgt_off[3];
+  DBuf<int2> cg[3], cgt[3];
   DBuf<float> eq_dw[2], eq_mask[2], eq_aff[2], msg[2], gmsg[2];
   DBuf<int> eq_e[2];
   DBuf<int> pair_slot;
@@ -725,14 +616,21 @@ void Engine::setup_3l()
     setup_layer(S.E[k], L.dense);
     S.zproj[k].upload(L.zproj);
     S.l0mask[k].upload(L.l0mask);
-    S.cg_v[k].upload(L.cg_v);
-    S.cgt_v[k].upload(L.cgt_v);
     S.rho_scale[k].upload(L.rho_scale);
-    S.lt[k].upload(L.lt);
+    for (size_t q = 0; q < L.lt.size(); q++)    // the kernels take the radial function of a harmonic from its place
+      if (L.lt[q] != (int) std::sqrt((double) q)) throw Unsupported("GRACE-3L: harmonics are expected in the order lm = l (l + 1) + m");
+    std::vector<int2> cg, cgt;
+    auto bits = [](float v) {
+      int u;
+      std::memcpy(&u, &v, 4);
+      return u;
+    };
+    for (size_t t = 0; t < L.cg_p.size(); t++) cg.push_back(make_int2((L.cg_p[t] / L.nlmi) << 16 | (L.cg_p[t] % L.nlmi), bits(L.cg_v[t])));
+    for (size_t t = 0; t < L.cgt_f.size(); t++) cgt.push_back(make_int2(L.cgt_f[t], bits(L.cgt_v[t])));
     S.cg_off[k].upload(L.cg_off);
-    S.cg_p[k].upload(L.cg_p);
     S.cgt_off[k].upload(L.cgt_off);
-    S.cgt_f[k].upload(L.cgt_f);
+    S.cg[k].upload(cg);
+    S.cgt[k].upload(cgt);
     if (k < 2) {
       S.eq_dw[k].upload(L.eq_dw);
       S.eq_mask[k].upload(L.eq_mask);
@@ -803,13 +701,10 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
     d.gmsg = k > 0 ? S.gmsg[k - 1].get() : nullptr;
     d.zproj = S.zproj[k].get();
     d.l0mask = S.l0mask[k].get();
-    d.lt = S.lt[k].get();
     d.cg_off = S.cg_off[k].get();
-    d.cg_p = S.cg_p[k].get();
     d.cgt_off = S.cgt_off[k].get();
-    d.cgt_f = S.cgt_f[k].get();
-    d.cg_v = S.cg_v[k].get();
-    d.cgt_v = S.cgt_v[k].get();
+    d.cg = S.cg[k].get();
+    d.cgt = S.cgt[k].get();
     d.N = Q.spline_n;
     d.C = L.C;
     d.nl = plan_.lmax + 1;
@@ -819,35 +714,48 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
     d.nel = plan_.n_elements;
     return d;
   };
-  // launch shape of the bond kernels of a layer: channel slice, tiles of the (ly, li) plane, threads, shared memory
-  struct Shape {
-    int cshift, nTI, threads, slices;
-    size_t smem_fwd, smem_bwd;
+  // launches of the bond kernels: a warp per 5 message functions (a layer without messages: 4 warps that share the bonds)
+  auto bonds_forward = [&](int k, float *A, int NC, int a0, int na) {
+    const Layer3Plan &L = Q.L[k];
+    const bool one = L.nlmi == 1;
+    const int nw = one ? 4 : std::min(S3_WARPS, (L.nlmi + S3_LIT - 1) / S3_LIT), nlm = plan_.nlm, nl = plan_.lmax + 1;
+    const size_t stage = sizeof(float) * (6 * (size_t) S3_NBS * nl * 32 + (size_t) S3_BB * ((nlm + 3) / 4 * 4)) + sizeof(S3Bond) * S3_BB;
+    const size_t sums = sizeof(float) * 32 * (size_t) nlm * nw * (one ? 1 : S3_LIT), smem = std::max(stage, sums);
+    const dim3 grid((L.C + 31) / 32, na);
+    auto go = [&](auto kernel) {
+      GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024));
+      before_launch("spbf3_fwd_kernel");
+      kernel<<<grid, 32 * nw, smem, dev().stream>>>(bonds, spbf(k), sht, A, NC, a0);
+      after_launch("spbf3_fwd_kernel");
+    };
+    switch (plan_.lmax) {
+      case 1: one ? go(spbf3_fwd_kernel<1, 1>) : go(spbf3_fwd_kernel<1, S3_LIT>); break;
+      case 2: one ? go(spbf3_fwd_kernel<2, 1>) : go(spbf3_fwd_kernel<2, S3_LIT>); break;
+      case 3: one ? go(spbf3_fwd_kernel<3, 1>) : go(spbf3_fwd_kernel<3, S3_LIT>); break;
+      default: one ? go(spbf3_fwd_kernel<4, 1>) : go(spbf3_fwd_kernel<4, S3_LIT>); break;
+    }
   };
-  auto shape = [&](const Layer3Plan &L) {
-    const int nTL = (plan_.nlm + S3_T - 1) / S3_T, nTI = (L.nlmi + S3_T - 1) / S3_T, groups = nTL * nTI;
-    int cshift = 5;
-    while (cshift > 2 && (L.C % (1 << cshift) != 0 || groups * (1 << cshift) > 832)) cshift--;
-    const int CC = 1 << cshift;
-    if (L.C % CC != 0 || groups * CC > 832) throw Unsupported("GRACE-3L: the coupled bond sums of a layer do not fit a thread block");
-    Shape s{};
-    s.cshift = cshift;
-    s.nTI = nTI;
-    s.threads = (groups * CC + 31) / 32 * 32;
-    s.slices = L.C / CC;
-    const size_t raw = 2 * (size_t) S3_NBS * (4 * (size_t) (plan_.lmax + 1) * CC + (size_t) L.nlmi * CC + CC) + plan_.nlm + L.nlmi + 8;    // the two staging buffers
-    s.smem_fwd = sizeof(float) * (raw + 8 * S3_BB + (size_t) S3_BB * plan_.nlm + S3_NBS * ((size_t) plan_.nlm * CC + (size_t) L.nlmi * CC) + (size_t) L.nfA * CC);
-    s.smem_bwd = sizeof(float) * (raw + 8 * S3_BB + 4 * (size_t) S3_BB * plan_.nlm +
-                                  S3_NBS * (3 * (size_t) plan_.nlm * CC + 2 * (size_t) L.nlmi * CC + plan_.nlm) + 8);
-    if (std::max(s.smem_fwd, s.smem_bwd) > 200 * 1024) throw Unsupported("GRACE-3L: the bond sums of a layer do not fit the shared memory");
-    return s;
+  auto bonds_reverse = [&](int k, const float *gA, int NC, int a0, int na) {
+    const Layer3Plan &L = Q.L[k];
+    const bool one = L.nlmi == 1;
+    const int nw = one ? 4 : std::min(S3_WARPS, (L.nlmi + S3_LIT - 1) / S3_LIT), nlm = plan_.nlm, nl = plan_.lmax + 1;
+    const size_t smem = sizeof(float) * (4 * (size_t) S3_BB * nlm + 8 * (size_t) S3_NBS * nl * 32 + 8 * S3_NBS + 32 * (size_t) L.nfA) +
+                        sizeof(S3Bond) * S3_BB + sizeof(double) * 6 * S3_NBS;
+    if (smem > 200 * 1024) throw Unsupported("GRACE-3L: the bond sums of a layer do not fit the shared memory");
+    const dim3 grid((L.C + 31) / 32, na);
+    auto go = [&](auto kernel) {
+      GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+      before_launch("spbf3_bwd_kernel");
+      kernel<<<grid, 32 * nw, smem, dev().stream>>>(bonds, spbf(k), sht, gA, NC, fv_.get(), vir_atom_.get(), a0);
+      after_launch("spbf3_bwd_kernel");
+    };
+    switch (plan_.lmax) {
+      case 1: one ? go(spbf3_bwd_kernel<1, 1>) : go(spbf3_bwd_kernel<1, S3_LIT>); break;
+      case 2: one ? go(spbf3_bwd_kernel<2, 1>) : go(spbf3_bwd_kernel<2, S3_LIT>); break;
+      case 3: one ? go(spbf3_bwd_kernel<3, 1>) : go(spbf3_bwd_kernel<3, S3_LIT>); break;
+      default: one ? go(spbf3_bwd_kernel<4, 1>) : go(spbf3_bwd_kernel<4, S3_LIT>); break;
+    }
   };
-  static bool attr_set = false;
-  if (!attr_set) {
-    GB_CUDA(cudaFuncSetAttribute(spbf3_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    GB_CUDA(cudaFuncSetAttribute(spbf3_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr_set = true;
-  }
   // Passes.  When the tensors of all three layers of all atoms fit the memory they are kept from the forward to the
   // reverse pass (arena k holds layer k).  Otherwise every layer runs in passes over atom chunks through one arena, and
   // the reverse pass of a layer evaluates the forward operations of a chunk again before it reverses them: the messages,
@@ -875,17 +783,6 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
     NC = std::max(4, NC / 4 * 4);
     for (int k = 1; k < 3; k++) S.arena[k].release();
   }
-  const bool simt_only = getenv("GRACE_B200_3L_MMA") == nullptr;    // read per evaluation
-  // GRACE_B200_3L_MMA=1: the forward bond sums as small matrix products on the tensor cores where the shape allows.  Same
-  // results; measured slower than the register-tile kernel so far (its operand staging, not the matrix instructions),
-  // so it is not the default
-  const size_t smem_mma = sizeof(float) * std::max<size_t>(2 * S3M_CH * S3M_CS + 3 + 8 * S3_BB + (size_t) S3_BB * plan_.nlm + 32 + 32,
-                                                            (size_t) S3M_CH * 32 * 33);
-  static bool mma_attr = false;
-  if (!simt_only && !mma_attr) {
-    GB_CUDA(cudaFuncSetAttribute(spbf3_fwd_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    mma_attr = true;
-  }
   // the arena of layer k bound for passes of NC atoms
   auto bind = [&](int k) {
     LayerEngine &E = S.E[k];
@@ -901,13 +798,9 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
   // forward operations of layer k for the atoms [a0, a0 + na); outputs: the message rows and the density sums
   auto forward = [&](int k, int a0, int na, bool outputs) {
     const Layer3Plan &L = Q.L[k];
-    const Shape sh = shape(L);
     LayerEngine &E = S.E[k];
     const std::vector<TensorDev> &T = E.tensors_host;
-    if (!simt_only && plan_.nlm <= 32 && L.nlmi <= 32 && L.C % S3M_CH == 0)
-      GB_LAUNCH(spbf3_fwd_mma_kernel, dim3(na, L.C / S3M_CH), 32 * S3M_CH, smem_mma, bonds, spbf(k), sht, T[L.tA].p, NC, a0);
-    else
-      GB_LAUNCH(spbf3_fwd_kernel, dim3(na, sh.slices), sh.threads, sh.smem_fwd, bonds, spbf(k), sht, T[L.tA].p, NC, sh.cshift, sh.nTI, a0);
+    bonds_forward(k, T[L.tA].p, NC, a0, na);
     run(E, L.dense.fwd, mu + a0, na, NC);
     if (!outputs) return;
     if (k < 2) {
@@ -919,7 +812,6 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
   // reverse operations of layer k for the atoms [a0, a0 + na), whose forward tensors are in the bound arena
   auto reverse = [&](int k, int a0, int na, float *base) {
     const Layer3Plan &L = Q.L[k];
-    const Shape sh = shape(L);
     LayerEngine &E = S.E[k];
     const std::vector<TensorDev> &T = E.tensors_host;
     if (L.dense.zero_grads)
@@ -930,8 +822,7 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
       GB_LAUNCH(eqnorm_bwd_kernel, na, 32 * EQ_WARPS, 0, e, T[L.tEQ].p, S.gmsg[k].get(), T[L.tGEQ].p, NC, a0);
     }
     run(E, L.dense.bwd, mu + a0, na, NC);
-    GB_LAUNCH(spbf3_bwd_kernel, dim3(na, sh.slices), sh.threads, sh.smem_bwd, bonds, spbf(k), sht, T[L.tGA].p, NC, fv_.get(), vir_atom_.get(),
-              sh.cshift, sh.nTI, a0);
+    bonds_reverse(k, T[L.tGA].p, NC, a0, na);
   };
   for (int k = 0; k < 2; k++) S.msg[k].ensure((size_t) n * Q.L[k].nfEQ * Q.L[k].cEQ);
   for (int k = 0; k < 3; k++) {

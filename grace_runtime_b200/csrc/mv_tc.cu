@@ -33,7 +33,7 @@ constexpr int NW = NTH / 32;
 constexpr int TMEM_COLS = 512;
 constexpr int MAX_TILES = 16;   // atom tiles a CTA holds accumulators for
 constexpr int MAX_TENSORS = 64;
-constexpr int MAX_ITEMS = 512, MAX_ROWS = 192;    // tables of an operation staged in shared memory
+constexpr int MAX_ITEMS = 512, MAX_ROWS = 256;    // tables of an operation staged in shared memory
 constexpr long long WAIT_CYCLES = 40000000LL;    // ~20 ms: far beyond any tile, far below a watchdog
 
 // byte offset of element (r, k) of a K-major operand tile with K columns (canonical layout, no swizzle)
