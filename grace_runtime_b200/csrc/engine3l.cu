@@ -28,17 +28,21 @@ struct Spbf3Dev {
   float *gmsg;               // [n][nlmi][C] its gradient, added to atomically (null: layer 1)
   const float *zproj;        // [n_elements][C]
   const float *l0mask;       // [nlmi]
-  const int *cg_off, *cgt_off;    // the couple by output function, and by (harmonic, message function) pair
-  const int2 *cg;            // (harmonic << 16 | message function, coefficient bits)
-  const int2 *cgt;           // (output function, coefficient bits)
+  // the couple as flat lists, one after the other for each round and warp (s3_list): cg in the order of the output
+  // functions, cgt in the order of the (harmonic, message function) pairs of the warp
+  const int2 *cg, *cgt;
+  const int *cg_off, *cgt_off;    // where the list of (round, warp) starts, [rounds warps + 1]
   int N, C, nl, nlm, nlmi, nfA, nel;
 };
 
 
 constexpr int S3_BB = 64;     // bonds whose harmonics and geometry are staged at once
-constexpr int S3_NBS = 8;     // bonds whose radial functions are evaluated together
-constexpr int S3_LIT = 5;     // message functions of a thread
-constexpr int S3_WARPS = 5;   // most warps of a CTA
+constexpr int S3_NBS = 4;     // bonds whose radial functions and messages travel together
+constexpr int S3_LIT = 7;     // message functions of a thread
+constexpr int S3_WARPS = 4;   // most warps of a CTA
+// warps of a CTA, and the message functions it holds at a time
+int s3_warps(int nlmi) { return nlmi == 1 ? 4 : std::min(S3_WARPS, (nlmi + S3_LIT - 1) / S3_LIT); }
+int s3_pitch(int nlmi) { return nlmi == 1 ? 1 : s3_warps(nlmi) * S3_LIT; }
 
 __device__ __forceinline__ void s3_cp16(void *dst_smem, const void *src)
 {
@@ -50,23 +54,23 @@ __device__ __forceinline__ void s3_cp_wait() { asm volatile("cp.async.wait_group
 // Geometry of a bond, worked out once per batch of bonds by one thread per bond (a chain of dependent global loads: record
 // -> element of the neighbour -> table of the pair) and kept in shared memory.
 struct __align__(16) S3Bond {
-  int j, muj;
   long long tab;    // offset of the bond's table row in floats, < 0: no table for this element pair, the bond is left out
+  long long row;    // offset of the neighbour's message row in floats
+  int muj;
   float t, r, rc;
-  int pad;
 };
 __device__ __forceinline__ S3Bond s3_bond(const BondsDev &b, const Spbf3Dev &L, const float4 &rec, int mui)
 {
   S3Bond o;
-  o.j = __float_as_int(rec.w);
-  o.muj = b.mu[o.j];
+  const int j = __float_as_int(rec.w);
+  o.muj = b.mu[j];
   o.r = sqrtf(rec.x * rec.x + rec.y * rec.y + rec.z * rec.z);
   o.rc = L.rc[mui * L.nel + o.muj];
   int k0;
   spline_locate(o.r / o.rc, L.N, k0, o.t);
   const int slot = L.pair_slot[mui * L.nel + o.muj];
   o.tab = slot < 0 ? -1 : (long long) slot * L.tab_stride + (long long) k0 * L.nl * L.C * 4;
-  o.pad = 0;
+  o.row = (long long) j * L.nlmi * L.C;
   return o;
 }
 
@@ -75,90 +79,172 @@ __device__ __forceinline__ S3Bond s3_bond(const BondsDev &b, const Spbf3Dev &L, 
 //     P[ly][li] = sum_j U[ly] I[li]         (forward),
 //     W[ly] = sum_li gP[ly][li] I[li],  dE/dmsg_j[li] = sum_ly gP[ly][li] U[ly]      (reverse, per bond),
 // 625 multiply-adds per bond and channel at lmax 4 (three times that in reverse).  A CTA works on one atom and 32 channels,
-// lane = channel; a warp owns 5 message functions and ALL harmonics of them, so that a thread keeps 25 x 5 sums (or their
-// gradient) in registers and one bond costs it 5 message loads, 5 radial values and the harmonics (16-byte broadcast reads)
-// for 125 multiply-adds (250 in reverse), where tiles of 5 x 5 over 25 warps needed 10 shared-memory reads for 25 and staged
-// U and I through shared memory.  The message rows go straight from global memory to the registers of the one warp that
-// needs them, a bond ahead.  Bound by instruction issue: about 190 (forward) and 450 (reverse) instructions per bond and
-// warp.  31,250 atoms, lmax 4, 64 channels, both message layers: see the table of measurements at spbf3_bwd_kernel.
+// lane = channel; a warp owns 7 message functions and ALL harmonics of them, so that a thread keeps 25 x 7 sums (or their
+// gradient) in registers and one bond costs it 7 messages, 5 radial values and the harmonics (16-byte broadcast reads) for
+// 175 multiply-adds (350 in reverse), where tiles of 5 x 5 over 25 warps needed 10 shared-memory reads for 25.  That fills
+// the register file with two warps per scheduler, balanced over the four of them; what the bonds need travels by asynchronous
+// copies a group of bonds ahead, and the number of instructions is what counts: no index arithmetic per bond, the couple as
+// flat lists read eight entries at a time, and in reverse pairs of harmonics through two-wide multiply-adds (forward they
+// gain nothing: the compiler copies the paired sums apart in every iteration).
 // A layer without messages has one function: the warps share the bonds instead (LIT = 1).
-
-// radial functions (and derivatives) of the bonds of a group: thread e of the CTA owns the values e, e + nth, ... of
-// [bond][l][channel]; the coefficients travel to its own piece of `raw` by asynchronous copies issued a group ahead
-__device__ __forceinline__ void s3_issue(const Spbf3Dev &L, const S3Bond *meta, int ns, int c0, float4 *raw, int tid, int nth)
-{
-  for (int e = tid; e < ns * L.nl * 32; e += nth) {
-    const int c = e & 31, sl = e >> 5, s = sl / L.nl, l = sl - s * L.nl;
-    const long long at = meta[s].tab;
-    if (at >= 0 && c0 + c < L.C) s3_cp16(raw + e, L.tab + at + 4 * ((long long) l * L.C + c0 + c));
-  }
-  s3_cp_commit();
-}
-template<bool GRAD>
-__device__ __forceinline__ void s3_radial(const Spbf3Dev &L, const S3Bond *meta, int ns, int c0, const float4 *raw, float *R, float *dR,
-                                          int tid, int nth)
-{
-  for (int e = tid; e < ns * L.nl * 32; e += nth) {
-    const int c = e & 31, s = (e >> 5) / L.nl;
-    float v = 0.0f, d = 0.0f;
-    if (meta[s].tab >= 0 && c0 + c < L.C) {
-      const float4 cf = raw[e];
-      const float t = meta[s].t;
-      v = cf.x + t * (cf.y + t * (cf.z + t * cf.w));
-      if (GRAD) d = (cf.y + t * (2.0f * cf.z + t * 3.0f * cf.w)) * (float) L.N;
-    }
-    R[e] = v;
-    if (GRAD) dR[e] = d;
-  }
-}
-
-// message functions li0 .. li0 + LIT of the neighbour of a bond, channel c
-template<int LIT>
-__device__ __forceinline__ void s3_message(const Spbf3Dev &L, const S3Bond &B, int li0, int c, bool in, unsigned masked, const float *mask,
-                                           float (&ic)[LIT])
-{
-#pragma unroll
-  for (int q = 0; q < LIT; q++)
-    ic[q] = L.msg && in && li0 + q < L.nlmi ? __ldg(L.msg + ((size_t) B.j * L.nlmi + li0 + q) * L.C + c) : 0.0f;
-  if (masked) {
-    const float z = in ? __ldg(L.zproj + (size_t) B.muj * L.C + c) : 0.0f;
-#pragma unroll
-    for (int q = 0; q < LIT; q++) ic[q] = fmaf(mask[q], z, ic[q]);
-  }
-}
+// 31,250 atoms, lmax 4, 64 channels, three layers (ms per evaluation, forward / reverse): tiles of 5 x 5 with staged operands
+// 84.6 / 260; 5 functions per warp, couple term by term 43.4 / 87.9; this form 26.3 / 72.2.
 
 template<int LMAX> struct S3 {
-  static constexpr int NLM = (LMAX + 1) * (LMAX + 1), NL = LMAX + 1, YLD = (NLM + 3) / 4 * 4;
+  static constexpr int NLM = (LMAX + 1) * (LMAX + 1), NL = LMAX + 1, NP = (NLM + 1) / 2;    // NP: pairs of harmonics
+  static constexpr int YLD = (NP + 1) / 2 * 4;                                             // floats of a bond's harmonics
+  __host__ __device__ static constexpr int l_of(int lm) { return lm < 1 ? 0 : lm < 4 ? 1 : lm < 9 ? 2 : lm < 16 ? 3 : 4; }
 };
 
-// A[f][a][c] = sum_q cg[q, f] P[q][c], q = ly nlmi + li
+// Radial functions (and derivatives) of the bonds of a group: a thread owns one channel of the functions l = warp, warp +
+// nw, ..; the coefficients travel to its own piece of `raw` by asynchronous copies issued a group ahead.  tabc: the table
+// from the thread's channel on.
+template<int NL>
+__device__ __forceinline__ void s3_issue(const float *tabc, int C, const S3Bond *meta, int ns, float4 *raw, int warp, int nw, int lane)
+{
+  for (int l = warp; l < NL; l += nw)
+#pragma unroll
+    for (int s = 0; s < S3_NBS; s++)
+      if (s < ns) s3_cp16(raw + (s * NL + l) * 32 + lane, tabc + max(meta[s].tab, 0LL) + 4 * l * C);
+  s3_cp_commit();
+}
+template<int NL, bool GRAD>
+__device__ __forceinline__ void s3_radial(float N, const S3Bond *meta, int ns, const float4 *raw, float *R, float *dR, int warp, int nw,
+                                          int lane)
+{
+  for (int l = warp; l < NL; l += nw)
+#pragma unroll
+    for (int s = 0; s < S3_NBS; s++) {
+      if (s >= ns) break;
+      const int e = (s * NL + l) * 32 + lane;
+      const float4 cf = raw[e];
+      const float t = meta[s].t;
+      const bool have = meta[s].tab >= 0;
+      R[e] = have ? cf.x + t * (cf.y + t * (cf.z + t * cf.w)) : 0.0f;
+      if (GRAD) dR[e] = have ? (cf.y + t * (2.0f * cf.z + t * 3.0f * cf.w)) * N : 0.0f;
+    }
+}
+
+// The warp's part of the message rows of a group of bonds: LIT functions (and the chemical weights, where the mask asks for
+// them) of 32 channels, by asynchronous copies into shared memory of the warp's own, a group ahead of their use.  Functions
+// beyond the model's repeat the last one and channels beyond the layer's are not copied: nothing reads what becomes of them.
+template<int LIT> struct S3Msg {
+  static constexpr int ROWS = LIT + 1, GROUP = S3_NBS * ROWS * 32;    // floats of a group
+  float mask[LIT];
+  bool masked;
+  __device__ void setup(const Spbf3Dev &L, int li0)
+  {
+    masked = false;
+#pragma unroll
+    for (int q = 0; q < LIT; q++) {
+      mask[q] = li0 + q < L.nlmi ? L.l0mask[li0 + q] : 0.0f;
+      masked = masked || mask[q] != 0.0f;
+    }
+  }
+  // chunk of 4 channels (lane & 7) of the rows lane >> 3, lane >> 3 + 4, ..
+  __device__ __forceinline__ void issue(const Spbf3Dev &L, const S3Bond *meta, int ns, int li0, int c0, float *buf, int lane) const
+  {
+    const int k = 4 * (lane & 7), r0 = lane >> 3;
+    if (c0 + k >= L.C) return;
+#pragma unroll
+    for (int s = 0; s < S3_NBS; s++) {
+      if (s >= ns) break;
+      const S3Bond &B = meta[s];
+      const float *m = L.msg + B.row + c0 + k;
+#pragma unroll
+      for (int r = 0; r < ROWS; r += 4) {
+        const int row = r + r0;
+        if (row < LIT && L.msg) s3_cp16(buf + (s * ROWS + row) * 32 + k, m + min(li0 + row, L.nlmi - 1) * L.C);
+        else if (row == LIT && masked) s3_cp16(buf + (s * ROWS + row) * 32 + k, L.zproj + B.muj * L.C + c0 + k);
+      }
+    }
+  }
+  __device__ __forceinline__ void get(const float *buf, int s, bool have, int lane, float (&ic)[LIT]) const
+  {
+#pragma unroll
+    for (int q = 0; q < LIT; q++) ic[q] = have ? buf[(s * ROWS + q) * 32 + lane] : 0.0f;
+    if (masked) {    // the same for the whole warp
+      const float z = buf[(s * ROWS + LIT) * 32 + lane];
+#pragma unroll
+      for (int q = 0; q < LIT; q++) ic[q] = fmaf(mask[q], z, ic[q]);
+    }
+  }
+};
+
+// A flat list of the couple: entries (source row | target + 1 << 16 where the target's sum ends, coefficient); target[32 lane]
+// of the sums go to `out`.  Eight entries at a time: their reads are in flight together, where a loop over the terms of one
+// target after the other is a chain of dependent reads (a third of the forward kernel's time).
+template<class Out>
+__device__ __forceinline__ void s3_list(const int2 *__restrict__ list, int k0, int k1, const float *src, int lane, Out &&out)
+{
+  float v = 0.0f;
+  for (int k = k0; k < k1; k += 8) {
+    int2 t[8];
+    float x[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) t[u] = __ldg(list + min(k + u, k1 - 1));
+#pragma unroll
+    for (int u = 0; u < 8; u++) x[u] = src[(t[u].x & 0xffff) * 32 + lane];
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      if (k + u >= k1) break;
+      v = fmaf(__int_as_float(t[u].y), x[u], v);
+      if (t[u].x >> 16) {
+        out((t[u].x >> 16) - 1, v);
+        v = 0.0f;
+      }
+    }
+  }
+}
+
+// pairs of fp32 values in a 64-bit register, for the two-wide multiply-add (as float2 the accumulators of a loop are copied
+// apart and together again)
+typedef unsigned long long s3_pair;
+__device__ __forceinline__ s3_pair s3_pack(float x, float y)
+{
+  s3_pair r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void s3_fma(s3_pair &d, s3_pair a, s3_pair b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
+__device__ __forceinline__ s3_pair s3_mul(s3_pair a, s3_pair b)
+{
+  s3_pair r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ s3_pair s3_dup(float v) { return s3_pack(v, v); }
+__device__ __forceinline__ float s3_sum(s3_pair p)
+{
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(p));
+  return x + y;
+}
+
+// A[f][a][c] = sum_q cg[q, f] P[q][c]
 template<int LMAX, int LIT>
 __global__ void __launch_bounds__(32 * S3_WARPS, 2) spbf3_fwd_kernel(BondsDev b, Spbf3Dev L, SHTable sht, float *__restrict__ A, int NA,
                                                                      int a0)
 {
   constexpr int NLM = S3<LMAX>::NLM, NL = S3<LMAX>::NL, YLD = S3<LMAX>::YLD;
   extern __shared__ __align__(16) float sm[];
-  float *Ps = sm;                                                  // [nlm nlmi][32], after the bond loop; below: during it
-  float4 *raw = reinterpret_cast<float4 *>(sm);                    // [NBS][nl][32]
+  float *Ps = sm;                                                  // [nlm][functions of a round][32], after the bond loop
+  float4 *raw = reinterpret_cast<float4 *>(sm);                    // during it: [NBS][nl][32]
   float *Rs = sm + 4 * S3_NBS * NL * 32;                           // [2][NBS][nl][32]
   float *Ys = Rs + 2 * S3_NBS * NL * 32;                           // [BB][YLD]
   S3Bond *meta = reinterpret_cast<S3Bond *>(Ys + S3_BB * YLD);     // [BB]
   const int nth = blockDim.x, nw = nth >> 5, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int ap = blockIdx.y, i = a0 + ap, c0 = blockIdx.x * 32, c = c0 + lane;
-  const bool in = c < L.C;
+  float *msg = reinterpret_cast<float *>(meta + S3_BB) + warp * 2 * S3Msg<LIT>::GROUP;    // [2] groups of the warp
+  const int ap = blockIdx.y, i = a0 + ap, c0 = blockIdx.x * 32, c = c0 + lane, C = L.C;
   const long long base = b.off[i];
   const int nb = b.cnt[i], mui = b.mu[i];
-  const int ntile = LIT == 1 ? 1 : (L.nlmi + LIT - 1) / LIT, nround = LIT == 1 ? 1 : (ntile + nw - 1) / nw;
-  float acc[NLM][LIT];
+  const int pitch = LIT == 1 ? 1 : nw * LIT, nround = (L.nlmi + pitch - 1) / pitch;
+  const float *tabc = L.tab + 4 * min(c, C - 1);
   for (int round = 0; round < nround; round++) {
-    const int li0 = LIT == 1 ? 0 : (round * nw + warp) * LIT;
-    float mask[LIT];
-    unsigned masked = 0;
-#pragma unroll
-    for (int q = 0; q < LIT; q++) {
-      mask[q] = li0 + q < L.nlmi ? L.l0mask[li0 + q] : 0.0f;
-      masked |= mask[q] != 0.0f;
-    }
+    const int li0 = LIT == 1 ? 0 : round * pitch + warp * LIT;
+    S3Msg<LIT> M;
+    M.setup(L, li0);
+    float acc[NLM][LIT];
 #pragma unroll
     for (int a = 0; a < NLM; a++)
 #pragma unroll
@@ -173,40 +259,39 @@ __global__ void __launch_bounds__(32 * S3_WARPS, 2) spbf3_fwd_kernel(BondsDev b,
         meta[e] = s3_bond(b, L, rec, mui);
       }
       __syncthreads();
-      s3_issue(L, meta, min(S3_NBS, nq), c0, raw, tid, nth);
-      float nxt[LIT];
-      if (LIT > 1) s3_message<LIT>(L, meta[0], li0, c, in, masked, mask, nxt);
+      M.issue(L, meta, min(S3_NBS, nq), li0, c0, msg, lane);
+      s3_issue<NL>(tabc, C, meta, min(S3_NBS, nq), raw, warp, nw, lane);
       for (int q = 0, k = 0; q < nq; q += S3_NBS, k ^= 1) {
         const int ns = min(S3_NBS, nq - q);
         float *R = Rs + k * S3_NBS * NL * 32;
+        const float *mg = msg + k * S3Msg<LIT>::GROUP;
         s3_cp_wait();
-        s3_radial<false>(L, meta + q, ns, c0, raw, R, nullptr, tid, nth);
-        if (q + S3_NBS < nq) s3_issue(L, meta + q + S3_NBS, min(S3_NBS, nq - q - S3_NBS), c0, raw, tid, nth);
+        s3_radial<NL, false>((float) L.N, meta + q, ns, raw, R, nullptr, warp, nw, lane);
         __syncthreads();    // R of this group is complete; the other half was last read before the barrier of the group before
+        if (q + S3_NBS < nq) {
+          const int nn = min(S3_NBS, nq - q - S3_NBS);
+          M.issue(L, meta + q + S3_NBS, nn, li0, c0, msg + (k ^ 1) * S3Msg<LIT>::GROUP, lane);
+          s3_issue<NL>(tabc, C, meta + q + S3_NBS, nn, raw, warp, nw, lane);
+        }
+#pragma unroll 1
         for (int s = LIT == 1 ? warp : 0; s < ns; s += LIT == 1 ? nw : 1) {
           float ic[LIT];
-          if (LIT == 1) s3_message<LIT>(L, meta[q + s], li0, c, in, masked, mask, ic);
-          else {
-#pragma unroll
-            for (int x = 0; x < LIT; x++) ic[x] = nxt[x];
-            if (q + s + 1 < nq) s3_message<LIT>(L, meta[q + s + 1], li0, c, in, masked, mask, nxt);
-          }
+          M.get(mg, s, L.msg != nullptr, lane, ic);
           const float4 *Y4 = reinterpret_cast<const float4 *>(Ys + (q + s) * YLD);
           float Rl[NL];
 #pragma unroll
           for (int l = 0; l < NL; l++) Rl[l] = R[(s * NL + l) * 32 + lane];
-          constexpr int L_OF[25] = {0, 1, 1, 1, 2, 2, 2, 2, 2, 3, 3, 3, 3, 3, 3, 3, 4, 4, 4, 4, 4, 4, 4, 4, 4};
 #pragma unroll
-          for (int y = 0; y < YLD / 4; y++) {
+          for (int y = 0; y < (NLM + 3) / 4; y++) {
             const float4 yv = Y4[y];
             const float ya[4] = {yv.x, yv.y, yv.z, yv.w};
 #pragma unroll
-            for (int x = 0; x < 4; x++) {
-              const int ly = 4 * y + x;
+            for (int h = 0; h < 4; h++) {
+              const int ly = 4 * y + h;
               if (ly >= NLM) continue;
-              const float u = ya[x] * Rl[L_OF[ly]];
+              const float u = ya[h] * Rl[S3<LMAX>::l_of(ly)];
 #pragma unroll
-              for (int z = 0; z < LIT; z++) acc[ly][z] = fmaf(u, ic[z], acc[ly][z]);
+              for (int x = 0; x < LIT; x++) acc[ly][x] = fmaf(u, ic[x], acc[ly][x]);
             }
           }
         }
@@ -215,70 +300,67 @@ __global__ void __launch_bounds__(32 * S3_WARPS, 2) spbf3_fwd_kernel(BondsDev b,
     // the couple: the sums of this round go to shared memory, and each function collects the pairs it is made of (a function
     // is added up by one thread per channel, across the rounds in global memory)
     __syncthreads();
-    const int pitch = LIT == 1 ? 1 : nw * LIT;
 #pragma unroll
     for (int a = 0; a < NLM; a++)
 #pragma unroll
       for (int q = 0; q < LIT; q++) Ps[(LIT == 1 ? warp * NLM + a : a * pitch + warp * LIT + q) * 32 + lane] = acc[a][q];
     __syncthreads();
-    for (int f = warp; f < L.nfA; f += nw) {
-      float v = 0.0f;
-      const int k1 = L.cg_off[f + 1];
-#pragma unroll 4
-      for (int k = L.cg_off[f]; k < k1; k++) {
-        const int2 t = __ldg(L.cg + k);    // (harmonic, message function), coefficient
-        const int ly = t.x >> 16, li = (t.x & 0xffff) - round * pitch;
-        if (LIT == 1) {
-          float p = 0.0f;
-          for (int w = 0; w < nw; w++) p += Ps[(w * NLM + ly) * 32 + lane];
-          v = fmaf(__int_as_float(t.y), p, v);
-        } else if (li >= 0 && li < pitch) {
-          v = fmaf(__int_as_float(t.y), Ps[(ly * pitch + li) * 32 + lane], v);
-        }
+    if (LIT == 1) {    // the warps' shares of the bonds
+      for (int a = warp; a < NLM; a += nw) {
+        float p = 0.0f;
+        for (int w = 0; w < nw; w++) p += Ps[(w * NLM + a) * 32 + lane];
+        Ps[a * 32 + lane] = p;
       }
-      float *o = A + ((size_t) f * NA + ap) * L.C + c;
-      if (in) *o = round > 0 ? *o + v : v;
+      __syncthreads();
     }
+    const int at = round * nw + warp;
+    s3_list(L.cg, L.cg_off[at], L.cg_off[at + 1], Ps, lane, [&](int f, float v) {
+      float *o = A + ((size_t) f * NA + ap) * C + c;
+      if (c < C) *o = round > 0 ? *o + v : v;
+    });
   }
 }
 
 // Reverse of the above from gA: bond forces and per-atom virial (added: the caller clears them before the first layer is
 // reversed), dE/dmsg of the neighbours.  Per bond a thread needs, beside W and dE/dmsg, its share of
 //     sum_ly,c W R_l dY_ly/du   and   dE/dx = sum_ly,c W Y_ly dR_l/dx,
-// both summed over the functions of its warp as they come (the radial values are taken out of the sums over m), so that
-// only four numbers per bond and warp are added over the lanes and none of W leaves the registers.
+// both summed over the functions of its warp as they come, so that only four numbers per bond and warp are added over the
+// lanes and none of W leaves the registers.
 template<int LMAX, int LIT>
 __global__ void __launch_bounds__(32 * S3_WARPS, 2) spbf3_bwd_kernel(BondsDev b, Spbf3Dev L, SHTable sht, const float *__restrict__ gA,
                                                                      int NA, float *__restrict__ fv, double *__restrict__ vir_atom,
                                                                      int a0)
 {
-  constexpr int NLM = S3<LMAX>::NLM, NL = S3<LMAX>::NL;
+  constexpr int NLM = S3<LMAX>::NLM, NL = S3<LMAX>::NL, NP = S3<LMAX>::NP;
   extern __shared__ __align__(16) float sm[];
-  float4 *G4 = reinterpret_cast<float4 *>(sm);                       // [BB][NLM] gradient of the harmonic, its value
-  float4 *raw = G4 + S3_BB * NLM;                                    // [NBS][nl][32]
+  float *gAs = sm;                                                   // [nfA][32]
+  float *gPs = gAs + 32 * L.nfA;                                     // [warps][half of nlm, LIT][32], before the bond loop; during it:
+  float4 *G4 = reinterpret_cast<float4 *>(gPs);                      // [BB][NP][2]: (x0 x1 y0 y1), (z0 z1 Y0 Y1) of a pair
+  float4 *raw = G4 + S3_BB * NP * 2;                                 // [NBS][nl][32]
   float *Rs = reinterpret_cast<float *>(raw + S3_NBS * NL * 32);     // [2][NBS][nl][32], then the derivatives
   float *dRs = Rs + 2 * S3_NBS * NL * 32;
   S3Bond *meta = reinterpret_cast<S3Bond *>(dRs + 2 * S3_NBS * NL * 32);    // [BB]
-  float *red = reinterpret_cast<float *>(meta + S3_BB);              // [2][NBS][4]
-  double *vir = reinterpret_cast<double *>(red + 2 * S3_NBS * 4);    // [NBS][6]
-  float *gAs = reinterpret_cast<float *>(vir + S3_NBS * 6);          // [nfA][32]
+  float *msg = reinterpret_cast<float *>(meta + S3_BB) + (threadIdx.x >> 5) * 2 * S3Msg<LIT>::GROUP;    // [2] groups of the warp
+  __shared__ float red[2][S3_NBS * 4];
+  __shared__ double vir[S3_NBS][6];
   const int nth = blockDim.x, nw = nth >> 5, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int ap = blockIdx.y, i = a0 + ap, c0 = blockIdx.x * 32, c = c0 + lane;
-  const bool in = c < L.C;
+  const int ap = blockIdx.y, i = a0 + ap, c0 = blockIdx.x * 32, c = c0 + lane, C = L.C;
+  const bool in = c < C;
   const long long base = b.off[i];
   const int nb = b.cnt[i], mui = b.mu[i];
-  const int ntile = LIT == 1 ? 1 : (L.nlmi + LIT - 1) / LIT, nround = LIT == 1 ? 1 : (ntile + nw - 1) / nw;
-  for (int f = warp; f < L.nfA; f += nw) gAs[f * 32 + lane] = in ? __ldg(gA + ((size_t) f * NA + ap) * L.C + c) : 0.0f;
-  for (int e = tid; e < S3_NBS * 6; e += nth) vir[e] = 0.0;
-  for (int e = tid; e < 2 * S3_NBS * 4; e += nth) red[e] = 0.0f;
-  __syncthreads();
-  // force and virial share of the bond `tid` of a group from the four sums of its warps
-  auto finish = [&](int at, int ns, float *r4) {
+  const int pitch = LIT == 1 ? 1 : nw * LIT, nround = (L.nlmi + pitch - 1) / pitch;
+  const float *tabc = L.tab + 4 * min(c, C - 1);
+  for (int f = warp; f < L.nfA; f += nw) gAs[f * 32 + lane] = in ? __ldg(gA + ((size_t) f * NA + ap) * C + c) : 0.0f;
+  if (tid < S3_NBS)
+    for (int k = 0; k < 6; k++) vir[tid][k] = 0.0;
+  for (int e = tid; e < 2 * S3_NBS * 4; e += nth) (&red[0][0])[e] = 0.0f;
+  // force and virial share of bond `tid` of the group at `at` of the batch q0, from the four sums of its warps
+  auto finish = [&](int q0, int at, int ns, float *r4) {
     if (tid >= ns) return;
     const S3Bond B = meta[at + tid];
     const float gx = r4[4 * tid], gy = r4[4 * tid + 1], gz = r4[4 * tid + 2], dedx = r4[4 * tid + 3];
     r4[4 * tid] = r4[4 * tid + 1] = r4[4 * tid + 2] = r4[4 * tid + 3] = 0.0f;
-    const long long slot = base + B.pad;
+    const long long slot = base + q0 + at + tid;
     const float4 rec = b.rec[slot];
     const float r = B.r, ir = 1.0f / r, ux = rec.x * ir, uy = rec.y * ir, uz = rec.z * ir;
     const float dEdr = dedx / B.rc, gr = gx * ux + gy * uy + gz * uz;
@@ -288,121 +370,129 @@ __global__ void __launch_bounds__(32 * S3_WARPS, 2) spbf3_bwd_kernel(BondsDev b,
     atomicAdd(o + 1, f1);
     atomicAdd(o + 2, f2);
     const double dx = -(double) ux * r, dy = -(double) uy * r, dz = -(double) uz * r;
-    double *v = vir + 6 * tid;
+    double *v = vir[tid];
     v[0] += dx * f0; v[1] += dy * f1; v[2] += dz * f2;
     v[3] += dx * f1; v[4] += dx * f2; v[5] += dy * f2;
   };
   for (int round = 0; round < nround; round++) {
-    const int li0 = LIT == 1 ? 0 : (round * nw + warp) * LIT;
-    float mask[LIT], gp[NLM][LIT];
-    unsigned masked = 0;
+    const int li0 = LIT == 1 ? 0 : round * pitch + warp * LIT;
+    S3Msg<LIT> M;
+    M.setup(L, li0);
+    // gP of the warp's functions from gA, through its own piece of shared memory
+    s3_pair gp[NP][LIT];
+    __syncthreads();    // gA is staged; what the round before left is no longer read
+    {
+      constexpr int HP = (NP + 1) / 2;    // half of the harmonics at a time
+      float *mine = gPs + warp * (2 * HP * LIT) * 32 + lane;
 #pragma unroll
-    for (int q = 0; q < LIT; q++) {
-      mask[q] = li0 + q < L.nlmi ? L.l0mask[li0 + q] : 0.0f;
-      masked |= mask[q] != 0.0f;
-    }
+      for (int half = 0; half < 2; half++) {
+        const int at = ((LIT == 1 ? 0 : round * nw + warp)) * 2 + half;
+        s3_list(L.cgt, L.cgt_off[at], L.cgt_off[at + 1], gAs, lane, [&](int p, float v) { mine[p * 32] = v; });
 #pragma unroll
-    for (int a = 0; a < NLM; a++)
+        for (int a = half * HP; a < (half ? NP : HP); a++)
 #pragma unroll
-      for (int q = 0; q < LIT; q++) {
-        float v = 0.0f;
-        if (li0 + q < L.nlmi) {
-          const int p = a * L.nlmi + li0 + q, k1 = __ldg(L.cgt_off + p + 1);
-          for (int k = __ldg(L.cgt_off + p); k < k1; k++) {
-            const int2 t = __ldg(L.cgt + k);    // function, coefficient
-            v = fmaf(__int_as_float(t.y), gAs[t.x * 32 + lane], v);
-          }
-        }
-        gp[a][q] = v;
+          for (int q = 0; q < LIT; q++)
+            gp[a][q] = s3_pack(mine[((2 * a - half * 2 * HP) * LIT + q) * 32], mine[((2 * a + 1 - half * 2 * HP) * LIT + q) * 32]);
       }
+    }
     for (int q0 = 0; q0 < nb; q0 += S3_BB) {
       const int nq = min(S3_BB, nb - q0);
       __syncthreads();    // what the batch before left is no longer read
       for (int e = tid; e < nq; e += nth) {
         const float4 rec = b.rec[base + q0 + e];
         const float ir = rsqrtf(rec.x * rec.x + rec.y * rec.y + rec.z * rec.z);
+        float *g = reinterpret_cast<float *>(G4 + e * NP * 2);
         sph_harm<LMAX, true>(sht, rec.x * ir, rec.y * ir, rec.z * ir, [&](int lm, float v, float gx, float gy, float gz) {
-          G4[e * NLM + lm] = make_float4(gx, gy, gz, v);
+          float *o = g + 8 * (lm >> 1) + (lm & 1);
+          o[0] = gx;
+          o[2] = gy;
+          o[4] = gz;
+          o[6] = v;
         });
-        S3Bond B = s3_bond(b, L, rec, mui);
-        B.pad = q0 + e;    // where its record is
-        meta[e] = B;
+        if (NLM & 1)
+          for (int k = 1; k < 8; k += 2) g[8 * (NP - 1) + k] = 0.0f;
+        meta[e] = s3_bond(b, L, rec, mui);
       }
       __syncthreads();
-      s3_issue(L, meta, min(S3_NBS, nq), c0, raw, tid, nth);
-      float nxt[LIT];
-      if (LIT > 1) s3_message<LIT>(L, meta[0], li0, c, in, masked, mask, nxt);
+      M.issue(L, meta, min(S3_NBS, nq), li0, c0, msg, lane);
+      s3_issue<NL>(tabc, C, meta, min(S3_NBS, nq), raw, warp, nw, lane);
       int k = 0;
       for (int q = 0; q < nq; q += S3_NBS, k ^= 1) {
         const int ns = min(S3_NBS, nq - q);
         float *R = Rs + k * S3_NBS * NL * 32, *dR = dRs + k * S3_NBS * NL * 32;
+        const float *mg = msg + k * S3Msg<LIT>::GROUP;
         s3_cp_wait();
-        s3_radial<true>(L, meta + q, ns, c0, raw, R, dR, tid, nth);
-        if (q + S3_NBS < nq) s3_issue(L, meta + q + S3_NBS, min(S3_NBS, nq - q - S3_NBS), c0, raw, tid, nth);
+        s3_radial<NL, true>((float) L.N, meta + q, ns, raw, R, dR, warp, nw, lane);
         __syncthreads();    // R of this group is complete, and so are the sums of the group before
-        if (q > 0) finish(q - S3_NBS, S3_NBS, red + (k ^ 1) * S3_NBS * 4);
+        if (q + S3_NBS < nq) {
+          const int nn = min(S3_NBS, nq - q - S3_NBS);
+          M.issue(L, meta + q + S3_NBS, nn, li0, c0, msg + (k ^ 1) * S3Msg<LIT>::GROUP, lane);
+          s3_issue<NL>(tabc, C, meta + q + S3_NBS, nn, raw, warp, nw, lane);
+        }
+        if (q > 0) finish(q0, q - S3_NBS, S3_NBS, red[k ^ 1]);
+#pragma unroll 1
         for (int s = LIT == 1 ? warp : 0; s < ns; s += LIT == 1 ? nw : 1) {
-          float ic[LIT], v[LIT];
-          const int j = meta[q + s].j;
-          if (LIT == 1) s3_message<LIT>(L, meta[q + s], li0, c, in, masked, mask, ic);
-          else {
-#pragma unroll
-            for (int x = 0; x < LIT; x++) ic[x] = nxt[x];
-            if (q + s + 1 < nq) s3_message<LIT>(L, meta[q + s + 1], li0, c, in, masked, mask, nxt);
-          }
-          const float4 *G = G4 + (q + s) * NLM;
-#pragma unroll
-          for (int x = 0; x < LIT; x++) v[x] = 0.0f;
-          float gx = 0.0f, gy = 0.0f, gz = 0.0f, dx = 0.0f;
+          float ic[LIT];
+          M.get(mg, s, L.msg != nullptr, lane, ic);
+          const ulonglong2 *G = reinterpret_cast<const ulonglong2 *>(G4 + (q + s) * NP * 2);
+          float Rl[NL], dRl[NL];
 #pragma unroll
           for (int l = 0; l < NL; l++) {
-            const float Rl = R[(s * NL + l) * 32 + lane], dRl = dR[(s * NL + l) * 32 + lane];
-            float lx = 0.0f, ly = 0.0f, lz = 0.0f, lr = 0.0f;
+            Rl[l] = R[(s * NL + l) * 32 + lane];
+            dRl[l] = dR[(s * NL + l) * 32 + lane];
+          }
+          s3_pair i2[LIT], v2[LIT], gx = s3_dup(0.0f), gy = gx, gz = gx, gr = gx;
 #pragma unroll
-            for (int m = l * l; m < (l + 1) * (l + 1); m++) {
-              const float4 g = G[m];
-              const float u = g.w * Rl;
-              float w = 0.0f;
+          for (int x = 0; x < LIT; x++) {
+            i2[x] = s3_dup(ic[x]);
+            v2[x] = s3_dup(0.0f);
+          }
 #pragma unroll
-              for (int x = 0; x < LIT; x++) {
-                w = fmaf(gp[m][x], ic[x], w);
-                v[x] = fmaf(gp[m][x], u, v[x]);
-              }
-              lx = fmaf(w, g.x, lx);
-              ly = fmaf(w, g.y, ly);
-              lz = fmaf(w, g.z, lz);
-              lr = fmaf(w, g.w, lr);
+          for (int p = 0; p < NP; p++) {
+            const int l0 = S3<LMAX>::l_of(2 * p), l1 = 2 * p + 1 < NLM ? S3<LMAX>::l_of(2 * p + 1) : l0;
+            const ulonglong2 g0 = G[2 * p], g1 = G[2 * p + 1];
+            const s3_pair Rp = s3_pack(Rl[l0], Rl[l1]), u = s3_mul(g1.y, Rp);
+            s3_pair w = s3_mul(gp[p][0], i2[0]);
+            s3_fma(v2[0], gp[p][0], u);
+#pragma unroll
+            for (int x = 1; x < LIT; x++) {
+              s3_fma(w, gp[p][x], i2[x]);
+              s3_fma(v2[x], gp[p][x], u);
             }
-            gx = fmaf(Rl, lx, gx);
-            gy = fmaf(Rl, ly, gy);
-            gz = fmaf(Rl, lz, gz);
-            dx = fmaf(dRl, lr, dx);
+            const s3_pair wr = s3_mul(w, Rp), wd = s3_mul(w, s3_pack(dRl[l0], dRl[l1]));
+            s3_fma(gx, wr, g0.x);
+            s3_fma(gy, wr, g0.y);
+            s3_fma(gz, wr, g1.x);
+            s3_fma(gr, wd, g1.y);
           }
           if (L.gmsg && in) {
+            float *o = L.gmsg + meta[q + s].row + c;
 #pragma unroll
             for (int x = 0; x < LIT; x++)
-              if (li0 + x < L.nlmi) atomicAdd(L.gmsg + ((size_t) j * L.nlmi + li0 + x) * L.C + c, v[x]);
+              if (li0 + x < L.nlmi) atomicAdd(o + (li0 + x) * C, s3_sum(v2[x]));
           }
           // the four sums over the lanes by one tree: two exchanges leave each lane one of them, three more add it up
           {
             const bool h = lane & 16, g = lane & 8;
-            const float a0_ = (h ? gz : gx) + __shfl_xor_sync(0xffffffffu, h ? gx : gz, 16);
-            const float a1_ = (h ? dx : gy) + __shfl_xor_sync(0xffffffffu, h ? gy : dx, 16);
-            float t = (g ? a1_ : a0_) + __shfl_xor_sync(0xffffffffu, g ? a0_ : a1_, 8);
+            const float sx = s3_sum(gx), sy = s3_sum(gy), sz = s3_sum(gz), sr = s3_sum(gr);
+            const float p0 = (h ? sz : sx) + __shfl_xor_sync(0xffffffffu, h ? sx : sz, 16);
+            const float p1 = (h ? sr : sy) + __shfl_xor_sync(0xffffffffu, h ? sy : sr, 16);
+            float t = (g ? p1 : p0) + __shfl_xor_sync(0xffffffffu, g ? p0 : p1, 8);
             t += __shfl_xor_sync(0xffffffffu, t, 4);
             t += __shfl_xor_sync(0xffffffffu, t, 2);
             t += __shfl_xor_sync(0xffffffffu, t, 1);
-            if ((lane & 7) == 0) atomicAdd(red + (k * S3_NBS + s) * 4 + (h ? 2 : 0) + (g ? 1 : 0), t);
+            if ((lane & 7) == 0) atomicAdd(&red[k][4 * s + (h ? 2 : 0) + (g ? 1 : 0)], t);
           }
         }
       }
       __syncthreads();
-      if (nq > 0) finish((nq - 1) / S3_NBS * S3_NBS, nq - (nq - 1) / S3_NBS * S3_NBS, red + (k ^ 1) * S3_NBS * 4);
+      const int last = (nq - 1) / S3_NBS * S3_NBS;
+      finish(q0, last, nq - last, red[k ^ 1]);
     }
   }
   if (tid < S3_NBS)
     for (int k = 0; k < 6; k++)
-      if (vir[6 * tid + k] != 0.0) atomicAdd(vir_atom + 6 * (size_t) i + k, vir[6 * tid + k]);
+      if (vir[tid][k] != 0.0) atomicAdd(vir_atom + 6 * (size_t) i + k, vir[tid][k]);
 }
 
 struct EqNormDev {
@@ -625,10 +715,43 @@ void Engine::setup_3l()
       std::memcpy(&u, &v, 4);
       return u;
     };
-    for (size_t t = 0; t < L.cg_p.size(); t++) cg.push_back(make_int2((L.cg_p[t] / L.nlmi) << 16 | (L.cg_p[t] % L.nlmi), bits(L.cg_v[t])));
-    for (size_t t = 0; t < L.cgt_f.size(); t++) cgt.push_back(make_int2(L.cgt_f[t], bits(L.cgt_v[t])));
-    S.cg_off[k].upload(L.cg_off);
-    S.cgt_off[k].upload(L.cgt_off);
+    const int nw = s3_warps(L.nlmi), pitch = s3_pitch(L.nlmi), nround = (L.nlmi + pitch - 1) / pitch, nlm = plan_.nlm;
+    const int lit = L.nlmi == 1 ? 1 : S3_LIT, hp = (nlm / 2 + nlm % 2 + 1) / 2 * 2;    // hp: harmonics of a half
+    if (nlm * pitch >= (1 << 16) || L.nfA >= (1 << 15)) throw Unsupported("GRACE-3L: the couple of a layer has too many functions");
+    // a target's last entry carries it; a target without entries gets one with coefficient 0
+    auto close = [&](std::vector<int2> &v, size_t from, int target) {
+      if (v.size() == from) v.push_back(make_int2(0, 0));
+      v.back().x |= (target + 1) << 16;
+    };
+    std::vector<int> cg_off, cgt_off;
+    for (int r = 0; r < nround; r++)
+      for (int w = 0; w < nw; w++) {
+        cg_off.push_back((int) cg.size());
+        for (int f = w; f < L.nfA; f += nw) {    // the output functions of the warp: sums of pairs
+          const size_t from = cg.size();
+          for (int t = L.cg_off[f]; t < L.cg_off[f + 1]; t++) {
+            const int ly = L.cg_p[t] / L.nlmi, li = L.cg_p[t] % L.nlmi;
+            if (li / pitch == r) cg.push_back(make_int2(ly * pitch + li % pitch, bits(L.cg_v[t])));
+          }
+          if (r == 0 || cg.size() > from) close(cg, from, f);
+        }
+        if (lit == 1 && w > 0) continue;
+        for (int half = 0; half < 2; half++) {    // the pairs of the warp: sums of the functions they feed
+          cgt_off.push_back((int) cgt.size());
+          for (int p = 0; p < hp * lit; p++) {
+            const int ly = half * hp + p / lit, li = (lit == 1 ? 0 : r * pitch + w * lit) + p % lit;
+            const size_t from = cgt.size();
+            if (ly < nlm && li < L.nlmi)
+              for (int t = L.cgt_off[ly * L.nlmi + li]; t < L.cgt_off[ly * L.nlmi + li + 1]; t++)
+                cgt.push_back(make_int2(L.cgt_f[t], bits(L.cgt_v[t])));
+            close(cgt, from, p);
+          }
+        }
+      }
+    cg_off.push_back((int) cg.size());
+    cgt_off.push_back((int) cgt.size());
+    S.cg_off[k].upload(cg_off);
+    S.cgt_off[k].upload(cgt_off);
     S.cg[k].upload(cg);
     S.cgt[k].upload(cgt);
     if (k < 2) {
@@ -718,8 +841,9 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
   auto bonds_forward = [&](int k, float *A, int NC, int a0, int na) {
     const Layer3Plan &L = Q.L[k];
     const bool one = L.nlmi == 1;
-    const int nw = one ? 4 : std::min(S3_WARPS, (L.nlmi + S3_LIT - 1) / S3_LIT), nlm = plan_.nlm, nl = plan_.lmax + 1;
-    const size_t stage = sizeof(float) * (6 * (size_t) S3_NBS * nl * 32 + (size_t) S3_BB * ((nlm + 3) / 4 * 4)) + sizeof(S3Bond) * S3_BB;
+    const int nw = s3_warps(L.nlmi), nlm = plan_.nlm, nl = plan_.lmax + 1, np = (nlm + 1) / 2;
+    const size_t group = (size_t) nw * 2 * S3_NBS * ((one ? 1 : S3_LIT) + 1) * 32;    // floats of the message buffers
+    const size_t stage = sizeof(float) * (6 * (size_t) S3_NBS * nl * 32 + (size_t) S3_BB * ((np + 1) / 2 * 4) + group) + sizeof(S3Bond) * S3_BB;
     const size_t sums = sizeof(float) * 32 * (size_t) nlm * nw * (one ? 1 : S3_LIT), smem = std::max(stage, sums);
     const dim3 grid((L.C + 31) / 32, na);
     auto go = [&](auto kernel) {
@@ -738,9 +862,11 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
   auto bonds_reverse = [&](int k, const float *gA, int NC, int a0, int na) {
     const Layer3Plan &L = Q.L[k];
     const bool one = L.nlmi == 1;
-    const int nw = one ? 4 : std::min(S3_WARPS, (L.nlmi + S3_LIT - 1) / S3_LIT), nlm = plan_.nlm, nl = plan_.lmax + 1;
-    const size_t smem = sizeof(float) * (4 * (size_t) S3_BB * nlm + 8 * (size_t) S3_NBS * nl * 32 + 8 * S3_NBS + 32 * (size_t) L.nfA) +
-                        sizeof(S3Bond) * S3_BB + sizeof(double) * 6 * S3_NBS;
+    const int nw = s3_warps(L.nlmi), nlm = plan_.nlm, nl = plan_.lmax + 1, np = (nlm + 1) / 2;
+    const size_t group = (size_t) nw * 2 * S3_NBS * ((one ? 1 : S3_LIT) + 1) * 32;
+    const size_t stage = sizeof(float) * (8 * (size_t) S3_BB * np + 8 * (size_t) S3_NBS * nl * 32 + group) + sizeof(S3Bond) * S3_BB;
+    const size_t grads = sizeof(float) * 32 * (size_t) ((np + 1) / 2 * 2) * nw * (one ? 1 : S3_LIT);
+    const size_t smem = sizeof(float) * 32 * (size_t) L.nfA + std::max(stage, grads);
     if (smem > 200 * 1024) throw Unsupported("GRACE-3L: the bond sums of a layer do not fit the shared memory");
     const dim3 grid((L.C + 31) / 32, na);
     auto go = [&](auto kernel) {
