@@ -670,12 +670,12 @@ def run_ours(args, rank, world, local_rank):
             gbs = by_atom * n_own / (v[1] / args.steps * 1e-3) / 1e9
             hbm_kernels[name] = {"achieved_GBs": gbs, "frac_of_measured_hbm": gbs / hbm_peak, "ms_per_step": v[1] / args.steps,
                                  "algorithmic_bytes_per_atom": by_atom}
-    # the per-element operations run as two kernels (reduces: a thread per atom; their adjoints: a lane per output float4)
-    elem_ms = sum(v[1] for k, v in kern if k.strip("()").split("<")[0] in ("mv_elem_tile_kernel", "mv_elem_wide_kernel"))
+    # the operations with per-element weights: the same kernel on atoms grouped by element
+    elem_ms = sum(v[1] for k, v in kern if k.strip("()").split("<")[0] == "mv_tc_element_kernel")
     if elem_ms > 0:
         by_atom = model.dense_stats["elementwise"][1]
         gbs = by_atom * n_own / (elem_ms / args.steps * 1e-3) / 1e9
-        hbm_kernels["mv_elem_tile_kernel + mv_elem_wide_kernel"] = {
+        hbm_kernels["mv_tc_element_kernel"] = {
             "achieved_GBs": gbs, "frac_of_measured_hbm": gbs / hbm_peak, "ms_per_step": elem_ms / args.steps,
             "algorithmic_bytes_per_atom": by_atom}
 

@@ -70,304 +70,9 @@ __global__ void __launch_bounds__(128) mv_kernel(MVDev op, const TensorDev *__re
   }
 }
 
-// Per-element weights (reduces over the central atom's element and their adjoints) for a tile of 128 atoms, one thread
-// per atom with all NQ x 4 output channels of a row in registers.  The atoms of the tile are taken in order of their
-// element, so the lanes of a warp mostly read the same weights (one broadcast shared-memory read serves them).  A CTA
-// walks the (row, item) pairs of its rows in groups of G items; the weight matrices of a group, for the elements
-// present in the tile, are staged in shared memory together - a weight is fetched from global memory once per tile and
-// element - through asynchronous copies into the half of a double buffer that the group before is not reading: the
-// fetch of a group runs under the arithmetic of the previous one and a group costs one barrier.  Same summation order
-// as mv_kernel.
-constexpr int ELEM_MAXS = 4;    // elements staged at a time (tiles with more walk the items once more per group of elements)
-constexpr int ELEM_GROUP = 4;   // most items whose weights are staged together
-constexpr int ELEM_TA = 128;
-
-__device__ __forceinline__ void cp_async16(void *smem_dst, const void *gmem_src)
-{
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned) __cvta_generic_to_shared(smem_dst)), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
-template<int NQ>
-__global__ void __launch_bounds__(ELEM_TA) mv_elem_tile_kernel(MVDev op, const TensorDev *__restrict__ T,
-                                                               const int *__restrict__ mu, int NA, int na, int n_in_max,
-                                                               int rows_per_cta, int G)
-{
-  extern __shared__ __align__(16) float wsm[];    // [2][G][ELEM_MAXS][n_in_max][NQ * 4]
-  __shared__ int s_slot[ELEM_TA], s_el[ELEM_TA], s_mu[ELEM_TA], s_order[ELEM_TA], s_cnt[ELEM_TA + 1], s_nsp;
-  const int a0 = blockIdx.x * ELEM_TA, nta = min(ELEM_TA, na - a0), t = threadIdx.x;
-  const int row_lo = blockIdx.y * rows_per_cta, row_hi = min(op.nrows, row_lo + rows_per_cta);
-  if (t < nta) s_mu[t] = mu[a0 + t];
-  __syncthreads();
-  if (t == 0) {    // distinct elements of the tile in order of first appearance, and the atoms grouped by them
-    int ns = 0;
-    for (int a = 0; a < nta; a++) {
-      const int e = s_mu[a];
-      int s = 0;
-      while (s < ns && s_el[s] != e) s++;
-      if (s == ns) { s_el[ns] = e; s_cnt[ns++] = 0; }
-      s_slot[a] = s;
-      s_cnt[s]++;
-    }
-    int at = 0;
-    for (int s = 0; s < ns; s++) { const int c = s_cnt[s]; s_cnt[s] = at; at += c; }
-    for (int a = 0; a < nta; a++) s_order[s_cnt[s_slot[a]]++] = a;
-    s_nsp = ns;
-  }
-  __syncthreads();
-  const bool active = t < nta;
-  const int p = active ? s_order[t] : 0;    // this thread's atom of the tile
-  const int nsp = s_nsp, slot = active ? s_slot[p] : -1;
-  const int i_lo = op.item_off[row_lo], i_hi = op.item_off[row_hi];
-  const int wstride = n_in_max * NQ;                      // float4 per (item of the group, element)
-  const int bstride = G * ELEM_MAXS * wstride;            // float4 per buffer
-  float4 *const w4 = reinterpret_cast<float4 *>(wsm);
-  const TensorDev dst = T[op.dst];
-  for (int s0 = 0; s0 < nsp; s0 += ELEM_MAXS) {
-    const int ng = min(ELEM_MAXS, nsp - s0);
-    const bool mine = slot >= s0 && slot < s0 + ng;
-    int row = row_lo;
-    float4 acc[NQ];
-#pragma unroll
-    for (int k = 0; k < NQ; k++) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto flush = [&]() {    // the sums of `row` are complete
-      if (mine) {
-        float *o = dst.p + ((size_t) op.row_out[row] * NA + a0 + p) * dst.C;
-        if ((dst.C & 3) == 0 && op.n_out == 4 * NQ) {
-#pragma unroll
-          for (int k = 0; k < NQ; k++) {
-            float4 v = acc[k];
-            if (op.accumulate) {
-              const float4 old = reinterpret_cast<const float4 *>(o)[k];
-              v.x += old.x; v.y += old.y; v.z += old.z; v.w += old.w;
-            }
-            reinterpret_cast<float4 *>(o)[k] = v;
-          }
-        } else {
-#pragma unroll
-          for (int k = 0; k < NQ; k++) {
-            const float v[4] = {acc[k].x, acc[k].y, acc[k].z, acc[k].w};
-            for (int q = 0; q < 4; q++)
-              if (4 * k + q < op.n_out) o[4 * k + q] = op.accumulate ? o[4 * k + q] + v[q] : v[q];
-          }
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < NQ; k++) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-      row++;
-    };
-    // asynchronous copies of the weights of the items it0 .. it0 + G of the elements s0 .. s0 + ng into buffer `buf`
-    auto stage = [&](int it0, int buf) {
-      const int nit = min(G, i_hi - it0);
-      for (int g = 0; g < nit; g++) {
-        const MVItem item = op.items[it0 + g];
-        const int per = item.n_in * NQ;
-        for (int q = t; q < ng * per; q += ELEM_TA) {
-          const int s = q / per, r = q - s * per;
-          cp_async16(w4 + (size_t) buf * bstride + (size_t) (g * ELEM_MAXS + s) * wstride + r,
-                     reinterpret_cast<const float4 *>(op.W + (size_t) s_el[s0 + s] * op.ty_stride + item.mat) + r);
-        }
-      }
-      cp_async_commit();
-    };
-    __syncthreads();    // the buffers of the previous group of elements are no longer read
-    if (i_lo < i_hi) stage(i_lo, 0);
-    int buf = 0;
-    for (int it0 = i_lo; it0 < i_hi; it0 += G, buf ^= 1) {
-      const int nit = min(G, i_hi - it0);
-      cp_async_wait_all();
-      __syncthreads();    // this group's weights are in place; the other buffer's readers are done
-      if (it0 + G < i_hi) stage(it0 + G, buf ^ 1);
-      for (int g = 0; g < nit; g++) {
-        while (it0 + g >= op.item_off[row + 1]) flush();
-        if (!mine) continue;
-        const MVItem item = op.items[it0 + g];
-        const TensorDev src = T[item.src];
-        const float *x = src.p + ((size_t) item.irow * NA + a0 + p) * src.C;
-        const float4 *w = w4 + (size_t) buf * bstride + (size_t) (g * ELEM_MAXS + slot - s0) * wstride;
-        float4 part[NQ];
-#pragma unroll
-        for (int k = 0; k < NQ; k++) part[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        auto one = [&](float xv, int n) {
-#pragma unroll
-          for (int k = 0; k < NQ; k++) {
-            const float4 wv = w[(size_t) n * NQ + k];
-            part[k].x = fmaf(xv, wv.x, part[k].x); part[k].y = fmaf(xv, wv.y, part[k].y);
-            part[k].z = fmaf(xv, wv.z, part[k].z); part[k].w = fmaf(xv, wv.w, part[k].w);
-          }
-        };
-        if (((src.C | item.n_in) & 3) == 0) {    // 16-byte activation loads, eight of them in flight
-          for (int n0 = 0; n0 < item.n_in; n0 += 32) {
-            float4 xv[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++)
-              xv[j] = n0 + 4 * j < item.n_in ? __ldg(reinterpret_cast<const float4 *>(x + n0) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-              if (n0 + 4 * j < item.n_in) {
-                one(xv[j].x, n0 + 4 * j); one(xv[j].y, n0 + 4 * j + 1); one(xv[j].z, n0 + 4 * j + 2); one(xv[j].w, n0 + 4 * j + 3);
-              }
-            }
-          }
-        } else {
-          for (int n = 0; n < item.n_in; n++) one(__ldg(x + n), n);
-        }
-#pragma unroll
-        for (int k = 0; k < NQ; k++) {
-          acc[k].x = fmaf(item.scale, part[k].x, acc[k].x); acc[k].y = fmaf(item.scale, part[k].y, acc[k].y);
-          acc[k].z = fmaf(item.scale, part[k].z, acc[k].z); acc[k].w = fmaf(item.scale, part[k].w, acc[k].w);
-        }
-      }
-    }
-    while (row < row_hi) flush();    // the last row, and rows without items
-  }
-}
-
-template<int NQ> void launch_elem(const MVDev &op, const TensorDev *tensors, const int *mu, int NA, int na)
-{
-  // items per group: both halves of the double buffer within ~56 KB, so that several CTAs share an SM
-  const size_t per_item = (size_t) ELEM_MAXS * op.unit_nmax * op.ldw * sizeof(float);
-  int G = ELEM_GROUP;
-  while (G > 1 && 2 * G * per_item > 56 * 1024) G--;
-  const size_t smem = 2 * G * per_item;
-  static size_t attr = 32 * 1024;    // static shared memory counts against the 48 KB a kernel gets without the attribute
-  if (smem > attr) {
-    GB_CUDA(cudaFuncSetAttribute(mv_elem_tile_kernel<NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr = 200 * 1024;
-  }
-  // rows of a tile go to one CTA unless the tiles alone cannot fill the GPU
-  const int tiles = (na + ELEM_TA - 1) / ELEM_TA, want = 16 * dev().sm_count;
-  const int gy = std::max(1, std::min(op.nrows, (want + tiles - 1) / tiles));
-  const int rows_per_cta = (op.nrows + gy - 1) / gy;
-  GB_LAUNCH((mv_elem_tile_kernel<NQ>), dim3(tiles, (op.nrows + rows_per_cta - 1) / rows_per_cta), ELEM_TA, smem, op, tensors, mu,
-            NA, na, op.unit_nmax, rows_per_cta, G);
-}
-
-// Per-element weights with wide outputs (the adjoints of the reduces: 9 - 17 inputs, 32 or 64 outputs per row): LPA =
-// n_out / 4 lanes per atom, each with one float4 of the output row, so that a row of an atom is written (and, when the
-// operation accumulates, read) as whole 128-byte lines; 32 / LPA atoms per warp, 8 warps per CTA, tiles of 128 atoms.
-// The weights of a group of output rows, for the elements present in the tile, are staged in shared memory; the inputs
-// of an atom are broadcast loads shared by its lanes.  Same summation order as mv_kernel.
-template<int LPA>
-__global__ void __launch_bounds__(256) mv_elem_wide_kernel(MVDev op, const TensorDev *__restrict__ T,
-                                                           const int *__restrict__ mu, int NA, int na, int n_in_max,
-                                                           int rows_per_cta, int G)
-{
-  constexpr int APW = 32 / LPA, APP = 8 * APW;    // atoms per warp and per pass of the CTA
-  extern __shared__ __align__(16) float wsm[];    // [G][ELEM_MAXS][n_in_max][LPA * 4]
-  __shared__ int s_slot[ELEM_TA], s_el[ELEM_TA], s_mu[ELEM_TA], s_nsp;
-  const int a0 = blockIdx.x * ELEM_TA, nta = min(ELEM_TA, na - a0), t = threadIdx.x;
-  const int row_lo = blockIdx.y * rows_per_cta, row_hi = min(op.nrows, row_lo + rows_per_cta);
-  if (t < nta) s_mu[t] = mu[a0 + t];
-  __syncthreads();
-  if (t == 0) {    // distinct elements of the tile in order of first appearance
-    int ns = 0;
-    for (int a = 0; a < nta; a++) {
-      const int e = s_mu[a];
-      int s = 0;
-      while (s < ns && s_el[s] != e) s++;
-      if (s == ns) s_el[ns++] = e;
-      s_slot[a] = s;
-    }
-    s_nsp = ns;
-  }
-  __syncthreads();
-  const int lane = t & 31, warp = t >> 5, kq = lane % LPA, asub = lane / LPA;
-  const int nsp = s_nsp, wstride = n_in_max * LPA;    // float4 per (item of the group, element)
-  float4 *const w4 = reinterpret_cast<float4 *>(wsm);
-  const TensorDev dst = T[op.dst];
-  for (int s0 = 0; s0 < nsp; s0 += ELEM_MAXS) {
-    const int ng = min(ELEM_MAXS, nsp - s0);
-    for (int r0 = row_lo; r0 < row_hi;) {
-      const int i_first = op.item_off[r0];
-      int r1 = r0 + 1;    // rows of the group: at most G items (a single row never has more: checked by the launcher)
-      while (r1 < row_hi && op.item_off[r1 + 1] - i_first <= G) r1++;
-      const int nit = op.item_off[r1] - i_first;
-      __syncthreads();    // the weights of the previous group are no longer read
-      for (int g = 0; g < nit; g++) {
-        const MVItem item = op.items[i_first + g];
-        const int per = item.n_in * LPA;
-        for (int q = t; q < ng * per; q += 256) {
-          const int s = q / per, r = q - s * per;
-          w4[(size_t) (g * ELEM_MAXS + s) * wstride + r] =
-              __ldg(reinterpret_cast<const float4 *>(op.W + (size_t) s_el[s0 + s] * op.ty_stride + item.mat) + r);
-        }
-      }
-      __syncthreads();
-      for (int ab = 0; ab < nta; ab += APP) {
-        const int ai = ab + warp * APW + asub;
-        if (ai >= nta) continue;
-        const int slot = s_slot[ai];
-        if (slot < s0 || slot >= s0 + ng) continue;
-        for (int row = r0; row < r1; row++) {
-          float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-          for (int it = op.item_off[row]; it < op.item_off[row + 1]; it++) {
-            const MVItem item = op.items[it];
-            const TensorDev src = T[item.src];
-            const float *x = src.p + ((size_t) item.irow * NA + a0 + ai) * src.C;
-            const float4 *w = w4 + (size_t) ((it - i_first) * ELEM_MAXS + slot - s0) * wstride + kq;
-            float4 part = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int n = 0; n < item.n_in; n++) {
-              const float xv = __ldg(x + n);
-              const float4 wv = w[(size_t) n * LPA];
-              part.x = fmaf(xv, wv.x, part.x); part.y = fmaf(xv, wv.y, part.y);
-              part.z = fmaf(xv, wv.z, part.z); part.w = fmaf(xv, wv.w, part.w);
-            }
-            acc.x = fmaf(item.scale, part.x, acc.x); acc.y = fmaf(item.scale, part.y, acc.y);
-            acc.z = fmaf(item.scale, part.z, acc.z); acc.w = fmaf(item.scale, part.w, acc.w);
-          }
-          float4 *o = reinterpret_cast<float4 *>(dst.p + ((size_t) op.row_out[row] * NA + a0 + ai) * dst.C) + kq;
-          if (op.accumulate) {
-            const float4 old = *o;
-            acc.x += old.x; acc.y += old.y; acc.z += old.z; acc.w += old.w;
-          }
-          *o = acc;
-        }
-      }
-      r0 = r1;
-    }
-  }
-}
-
-template<int LPA> bool launch_elem_wide(const MVDev &op, const TensorDev *tensors, const int *mu, int NA, int na)
-{
-  const size_t per_item = (size_t) ELEM_MAXS * op.unit_nmax * op.ldw * sizeof(float);
-  const int G = (int) std::min<size_t>(16, (40 * 1024) / per_item);
-  if (G < 1 || op.max_row_items > G) return false;
-  const size_t smem = G * per_item;
-  const int tiles = (na + ELEM_TA - 1) / ELEM_TA, want = 8 * dev().sm_count;
-  const int gy = std::max(1, std::min(op.nrows, (want + tiles - 1) / tiles));
-  const int rows_per_cta = (op.nrows + gy - 1) / gy;
-  GB_LAUNCH((mv_elem_wide_kernel<LPA>), dim3(tiles, (op.nrows + rows_per_cta - 1) / rows_per_cta), 256, smem, op, tensors, mu, NA,
-            na, op.unit_nmax, rows_per_cta, G);
-  return true;
-}
-
 void launch_mv(const MVDev &op, const TensorDev *tensors, const int *mu, int NA, int na)
 {
   if (op.nrows == 0 || na == 0) return;
-  // wide per-element operations (adjoints of the reduces): channel-parallel form with whole-line stores
-  static const bool nowide = getenv("GRACE_B200_ELEM_NOWIDE") != nullptr;
-  if (!nowide && op.elem && op.ldw == op.n_out && op.dst_C == op.n_out && (op.ty_stride & 3) == 0 && op.unit_nmax > 0 &&
-      op.unit_nmax <= 20) {
-    if (op.n_out == 32 && launch_elem_wide<8>(op, tensors, mu, NA, na)) return;
-    if (op.n_out == 64 && launch_elem_wide<16>(op, tensors, mu, NA, na)) return;
-  }
-  if (op.elem && (op.ldw & 3) == 0 && (op.ty_stride & 3) == 0 && op.unit_nmax > 0 &&
-      (size_t) 2 * ELEM_MAXS * op.unit_nmax * op.ldw * sizeof(float) <= 192 * 1024) {
-    switch (op.ldw >> 2) {
-      case 1: launch_elem<1>(op, tensors, mu, NA, na); return;
-      case 2: launch_elem<2>(op, tensors, mu, NA, na); return;
-      case 3: launch_elem<3>(op, tensors, mu, NA, na); return;
-      case 4: launch_elem<4>(op, tensors, mu, NA, na); return;
-      case 5: launch_elem<5>(op, tensors, mu, NA, na); return;
-      case 8: launch_elem<8>(op, tensors, mu, NA, na); return;
-      case 12: launch_elem<12>(op, tensors, mu, NA, na); return;
-      case 16: launch_elem<16>(op, tensors, mu, NA, na); return;
-      default: break;    // other widths: the per-atom kernel below
-    }
-  }
   int KP = 8;
   while (KP < op.n_out) KP *= 2;
   if (KP > 128) throw Unsupported("dense network: more than 128 channels are not supported");
@@ -408,11 +113,14 @@ __global__ void __launch_bounds__(256) prod_kernel(ProdDev op, const TensorDev *
 // memory once (coalesced, TA x C contiguous floats per function) however many terms read it, and the term loop runs on
 // shared memory.  srcB == srcA or srcB < 0: one staged tensor.
 __global__ void __launch_bounds__(256) prod_tile_kernel(ProdDev op, const TensorDev *__restrict__ T, int NA, int na, int TA,
-                                                        int nfA, int nfB, int C, int nterms)
+                                                        int nfA, int nfB, int C)
 {
   extern __shared__ __align__(16) float psm[];
   const int C4 = C >> 2, TAC4 = TA * C4, t = threadIdx.x;
   const int a0 = blockIdx.x * TA, nta = min(TA, na - a0);
+  const int per = (op.nrows + gridDim.y - 1) / gridDim.y, row_lo = per * blockIdx.y, row_hi = min(op.nrows, row_lo + per);
+  if (row_lo >= row_hi) return;
+  const int term0 = op.term_off[row_lo], nterms = op.term_off[row_hi] - term0;
   float4 *sA = reinterpret_cast<float4 *>(psm);
   float4 *sB = sA + (size_t) nfA * TAC4;
   int4 *sT = reinterpret_cast<int4 *>(sB + (size_t) nfB * TAC4);    // per term: row offsets of both operands, coefficient
@@ -440,7 +148,7 @@ __global__ void __launch_bounds__(256) prod_tile_kernel(ProdDev op, const Tensor
     stage(T[op.srcA].p, sA, nfA);
     if (two) stage(T[op.srcB].p, sB, nfB);
     for (int idx = t; idx < nterms; idx += 256) {
-      const ProdTerm tm = op.terms[idx];
+      const ProdTerm tm = op.terms[term0 + idx];
       sT[idx] = make_int4(tm.a * TAC4, tm.b * TAC4, __float_as_int(tm.coef), 0);
     }
   }
@@ -452,8 +160,8 @@ __global__ void __launch_bounds__(256) prod_tile_kernel(ProdDev op, const Tensor
   // broadcast 16-byte read) serves two positions; the products are packed two-wide FMAs (the same roundings as
   // fmaf(coef * a, b, acc) per channel)
   auto f2 = [](float x, float y) { return make_float2(x, y); };
-  for (int row = warp; row < op.nrows; row += 8) {
-    const int t0 = op.term_off[row], t1 = op.term_off[row + 1];
+  for (int row = row_lo + warp; row < row_hi; row += 8) {
+    const int t0 = op.term_off[row] - term0, t1 = op.term_off[row + 1] - term0;
     const bool add = op.accumulate && !(op.row_first && op.row_first[row]);
     float4 *orow = reinterpret_cast<float4 *>(D + ((size_t) op.row_out[row] * NA + a0) * C);
     for (int r = lane; r < nvalid; r += 64) {
@@ -513,7 +221,11 @@ void launch_prod(const ProdDev &op, const TensorDev *tensors, int NA, int na, in
     {    // a warp walks a row 64 float4 at a time: tiles whose rows are a multiple of that leave no lane idle
       const int unit = std::max(1, 64 / (C >> 2));
       if (TA > unit) TA = TA / unit * unit;
+      while (TA >= 2 * unit && (na + TA - 1) / TA < dev().sm_count) TA = TA / 2 / unit * unit;    // few atoms: more tiles
     }
+    // and where the tiles alone leave the GPU idle, the rows of a tile go to several CTAs (54 atoms: 12 -> 7 us a product)
+    const int tiles = TA >= 1 ? (na + TA - 1) / TA : 1;
+    const int gy = std::max(1, std::min((op.nrows + 3) / 4, 2 * dev().sm_count / tiles));
     if (TA >= 1) {
       const size_t smem = fixed + (size_t) TA * per_atom;
       static size_t attr = 48 * 1024;
@@ -521,7 +233,7 @@ void launch_prod(const ProdDev &op, const TensorDev *tensors, int NA, int na, in
         GB_CUDA(cudaFuncSetAttribute(prod_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) large));
         attr = large;
       }
-      GB_LAUNCH(prod_tile_kernel, (na + TA - 1) / TA, 256, smem, op, tensors, NA, na, TA, nfA, two ? nfB : 0, C, nterms);
+      GB_LAUNCH(prod_tile_kernel, dim3(tiles, gy), 256, smem, op, tensors, NA, na, TA, nfA, two ? nfB : 0, C);
       return;
     }
   }
@@ -530,43 +242,70 @@ void launch_prod(const ProdDev &op, const TensorDev *tensors, int NA, int na, in
   GB_LAUNCH(prod_kernel, grid, 256, 0, op, tensors, row_len, act_len);
 }
 
-// ---- readouts (fp64, one thread per atom) ---------------------------------------------------------------------
-__global__ void __launch_bounds__(64) readout_1l_kernel(ReadoutDev r, const float *__restrict__ rho, float *grho,
-                                                        const int *__restrict__ mu, double *e_atom, int NA, int na,
-                                                        int a0, int want_grad, const int *__restrict__ ilist)
+// ---- readouts (fp64) -------------------------------------------------------------------------------------------
+// A thread per atom is a chain of a thousand dependent fp64 instructions, 88 us however few the atoms; a warp per atom is
+// done in 20 us but takes five times the machine (GRACE-2L, 1,024,000 atoms: 10.4 against 2.2 ms).  The line is where the two
+// meet.
+constexpr int READOUT_WARP_ATOMS = 8192;
+
+template<bool WARP>
+__global__ void __launch_bounds__(128) readout_1l_kernel(ReadoutDev r, const float *__restrict__ rho, float *grho,
+                                                         const int *__restrict__ mu, double *e_atom, int NA, int na, int a0,
+                                                         int want_grad, const int *__restrict__ ilist)
 {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  const int a = WARP ? blockIdx.x * 4 + (threadIdx.x >> 5) : blockIdx.x * 128 + threadIdx.x;
   if (a >= na) return;
   const int i = ilist ? ilist[a0 + a] : a0 + a;    // the atom of chunk position a
-  e_atom[i] = readout_1l_atom(r, rho + (size_t) a * r.nrho, mu[i], grho + (size_t) a * r.nrho, want_grad, r.owned(i));
+  const float *x = rho + (size_t) a * r.nrho;
+  float *g = grho + (size_t) a * r.nrho;
+  if (WARP) {
+    const double e = readout_1l_warp(r, x, mu[i], g, want_grad, r.owned(i));
+    if ((threadIdx.x & 31) == 0) e_atom[i] = e;
+  } else {
+    e_atom[i] = readout_1l_atom(r, x, mu[i], g, want_grad, r.owned(i));
+  }
 }
 
 void launch_readout_1l(const ReadoutDev &r, const float *rho, float *grho, const int *mu, double *e_atom, int NA,
                        int na, int a0, int want_grad, const int *ilist)
 {
   if (na == 0) return;
-  GB_LAUNCH(readout_1l_kernel, (na + 63) / 64, 64, 0, r, rho, grho, mu, e_atom, NA, na, a0, want_grad, ilist);
+  if (na < READOUT_WARP_ATOMS)
+    GB_LAUNCH((readout_1l_kernel<true>), (na + 3) / 4, 128, 0, r, rho, grho, mu, e_atom, NA, na, a0, want_grad, ilist);
+  else
+    GB_LAUNCH((readout_1l_kernel<false>), (na + 127) / 128, 128, 0, r, rho, grho, mu, e_atom, NA, na, a0, want_grad, ilist);
 }
 
-__global__ void __launch_bounds__(64) readout_2l_kernel(ReadoutDev r, const float *__restrict__ rho_rows,
-                                                        const float *__restrict__ I2, double *grho_rows, float *gI2,
-                                                        const int *__restrict__ mu, double *e_atom, int NA, int na,
-                                                        int a0, int want_grad, const int *__restrict__ ilist)
+template<bool WARP>
+__global__ void __launch_bounds__(128) readout_2l_kernel(ReadoutDev r, const float *__restrict__ rho_rows,
+                                                         const float *__restrict__ I2, double *grho_rows, float *gI2,
+                                                         const int *__restrict__ mu, double *e_atom, int NA, int na, int a0,
+                                                         int want_grad, const int *__restrict__ ilist)
 {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  const int a = WARP ? blockIdx.x * 4 + (threadIdx.x >> 5) : blockIdx.x * 128 + threadIdx.x;
   if (a >= na) return;
   const int nr = r.nrho;
   const size_t i = ilist ? (size_t) ilist[a0 + a] : (size_t) (a0 + a);    // the atom of chunk position a
-  e_atom[i] = readout_2l_atom(r, rho_rows + i * nr, I2 + (size_t) a * nr, mu[i], grho_rows + i * nr, gI2 + (size_t) a * nr,
-                              want_grad, r.owned((long long) i));
+  const bool own = r.owned((long long) i);
+  if (WARP) {
+    const double e = readout_2l_warp(r, rho_rows + i * nr, I2 + (size_t) a * nr, mu[i], grho_rows + i * nr, gI2 + (size_t) a * nr,
+                                     want_grad, own);
+    if ((threadIdx.x & 31) == 0) e_atom[i] = e;
+  } else {
+    e_atom[i] = readout_2l_atom(r, rho_rows + i * nr, I2 + (size_t) a * nr, mu[i], grho_rows + i * nr, gI2 + (size_t) a * nr,
+                                want_grad, own);
+  }
 }
 
 void launch_readout_2l(const ReadoutDev &r, const float *rho_rows, const float *I2, double *grho_rows, float *gI2,
                        const int *mu, double *e_atom, int NA, int na, int a0, int want_grad, const int *ilist)
 {
   if (na == 0) return;
-  GB_LAUNCH(readout_2l_kernel, (na + 63) / 64, 64, 0, r, rho_rows, I2, grho_rows, gI2, mu, e_atom, NA, na, a0,
-            want_grad, ilist);
+  if (na < READOUT_WARP_ATOMS)
+    GB_LAUNCH((readout_2l_kernel<true>), (na + 3) / 4, 128, 0, r, rho_rows, I2, grho_rows, gI2, mu, e_atom, NA, na, a0, want_grad, ilist);
+  else
+    GB_LAUNCH((readout_2l_kernel<false>), (na + 127) / 128, 128, 0, r, rho_rows, I2, grho_rows, gI2, mu, e_atom, NA, na, a0, want_grad,
+              ilist);
 }
 
 // out[a] = v[list[a]]

@@ -117,7 +117,7 @@ void after_launch(const char *name)
 }
 
 namespace {
-constexpr size_t POOL_BLOCK = (size_t) 256 << 20, POOL_TOTAL = (size_t) 1 << 30;
+constexpr size_t POOL_BLOCK = (size_t) 1 << 30, POOL_TOTAL = (size_t) 4 << 30;
 std::mutex g_pool_mu;
 std::multimap<size_t, void *> g_pool;    // free blocks by size
 std::map<void *, size_t> g_block;        // size of every block that came from the driver

@@ -66,7 +66,7 @@ std::string profile_report();
     ::gb::after_launch(#kernel);                                                    \
   } while (0)
 
-// Device memory of the library.  Freed blocks of up to 256 MB stay in a pool of at most 1 GB and serve later requests
+// Device memory of the library.  Freed blocks of up to 1 GB stay in a pool of at most 4 GB and serve later requests
 // of about their size: a Batch that gives its buffers back after every call (the default of the interface) otherwise
 // pays the driver's allocation and release, which synchronise the device, for every buffer of every call (24 structures
 // of GRACE-2L: 7.8 ms per call for 2.8 ms of kernels).  All work on the blocks runs on the library's one stream, so a

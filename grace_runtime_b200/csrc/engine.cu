@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <set>
 
 namespace gb {
 
@@ -152,9 +153,6 @@ void Engine::setup_layer(LayerEngine &E, const LayerPlan &P)
     d.accumulate = o.accumulate;
     d.elem = o.elem;
     d.dst = o.dst;
-    d.dst_C = P.tensors[o.dst].channels;
-    d.max_row_items = 0;
-    for (size_t r = 0; r + 1 < o.item_off.size(); r++) d.max_row_items = std::max(d.max_row_items, o.item_off[r + 1] - o.item_off[r]);
     E.mv.push_back(d);
   }
   for (size_t q = 0; q < P.prod.size(); q++) {
@@ -171,21 +169,7 @@ void Engine::setup_layer(LayerEngine &E, const LayerPlan &P)
     d.srcB = o.srcB;
     E.prod.push_back(d);
   }
-  // tensor-core form of the operations with shared weights
-  {
-    double covered = 0.0, all = 0.0;
-    E.mv_tc.clear();
-    E.mv_tc.resize(P.mv.size());
-    for (size_t q = 0; q < P.mv.size(); q++) {
-      const double fl = (int) q == P.uq_mv ? 0.0 : P.mv[q].flops_per_atom();    // the UQ projection is not part of a step
-      all += fl;
-      if (MVTensorCore::eligible(P.mv[q], P.tensors)) {
-        E.mv_tc[q].setup(P.mv[q]);
-        covered += fl;
-      }
-    }
-    E.tc_flop_share = all > 0.0 ? covered / all : 0.0;
-  }
+  setup_steps(E, P);
   // tensors: values first, then the gradients that are zeroed per chunk (one contiguous range)
   E.toff.assign(P.tensors.size(), 0);
   long long at = 0;
@@ -201,6 +185,112 @@ void Engine::setup_layer(LayerEngine &E, const LayerPlan &P)
   E.per_atom = at;
   E.tensors.set_label("engine:tensor_table");
   E.tensors_host.assign(P.tensors.size(), TensorDev{nullptr, 0});
+}
+
+// The launches of a layer's programs.  An MV operation joins an earlier launch of its shape when it may as well run there: it
+// reads nothing that launch or a later one writes, and no other step in between touches what it writes.  A row two
+// operations of a launch write gets the items of both (one read and one write of it less).
+void Engine::setup_steps(LayerEngine &E, const LayerPlan &P)
+{
+  double covered = 0.0, all = 0.0;
+  auto build = [&](const Program &prog, std::vector<LayerEngine::Step> &steps) {
+    struct Touch {
+      std::vector<int> reads;
+      std::map<int, std::vector<int>> writes;    // tensor -> rows
+    };
+    auto touch_of = [&](const Op &o) {
+      Touch t;
+      if (o.kind == Op::MV) {
+        for (const MVItem &it : P.mv[o.index].items) t.reads.push_back(it.src);
+        t.writes[P.mv[o.index].dst] = P.mv[o.index].row_out;
+      } else {
+        const ProdOp &q = P.prod[o.index];
+        t.reads.push_back(q.srcA);
+        if (q.srcB >= 0) t.reads.push_back(q.srcB);
+        t.writes[q.dst] = q.row_out;
+      }
+      std::sort(t.reads.begin(), t.reads.end());
+      t.reads.erase(std::unique(t.reads.begin(), t.reads.end()), t.reads.end());
+      return t;
+    };
+    auto has = [](const std::vector<int> &v, int x) { return std::find(v.begin(), v.end(), x) != v.end(); };
+    auto overlap = [&](const Touch &a, const Touch &b) {
+      for (const auto &w : a.writes) {
+        auto f = b.writes.find(w.first);
+        if (f == b.writes.end()) continue;
+        for (int r : w.second)
+          if (has(f->second, r)) return true;
+      }
+      return false;
+    };
+    auto crosses = [&](const Touch &a, const Touch &b) {    // one reads what the other writes
+      for (const auto &w : a.writes)
+        if (has(b.reads, w.first)) return true;
+      for (const auto &w : b.writes)
+        if (has(a.reads, w.first)) return true;
+      return false;
+    };
+    std::vector<Touch> touched;
+    steps.clear();
+    for (const Op &o : prog.ops) {
+      const Touch t = touch_of(o);
+      const bool tc = o.kind == Op::MV && MVTensorCore::eligible(P.mv[o.index], P.tensors);
+      int into = -1;
+      if (o.kind == Op::MV) {
+        const double fl = P.mv[o.index].flops_per_atom();
+        all += fl;
+        if (tc) covered += fl;
+      }
+      for (int g = (int) steps.size() - 1; tc && g >= 0 && into < 0; g--) {
+        LayerEngine::Step &st = steps[g];
+        if (crosses(t, touched[g])) break;
+        const MVOp &m = P.mv[o.index];
+        bool same = st.kind == Op::MV && MVTensorCore::eligible(P.mv[st.ops[0]], P.tensors) && P.mv[st.ops[0]].elem == m.elem &&
+                    MVTensorCore::padded_k(P.mv[st.ops[0]]) == MVTensorCore::padded_k(m) &&
+                    MVTensorCore::padded_n(P.mv[st.ops[0]].n_out) == MVTensorCore::padded_n(m.n_out);
+        if (same) {
+          size_t rows = m.row_out.size(), items = m.items.size();
+          for (int q : st.ops) {
+            rows += P.mv[q].row_out.size();
+            items += P.mv[q].items.size();
+          }
+          same = rows <= MVTensorCore::MAX_ROWS && items <= MVTensorCore::MAX_ITEMS && (m.accumulate || !overlap(t, touched[g]));
+        }
+        if (same) into = g;
+        else if (overlap(t, touched[g])) break;
+      }
+      if (into >= 0) {
+        steps[into].ops.push_back(o.index);
+        touched[into].reads.insert(touched[into].reads.end(), t.reads.begin(), t.reads.end());
+        for (const auto &w : t.writes) {
+          auto &v = touched[into].writes[w.first];
+          v.insert(v.end(), w.second.begin(), w.second.end());
+        }
+      } else {
+        LayerEngine::Step st;
+        st.kind = o.kind;
+        st.ops = {o.index};
+        st.elem = o.kind == Op::MV && P.mv[o.index].elem;
+        steps.push_back(std::move(st));
+        touched.push_back(t);
+      }
+    }
+    for (LayerEngine::Step &st : steps)
+      if (st.kind == Op::MV && MVTensorCore::eligible(P.mv[st.ops[0]], P.tensors)) {
+        std::vector<const MVOp *> ops;
+        std::vector<const float *> W;
+        for (int q : st.ops) {
+          ops.push_back(&P.mv[q]);
+          W.push_back(E.mv[q].W);
+        }
+        st.tc = std::make_unique<MVTensorCore>();
+        st.tc->setup(ops, W, plan_.n_elements);
+      }
+  };
+  build(P.fwd, E.fwd);
+  build(P.bwd, E.bwd);
+  if (P.uq_mv >= 0 && MVTensorCore::eligible(P.mv[P.uq_mv], P.tensors)) E.uq_tc.setup({&P.mv[P.uq_mv]}, {E.mv[P.uq_mv].W}, 1);
+  E.tc_flop_share = all > 0.0 ? covered / all : 0.0;
 }
 
 Engine::Engine(const GraceModel &m, int spline_n) : plan_(build_plan(m, spline_n > 0 ? spline_n : 1024))
@@ -331,7 +421,7 @@ void Engine::dense_stats(double *o) const
         by += 4.0 * it.n_in;
       }
       by += 4.0 * m.n_out * (double) m.row_out.size() * (m.accumulate ? 2.0 : 1.0);
-      const int k = E->mv_tc[q].ready() ? 0 : 4;
+      const int k = m.elem ? 4 : 0;
       o[k] += fl;
       o[k + 1] += by;
     }
@@ -365,14 +455,17 @@ double Engine::per_atom_bytes(int64_t n_eval) const
   return 4.0 * (double) std::max(L1_.per_atom, L2_.per_atom);
 }
 
+constexpr double SMALL_WORK = 2e9;    // bytes
+
 int Engine::auto_chunk(int64_t n) const
 {
   if (plan_.layers == 3) return (int) std::max<int64_t>(n, 1);    // one pass
   // per-operation passes: large enough that the atom tiles of a pass fill the GPU, small enough to bound the work memory
   const int64_t most = std::min<int64_t>(std::max<int64_t>(n, 1), use_fused(n) ? ((int64_t) 1 << 22) : (use_tc(n) ? 524288 : 32768));
   const double held = 4.0 * (double) arena_.capacity(), per = per_atom_bytes(n);
-  // what the work buffer already holds needs no look at the free memory (a driver call of 10 us and more per evaluation)
-  if ((double) most * per <= held) return (int) most;
+  // what the work buffer already holds, or is small on this GPU, needs no look at the free memory (a driver call of 10 us, at
+  // times of 10 ms; should it not fit all the same, the call is repeated with smaller passes)
+  if ((double) most * per <= std::max(held, SMALL_WORK)) return (int) most;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = (size_t) 8 << 30;
   const int64_t c = (int64_t) ((0.35 * (double) free_b + held) / per);
@@ -451,27 +544,34 @@ void Engine::gather_message_gradients(NeighborList &nl, const float *slots, cons
                          R.nlocal >= 0 ? nl.perm() : nullptr, R.nlocal);
 }
 
-void Engine::run(LayerEngine &E, const Program &prog, const int *mu, int NA, int stride)
+void Engine::run(LayerEngine &E, bool forward, NeighborList &nl, const int *mu, int64_t a0, int na, int stride)
 {
-  // NA here is the number of atoms in use; stride: the atom stride of the layer's chunk tensors
-  const int arena_NA_ = stride;
   static const bool tag_ops = getenv("GRACE_B200_PROFILE_OPS") != nullptr;
-  for (const Op &o : prog.ops) {
-    if (tag_ops) launch_tag(o.kind == Op::MV ? E.plan->mv[o.index].name.c_str() : E.plan->prod[o.index].name.c_str());
-    if (o.kind == Op::MV) {
-      if (tc_now_ && E.mv_tc[o.index].ready())
-        E.mv_tc[o.index].launch(E.mv[o.index], E.tensors.get(), (int) E.tensors_host.size(), arena_NA_, NA, tc_error_.get());
-      else launch_mv(E.mv[o.index], E.tensors.get(), mu, arena_NA_, NA);
-    } else {
-      const ProdDev &pd = E.prod[o.index];
-      const auto &ts = E.plan->tensors;
-      const int C = ts[pd.dst].channels;
-      const bool same = ts[pd.srcA].channels == C && (pd.srcB < 0 || ts[pd.srcB].channels == C);
-      launch_prod(pd, E.tensors.get(), arena_NA_, NA, C, same ? ts[pd.srcA].nfuncs : 0,
-                  pd.srcB >= 0 ? ts[pd.srcB].nfuncs : 0, (int) E.plan->prod[o.index].terms.size());
-    }
+  const auto &ts = E.plan->tensors;
+  auto product = [&](int q) {
+    const ProdDev &pd = E.prod[q];
+    const int C = ts[pd.dst].channels;
+    const bool same = ts[pd.srcA].channels == C && (pd.srcB < 0 || ts[pd.srcB].channels == C);
+    launch_prod(pd, E.tensors.get(), stride, na, C, same ? ts[pd.srcA].nfuncs : 0, pd.srcB >= 0 ? ts[pd.srcB].nfuncs : 0,
+                (int) E.plan->prod[q].terms.size());
+  };
+  for (const LayerEngine::Step &st : forward ? E.fwd : E.bwd) {
+    if (tag_ops) launch_tag(st.kind == Op::MV ? E.plan->mv[st.ops[0]].name.c_str() : E.plan->prod[st.ops[0]].name.c_str());
+    if (st.kind == Op::PROD) product(st.ops[0]);
+    else if (tc_now_ && st.tc)
+      st.tc->launch(E.tensors.get(), (int) E.tensors_host.size(), stride, na, tc_error_.get(),
+                    st.elem ? &nl.element_order(mu, a0, na, plan_.n_elements) : nullptr);
+    else
+      for (int q : st.ops) launch_mv(E.mv[q], E.tensors.get(), mu, stride, na);
   }
   if (tag_ops) launch_tag(nullptr);
+}
+
+void Engine::uq_project(LayerEngine &E, const int *mu, int na, int stride)
+{
+  if (tc_now_ && E.uq_tc.ready())
+    E.uq_tc.launch(E.tensors.get(), (int) E.tensors_host.size(), stride, na, tc_error_.get(), nullptr);
+  else launch_mv(E.mv[E.plan->uq_mv], E.tensors.get(), mu, stride, na);
 }
 
 // UQ of GRACE-2L, layer 1 (after the forward program of a chunk of layer 1): projection of the rho block, kept per atom
@@ -480,9 +580,7 @@ void Engine::uq_layer1(const int *mu, int64_t a0, int na, int stride)
 {
   const LayerPlan &P = *L1_.plan;
   const int q = P.uq_mv;
-  if (tc_now_ && L1_.mv_tc[q].ready())
-    L1_.mv_tc[q].launch(L1_.mv[q], L1_.tensors.get(), (int) L1_.tensors_host.size(), stride, na, tc_error_.get());
-  else launch_mv(L1_.mv[q], L1_.tensors.get(), mu, stride, na);
+  uq_project(L1_, mu, na, stride);
   launch_uq_norm(L1_.mv[q], L1_.tensors.get(), stride, na, uq_n2b_.get() + a0);
   launch_rows_from_chunk(L1_.tensors_host[P.tUQ].p, uq_z1_.get(), 1, plan_.uq.rp_dim, stride, na, (int) a0);
 }
@@ -492,9 +590,7 @@ void Engine::uq_last(LayerEngine &E, const int *mu, int64_t a0, int na, int stri
 {
   const LayerPlan &P = *E.plan;
   const int q = P.uq_mv;
-  if (tc_now_ && E.mv_tc[q].ready())
-    E.mv_tc[q].launch(E.mv[q], E.tensors.get(), (int) E.tensors_host.size(), stride, na, tc_error_.get());
-  else launch_mv(E.mv[q], E.tensors.get(), mu + a0, stride, na);
+  uq_project(E, mu + a0, na, stride);
   launch_uq_norm(E.mv[q], E.tensors.get(), stride, na, uq_n2a_.get() + a0);
   const bool two = plan_.layers == 2;
   double *o = uq_out_.get();
@@ -803,7 +899,7 @@ void Engine::evaluate_chunked(NeighborList &nl, bool energy_only, int NA, StageT
     const size_t need = (size_t) L1_.per_atom * (size_t) w1 * sizeof(float);
     const size_t held = arena1_.capacity() * sizeof(float);
     if (w1 < ((int64_t) 1 << 30) &&
-        (need <= held || (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && need <= (size_t) (0.45 * (double) free_b) + held))) {
+        (need <= std::max(held, (size_t) SMALL_WORK) || (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && need <= (size_t) (0.45 * (double) free_b) + held))) {
       try {
         base1 = arena1_.ensure((size_t) L1_.per_atom * (size_t) w1);
         NA1 = (int) w1;
@@ -842,14 +938,14 @@ void Engine::evaluate_chunked(NeighborList &nl, bool energy_only, int NA, StageT
       const int na = (int) std::min<int64_t>(NA, s0.hi - a0);
       if (tm) tm->begin(StageTimer::FWD);
       launch_bond_fwd(P.lmax, bonds0, L, T1(P.L1.tQ), NA, (int) a0, na);
-      run(L1_, P.L1.fwd, s0.mu + a0, na, NA);
+      run(L1_, true, nl, s0.mu + a0, a0, na, NA);
       if (uq_now_) uq_last(L1_, mu, a0, na, NA, n);
       launch_readout_1l(readout_, T1(P.t1_rho), T1(P.t1_grho), mu, e_atom_.get(), NA, na, (int) a0, !energy_only, s0.ilist);
       if (tm) tm->end(StageTimer::FWD);
       if (energy_only) continue;
       if (tm) tm->begin(StageTimer::BWD);
       zero_grads(L1_, arena_.get(), NA);
-      run(L1_, P.L1.bwd, s0.mu + a0, na, NA);
+      run(L1_, false, nl, s0.mu + a0, a0, na, NA);
       launch_bond_bwd(P.lmax, bonds0, L, T1(P.L1.tGQ), NA, (int) a0, na, fv, vir_atom_.get(), 0);
       if (tm) tm->end(StageTimer::BWD);
     }
@@ -873,7 +969,7 @@ void Engine::evaluate_chunked(NeighborList &nl, bool energy_only, int NA, StageT
     for (int64_t a0 = s1.lo; a0 < s1.hi; a0 += step1) {
       const int na = (int) std::min<int64_t>(step1, s1.hi - a0);
       { TagScope tg("layer1"); launch_bond_fwd(P.lmax, bonds1, La, T1(P.L1.tQ), S1, (int) a0, na); }
-      run(L1_, P.L1.fwd, s1.mu + a0, na, S1);
+      run(L1_, true, nl, s1.mu + a0, a0, na, S1);
       if (uq_now_) uq_layer1(mu + a0, a0, na, S1);
       launch_rows_from_chunk(T1(P.t1_I), I_rows_.get(), nI, CR, S1, na, (int) a0, s1.ilist);
       launch_rows_from_chunk(T1(P.t1_rho), rho_rows_.get(), 1, nrho, S1, na, (int) a0, s1.ilist);
@@ -885,7 +981,7 @@ void Engine::evaluate_chunked(NeighborList &nl, bool energy_only, int NA, StageT
       const int na = (int) std::min<int64_t>(NA, s0.hi - a0);
       if (tm) tm->begin(StageTimer::FWD);
       { TagScope tg("layer2"); launch_bond_fwd(P.lmax, bonds0, Lb, T2(P.L2.tQ), NA, (int) a0, na); }
-      run(L2_, P.L2.fwd, s0.mu + a0, na, NA);
+      run(L2_, true, nl, s0.mu + a0, a0, na, NA);
       if (uq_now_) uq_last(L2_, mu, a0, na, NA, n);
       launch_readout_2l(readout_, rho_rows_.get(), T2(P.t2_I2), grho_rows_.get(), T2(P.t2_gI2), mu, e_atom_.get(), NA,
                         na, (int) a0, !energy_only, s0.ilist);
@@ -893,7 +989,7 @@ void Engine::evaluate_chunked(NeighborList &nl, bool energy_only, int NA, StageT
       if (energy_only) continue;
       if (tm) tm->begin(StageTimer::BWD);
       zero_grads(L2_, arena_.get(), NA);
-      run(L2_, P.L2.bwd, s0.mu + a0, na, NA);
+      run(L2_, false, nl, s0.mu + a0, a0, na, NA);
       { TagScope tg("layer2"); launch_bond_bwd(P.lmax, bonds0, Lb, T2(P.L2.tGQ), NA, (int) a0, na, fv, vir_atom_.get(), 0); }
       if (tm) tm->end(StageTimer::BWD);
     }
@@ -906,12 +1002,12 @@ void Engine::evaluate_chunked(NeighborList &nl, bool energy_only, int NA, StageT
         const int na = (int) std::min<int64_t>(step1, s1.hi - a0);
         if (!base1) {    // the tensors of layer 1 were overwritten by layer 2: evaluate it again
           launch_bond_fwd(P.lmax, bonds1, La, T1(P.L1.tQ), S1, (int) a0, na);
-          run(L1_, P.L1.fwd, s1.mu + a0, na, S1);
+          run(L1_, true, nl, s1.mu + a0, a0, na, S1);
         }
         zero_grads(L1_, abase1, S1);
         launch_chunk_from_rows(T1(P.t1_gI), gI_rows_.get(), nI, CR, S1, na, (int) a0, s1.ilist);
         launch_chunk_from_rows_f64(T1(P.t1_grho), grho_rows_.get(), 1, nrho, S1, na, (int) a0, s1.ilist);
-        run(L1_, P.L1.bwd, s1.mu + a0, na, S1);
+        run(L1_, false, nl, s1.mu + a0, a0, na, S1);
         { TagScope tg("layer1"); launch_bond_bwd(P.lmax, bonds1, La, T1(P.L1.tGQ), S1, (int) a0, na, fv, vir_atom_.get(), 1); }
       }
       if (tm) tm->end(StageTimer::BWD);
@@ -1256,6 +1352,7 @@ SystemObj::SystemObj(std::shared_ptr<ModelObj> m, const std::vector<std::string>
   for (int a : t2m_)
     for (int b : t2m_) cutoff_ = std::max(cutoff_, model_->model.pair_cutoff(a, b));
   label_ws(ws_);
+  nl_.set_kinds((int) std::set<int>(t2m_.begin(), t2m_.end()).size());
 }
 
 void SystemObj::release()
@@ -1460,6 +1557,7 @@ EngineRunObj::EngineRunObj(std::shared_ptr<ModelObj> m, const std::vector<std::s
   for (int a : t2m_)
     for (int b : t2m_) cutoff_ = std::max(cutoff_, model_->model.pair_cutoff(a, b));
   label_ws(ws_);
+  nl_.set_kinds((int) std::set<int>(t2m_.begin(), t2m_.end()).size());
 }
 
 int EngineRunObj::comm_width() const { return engine_->plan().layers == 2 ? engine_->plan().nI * engine_->plan().cr : 0; }
@@ -1532,6 +1630,7 @@ BatchObj::BatchObj(std::shared_ptr<ModelObj> m, const std::vector<std::string> &
   for (int a : t2m_)
     for (int b : t2m_) cutoff_ = std::max(cutoff_, model_->model.pair_cutoff(a, b));
   label_ws(ws_);
+  nl_.set_kinds((int) std::set<int>(t2m_.begin(), t2m_.end()).size());
 }
 
 void BatchObj::release()

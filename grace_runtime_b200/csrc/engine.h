@@ -45,8 +45,16 @@ struct LayerEngine {
   int fused_TA = 0;           // atoms per tile that fit the shared memory (0: the layer does not fit)
   int fused_NG = 2;           // warp groups per CTA the layer runs with (2, or 1 when two would get one atom each)
   long long q_floats = 0;     // floats per atom of the bond-sum tensor
-  // tensor-core form of each MV operation on chunk tensors (mv_tc.cu); not ready: the operation runs as mv_kernel
-  std::vector<MVTensorCore> mv_tc;
+  // the programs as launches on chunk tensors: an MV step is a group of operations in one tensor-core launch (mv_tc.cu), or
+  // one operation outside its shapes (mv_kernel); a PROD step is one product
+  struct Step {
+    Op::Kind kind;
+    std::vector<int> ops;    // indices into the plan's mv / prod
+    std::unique_ptr<MVTensorCore> tc;    // null: launch_mv of ops[0]
+    bool elem = false;
+  };
+  std::vector<Step> fwd, bwd;
+  MVTensorCore uq_tc;            // the UQ projection
   double tc_flop_share = 0.0;    // share of the layer's MV flops the tensor-core kernel covers
 };
 
@@ -136,20 +144,22 @@ class Engine {
   UqDev uq_dev_{};
   bool uq_now_ = false;    // the evaluation in progress computes the UQ outputs
   void uq_layer1(const int *mu, int64_t a0, int na, int stride);
+  void uq_project(LayerEngine &E, const int *mu, int na, int stride);
   void uq_last(LayerEngine &E, const int *mu, int64_t a0, int na, int stride, int64_t n);
   int arena_NA_ = 0;
   void setup_layer(LayerEngine &E, const LayerPlan &P);
   void setup_fused(LayerEngine &E, const LayerPlan &P);
   bool fused_ = false;        // both layers fit the fused shared-memory kernel
-  // Dense-network path of an evaluation.  Large evaluations stream the network operation by operation over chunk
-  // tensors in global memory with the FC layers on the tensor cores (atoms are the long GEMM dimension: 128-atom
-  // tiles fill an MMA); small ones (too few atom tiles to fill the GPU) and shapes the tensor-core kernel does not
-  // cover run as the fused shared-memory kernel.  GRACE_B200_DENSE = fused | tc | ops overrides (ops: every operation
-  // as its SIMT kernel).
+  // Dense-network path of an evaluation.  The network runs operation by operation over chunk tensors in global memory, every
+  // MV operation on the tensor cores (atoms are the long GEMM dimension: 128-atom tiles fill an MMA, and where the tiles are
+  // few the output rows go to different SMs); structures of a few hundred atoms, whose operations are too short for their
+  // launches, run as the fused shared-memory kernel.  The line is where both take the same time (GRACE-1L 2,000 atoms 0.40
+  // against 0.43 ms, GRACE-2L 108 atoms 0.49 against 0.41, 3,264 atoms 1.7 against 2.6).  GRACE_B200_DENSE = fused | tc |
+  // ops overrides (ops: every operation as its SIMT kernel).
   enum class Dense { Auto, Fused, Tc, Ops };
   Dense dense_ = Dense::Auto;
   bool tc_ready_ = false;
-  int64_t tc_min_atoms_ = 16384;
+  int64_t tc_min_atoms_ = 512;
   DBuf<int> tc_error_;
   bool use_fused(int64_t n_eval) const;
   bool use_tc(int64_t n_eval) const;
@@ -167,7 +177,10 @@ class Engine {
   void evaluate_chunked(NeighborList &nl, bool energy_only, int NA, StageTimer *tm, const ActiveRanges &R);
   void run_fused(LayerEngine &E, int mode, int NA, int a0, int na, const int *mu, const int *ilist, float *saved = nullptr);
   void bind_arena(LayerEngine &E, float *base, int NA);
-  void run(LayerEngine &E, const Program &prog, const int *mu, int NA, int stride);
+  // operations of one direction for `na` atoms with elements mu, chunk tensors of atom stride `stride`; list position a0 of
+  // the first atom (the grouping by element is kept with the list)
+  void run(LayerEngine &E, bool forward, NeighborList &nl, const int *mu, int64_t a0, int na, int stride);
+  void setup_steps(LayerEngine &E, const LayerPlan &P);
   DBuf<float> arena1_;               // chunk tensors of layer 1 for all of its atoms (GRACE-2L on the per-operation path)
   const float *arena1_bound_ = nullptr;
   int arena1_NA_ = 0;

@@ -805,8 +805,7 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
   const BondsDev bonds = nl.bonds();
   const int *mu = bonds.mu;
   const SHTable sht = sh_table_host();
-  // large evaluations: the projections, reduces and FCs with 16 / 32 / 64 channels as tensor-core grouped GEMMs (mv_tc.cu)
-  tc_now_ = dense_ == Dense::Tc || (n >= tc_min_atoms_ && dense_ == Dense::Auto);
+  tc_now_ = dense_ == Dense::Tc || dense_ == Dense::Auto;    // the projections, reduces and FCs as tensor-core grouped GEMMs (mv_tc.cu)
   // every bond needs the radial table of its element pair: the species of every System / Batch of this engine were
   // prepared when it was created (prepare_species); a bond of a pair without a table is left out by the kernels
   if (tm) tm->begin(StageTimer::FWD);
@@ -927,7 +926,7 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
     LayerEngine &E = S.E[k];
     const std::vector<TensorDev> &T = E.tensors_host;
     bonds_forward(k, T[L.tA].p, NC, a0, na);
-    run(E, L.dense.fwd, mu + a0, na, NC);
+    run(E, true, nl, mu + a0, a0, na, NC);
     if (!outputs) return;
     if (k < 2) {
       const EqNormDev e{S.eq_dw[k].get(), S.eq_mask[k].get(), S.eq_aff[k].get(), S.eq_e[k].get(), L.nfEQ, L.cEQ, L.eq_center, L.eq_eps};
@@ -947,7 +946,7 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
       const EqNormDev e{S.eq_dw[k].get(), S.eq_mask[k].get(), S.eq_aff[k].get(), S.eq_e[k].get(), L.nfEQ, L.cEQ, L.eq_center, L.eq_eps};
       GB_LAUNCH(eqnorm_bwd_kernel, na, 32 * EQ_WARPS, 0, e, T[L.tEQ].p, S.gmsg[k].get(), T[L.tGEQ].p, NC, a0);
     }
-    run(E, L.dense.bwd, mu + a0, na, NC);
+    run(E, false, nl, mu + a0, a0, na, NC);
     bonds_reverse(k, T[L.tGA].p, NC, a0, na);
   };
   for (int k = 0; k < 2; k++) S.msg[k].ensure((size_t) n * Q.L[k].nfEQ * Q.L[k].cEQ);

@@ -1,4 +1,4 @@
-// FC layers, non-element reduces and their adjoints of the dense network on the 5th-generation tensor cores.
+// FC layers, reduces and their adjoints of the dense network on the 5th-generation tensor cores.
 //
 // On chunk tensors [function][atom][channel] an operation  out[row] (+)= sum_items scale * W_item^T x[item]  is a
 // grouped GEMM whose long dimension is the atoms: for an output row and a tile of 128 atoms,
@@ -6,11 +6,18 @@
 // with X_item a contiguous block of the source tensor.  A CTA owns up to 256 / n_out atom tiles at a time and keeps two
 // sets of fp32 accumulators for them in tensor memory; for every item of the row its producer warps write the tile's
 // activations as hi + lo operand images into a ring of shared-memory stages (canonical K-major layout, 8-row x 16-byte
-// core matrices), the item's weight image (split on the host once) arrives by one bulk asynchronous copy, and one
-// thread issues tcgen05.mma kind::tf32 M = 128, N = n_out: a b ~ a_lo b_hi + a_hi b_lo + a_hi b_hi keeps fp32-level
+// core matrices), the item's weight image (split once when the model is loaded) arrives by one bulk asynchronous copy, and
+// one thread issues tcgen05.mma kind::tf32 M = 128, N = n_out: a b ~ a_lo b_hi + a_hi b_lo + a_hi b_hi keeps fp32-level
 // accuracy.  The global loads of the next two tiles are in flight in registers while a tile is written, all items of a
 // row accumulate in tensor memory, and the epilogue warps write each output row once while the next row's matrix
 // instructions run.
+// Widths are padded with zeros to K = 16, 32 or 64 and N a multiple of 16, so every operation of up to 64 inputs runs here.
+// Operations whose weights depend on the central atom's element (the reduces to densities and messages, their adjoints) take
+// tiles of atoms of ONE element: the atoms are gathered through an index (ElemOrder) that groups them by element, a row of
+// 9 - 64 channels each, and the weight image is chosen per tile.  With the elements mixed in a tile the weights of every
+// element present passed through shared memory: 557,000 atoms of 89 elements 82 ms, 1,024,000 atoms of 3 elements 20.7 ms per
+// evaluation of GRACE-2L; grouped 11.0 and 17.7 ms.
+// Independent operations of the same shape are one launch (plan.h MVGroup): rows carry their tensor and whether they add.
 // Same mathematics as mv_kernel (chain.cu); reference: fc_fwd / mv_batch, libgrace/include/grace/fused_cpu.h:294-356,
 // GPU fc_fwd4 libgrace/include/grace/kk/fused_dense.h:441-495.
 //
@@ -33,7 +40,7 @@ constexpr int NW = NTH / 32;
 constexpr int TMEM_COLS = 512;
 constexpr int MAX_TILES = 16;   // atom tiles a CTA holds accumulators for
 constexpr int MAX_TENSORS = 64;
-constexpr int MAX_ITEMS = 512, MAX_ROWS = 256;    // tables of an operation staged in shared memory
+constexpr int MAX_ITEMS = MVTensorCore::MAX_ITEMS, MAX_ROWS = MVTensorCore::MAX_ROWS;    // tables of an operation staged in shared memory
 constexpr long long WAIT_CYCLES = 40000000LL;    // ~20 ms: far beyond any tile, far below a watchdog
 
 // byte offset of element (r, k) of a K-major operand tile with K columns (canonical layout, no swizzle)
@@ -125,7 +132,7 @@ template<int K> struct TileRegs {
 // arrivals).  A wait that runs out raises `abort`, which every other wait sees, and all roles leave together.
 constexpr int NPROD = NTH, NTHREADS = NTH + 32 + 128;
 
-template<int K, int CB, int S>
+template<int K, int CB, int S, bool ELEM>
 __global__ void __launch_bounds__(NTHREADS, 1) mv_tc_kernel(MVTCDev op, const TensorDev *__restrict__ Tg, int ntensors, int NA,
                                                             int na, int TB, int tmem_cols, int *error)
 {
@@ -139,16 +146,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) mv_tc_kernel(MVTCDev op, const Te
   __shared__ TensorDev s_T[MAX_TENSORS];
   // the operation's tables: every role walks them once per fill, so they live in shared memory
   __shared__ MVItem s_items[MAX_ITEMS];
-  __shared__ int s_item_off[MAX_ROWS + 1], s_row_out[MAX_ROWS];
+  __shared__ MVRowDev s_rows[MAX_ROWS];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const int N = op.n_out;
+  const int N = op.N;
   const int W_BYTES = N * K * 4;                         // one image of a weight matrix
   char *A_st = smem;                                     // stage s at s * 2 * A_BYTES: hi, then lo
   char *W_st = smem + (size_t) S * 2 * A_BYTES;          // buffer b at b * 2 * W_BYTES: hi, then lo
   float *tr_all = reinterpret_cast<float *>(W_st + (size_t) S * 2 * W_BYTES);    // transpose buffers of the epilogue warps
   for (int q = t; q < ntensors; q += NTHREADS) s_T[q] = Tg[q];
-  for (int q = t; q <= op.nrows; q += NTHREADS) s_item_off[q] = op.item_off[q];
-  for (int q = t; q < op.nrows; q += NTHREADS) s_row_out[q] = op.row_out[q];
+  for (int q = t; q < op.nrows; q += NTHREADS) s_rows[q] = op.rows[q];
   for (int q = t; q < op.nitems; q += NTHREADS) s_items[q] = op.items[q];
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(tmem_cols) : "memory");
@@ -171,7 +177,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mv_tc_kernel(MVTCDev op, const Te
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const unsigned tmem = s_tmem;
-  const int ntiles = (na + TM - 1) / TM, per_round = gridDim.x * TB;
+  const int ntiles = ELEM ? op.tiles[0] : (na + TM - 1) / TM, per_round = gridDim.x * TB;
   volatile int *abort_flag = &s_abort;
 
   // bounded wait that also gives up when another role did
@@ -196,8 +202,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) mv_tc_kernel(MVTCDev op, const Te
     c.valid = tile0 < ntiles && row < op.nrows;
     if (!c.valid) return;
     c.nt = min(TB, ntiles - tile0);
-    c.i0 = c.it = s_item_off[row];
-    c.i1 = s_item_off[row + 1];
+    c.i0 = c.it = s_rows[row].i0;
+    c.i1 = s_rows[row].i1;
     c.tt = 0;
   };
   auto advance = [&](Cursor &c) {
@@ -222,16 +228,34 @@ __global__ void __launch_bounds__(NTHREADS, 1) mv_tc_kernel(MVTCDev op, const Te
 
   if (warp < NW) {
     // ---------------- producers ----------------
+    // grouped atoms: this thread's two rows of the tile at hand (the tile stays while the items of all rows pass)
+    int tile_of_rows = -1, arow[2] = {-1, -1};
     auto load_tile = [&](const Cursor &c, TR &r) {
       const MVItem item = s_items[c.it];
       const TensorDev src = s_T[item.src];
-      const int atom0 = (c.tile0 + c.tt) * TM, valid = min(TM, na - atom0);
-      const float *base = src.p + ((size_t) item.irow * NA + atom0) * src.C;
+      const int atom0 = (c.tile0 + c.tt) * TM, valid = ELEM ? TM : min(TM, na - atom0);
+      const float *base = src.p + (size_t) item.irow * NA * src.C;
+      const bool vec = ((src.C | item.n_in) & 3) == 0;
+      if (ELEM && tile_of_rows != c.tile0 + c.tt) {
+        tile_of_rows = c.tile0 + c.tt;
+        arow[0] = __ldg(op.order + atom0 + warp * 8 + (lane & 7));
+        arow[1] = __ldg(op.order + atom0 + (warp + NW) * 8 + (lane & 7));
+      }
 #pragma unroll
       for (int j = 0; j < PER; j++) {
         const int u = warp + NW * j, row = (u % 16) * 8 + (lane & 7), c4 = (u / 16) * 4 + (lane >> 3);
-        r.v[j] = (u < UNITS && row < valid && c4 < K4) ? __ldg(reinterpret_cast<const float4 *>(base + (size_t) row * src.C) + c4)
-                                                        : make_float4(0.f, 0.f, 0.f, 0.f);
+        r.v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (u >= UNITS || row >= valid || 4 * c4 >= item.n_in) continue;
+        const int a = ELEM ? arow[j & 1] : atom0 + row;    // (16 groups of rows, NW = 8 warps: even and odd j)
+        if (ELEM && a < 0) continue;
+        const float *x = base + (size_t) a * src.C + 4 * c4;
+        if (vec) r.v[j] = __ldg(reinterpret_cast<const float4 *>(x));
+        else {
+          r.v[j].x = __ldg(x);
+          if (4 * c4 + 1 < item.n_in) r.v[j].y = __ldg(x + 1);
+          if (4 * c4 + 2 < item.n_in) r.v[j].z = __ldg(x + 2);
+          if (4 * c4 + 3 < item.n_in) r.v[j].w = __ldg(x + 3);
+        }
       }
     };
     Cursor cur, nxt, nxt2;
@@ -262,13 +286,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) mv_tc_kernel(MVTCDev op, const Te
       }
       GB_TICK(tp_, 0);
       const MVItem item = s_items[cur.it];
-      if (cur.tt == 0) {    // first tile of an item: its weight image (hi + lo, byte for byte the operand layout)
+      if (ELEM || cur.tt == 0) {    // first tile of an item (every tile of its own element): its weight image (hi + lo)
         item_no++;
         if (t == 0) {
           // one bulk asynchronous copy; its bytes are counted by this stage's `full` barrier, so the matrix instructions
           // of the fill start when the image and the 256 arrivals are there, and no producer waits for the copy
           const unsigned bar = smem_u32(&s_full[s]), dst = smem_u32(W_st + (size_t) (item_no % S) * 2 * W_BYTES);
-          const char *src = op.images + (size_t) item.mat * 2 * W_BYTES;
+          const int e = ELEM ? __ldg(op.tiles + 1 + cur.tile0 + cur.tt) : 0;
+          const char *src = op.images + ((size_t) e * op.nmat + item.mat) * 2 * W_BYTES;
           asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"((unsigned) (2 * W_BYTES)) : "memory");
           asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                        ::"r"(dst), "l"(src), "r"((unsigned) (2 * W_BYTES)), "r"(bar) : "memory");
@@ -321,7 +346,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mv_tc_kernel(MVTCDev op, const Te
       while (cur.valid && ok) {
         GB_TICK(tm_, 3);
         const int s = fill % S, set = rowc & 1;
-        if (cur.tt == 0) item_no++;
+        if (ELEM || cur.tt == 0) item_no++;
         if (cur.it == cur.i0 && cur.tt == 0 && rowc >= 2) {    // first fill of a row: its accumulators were read out
           ok = wait(&s_accempty[set], (unsigned) ((rowc / 2 - 1) & 1));
           if (!ok) break;
@@ -335,8 +360,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) mv_tc_kernel(MVTCDev op, const Te
         const unsigned b_hi = smem_u32(W_st + (size_t) (item_no % S) * 2 * W_BYTES);
         const unsigned long long dA[2] = {make_desc(a_hi, K), make_desc(a_hi + A_BYTES, K)};
         const unsigned long long dB[2] = {make_desc(b_hi, K), make_desc(b_hi + W_BYTES, K)};
-        const unsigned d = tmem + (unsigned) ((set * TB + cur.tt) * N);
-        const bool acc0 = cur.it != cur.i0;
+        const int sub = ELEM ? (cur.it - cur.i0) % op.sub : 0;
+        const unsigned d = tmem + (unsigned) (((set * TB + cur.tt) * op.sub + sub) * N);
+        const bool acc0 = ELEM ? cur.it - cur.i0 >= op.sub : cur.it != cur.i0;
 #pragma unroll
         for (int pass = 0; pass < 3; pass++) {    // small terms first: a_lo b_hi, a_hi b_lo, a_hi b_hi
           const unsigned long long a = dA[pass == 0 ? 1 : 0], b = dB[pass == 1 ? 1 : 0];
@@ -367,7 +393,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) mv_tc_kernel(MVTCDev op, const Te
     const int ew = warp & 3;    // the quarter of the tensor-memory lanes this warp may read (warp id modulo 4)
     float *tr = tr_all + ew * (32 * (CB + 4));
     constexpr int LPR = CB / 4, RPI = 32 / LPR;    // lanes per atom row, atom rows per store instruction
-    const TensorDev dstT = s_T[op.dst];
     Cursor cur;
     start(cur, blockIdx.x * TB, blockIdx.y);
     int rowc = 0;
@@ -381,44 +406,69 @@ __global__ void __launch_bounds__(NTHREADS, 1) mv_tc_kernel(MVTCDev op, const Te
       if (!ok) break;
       GB_TICK(te_, 0);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int orow = s_row_out[cur.row], nblk = N / CB;
-      const int nb = cur.nt * nblk;
-      // the old values of an accumulating operation are fetched one block ahead of the block being written
+      const MVRowDev row = s_rows[cur.row];
+      const TensorDev dstT = s_T[row.dst];
+      float *const out = dstT.p + (size_t) row.out * NA * dstT.C;
+      const int nblk = N / CB, nb = cur.nt * nblk;
+      const bool vec = ((dstT.C | row.n_out) & 3) == 0;
+      // atom of row r of this warp's quarter of tile tt, -1: none
+      auto atom_of = [&](int tt, int r) {
+        const int at = (cur.tile0 + tt) * TM + ew * 32 + r;
+        return ELEM ? __ldg(op.order + at) : at < na ? at : -1;
+      };
+      // the old values of an accumulating row are fetched one block ahead of the block being written
       float4 old[32 / RPI], oldn[32 / RPI];
       auto load_old = [&](int b, float4 (&o)[32 / RPI]) {
-        const int tt = b / nblk, c0 = (b - tt * nblk) * CB, atom0 = (cur.tile0 + tt) * TM + ew * 32;
+        const int tt = b / nblk, c0 = (b - tt * nblk) * CB;
 #pragma unroll
         for (int j = 0; j < 32 / RPI; j++) {
-          const int r = j * RPI + lane / LPR, cq = lane % LPR;
-          o[j] = (b < nb && atom0 + r < na) ? __ldcg(reinterpret_cast<const float4 *>(dstT.p + ((size_t) orow * NA + atom0 + r) * dstT.C + c0) + cq)
-                                            : make_float4(0.f, 0.f, 0.f, 0.f);
+          const int cq = lane % LPR, a = b < nb && c0 + 4 * cq < row.n_out ? atom_of(tt, j * RPI + lane / LPR) : -1;
+          o[j] = a >= 0 ? __ldcg(reinterpret_cast<const float4 *>(out + (size_t) a * dstT.C + c0) + cq) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
       };
-      if (op.accumulate) load_old(0, oldn);
+      if (row.accumulate && vec) load_old(0, oldn);
       for (int b = 0; b < nb; b++) {
         const int tt = b / nblk, c0 = (b - tt * nblk) * CB;
         float v[CB];
-        tmem_ld<CB>(tmem + ((unsigned) (ew * 32) << 16) + (unsigned) ((set * TB + tt) * N + c0), v);
+        const unsigned at = tmem + ((unsigned) (ew * 32) << 16) + (unsigned) ((set * TB + tt) * op.sub * N + c0);
+        tmem_ld<CB>(at, v);
+        if (ELEM)
+          for (int k = 1; k < min(op.sub, row.i1 - row.i0); k++) {    // the other accumulators of the row
+            float w[CB];
+            tmem_ld<CB>(at + (unsigned) (k * N), w);
+#pragma unroll
+            for (int q = 0; q < CB; q++) v[q] += w[q];
+          }
         __syncwarp();
 #pragma unroll
         for (int q = 0; q < CB / 4; q++)
           *reinterpret_cast<float4 *>(tr + lane * (CB + 4) + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
         __syncwarp();
-        const int atom0 = (cur.tile0 + tt) * TM + ew * 32;
-        if (op.accumulate) {
+        if (!vec) {    // rows of a width that is no multiple of 4: value by value
+          const int w = min(CB, row.n_out - c0);
+          for (int e = lane; e < 32 * w; e += 32) {
+            const int r = e / w, c = e - r * w, a = atom_of(tt, r);
+            if (a < 0) continue;
+            float *o = out + (size_t) a * dstT.C + c0 + c;
+            const float x = tr[r * (CB + 4) + c];
+            *o = row.accumulate ? *o + x : x;
+          }
+          continue;
+        }
+        if (row.accumulate) {
 #pragma unroll
           for (int j = 0; j < 32 / RPI; j++) old[j] = oldn[j];
           load_old(b + 1, oldn);
         }
 #pragma unroll
         for (int j = 0; j < 32 / RPI; j++) {
-          const int r = j * RPI + lane / LPR, cq = lane % LPR;
-          if (atom0 + r < na) {
+          const int r = j * RPI + lane / LPR, cq = lane % LPR, a = c0 + 4 * cq < row.n_out ? atom_of(tt, r) : -1;
+          if (a >= 0) {
             float4 w = *reinterpret_cast<const float4 *>(tr + r * (CB + 4) + 4 * cq);
-            if (op.accumulate) {
+            if (row.accumulate) {
               w.x += old[j].x; w.y += old[j].y; w.z += old[j].z; w.w += old[j].w;
             }
-            reinterpret_cast<float4 *>(dstT.p + ((size_t) orow * NA + atom0 + r) * dstT.C + c0)[cq] = w;
+            reinterpret_cast<float4 *>(out + (size_t) a * dstT.C + c0)[cq] = w;
           }
         }
       }
@@ -448,122 +498,304 @@ size_t smem_bytes(int K, int N, int S)
 
 int stages_for(int K, int N) { return smem_bytes(K, N, 4) <= 200 * 1024 ? 4 : 2; }
 
-template<int K, int CB, int S>
+template<int K, int CB, int S, bool ELEM>
 void launch_s(const MVTCDev &op, const TensorDev *T, int ntensors, int NA, int na, int TB, int tmem_cols, dim3 grid, int *error)
 {
-  const size_t smem = smem_bytes(K, op.n_out, S);
+  const size_t smem = smem_bytes(K, op.N, S);
   static size_t attr = 0;
   if (smem > attr) {
-    GB_CUDA(cudaFuncSetAttribute((mv_tc_kernel<K, CB, S>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+    GB_CUDA(cudaFuncSetAttribute((mv_tc_kernel<K, CB, S, ELEM>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
     attr = smem;
   }
-  GB_LAUNCH((mv_tc_kernel<K, CB, S>), grid, NTHREADS, smem, op, T, ntensors, NA, na, TB, tmem_cols, error);
+  const char *name = ELEM ? "mv_tc_element_kernel" : "mv_tc_kernel";
+  before_launch(name);
+  mv_tc_kernel<K, CB, S, ELEM><<<grid, NTHREADS, smem, dev().stream>>>(op, T, ntensors, NA, na, TB, tmem_cols, error);
+  after_launch(name);
 }
 
-template<int K> void launch_k(const MVTCDev &op, const TensorDev *T, int ntensors, int NA, int na, int TB, dim3 grid, int *error)
+template<int K, bool ELEM> void launch_k(const MVTCDev &op, const TensorDev *T, int ntensors, int NA, int na, int TB, dim3 grid, int *error)
 {
   int tmem_cols = 32;    // a power of two that holds two sets of accumulators of TB tiles
-  while (tmem_cols < 2 * TB * op.n_out) tmem_cols *= 2;
-  const bool s4 = stages_for(K, op.n_out) == 4;
-  if (op.n_out % 32 == 0) {
-    if (s4) launch_s<K, 32, 4>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
-    else launch_s<K, 32, 2>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+  while (tmem_cols < 2 * TB * op.sub * op.N) tmem_cols *= 2;
+  const bool s4 = stages_for(K, op.N) == 4;
+  if (op.N % 32 == 0) {
+    if (s4) launch_s<K, 32, 4, ELEM>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+    else launch_s<K, 32, 2, ELEM>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
   } else {
-    if (s4) launch_s<K, 16, 4>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
-    else launch_s<K, 16, 2>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+    if (s4) launch_s<K, 16, 4, ELEM>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+    else launch_s<K, 16, 2, ELEM>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
   }
+}
+
+template<bool ELEM> void launch_e(int K, const MVTCDev &op, const TensorDev *T, int ntensors, int NA, int na, int TB, dim3 grid, int *error)
+{
+  switch (K) {
+    case 16: launch_k<16, ELEM>(op, T, ntensors, NA, na, TB, grid, error); break;
+    case 32: launch_k<32, ELEM>(op, T, ntensors, NA, na, TB, grid, error); break;
+    case 64: launch_k<64, ELEM>(op, T, ntensors, NA, na, TB, grid, error); break;
+    default: throw DeviceError("tensor-core FC: unsupported input width");
+  }
+}
+
+// operand images of the matrices of an operation: B[n][k] = W[k][n], hi (rounded to tf32) then lo, zero beyond the matrix;
+// grid (matrices, elements)
+__global__ void __launch_bounds__(256) mv_images_kernel(const float *__restrict__ W, const int4 *__restrict__ mats, long long ty_stride,
+                                                        int K, int N, char *images, int nmat, int first)
+{
+  const int4 m = mats[blockIdx.x];    // offset, rows, row stride, columns
+  const float *M = W + (long long) blockIdx.y * ty_stride + m.x;
+  char *o = images + ((size_t) blockIdx.y * nmat + first + blockIdx.x) * 2 * N * K * 4;
+  for (int e = threadIdx.x; e < N * K; e += 256) {
+    const int n = e / K, k = e - n * K;
+    const float w = k < m.y && n < m.w ? M[(long long) k * m.z + n] : 0.0f;
+    const unsigned h = (__float_as_uint(w) + 0x1000u) & 0xffffe000u;    // nearest tf32 (10-bit mantissa)
+    const unsigned l = (__float_as_uint(w - __uint_as_float(h)) + 0x1000u) & 0xffffe000u;
+    const int at = tile_off(n, k, K);
+    *reinterpret_cast<unsigned *>(o + at) = h;
+    *reinterpret_cast<unsigned *>(o + (size_t) N * K * 4 + at) = l;
+  }
+}
+
+// Atoms by element, every element padded to whole tiles.  order [tiles x 128]: atom or -1; tiles: their number, then the
+// element of each.  One block, no barrier per atom: a warp owns a stretch of the atoms, counts its elements, and after a scan
+// over the warps hands out its places in order (lanes that hold the same element take consecutive ones).
+constexpr int ORDER_EL = 256;    // most elements
+__global__ void __launch_bounds__(1024) elem_order_kernel(const int *__restrict__ mu, int na, int nel, int tiles_max, int *order, int *tiles)
+{
+  extern __shared__ int cnt[];    // [32 warps][nel]: counts, then the next place of the warp
+  __shared__ int at[ORDER_EL + 1];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, seg = (na + 1023) / 1024 * 32;
+  const int a_lo = warp * seg, a_hi = min(na, a_lo + seg);
+  for (int q = t; q < 32 * nel; q += 1024) cnt[q] = 0;
+  for (int q = t; q < tiles_max * TM; q += 1024) order[q] = -1;
+  __syncthreads();
+  for (int a = a_lo + lane; a < a_hi; a += 32) atomicAdd(&cnt[warp * nel + mu[a]], 1);
+  __syncthreads();
+  for (int e = t; e < nel; e += 1024) {
+    int n = 0;
+    for (int w = 0; w < 32; w++) {
+      const int c = cnt[w * nel + e];
+      cnt[w * nel + e] = n;
+      n += c;
+    }
+    at[e] = (n + TM - 1) / TM;
+  }
+  __syncthreads();
+  if (t == 0) {
+    int tile = 0;
+    for (int e = 0; e < nel; e++) {
+      const int k = at[e];
+      at[e] = tile;
+      tile += k;
+    }
+    at[nel] = tile;
+    tiles[0] = min(tile, tiles_max);
+  }
+  __syncthreads();
+  for (int e = t; e < nel; e += 1024)
+    for (int k = at[e]; k < min(at[e + 1], tiles_max); k++) tiles[1 + k] = e;
+  for (int a0 = a_lo; a0 < a_hi; a0 += 32) {
+    const int a = a0 + lane, e = a < a_hi ? mu[a] : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, e);
+    const int lead = __ffs(same) - 1;
+    int base = 0;
+    if (e >= 0 && lane == lead) {
+      base = cnt[warp * nel + e];
+      cnt[warp * nel + e] = base + __popc(same);
+    }
+    base = __shfl_sync(0xffffffffu, base, lead);
+    const int place = e < 0 ? tiles_max * TM : at[e] * TM + base + __popc(same & ((1u << lane) - 1u));
+    if (place < tiles_max * TM) order[place] = a;
+    __syncwarp();
+  }
+}
+
+// the same for many atoms: counts and places by blocks of 1024 atoms
+__global__ void __launch_bounds__(1024) elem_count_kernel(const int *__restrict__ mu, int na, int nel, int *count)
+{
+  __shared__ int cnt[ORDER_EL];
+  const int t = threadIdx.x, a = blockIdx.x * 1024 + t;
+  for (int e = t; e < nel; e += 1024) cnt[e] = 0;
+  __syncthreads();
+  if (a < na) atomicAdd(&cnt[mu[a]], 1);
+  __syncthreads();
+  for (int e = t; e < nel; e += 1024)
+    if (cnt[e]) atomicAdd(count + e, cnt[e]);
+}
+__global__ void __launch_bounds__(1024) elem_tiles_kernel(int *count, int nel, int tiles_max, int *tiles)
+{
+  __shared__ int at[ORDER_EL + 1];
+  if (threadIdx.x == 0) {
+    int tile = 0;
+    for (int e = 0; e < nel; e++) {
+      at[e] = tile;
+      tile += (count[e] + TM - 1) / TM;
+    }
+    at[nel] = tile;
+    tiles[0] = min(tile, tiles_max);
+  }
+  __syncthreads();
+  for (int e = 0; e < nel; e++)
+    for (int k = at[e] + threadIdx.x; k < min(at[e + 1], tiles_max); k += 1024) tiles[1 + k] = e;
+  for (int e = threadIdx.x; e < nel; e += 1024) count[e] = at[e] * TM;    // where the next atom of the element goes
+}
+__global__ void __launch_bounds__(1024) elem_place_kernel(const int *__restrict__ mu, int na, int nel, int tiles_max, int *next, int *order)
+{
+  __shared__ int cnt[ORDER_EL], base[ORDER_EL];
+  const int t = threadIdx.x, a = blockIdx.x * 1024 + t;
+  for (int e = t; e < nel; e += 1024) cnt[e] = 0;
+  __syncthreads();
+  const int e = a < na ? mu[a] : 0;
+  int rank = 0;
+  if (a < na) rank = atomicAdd(&cnt[e], 1);
+  __syncthreads();
+  for (int q = t; q < nel; q += 1024)
+    if (cnt[q]) base[q] = atomicAdd(next + q, cnt[q]);
+  __syncthreads();
+  if (a < na && base[e] + rank < tiles_max * TM) order[base[e] + rank] = a;
 }
 
 }    // namespace
 
-bool MVTensorCore::eligible(const MVOp &o, const std::vector<TensorSpec> &tensors)
+void ElemOrder::make(const int *mu, int na, int nel, int kinds)
 {
-  if (o.elem || o.items.empty() || o.row_out.empty()) return false;
-  if ((int) tensors.size() > MAX_TENSORS || (int) o.items.size() > MAX_ITEMS || (int) o.row_out.size() > MAX_ROWS) return false;
-  const int K = o.items[0].n_in;
-  if (K != 8 && K != 16 && K != 32 && K != 64) return false;
-  if (o.n_out % 16 != 0 || o.n_out < 16 || o.n_out > 256) return false;
-  if (tensors[o.dst].channels % 4 != 0 || tensors[o.dst].channels < o.n_out) return false;
-  for (const MVItem &it : o.items)
-    if (it.n_in != K || tensors[it.src].channels % 4 != 0 || tensors[it.src].channels < K) return false;
-  for (size_t r = 0; r + 1 < o.item_off.size(); r++)
-    if (o.item_off[r + 1] == o.item_off[r]) return false;    // a row without items has no accumulator to write
-  return smem_bytes(K, o.n_out, 2) <= 220 * 1024;
+  if (nel > ORDER_EL) throw Unsupported("models with more than 256 elements are not supported");
+  tiles_max = (na + TM - 1) / TM + std::min(kinds, na);
+  order_.set_label("nlist:element_order");
+  tiles_.set_label("nlist:element_order");
+  order_.ensure((size_t) tiles_max * TM);
+  tiles_.ensure((size_t) tiles_max + 1);
+  if (na <= 8192) {    // one block of 10 us against four launches
+    GB_LAUNCH(elem_order_kernel, 1, 1024, sizeof(int) * 32 * nel, mu, na, nel, tiles_max, order_.get(), tiles_.get());
+    return;
+  }
+  next_.set_label("nlist:element_order");
+  next_.ensure(ORDER_EL);
+  GB_CUDA(cudaMemsetAsync(next_.get(), 0, sizeof(int) * ORDER_EL, dev().stream));
+  GB_CUDA(cudaMemsetAsync(order_.get(), 0xff, sizeof(int) * (size_t) tiles_max * TM, dev().stream));
+  const int nb = (na + 1023) / 1024;
+  GB_LAUNCH(elem_count_kernel, nb, 1024, 0, mu, na, nel, next_.get());
+  GB_LAUNCH(elem_tiles_kernel, 1, 1024, 0, next_.get(), nel, tiles_max, tiles_.get());
+  GB_LAUNCH(elem_place_kernel, nb, 1024, 0, mu, na, nel, tiles_max, next_.get(), order_.get());
 }
 
-void MVTensorCore::setup(const MVOp &o)
+int MVTensorCore::padded_k(const MVOp &o)
 {
-  K_ = o.items[0].n_in;
-  const int N = o.n_out, K = K_;
-  // one operand image per distinct matrix: B[n][k] = W[k][n] as tf32 hi, then lo (canonical K-major layout)
-  std::map<int, int> index;
-  std::vector<char> img;
-  std::vector<MVItem> items = o.items;
-  for (MVItem &it : items) {
-    auto f = index.find(it.mat);
-    if (f == index.end()) {
-      const int id = (int) index.size();
-      f = index.emplace(it.mat, id).first;
-      std::vector<char> hi((size_t) N * K * 4, 0), lo((size_t) N * K * 4, 0);
-      for (int n = 0; n < N; n++)
-        for (int k = 0; k < K; k++) {
-          const float w = o.W[(size_t) it.mat + (size_t) k * o.ldw + n];
-          unsigned u;
-          std::memcpy(&u, &w, 4);
-          u = (u + 0x1000u) & 0xffffe000u;    // round to nearest tf32 (10-bit mantissa)
-          float h;
-          std::memcpy(&h, &u, 4);
-          const float r = w - h;
-          unsigned v;
-          std::memcpy(&v, &r, 4);
-          v = (v + 0x1000u) & 0xffffe000u;
-          std::memcpy(hi.data() + tile_off(n, k, K), &u, 4);
-          std::memcpy(lo.data() + tile_off(n, k, K), &v, 4);
-        }
-      img.insert(img.end(), hi.begin(), hi.end());
-      img.insert(img.end(), lo.begin(), lo.end());
-    }
-    it.mat = f->second;    // image index instead of the offset in the fp32 weights
+  int k = 0;
+  for (const MVItem &it : o.items) k = std::max(k, it.n_in);
+  return k <= 16 ? 16 : k <= 32 ? 32 : k <= 64 ? 64 : 0;
+}
+
+bool MVTensorCore::eligible(const MVOp &o, const std::vector<TensorSpec> &tensors)
+{
+  if (o.items.empty() || o.row_out.empty()) return false;
+  if ((int) tensors.size() > MAX_TENSORS || (int) o.items.size() > MAX_ITEMS || (int) o.row_out.size() > MAX_ROWS) return false;
+  const int K = padded_k(o), N = padded_n(o.n_out);
+  if (K == 0 || N > 256) return false;
+  for (size_t r = 0; r + 1 < o.item_off.size(); r++)
+    if (o.item_off[r + 1] == o.item_off[r]) return false;    // a row without items has no accumulator to write
+  // beside the tables of an operation (17 KB of static shared memory)
+  return smem_bytes(K, N, 2) <= 211 * 1024;
+}
+
+void MVTensorCore::setup(const std::vector<const MVOp *> &ops, const std::vector<const float *> &W, int n_elements)
+{
+  K_ = N_ = 0;
+  elem_ = ops[0]->elem;
+  for (const MVOp *o : ops) {
+    K_ = std::max(K_, padded_k(*o));
+    N_ = std::max(N_, padded_n(o->n_out));
   }
+  // rows of all operations; a row that several of them write gets the items of all (the first decides whether it adds)
+  std::map<std::pair<int, int>, int> index;
+  std::vector<MVRowDev> rows;
+  std::vector<std::vector<MVItem>> row_items;
+  std::vector<std::vector<int4>> mats(ops.size());
+  int first = 0;
+  for (size_t q = 0; q < ops.size(); q++) {
+    const MVOp &o = *ops[q];
+    std::map<int, int> image;    // distinct matrices of the operation
+    for (size_t r = 0; r < o.row_out.size(); r++) {
+      auto key = std::make_pair(o.dst, o.row_out[r]);
+      auto f = index.find(key);
+      if (f == index.end()) {
+        f = index.emplace(key, (int) rows.size()).first;
+        rows.push_back(MVRowDev{(short) o.dst, (short) o.row_out[r], (short) (o.accumulate ? 1 : 0), (short) o.n_out, 0, 0});
+        row_items.emplace_back();
+      }
+      for (int i = o.item_off[r]; i < o.item_off[r + 1]; i++) {
+        MVItem it = o.items[i];
+        auto g = image.find(it.mat);
+        if (g == image.end()) {
+          g = image.emplace(it.mat, first + (int) mats[q].size()).first;
+          mats[q].push_back(make_int4(it.mat, it.n_in, o.ldw, o.n_out));
+        }
+        it.mat = g->second;    // image index instead of the offset in the fp32 weights
+        row_items[f->second].push_back(it);
+      }
+    }
+    first += (int) mats[q].size();
+  }
+  nmat_ = first;
+  std::vector<MVItem> items;
+  for (size_t r = 0; r < rows.size(); r++) {
+    rows[r].i0 = (int) items.size();
+    items.insert(items.end(), row_items[r].begin(), row_items[r].end());
+    rows[r].i1 = (int) items.size();
+  }
+  nrows_ = (int) rows.size();
+  nitems_ = (int) items.size();
   images_.set_label("engine:weights_tf32");
   items_.set_label("engine:tables");
-  images_.ensure(img.size());
-  GB_CUDA(cudaMemcpyAsync(images_.get(), img.data(), img.size(), cudaMemcpyHostToDevice, dev().stream));
+  rows_.set_label("engine:tables");
+  const int ne = elem_ ? n_elements : 1;
+  images_.ensure((size_t) ne * nmat_ * 2 * N_ * K_ * 4);
   items_.upload(items);
-  nitems_ = (int) items.size();
-  GB_CUDA(cudaStreamSynchronize(dev().stream));
+  rows_.upload(rows);
+  first = 0;
+  DBuf<int4> d;
+  for (size_t q = 0; q < ops.size(); q++) {
+    d.upload(mats[q]);
+    GB_LAUNCH(mv_images_kernel, dim3((unsigned) mats[q].size(), ne), 256, 0, W[q], d.get(), (long long) ops[q]->ty_stride, K_, N_,
+              images_.get(), nmat_, first);
+    first += (int) mats[q].size();
+    GB_CUDA(cudaStreamSynchronize(dev().stream));
+  }
   ready_ = true;
 }
 
-void MVTensorCore::launch(const MVDev &d, const TensorDev *tensors, int ntensors, int NA, int na, int *error) const
+void MVTensorCore::launch(const TensorDev *tensors, int ntensors, int NA, int na, int *error, const ElemOrder *order) const
 {
   if (!ready_) throw DeviceError("tensor-core FC used before its set-up");
-  if (d.nrows == 0 || na == 0) return;
+  if (nrows_ == 0 || na == 0) return;
   MVTCDev op{};
-  op.row_out = d.row_out;
-  op.item_off = d.item_off;
+  op.rows = rows_.get();
   op.items = items_.get();
   op.images = images_.get();
-  op.n_out = d.n_out;
-  op.nrows = d.nrows;
+  op.N = N_;
+  op.nrows = nrows_;
   op.nitems = nitems_;
-  op.accumulate = d.accumulate;
-  op.dst = d.dst;
+  op.nmat = nmat_;
+  int ntiles = (na + TM - 1) / TM;
+  if (elem_) {
+    if (!order) throw DeviceError("tensor-core FC: the order of the atoms by element is missing");
+    op.order = order->order_.get();
+    op.tiles = order->tiles_.get();
+    ntiles = order->tiles_max;
+  }
   // one CTA per SM; two sets of accumulators share the 512 tensor-memory columns
-  const int ntiles = (na + TM - 1) / TM, G = dev().sm_count;
-  const int tb_max = std::max(1, std::min(MAX_TILES, TMEM_COLS / 2 / d.n_out));
+  const int G = dev().sm_count;
+  // The rows of reduces over the element are sums of up to 89 items.  The tensor cores cut off what they add (towards zero,
+  // one bit of 2^-24 per instruction and accumulator), which over hundreds of instructions becomes a bias of 1e-5: such a row
+  // spreads its items over as many accumulators as there are columns for, and the epilogue adds them with rounding.
+  op.sub = elem_ ? std::max(1, std::min(16, TMEM_COLS / 2 / N_)) : 1;
+  const int tb_max = elem_ ? 1 : std::max(1, std::min(MAX_TILES, TMEM_COLS / 2 / N_));
   const int rounds = (ntiles + G * tb_max - 1) / (G * tb_max);
   const int TB = std::max(1, std::min(tb_max, (ntiles + G * rounds - 1) / (G * rounds)));
   const int gx = std::min(G, (ntiles + TB - 1) / TB);
-  const int gy = std::max(1, std::min(d.nrows, G / gx));
-  const dim3 grid(gx, gy);
-  switch (K_) {
-    case 8: launch_k<8>(op, tensors, ntensors, NA, na, TB, grid, error); break;
-    case 16: launch_k<16>(op, tensors, ntensors, NA, na, TB, grid, error); break;
-    case 32: launch_k<32>(op, tensors, ntensors, NA, na, TB, grid, error); break;
-    case 64: launch_k<64>(op, tensors, ntensors, NA, na, TB, grid, error); break;
-    default: throw DeviceError("tensor-core FC: unsupported input width");
-  }
+  const int gy = std::max(1, std::min(nrows_, G / gx));
+  if (elem_) launch_e<true>(K_, op, tensors, ntensors, NA, na, TB, dim3(gx, gy), error);
+  else launch_e<false>(K_, op, tensors, ntensors, NA, na, TB, dim3(gx, gy), error);
 }
 
 }    // namespace gb

@@ -561,6 +561,7 @@ void NeighborList::build(int nsys, const int *natoms, int64_t n, const double *d
   n_ = 0;
   nslots_ = 0;
   nsys_ = nsys;
+  orders_.clear();
   st_.assign(nsys, NLStructHost{});
   std::vector<double> heights(3 * (size_t) nsys);
   int64_t at = 0;
@@ -750,6 +751,7 @@ void NeighborList::adopt(int nlocal, int nall, const int *d_mu, const int *d_num
   const int64_t n = nall;
   nsys_ = 1;
   external_ = true;
+  orders_.clear();
   st_.assign(1, NLStructHost{});
   NLStructHost &S = st_[0];
   const double eye[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
@@ -840,8 +842,18 @@ void NeighborList::export_host(std::vector<int> &bi, std::vector<int> &bj, std::
     }
 }
 
+const ElemOrder &NeighborList::element_order(const int *mu, int64_t a0, int na, int nel)
+{
+  for (const OrderOf &o : orders_)
+    if (o.mu == mu && o.a0 == a0 && o.na == na) return *o.order;
+  orders_.push_back(OrderOf{mu, a0, na, std::make_unique<ElemOrder>()});
+  orders_.back().order->make(mu, na, nel, std::min(kinds_, nel));
+  return *orders_.back().order;
+}
+
 void NeighborList::release()
 {
+  orders_.clear();
   frac_.release(); xs_.release(); xbuild_.release(); lohi_.release(); img_.release(); img_s_.release();
   sid_.release(); sid_s_.release(); binid_.release(); b3_s_.release(); count_.release();
   members_.release(); perm_.release(); mu_s_.release(); cnt_full_.release(); cnt_.release(); nbr_j_.release();

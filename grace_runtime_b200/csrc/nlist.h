@@ -9,7 +9,9 @@
 
 #include "device.h"
 #include "kernels.h"
+#include "mv_tc.h"
 
+#include <memory>
 #include <vector>
 
 namespace gb {
@@ -51,6 +53,10 @@ class NeighborList {
   // device: two error words, [0] raised by prepare() (2: a bond of length 0), [1] by the build (4: no reverse bond)
   const int *flag() const { return flag_.get(); }
   const double *build_positions() const { return xbuild_.get(); }    // device: the caller's positions of the last build
+  // most different elements among the atoms (the species of the System or Batch)
+  void set_kinds(int kinds) { kinds_ = kinds; }
+  // the atoms [0, na) of a chunk with elements mu (device), grouped by element; made once per list and chunk
+  const ElemOrder &element_order(const int *mu, int64_t a0, int na, int nel);
   void release();
   size_t bytes() const;
   // diagnostics: the list of the last build (radius cutoff + skin) on the host, in the caller's atom order and frame:
@@ -58,6 +64,14 @@ class NeighborList {
   void export_host(std::vector<int> &bi, std::vector<int> &bj, std::vector<int> &bS) const;
 
  private:
+  struct OrderOf {
+    const int *mu;
+    int64_t a0;
+    int na;
+    std::unique_ptr<ElemOrder> order;
+  };
+  std::vector<OrderOf> orders_;    // of the present list
+  int kinds_ = 1 << 30;
   int64_t n_ = 0, nslots_ = 0;
   int nsys_ = 0;
   bool external_ = false;
