@@ -14,8 +14,6 @@
 // allocated the shares are added with fp32 atomics, as the reference does.
 #include "bond_common.cuh"
 
-#include <cstdlib>
-
 namespace gb {
 
 namespace {
@@ -221,146 +219,63 @@ __global__ void __launch_bounds__(128) bond_bwd_kernel(BondsDev b, LayerDev L, S
   }
 }
 
-// The same for layers that couple message functions in (NIT > 1) with at most 16 channels: a whole warp per bond, lane
-// = (channel n, half h) with the lm of the bond sums split between the halves (lm = 2 k + h), so that a lane keeps
-// NIT x NLM / 2 gradients in registers instead of NIT x NLM (twice the resident warps) and the two halves share the
-// work of a bond.  Per lm the lane forms h = sum_I msg_I gQ[I][lm] once; with R and dR/dx of the lm's degree
-// (selected per lm) everything is linear in h:
-//   dE/dx += dR_l Y_lm h,   g += R_l h grad Y_lm,   dE/dmsg_I += R_l Y_lm gQ[I][lm].
-template<int LMAX, int NIT>
-__global__ void __launch_bounds__(128) bond_bwd_split_kernel(BondsDev b, LayerDev L, SHTable sht, const float *__restrict__ gQ,
-                                                             int NA, int a0, float *__restrict__ fv,
-                                                             double *__restrict__ vir_atom, int add)
+// What the kernels with two channels per lane stage per bond.  A row holds (y y gx gx) (gy gy gz gz) per harmonic, an odd number
+// of 16-byte words so that the threads which write the rows of different bonds meet no bank conflict.
+template<int ROW, int EB> struct BwdStage {
+  float4 Y[EB][ROW];
+  float4 u[EB], fe[EB];    // rhat, r;  g, dE/dx
+  int4 meta[EB];           // interval, element, offset, neighbour
+  float scale[EB];         // intervals per length: N / rcut of the pair
+  int cs[EB];
+  double vred[4][6];
+};
+
+template<int LMAX, class S, class Place>
+__device__ __forceinline__ void bwd_stage(S &s, int e, const BondsDev &b, const LayerDev &L, const SHTable &sht, long long slot, int mui, Place place)
 {
-  constexpr int NL = LMAX + 1, NLM = NL * NL, NK = (NLM + 1) / 2;
-  __shared__ float4 YG[EBB][NLM];
-  __shared__ float su[EBB][4];     // rhat, r
-  __shared__ float srci[EBB], st[EBB];
-  __shared__ int sk[EBB], smu[EBB], sj[EBB], scs[EBB];
-  __shared__ float fe[EBB][4];     // g (3), dE/dx
-  __shared__ double vred[4][6];
+  const float4 rec = b.rec[slot];
+  const float r = sqrtf(rec.x * rec.x + rec.y * rec.y + rec.z * rec.z), ir = 1.0f / r;
+  const int j = __float_as_int(rec.w), muj = b.mu[j];
+  const float rc = L.rc[mui * L.n_elements + muj];
+  int k;
+  float t;
+  spline_locate(r / rc, L.N, k, t);
+  s.meta[e] = make_int4(k, muj, __float_as_int(t), j);
+  s.cs[e] = b.cslot[slot];
+  s.scale[e] = (float) L.N / rc;
+  s.u[e] = make_float4(rec.x * ir, rec.y * ir, rec.z * ir, r);
+  float4 *y = s.Y[e];
+  sph_harm<LMAX, true>(sht, rec.x * ir, rec.y * ir, rec.z * ir, [&](int lm, float v, float gx, float gy, float gz) {
+    const int at = place(lm);
+    y[2 * at] = make_float4(v, v, gx, gx);
+    y[2 * at + 1] = make_float4(gy, gy, gz, gz);
+  });
+}
 
-  const int a = blockIdx.x, i = b.ilist ? b.ilist[a0 + a] : a0 + a, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-  const int n = lane & 15, h = lane >> 4;
-  const long long base = b.off[i];
-  const int nb = b.cnt[i];
-  const int mui = b.mu[i];
-  const int C = L.C, nel = L.n_elements;
-  const float fN = (float) L.N;
-  double vir[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  // gradients of this lane's channel and lm's: g[I][k] = gQ[(I, 2 k + h)][n]
-  float g[NIT][NK];
-#pragma unroll
-  for (int I = 0; I < NIT; I++)
-#pragma unroll
-    for (int k = 0; k < NK; k++) {
-      const int q = 2 * k + h;
-      g[I][k] = (n < C && q < NLM && I <= L.n_msg) ? __ldg(gQ + ((size_t) (I * NLM + q) * NA + a) * C + n) : 0.0f;
-    }
+// bond force to its slot, virial of the bonds this thread finishes
+template<class S>
+__device__ __forceinline__ void bwd_finish(const S &s, int e, float *__restrict__ fv, int add, double (&vir)[6])
+{
+  const float4 u = s.u[e], g = s.fe[e];
+  const float dEdr = g.w * s.scale[e], gr = g.x * u.x + g.y * u.y + g.z * u.z, ir = 1.0f / u.w;
+  const float f0 = dEdr * u.x + (g.x - gr * u.x) * ir;
+  const float f1 = dEdr * u.y + (g.y - gr * u.y) * ir;
+  const float f2 = dEdr * u.z + (g.z - gr * u.z) * ir;
+  float *o = fv + 3 * (size_t) s.cs[e];
+  if (add) { o[0] += f0; o[1] += f1; o[2] += f2; }
+  else { o[0] = f0; o[1] = f1; o[2] = f2; }
+  const double dx = -(double) u.x * u.w, dy = -(double) u.y * u.w, dz = -(double) u.z * u.w;
+  vir[0] += dx * f0; vir[1] += dy * f1; vir[2] += dz * f2;
+  vir[3] += dx * f1; vir[4] += dx * f2; vir[5] += dy * f2;
+}
 
-  for (int b0 = 0; b0 < nb; b0 += EBB) {
-    const int nbat = min(EBB, nb - b0);
-    for (int e = tid; e < nbat; e += 128) {
-      const float4 rec = b.rec[base + b0 + e];
-      const float r = sqrtf(rec.x * rec.x + rec.y * rec.y + rec.z * rec.z), ir = 1.0f / r;
-      const int j = __float_as_int(rec.w);
-      const int muj = b.mu[j];
-      const float rc = L.rc[mui * nel + muj];
-      int k;
-      float t;
-      spline_locate(r / rc, L.N, k, t);
-      sk[e] = k; st[e] = t; smu[e] = muj; sj[e] = j;
-      scs[e] = b.cslot[base + b0 + e];
-      srci[e] = 1.0f / rc;
-      su[e][0] = rec.x * ir; su[e][1] = rec.y * ir; su[e][2] = rec.z * ir; su[e][3] = r;
-      float4 *yg = YG[e];
-      sph_harm<LMAX, true>(sht, rec.x * ir, rec.y * ir, rec.z * ir,
-                           [&](int lm, float v, float gx, float gy, float gz) { yg[lm] = make_float4(v, gx, gy, gz); });
-    }
-    __syncthreads();
-    for (int e = w; e < nbat; e += 4) {    // a warp per bond
-      float gx = 0.0f, gy = 0.0f, gz = 0.0f, dedx = 0.0f;
-      float gm[NIT];
-#pragma unroll
-      for (int I = 0; I < NIT; I++) gm[I] = 0.0f;
-      if (n < C) {
-        const int k0 = sk[e], muj = smu[e], j = sj[e];
-        const float t = st[e];
-        const float4 *yg = YG[e];
-        float R[NL], dR[NL];
-        const float4 *cf = reinterpret_cast<const float4 *>(L.tab) + (size_t) k0 * NL * C + n;
-#pragma unroll
-        for (int l = 0; l < NL; l++) {
-          const float4 c = __ldg(cf + l * C);
-          R[l] = c.x + t * (c.y + t * (c.z + t * c.w));
-          dR[l] = (c.y + t * (2.0f * c.z + t * 3.0f * c.w)) * fN;
-        }
-        float m[NIT];
-#pragma unroll
-        for (int I = 0; I < NIT; I++) {
-          m[I] = 0.0f;
-          if (I < L.n_msg) m[I] = __ldg(L.msg + ((size_t) j * L.n_msg + I) * C + n);
-          else if (I == L.n_msg) m[I] = __ldg(L.z + (size_t) muj * C + n);
-        }
-#pragma unroll
-        for (int k = 0; k < NK; k++) {
-          // degree of lm = 2 k (h = 0) and lm = 2 k + 1 (h = 1): compile-time constants, selected per lane
-          constexpr auto deg = [](int q) { int l = 0; while ((l + 1) * (l + 1) <= q) l++; return l; };
-          const int q = 2 * k + h;
-          const int l0 = deg(2 * k), l1 = deg(2 * k + 1 < NLM ? 2 * k + 1 : NLM - 1);
-          const float Rl = h ? R[l1] : R[l0], dRl = h ? dR[l1] : dR[l0];
-          if (q < NLM) {
-            const float4 y4 = yg[q];
-            float hq = 0.0f;
-#pragma unroll
-            for (int I = 0; I < NIT; I++) hq = fmaf(m[I], g[I][k], hq);
-            dedx = fmaf(dRl * y4.x, hq, dedx);
-            const float p = Rl * hq;
-            gx = fmaf(p, y4.y, gx);
-            gy = fmaf(p, y4.z, gy);
-            gz = fmaf(p, y4.w, gz);
-            const float ry = Rl * y4.x;
-#pragma unroll
-            for (int I = 0; I < NIT; I++) gm[I] = fmaf(ry, g[I][k], gm[I]);
-          }
-        }
-      }
-      // dE/dmsg: the two halves of a channel add up; force terms: all lanes
-#pragma unroll
-      for (int I = 0; I < NIT; I++) gm[I] += __shfl_xor_sync(0xffffffffu, gm[I], 16);
-      if (h == 0 && n < C) {
-#pragma unroll
-        for (int I = 0; I < NIT; I++)
-          if (I < L.n_msg) {
-            if (L.gmsg_slot) L.gmsg_slot[((size_t) scs[e] * L.n_msg + I) * C + n] = gm[I];
-            else atomicAdd(L.gmsg + ((size_t) sj[e] * L.n_msg + I) * C + n, gm[I]);
-          }
-      }
-      const float tot = group_sum4<32>(gx, gy, gz, dedx, lane);
-      if ((lane & 7) == 0) fe[e][lane >> 3] = tot;
-    }
-    __syncthreads();
-    for (int e = tid; e < nbat; e += 128) {
-      const float ux = su[e][0], uy = su[e][1], uz = su[e][2], r = su[e][3];
-      const float gxx = fe[e][0], gyy = fe[e][1], gzz = fe[e][2];
-      const float dEdr = fe[e][3] * srci[e];
-      const float gr = gxx * ux + gyy * uy + gzz * uz, ir = 1.0f / r;
-      const float f0 = dEdr * ux + (gxx - gr * ux) * ir;
-      const float f1 = dEdr * uy + (gyy - gr * uy) * ir;
-      const float f2 = dEdr * uz + (gzz - gr * uz) * ir;
-      float *o = fv + 3 * (size_t) scs[e];
-      if (add) { o[0] += f0; o[1] += f1; o[2] += f2; }
-      else { o[0] = f0; o[1] = f1; o[2] = f2; }
-      const double dx = -(double) ux * r, dy = -(double) uy * r, dz = -(double) uz * r;
-      vir[0] += dx * f0; vir[1] += dy * f1; vir[2] += dz * f2;
-      vir[3] += dx * f1; vir[4] += dx * f2; vir[5] += dy * f2;
-    }
-    __syncthreads();
-  }
+__device__ __forceinline__ void bwd_virial(double (&vred)[4][6], double (&vir)[6], double *__restrict__ vir_atom, int i, int add)
+{
+  const int tid = threadIdx.x;
 #pragma unroll
   for (int k = 0; k < 6; k++) {
     for (int s = 16; s > 0; s >>= 1) vir[k] += __shfl_xor_sync(0xffffffffu, vir[k], s);
-    if (lane == 0) vred[w][k] = vir[k];
+    if ((tid & 31) == 0) vred[tid >> 5][k] = vir[k];
   }
   __syncthreads();
   if (tid < 6) {
@@ -368,6 +283,206 @@ __global__ void __launch_bounds__(128) bond_bwd_split_kernel(BondsDev b, LayerDe
     double *o = vir_atom + 6 * (size_t) i + tid;
     *o = add ? *o + v : v;
   }
+}
+
+// bonds per round: the 78 of a dense metal inside 6 Angstrom at lmax 3, four or five blocks per SM
+template<int LMAX> __host__ __device__ constexpr int bwd_bonds() { return LMAX <= 3 ? 80 : 64; }
+template<int LMAX> using PairStage = BwdStage<2 * (LMAX + 1) * (LMAX + 1) + 1, bwd_bonds<LMAX>()>;
+template<int LMAX> using MsgStage = BwdStage<4 * LmSplit<LMAX>::NK + 1, bwd_bonds<LMAX>()>;
+
+// Layers without message functions and with an even number of channels: LPB lanes per bond, two channels per lane, 32 / LPB
+// bonds per warp at a time, with the gradients of its channels in a lane's registers.  With the chemical weight folded into
+// the radial functions a harmonic costs four packed FMAs per lane and bond.
+template<int LMAX, int LPB>
+__global__ void __launch_bounds__(128) bond_bwd_pair_kernel(BondsDev b, LayerDev L, SHTable sht, const float *__restrict__ gQ, int NA, int a0,
+                                                            float *__restrict__ fv, double *__restrict__ vir_atom, int add)
+{
+  constexpr int NL = LMAX + 1, NLM = NL * NL, BPW = 32 / LPB, EB = bwd_bonds<LMAX>();
+  extern __shared__ __align__(16) char smem[];
+  PairStage<LMAX> &s = *reinterpret_cast<PairStage<LMAX> *>(smem);
+  const int a = blockIdx.x, i = b.ilist ? b.ilist[a0 + a] : a0 + a, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const int c = lane % LPB, sub = lane / LPB;
+  const long long base = b.off[i];
+  const int nb = b.cnt[i], mui = b.mu[i], C = L.C, C2 = C >> 1;
+  const int rounds = max(1, (nb + EB - 1) / EB), per = (nb + rounds - 1) / rounds;
+  double vir[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  float2 g[NLM];
+#pragma unroll
+  for (int q = 0; q < NLM; q++)
+    g[q] = c < C2 ? __ldg(reinterpret_cast<const float2 *>(gQ + ((size_t) q * NA + a) * C) + c) : make_float2(0.f, 0.f);
+
+  for (int b0 = 0; b0 < nb; b0 += per) {
+    const int nbat = min(per, nb - b0);
+    for (int e = tid; e < nbat; e += 128) bwd_stage<LMAX>(s, e, b, L, sht, base + b0 + e, mui, [](int lm) { return lm; });
+    __syncthreads();
+    for (int e0 = w * BPW; e0 < nbat; e0 += 4 * BPW) {
+      const int e = e0 + sub;
+      float2 gx = make_float2(0.f, 0.f), gy = gx, gz = gx, dedx = gx;
+      if (e < nbat && c < C2) {
+        const int4 m = s.meta[e];
+        const float tt = __int_as_float(m.z);
+        const float2 t = pair_of(tt), t_2 = pair_of(2.0f * tt), t_15 = pair_of(1.5f * tt);
+        const float4 *cf = reinterpret_cast<const float4 *>(L.tab) + (size_t) m.x * NL * C + c;
+        const float2 z = __ldg(reinterpret_cast<const float2 *>(L.z + (size_t) m.y * C) + c);
+        const float4 *y = s.Y[e];
+#pragma unroll
+        for (int l = 0; l < NL; l++) {
+          const float4 xy = __ldg(cf + l * C), zw = __ldg(cf + l * C + C2);
+          float2 T = make_float2(0.f, 0.f), vx = T, vy = T, vz = T;
+#pragma unroll
+          for (int q = l * l; q < (l + 1) * (l + 1); q++) {
+            const float4 A = y[2 * q], B = y[2 * q + 1];
+            T = __ffma2_rn(lo2(A), g[q], T);
+            vx = __ffma2_rn(hi2(A), g[q], vx);
+            vy = __ffma2_rn(lo2(B), g[q], vy);
+            vz = __ffma2_rn(hi2(B), g[q], vz);
+          }
+          const float2 R = pair_value(xy, zw, t);
+          dedx = __ffma2_rn(T, pair_slope(xy, zw, t_2, t_15), dedx);
+          gx = __ffma2_rn(R, vx, gx);
+          gy = __ffma2_rn(R, vy, gy);
+          gz = __ffma2_rn(R, vz, gz);
+        }
+        gx = __fmul2_rn(gx, z);
+        gy = __fmul2_rn(gy, z);
+        gz = __fmul2_rn(gz, z);
+        dedx = __fmul2_rn(dedx, z);
+      }
+      const float tot = group_sum4<LPB>(gx.x + gx.y, gy.x + gy.y, gz.x + gz.y, dedx.x + dedx.y, c);
+      if (e < nbat && (c & (LPB / 4 - 1)) == 0) reinterpret_cast<float *>(s.fe + e)[c / (LPB / 4)] = tot;
+    }
+    __syncthreads();
+    for (int e = tid; e < nbat; e += 128) bwd_finish(s, e, fv, add, vir);
+    __syncthreads();
+  }
+  bwd_virial(s.vred, vir, vir_atom, i, add);
+}
+
+// Layers with four message functions and at most 16 channels (an even number): 16 lanes per bond, lane = (group h of
+// harmonics, channel pair c), two bonds per warp at a time; the gradients of 5 message functions x NK harmonics x two channels
+// in a lane's registers.  Per harmonic the lane forms h = sum_I msg_I gQ[I][lm] once; with R and dR/dx of the harmonic's degree
+// everything is linear in h:
+//   dE/dx += dR_l Y_lm h,   g += R_l h grad Y_lm,   dE/dmsg_I += R_l Y_lm gQ[I][lm].
+// One channel per lane took 447 issued instructions per bond and was bound by them.
+template<int LMAX>
+__global__ void __launch_bounds__(128) bond_bwd_msg_kernel(BondsDev b, LayerDev L, SHTable sht, const float *__restrict__ gQ, int NA, int a0,
+                                                           float *__restrict__ fv, double *__restrict__ vir_atom, int add)
+{
+  using SP = LmSplit<LMAX>;
+  constexpr int NL = LMAX + 1, NLM = NL * NL, NI = 5, NK = SP::NK, EB = bwd_bonds<LMAX>();
+  extern __shared__ __align__(16) char smem[];
+  MsgStage<LMAX> &s = *reinterpret_cast<MsgStage<LMAX> *>(smem);
+  const int a = blockIdx.x, i = b.ilist ? b.ilist[a0 + a] : a0 + a, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const int c = lane & 7, h = (lane >> 3) & 1, sub = lane >> 4;
+  const long long base = b.off[i];
+  const int nb = b.cnt[i], mui = b.mu[i], C = L.C, C2 = C >> 1;
+  const int rounds = max(1, (nb + EB - 1) / EB), per = (nb + rounds - 1) / rounds;
+  double vir[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  float2 g[NI][NK];
+#pragma unroll
+  for (int k = 0; k < NK; k++) {
+    const int q = h ? SP::lm(1, k) : SP::lm(0, k);
+#pragma unroll
+    for (int I = 0; I < NI; I++)
+      g[I][k] = q >= 0 && c < C2 ? __ldg(reinterpret_cast<const float2 *>(gQ + ((size_t) (I * NLM + q) * NA + a) * C) + c)
+                                 : make_float2(0.f, 0.f);
+  }
+
+  for (int b0 = 0; b0 < nb; b0 += per) {
+    const int nbat = min(per, nb - b0);
+    for (int e = tid; e < nbat; e += 128) {
+      constexpr LmPlaces<LMAX> places;
+      bwd_stage<LMAX>(s, e, b, L, sht, base + b0 + e, mui, [&](int lm) { return places.v[lm]; });
+#pragma unroll
+      for (int hk = 0; hk < 2 * NK; hk++)    // positions without a harmonic
+        if (SP::lm(hk / NK, hk % NK) < 0) s.Y[e][2 * hk] = s.Y[e][2 * hk + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+    for (int e0 = 2 * w; e0 < nbat; e0 += 8) {
+      const int e = e0 + sub;
+      const bool work = e < nbat && c < C2;
+      float2 gx = make_float2(0.f, 0.f), gy = gx, gz = gx, dedx = gx, gm[4] = {gx, gx, gx, gx};
+      int j = 0;
+      if (work) {
+        const int4 m = s.meta[e];
+        j = m.w;
+        const float tt = __int_as_float(m.z);
+        const float2 t = pair_of(tt), t_2 = pair_of(2.0f * tt), t_15 = pair_of(1.5f * tt);
+        const float4 *cf = reinterpret_cast<const float4 *>(L.tab) + (size_t) m.x * NL * C + c;
+        const float2 *msg = reinterpret_cast<const float2 *>(L.msg + (size_t) j * 4 * C) + c;
+        float2 R[SP::NS], dR[SP::NS], mm[NI];
+#pragma unroll
+        for (int q = 0; q < SP::NS; q++) {
+          constexpr auto some = [](int l) { return l < 0 ? 0 : l; };
+          const int l = h ? some(SP::degree(1, q)) : some(SP::degree(0, q));
+          const float4 xy = __ldg(cf + l * C), zw = __ldg(cf + l * C + C2);
+          R[q] = pair_value(xy, zw, t);
+          dR[q] = pair_slope(xy, zw, t_2, t_15);
+        }
+#pragma unroll
+        for (int I = 0; I < 4; I++) mm[I] = __ldg(msg + I * C2);
+        mm[4] = __ldg(reinterpret_cast<const float2 *>(L.z + (size_t) m.y * C) + c);
+        const float4 *y = s.Y[e] + h * 2 * NK;
+#pragma unroll
+        for (int k = 0; k < NK; k++) {
+          constexpr auto bound = [](int q) { return q < SP::NS ? q : SP::NS - 1; };
+          const int s0 = bound(SP::slot(0, k)), s1 = bound(SP::slot(1, k));
+          const float2 Rk = s0 == s1 ? R[s0] : h ? R[s1] : R[s0], dRk = s0 == s1 ? dR[s0] : h ? dR[s1] : dR[s0];
+          const float4 A = y[2 * k], B = y[2 * k + 1];
+          float2 hq = __fmul2_rn(mm[0], g[0][k]);
+#pragma unroll
+          for (int I = 1; I < NI; I++) hq = __ffma2_rn(mm[I], g[I][k], hq);
+          const float2 p = __fmul2_rn(Rk, hq), ry = __fmul2_rn(Rk, lo2(A));
+          dedx = __ffma2_rn(__fmul2_rn(dRk, lo2(A)), hq, dedx);
+          gx = __ffma2_rn(p, hi2(A), gx);
+          gy = __ffma2_rn(p, lo2(B), gy);
+          gz = __ffma2_rn(p, hi2(B), gz);
+#pragma unroll
+          for (int I = 0; I < 4; I++) gm[I] = __ffma2_rn(ry, g[I][k], gm[I]);
+        }
+      }
+      // dE/dmsg: each group of harmonics takes two of the message functions and gets the other group's part of them
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const float2 give = h ? gm[q] : gm[2 + q];
+        float2 keep = h ? gm[2 + q] : gm[q];
+        keep.x += __shfl_xor_sync(0xffffffffu, give.x, 8);
+        keep.y += __shfl_xor_sync(0xffffffffu, give.y, 8);
+        if (work) {
+          const int at = (2 * h + q) * C + 2 * c;
+          if (L.gmsg_slot) *reinterpret_cast<float2 *>(L.gmsg_slot + (size_t) s.cs[e] * 4 * C + at) = keep;
+          else {
+            atomicAdd(L.gmsg + (size_t) j * 4 * C + at, keep.x);
+            atomicAdd(L.gmsg + (size_t) j * 4 * C + at + 1, keep.y);
+          }
+        }
+      }
+      const float tot = group_sum4<16>(gx.x + gx.y, gy.x + gy.y, gz.x + gz.y, dedx.x + dedx.y, lane & 15);
+      if (e < nbat && (lane & 3) == 0) reinterpret_cast<float *>(s.fe + e)[(lane & 15) >> 2] = tot;
+    }
+    __syncthreads();
+    for (int e = tid; e < nbat; e += 128) bwd_finish(s, e, fv, add, vir);
+    __syncthreads();
+  }
+  bwd_virial(s.vred, vir, vir_atom, i, add);
+}
+
+template<class Stage, class F> size_t pair_smem(F *kernel, size_t &attr)
+{
+  const size_t n = sizeof(Stage);
+  if (n > attr) {
+    GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) n));
+    attr = n;
+  }
+  return n;
+}
+
+template<int LMAX, int LPB>
+void launch_pair(const BondsDev &b, const LayerDev &L, const float *gQ, int NA, int a0, int na, float *fv, double *vir_atom, int add)
+{
+  static size_t attr = 48 * 1024;
+  const size_t smem = pair_smem<PairStage<LMAX>>(bond_bwd_pair_kernel<LMAX, LPB>, attr);
+  GB_LAUNCH((bond_bwd_pair_kernel<LMAX, LPB>), na, 128, smem, b, L, sh_table_host(), gQ, NA, a0, fv, vir_atom, add);
 }
 
 template<int LMAX, int NIT, int NCH, int LPE>
@@ -384,10 +499,18 @@ void launch_l(const BondsDev &b, const LayerDev &L, const float *gQ, int NA, int
 {
   const int C = L.C, nI = L.n_msg + 1;
   if (C > 64) throw Unsupported("bond sums with more than 64 channels are not supported");
+  if (L.pairs) {
+    if (L.n_msg) {
+      static size_t attr = 48 * 1024;
+      const size_t smem = pair_smem<MsgStage<LMAX>>(bond_bwd_msg_kernel<LMAX>, attr);
+      GB_LAUNCH(bond_bwd_msg_kernel<LMAX>, na, 128, smem, b, L, sh_table_host(), gQ, NA, a0, fv, vir_atom, add);
+    } else if (C > 32) launch_pair<LMAX, 32>(b, L, gQ, NA, a0, na, fv, vir_atom, add);
+    else if (C > 16) launch_pair<LMAX, 16>(b, L, gQ, NA, a0, na, fv, vir_atom, add);
+    else launch_pair<LMAX, 8>(b, L, gQ, NA, a0, na, fv, vir_atom, add);
+    return;
+  }
   if (C > 32) launch_t<LMAX, 1, 2, 32>(b, L, gQ, NA, a0, na, fv, vir_atom, add);
   else if (C > 16) { if (nI == 5) launch_t<LMAX, 5, 1, 32>(b, L, gQ, NA, a0, na, fv, vir_atom, add); else launch_t<LMAX, 1, 1, 32>(b, L, gQ, NA, a0, na, fv, vir_atom, add); }
-  else if (nI == 5 && !L.Rex && !getenv("GRACE_B200_BOND_NOSPLIT"))
-    GB_LAUNCH((bond_bwd_split_kernel<LMAX, 5>), na, 128, 0, b, L, sh_table_host(), gQ, NA, a0, fv, vir_atom, add);
   else { if (nI == 5) launch_t<LMAX, 5, 1, 16>(b, L, gQ, NA, a0, na, fv, vir_atom, add); else launch_t<LMAX, 1, 1, 16>(b, L, gQ, NA, a0, na, fv, vir_atom, add); }
 }
 

@@ -81,6 +81,80 @@ __device__ __forceinline__ float group_sum4(float v0, float v1, float v2, float 
   return v;
 }
 
+// ---- two channels per lane -------------------------------------------------------------------------------------
+// The kernels of layers with an even number of channels keep two neighbouring channels in a lane: every sum is a packed
+// two-wide FMA, a bond takes half the lanes and a warp works on several bonds at once.  Factors that are the same for both
+// channels (harmonics) are staged in shared memory twice side by side, so that no instruction goes into pairing them.
+__device__ __forceinline__ float2 pair_of(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
+
+// radial functions of a channel pair from the table of pairs (rows of x x y y, then of z z w w: a load instruction of a bond covers a contiguous
+// row; with the two quadruples of a pair side by side the lanes are 32 bytes apart and the kernels a fifth slower)
+__device__ __forceinline__ float2 pair_value(float4 xy, float4 zw, float2 t)
+{
+  return __ffma2_rn(t, __ffma2_rn(t, __ffma2_rn(t, hi2(zw), lo2(zw)), hi2(xy)), lo2(xy));
+}
+// their derivative by the interval's offset: y + 2 t (z + 1.5 t w)
+__device__ __forceinline__ float2 pair_slope(float4 xy, float4 zw, float2 t_2, float2 t_15)
+{
+  return __ffma2_rn(t_2, __ffma2_rn(t_15, hi2(zw), lo2(zw)), hi2(xy));
+}
+
+// Layers with four message functions split the harmonics of a bond between two groups of lanes, by whole degrees so that a
+// group needs the radial functions of its own degrees only: lmax 3: {3, 0} and {2, 1}, eight harmonics each.  Position k of
+// group h holds lm(h, k) of the degree in slot(h, k); where the groups hold another slot at a position, the lane selects.
+template<int LMAX> struct LmSplit {
+  static constexpr int NL = LMAX + 1, NLM = NL * NL;
+  static constexpr int NS = LMAX == 1 ? 1 : LMAX == 4 ? 3 : 2;       // degrees of a group, at most
+  static constexpr int NK = LMAX == 1 ? 3 : LMAX == 2 ? 5 : LMAX == 3 ? 8 : 13;
+  // degree of slot s of group h, -1: none
+  static constexpr __host__ __device__ int degree(int h, int s)
+  {
+    if (LMAX == 1) return s == 0 ? (h ? 0 : 1) : -1;
+    if (LMAX == 2) return h ? (s < 2 ? 1 - s : -1) : s == 0 ? 2 : -1;
+    if (LMAX == 3) return s > 1 ? -1 : h ? 2 - s : s == 0 ? 3 : 0;
+    return h ? (s == 0 ? 3 : s == 1 ? 2 : 0) : s == 0 ? 4 : s == 1 ? 1 : -1;
+  }
+  static constexpr __host__ __device__ int slot(int h, int k)    // NS: no harmonic at the position
+  {
+    int at = 0;
+    for (int s = 0; s < NS; s++) {
+      const int l = degree(h, s);
+      if (l < 0) break;
+      at += 2 * l + 1;
+      if (k < at) return s;
+    }
+    return NS;
+  }
+  static constexpr __host__ __device__ int lm(int h, int k)      // -1: none
+  {
+    int at = 0;
+    for (int s = 0; s < NS; s++) {
+      const int l = degree(h, s);
+      if (l < 0) break;
+      if (k < at + 2 * l + 1) return l * l + k - at;
+      at += 2 * l + 1;
+    }
+    return -1;
+  }
+  static constexpr __host__ __device__ int place(int q)          // h NK + k of harmonic q
+  {
+    for (int h = 0; h < 2; h++)
+      for (int k = 0; k < NK; k++)
+        if (lm(h, k) == q) return h * NK + k;
+    return -1;
+  }
+};
+// place() at compile time, for the loops over harmonics whose index is a constant only after unrolling
+template<int LMAX> struct LmPlaces {
+  int v[25];
+  constexpr LmPlaces() : v{}
+  {
+    for (int q = 0; q < 25; q++) v[q] = q < LmSplit<LMAX>::NLM ? LmSplit<LMAX>::place(q) : -1;
+  }
+};
+
 // interval k and offset t of x = r / rcut in a table of N intervals (libgrace/include/grace/fused_cpu.h:1052-1058)
 __device__ __forceinline__ void spline_locate(float x, int N, int &k, float &t)
 {

@@ -88,7 +88,19 @@ void Engine::setup_layer(LayerEngine &E, const LayerPlan &P)
   E.plan = &P;
   E.tab.set_label("engine:radial_table");
   E.z.set_label("engine:chemical_weights");
-  E.tab.upload(P.radial.tab);
+  E.pairs = !exact_ && bond_pairs(P.C, P.n_msg);
+  if (E.pairs) {    // the coefficients of two neighbouring channels side by side: x x y y of all pairs, then z z w w
+    const std::vector<float> &src = P.radial.tab;
+    std::vector<float> tab(src.size());
+    const size_t C = (size_t) P.C;
+    for (size_t row = 0; row < src.size(); row += 4 * C)
+      for (size_t n = 0; n < C; n++)
+        for (size_t q = 0; q < 4; q++) tab[row + (q / 2) * 2 * C + (n / 2) * 4 + (q % 2) * 2 + n % 2] = src[row + 4 * n + q];
+    E.tab.upload(tab);
+    GB_CUDA(cudaStreamSynchronize(dev().stream));    // the upload reads a vector of this scope
+  } else {
+    E.tab.upload(P.radial.tab);
+  }
   E.z.upload(P.z);
   // all index tables of the layer in one buffer each (the fused kernel copies them to shared memory as a whole)
   std::vector<int> itab;
@@ -502,6 +514,7 @@ LayerDev Engine::layer_dev(const LayerEngine &E) const
   L.gmsg = nullptr;
   L.gmsg_slot = nullptr;
   L.N = E.plan->radial.N;
+  L.pairs = E.pairs;
   L.C = E.plan->C;
   L.n_msg = E.plan->n_msg;
   L.n_elements = plan_.n_elements;

@@ -24,6 +24,7 @@ struct State3L;    // device state of a GRACE-3L model (engine3l.cu)
 struct LayerEngine {
   const LayerPlan *plan = nullptr;
   DBuf<float> tab, z;
+  bool pairs = false;        // bond sums with two channels per lane: tab holds channel pairs (bond_pairs)
   DBuf<int> itab;            // row / offset tables of every operation
   DBuf<MVItem> items;
   DBuf<ProdTerm> terms;

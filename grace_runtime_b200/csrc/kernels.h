@@ -50,7 +50,7 @@ struct BondsDev {
 
 // per layer: radial table, chemical weights, messages
 struct LayerDev {
-  const float *tab;        // [N][nl][C][4]: cubic Hermite coefficients
+  const float *tab;        // [N][nl][C][4]: cubic Hermite coefficients; with `pairs` [N][nl][2][C / 2][4], x x y y and z z w w of channel pairs
   const float *z;          // [n_elements][C]
   const float *rc;         // [n_elements][n_elements] pair cutoffs
   const float *msg;        // [n][n_msg][C] message rows of all atoms (layer 2) or null
@@ -60,7 +60,11 @@ struct LayerDev {
   int N, C, n_msg, n_elements;
   // exact radial MLP instead of the tables: value and d/dx per list slot, [slot][l][C] (null: tables)
   const float *Rex, *dRex;
+  bool pairs;              // the kernels with two channels per lane (bond_pairs)
 };
+// layers whose bond sums run with two channels per lane: an even number of channels (8-byte rows), and either no message
+// functions or the four of GRACE-2L.  Odd widths, other numbers of messages and the exact radial MLP take the general kernels.
+inline bool bond_pairs(int C, int n_msg) { return C % 2 == 0 && (n_msg == 0 ? C <= 64 : n_msg == 4 && C <= 16); }
 
 // element of a tensor: p[(f * NA + a) * C + c]; NA: atom stride of the chunk tensors, na <= NA: atoms in use
 void launch_mv(const MVDev &op, const TensorDev *tensors, const int *mu, int NA, int na);
