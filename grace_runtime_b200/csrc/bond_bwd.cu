@@ -247,8 +247,8 @@ __device__ __forceinline__ void bwd_stage(S &s, int e, const BondsDev &b, const 
   float4 *y = s.Y[e];
   sph_harm<LMAX, true>(sht, rec.x * ir, rec.y * ir, rec.z * ir, [&](int lm, float v, float gx, float gy, float gz) {
     const int at = place(lm);
-    y[2 * at] = make_float4(v, v, gx, gx);
-    y[2 * at + 1] = make_float4(gy, gy, gz, gz);
+    y[at] = make_float4(v, v, gx, gx);
+    y[at + 1] = make_float4(gy, gy, gz, gz);
   });
 }
 
@@ -285,19 +285,27 @@ __device__ __forceinline__ void bwd_virial(double (&vred)[4][6], double (&vir)[6
   }
 }
 
-// bonds per round: the 78 of a dense metal inside 6 Angstrom at lmax 3, four or five blocks per SM
-template<int LMAX> __host__ __device__ constexpr int bwd_bonds() { return LMAX <= 3 ? 80 : 64; }
-template<int LMAX> using PairStage = BwdStage<2 * (LMAX + 1) * (LMAX + 1) + 1, bwd_bonds<LMAX>()>;
-template<int LMAX> using MsgStage = BwdStage<4 * LmSplit<LMAX>::NK + 1, bwd_bonds<LMAX>()>;
+// Blocks per SM the kernels are compiled for and bonds per round, so that registers and shared memory allow the same number.
+// They wait for the table and for shared memory most of the time: warps in flight count for more than a few spilled registers.
+template<int LMAX> __host__ __device__ constexpr int pair_blocks() { return 4; }
+template<int LMAX> __host__ __device__ constexpr int pair_bonds() { return LMAX <= 3 ? 78 : 60; }
+template<int LMAX> __host__ __device__ constexpr int msg_blocks() { return LMAX <= 3 ? 3 : 2; }
+template<int LMAX> __host__ __device__ constexpr int msg_bonds() { return LMAX <= 3 ? 80 : 64; }
+template<int LMAX> using PairStage = BwdStage<2 * (LMAX + 1) * (LMAX + 1) + 1, pair_bonds<LMAX>()>;
+// The four 16-byte words a load instruction of the message kernel reads, (bond, group of harmonics), lie in different banks: the
+// groups are an odd number of words apart and the bonds three.
+template<int LMAX> __host__ __device__ constexpr int msg_half() { return 2 * LmSplit<LMAX>::NK + 1; }
+template<int LMAX> __host__ __device__ constexpr int msg_row() { return 2 * msg_half<LMAX>() + (8 + 3 - 2 * msg_half<LMAX>() % 8) % 8; }
+template<int LMAX> using MsgStage = BwdStage<msg_row<LMAX>(), msg_bonds<LMAX>()>;
 
 // Layers without message functions and with an even number of channels: LPB lanes per bond, two channels per lane, 32 / LPB
 // bonds per warp at a time, with the gradients of its channels in a lane's registers.  With the chemical weight folded into
 // the radial functions a harmonic costs four packed FMAs per lane and bond.
 template<int LMAX, int LPB>
-__global__ void __launch_bounds__(128) bond_bwd_pair_kernel(BondsDev b, LayerDev L, SHTable sht, const float *__restrict__ gQ, int NA, int a0,
+__global__ void __launch_bounds__(128, pair_blocks<LMAX>()) bond_bwd_pair_kernel(BondsDev b, LayerDev L, SHTable sht, const float *__restrict__ gQ, int NA, int a0,
                                                             float *__restrict__ fv, double *__restrict__ vir_atom, int add)
 {
-  constexpr int NL = LMAX + 1, NLM = NL * NL, BPW = 32 / LPB, EB = bwd_bonds<LMAX>();
+  constexpr int NL = LMAX + 1, NLM = NL * NL, BPW = 32 / LPB, EB = pair_bonds<LMAX>();
   extern __shared__ __align__(16) char smem[];
   PairStage<LMAX> &s = *reinterpret_cast<PairStage<LMAX> *>(smem);
   const int a = blockIdx.x, i = b.ilist ? b.ilist[a0 + a] : a0 + a, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
@@ -313,7 +321,7 @@ __global__ void __launch_bounds__(128) bond_bwd_pair_kernel(BondsDev b, LayerDev
 
   for (int b0 = 0; b0 < nb; b0 += per) {
     const int nbat = min(per, nb - b0);
-    for (int e = tid; e < nbat; e += 128) bwd_stage<LMAX>(s, e, b, L, sht, base + b0 + e, mui, [](int lm) { return lm; });
+    for (int e = tid; e < nbat; e += 128) bwd_stage<LMAX>(s, e, b, L, sht, base + b0 + e, mui, [](int lm) { return 2 * lm; });
     __syncthreads();
     for (int e0 = w * BPW; e0 < nbat; e0 += 4 * BPW) {
       const int e = e0 + sub;
@@ -365,11 +373,11 @@ __global__ void __launch_bounds__(128) bond_bwd_pair_kernel(BondsDev b, LayerDev
 //   dE/dx += dR_l Y_lm h,   g += R_l h grad Y_lm,   dE/dmsg_I += R_l Y_lm gQ[I][lm].
 // One channel per lane took 447 issued instructions per bond and was bound by them.
 template<int LMAX>
-__global__ void __launch_bounds__(128) bond_bwd_msg_kernel(BondsDev b, LayerDev L, SHTable sht, const float *__restrict__ gQ, int NA, int a0,
+__global__ void __launch_bounds__(128, msg_blocks<LMAX>()) bond_bwd_msg_kernel(BondsDev b, LayerDev L, SHTable sht, const float *__restrict__ gQ, int NA, int a0,
                                                            float *__restrict__ fv, double *__restrict__ vir_atom, int add)
 {
   using SP = LmSplit<LMAX>;
-  constexpr int NL = LMAX + 1, NLM = NL * NL, NI = 5, NK = SP::NK, EB = bwd_bonds<LMAX>();
+  constexpr int NL = LMAX + 1, NLM = NL * NL, NI = 5, NK = SP::NK, EB = msg_bonds<LMAX>(), HALF = msg_half<LMAX>();
   extern __shared__ __align__(16) char smem[];
   MsgStage<LMAX> &s = *reinterpret_cast<MsgStage<LMAX> *>(smem);
   const int a = blockIdx.x, i = b.ilist ? b.ilist[a0 + a] : a0 + a, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
@@ -392,10 +400,16 @@ __global__ void __launch_bounds__(128) bond_bwd_msg_kernel(BondsDev b, LayerDev 
     const int nbat = min(per, nb - b0);
     for (int e = tid; e < nbat; e += 128) {
       constexpr LmPlaces<LMAX> places;
-      bwd_stage<LMAX>(s, e, b, L, sht, base + b0 + e, mui, [&](int lm) { return places.v[lm]; });
+      bwd_stage<LMAX>(s, e, b, L, sht, base + b0 + e, mui, [&](int lm) {
+        const int at = places.v[lm];
+        return at < NK ? 2 * at : HALF + 2 * (at - NK);
+      });
 #pragma unroll
       for (int hk = 0; hk < 2 * NK; hk++)    // positions without a harmonic
-        if (SP::lm(hk / NK, hk % NK) < 0) s.Y[e][2 * hk] = s.Y[e][2 * hk + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (SP::lm(hk / NK, hk % NK) < 0) {
+          float4 *none = s.Y[e] + hk / NK * HALF + hk % NK * 2;
+          none[0] = none[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
     }
     __syncthreads();
     for (int e0 = 2 * w; e0 < nbat; e0 += 8) {
@@ -422,7 +436,7 @@ __global__ void __launch_bounds__(128) bond_bwd_msg_kernel(BondsDev b, LayerDev 
 #pragma unroll
         for (int I = 0; I < 4; I++) mm[I] = __ldg(msg + I * C2);
         mm[4] = __ldg(reinterpret_cast<const float2 *>(L.z + (size_t) m.y * C) + c);
-        const float4 *y = s.Y[e] + h * 2 * NK;
+        const float4 *y = s.Y[e] + h * HALF;
 #pragma unroll
         for (int k = 0; k < NK; k++) {
           constexpr auto bound = [](int q) { return q < SP::NS ? q : SP::NS - 1; };

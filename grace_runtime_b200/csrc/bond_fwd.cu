@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(128) bond_fwd_kernel(BondsDev b, LayerDev L, S
 // lane, 32 / LPB bonds per warp at a time.  Bound by the radial table: a bond reads NL C coefficient quadruples (2 KB at
 // lmax 3, 32 channels) out of 2 MB, and the kernel moves them at the rate of the L1 and L2 caches.
 template<int LMAX, int LPB>
-__global__ void __launch_bounds__(128) bond_fwd_pair_kernel(BondsDev b, LayerDev L, SHTable sht, float *__restrict__ Q, int NA, int a0)
+__global__ void __launch_bounds__(128, LMAX <= 3 ? 8 : 5) bond_fwd_pair_kernel(BondsDev b, LayerDev L, SHTable sht, float *__restrict__ Q, int NA, int a0)
 {
   constexpr int NL = LMAX + 1, NLM = NL * NL, NP = (NLM + 1) / 2, ROW = NP | 1, BPW = 32 / LPB;    // odd rows: no bank conflicts
   constexpr int Y_F4 = EB * ROW, RED_F4 = 4 * NLM * LPB / 2, BUF = Y_F4 > RED_F4 ? Y_F4 : RED_F4;
