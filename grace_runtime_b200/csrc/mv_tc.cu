@@ -109,6 +109,22 @@ template<> __device__ __forceinline__ void tmem_ld<16>(unsigned taddr, float (&v
   for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
+// 16 columns of 32 tensor-memory lanes (two 16-lane loads and one wait).  A thread gets, for groups j of 8 columns, columns
+// 8 j + 2 (lane & 3) and the next of the rows lane / 4 (v[4 j], v[4 j + 1]) and lane / 4 + 8 (v[4 j + 2], v[4 j + 3]), then the
+// same of rows + 16 behind the first 8 values: a store of two columns by the warp fills whole 32-byte sectors of 8 rows.
+__device__ __forceinline__ void tmem_ld_rows(unsigned taddr, float (&v)[16])
+{
+  unsigned r[16];
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%16];\n\t"
+               "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%17];\n\t"
+               "tcgen05.wait::ld.sync.aligned;"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                 "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(taddr), "r"(taddr + (16u << 16)) : "memory");
+#pragma unroll
+  for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+}
+
 // position in the loop nest (round of tiles, output row, item of the row, tile of the round)
 struct Cursor {
   int tile0, nt, row, it, i0, i1, tt;
@@ -125,19 +141,25 @@ template<int K> struct TileRegs {
 
 // Warp-specialised: warps 0-7 produce (global loads two tiles ahead in registers, tf32 hi / lo operand images of a tile
 // into one of S shared-memory stages, the weight image of an item into a ring of S buffers), warp 8 issues the matrix
-// instructions (one thread; nothing else runs on its critical path), warps 9-12 move finished accumulators from tensor
+// instructions (one thread; nothing else runs on its critical path), the warps from 9 on move finished accumulators from tensor
 // memory to global memory.  Two sets of accumulators (TB tiles x n_out columns each) take turns, so the epilogue of a
 // row overlaps the matrix instructions of the next.  Hand-offs are mbarriers: full[s] (256 producer arrivals) / empty[s]
-// (tcgen05.commit) per stage, accfull[set] (tcgen05.commit after the last item of a row) / accempty[set] (128 epilogue
-// arrivals).  A wait that runs out raises `abort`, which every other wait sees, and all roles leave together.
-constexpr int NPROD = NTH, NTHREADS = NTH + 32 + 128;
+// (tcgen05.commit) per stage, accfull[set] (tcgen05.commit after the last item of a row) / accempty[set] (every
+// epilogue thread).  A wait that runs out raises `abort`, which every other wait sees, and all roles leave together.
+constexpr int NPROD = NTH;
+// grouped atoms: two epilogue warps per quarter of the lanes (the sums over several accumulators and the scattered rows take longer
+// than the matrix instructions of a row: 1,024,000 atoms, 16 inputs, 9.4 -> 6.3 ms).  17 warps leave 96 registers per thread, not
+// enough for producers that hold two tiles of 64 channels (1.87 -> 2.13 ms) or for the other epilogue
+__host__ __device__ constexpr int epilogue_threads(int K, bool elem) { return elem && K < 64 ? 256 : 128; }
+__host__ __device__ constexpr int block_threads(int K, bool elem) { return NTH + 32 + epilogue_threads(K, elem); }
 
 template<int K, int CB, int S, bool ELEM>
-__global__ void __launch_bounds__(NTHREADS, 1) mv_tc_kernel(MVTCDev op, const TensorDev *__restrict__ Tg, int ntensors, int NA,
+__global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDev op, const TensorDev *__restrict__ Tg, int ntensors, int NA,
                                                             int na, int TB, int tmem_cols, int *error)
 {
   using TR = TileRegs<K>;
   constexpr int K4 = TR::K4, UNITS = TR::UNITS, PER = TR::PER;
+  constexpr int NEPI = epilogue_threads(K, ELEM), NTHREADS = block_threads(K, ELEM);
   constexpr int A_BYTES = TM * K * 4;    // one image (hi or lo) of an activation tile
   extern __shared__ __align__(1024) char smem[];
   __shared__ unsigned long long s_full[S], s_empty[S], s_accfull[2], s_accempty[2];
@@ -167,7 +189,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mv_tc_kernel(MVTCDev op, const Te
     }
     for (int s = 0; s < 2; s++) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_accfull[s])) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 128;" ::"r"(smem_u32(&s_accempty[s])) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&s_accempty[s])), "r"(NEPI) : "memory");
     }
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -391,6 +413,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mv_tc_kernel(MVTCDev op, const Te
     // Each warp moves blocks of 32 atoms x CB columns of its tensor-memory lanes: registers (a lane holds one atom's
     // columns) -> a padded transpose buffer of its own -> global memory with whole 128-byte lines per store
     const int ew = warp & 3;    // the quarter of the tensor-memory lanes this warp may read (warp id modulo 4)
+    const int half = (warp - NW - 1) >> 2;    // grouped atoms: the warps of a quarter take the blocks in turn
     float *tr = tr_all + ew * (32 * (CB + 4));
     constexpr int LPR = CB / 4, RPI = 32 / LPR;    // lanes per atom row, atom rows per store instruction
     Cursor cur;
@@ -410,65 +433,110 @@ __global__ void __launch_bounds__(NTHREADS, 1) mv_tc_kernel(MVTCDev op, const Te
       const TensorDev dstT = s_T[row.dst];
       float *const out = dstT.p + (size_t) row.out * NA * dstT.C;
       const int nblk = N / CB, nb = cur.nt * nblk;
-      const bool vec = ((dstT.C | row.n_out) & 3) == 0;
-      // atom of row r of this warp's quarter of tile tt, -1: none
-      auto atom_of = [&](int tt, int r) {
-        const int at = (cur.tile0 + tt) * TM + ew * 32 + r;
-        return ELEM ? __ldg(op.order + at) : at < na ? at : -1;
-      };
-      // the old values of an accumulating row are fetched one block ahead of the block being written
-      float4 old[32 / RPI], oldn[32 / RPI];
-      auto load_old = [&](int b, float4 (&o)[32 / RPI]) {
-        const int tt = b / nblk, c0 = (b - tt * nblk) * CB;
+      if constexpr (ELEM) {    // rows of single atoms, 32-byte sectors straight from registers
+        const bool vec = ((dstT.C | row.n_out) & 1) == 0;
+        for (int b = half; b < nb; b += NEPI / 128) {
+          const int tt = b / nblk, c0 = (b - tt * nblk) * CB;
+          int at[4];    // atoms of the thread's rows lane / 4 + 8 q, -1: none
 #pragma unroll
-        for (int j = 0; j < 32 / RPI; j++) {
-          const int cq = lane % LPR, a = b < nb && c0 + 4 * cq < row.n_out ? atom_of(tt, j * RPI + lane / LPR) : -1;
-          o[j] = a >= 0 ? __ldcg(reinterpret_cast<const float4 *>(out + (size_t) a * dstT.C + c0) + cq) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-      };
-      if (row.accumulate && vec) load_old(0, oldn);
-      for (int b = 0; b < nb; b++) {
-        const int tt = b / nblk, c0 = (b - tt * nblk) * CB;
-        float v[CB];
-        const unsigned at = tmem + ((unsigned) (ew * 32) << 16) + (unsigned) ((set * TB + tt) * op.sub * N + c0);
-        tmem_ld<CB>(at, v);
-        if (ELEM)
+          for (int q = 0; q < 4; q++) {
+            const int r = (cur.tile0 + tt) * TM + ew * 32 + 8 * q + (lane >> 2);
+            at[q] = __ldg(op.order + r);
+          }
+          float *const o = out + c0 + 2 * (lane & 3);
+          // value pair p: columns c0 + 8 j + 2 (lane & 3) and the next of row q
+          auto row_of = [](int p) { return p / (CB / 4) * 2 + (p & 1); };
+          auto col_of = [](int p) { return p % (CB / 4) / 2 * 8; };
+          float2 old[CB / 2];
+          if (row.accumulate && vec) {
+#pragma unroll
+            for (int p = 0; p < CB / 2; p++) {
+              const int a = at[row_of(p)];
+              old[p] = a >= 0 && c0 + col_of(p) + 2 * (lane & 3) < row.n_out
+                           ? __ldcg(reinterpret_cast<const float2 *>(o + (size_t) a * dstT.C + col_of(p))) : make_float2(0.f, 0.f);
+            }
+          }
+          float v[CB];
+          const unsigned from = tmem + ((unsigned) (ew * 32) << 16) + (unsigned) ((set * TB + tt) * op.sub * N + c0);
+          tmem_ld_rows(from, v);
           for (int k = 1; k < min(op.sub, row.i1 - row.i0); k++) {    // the other accumulators of the row
             float w[CB];
-            tmem_ld<CB>(at + (unsigned) (k * N), w);
+            tmem_ld_rows(from + (unsigned) (k * N), w);
 #pragma unroll
             for (int q = 0; q < CB; q++) v[q] += w[q];
           }
-        __syncwarp();
 #pragma unroll
-        for (int q = 0; q < CB / 4; q++)
-          *reinterpret_cast<float4 *>(tr + lane * (CB + 4) + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-        __syncwarp();
-        if (!vec) {    // rows of a width that is no multiple of 4: value by value
-          const int w = min(CB, row.n_out - c0);
-          for (int e = lane; e < 32 * w; e += 32) {
-            const int r = e / w, c = e - r * w, a = atom_of(tt, r);
-            if (a < 0) continue;
-            float *o = out + (size_t) a * dstT.C + c0 + c;
-            const float x = tr[r * (CB + 4) + c];
-            *o = row.accumulate ? *o + x : x;
-          }
-          continue;
-        }
-        if (row.accumulate) {
-#pragma unroll
-          for (int j = 0; j < 32 / RPI; j++) old[j] = oldn[j];
-          load_old(b + 1, oldn);
-        }
-#pragma unroll
-        for (int j = 0; j < 32 / RPI; j++) {
-          const int r = j * RPI + lane / LPR, cq = lane % LPR, a = c0 + 4 * cq < row.n_out ? atom_of(tt, r) : -1;
-          if (a >= 0) {
-            float4 w = *reinterpret_cast<const float4 *>(tr + r * (CB + 4) + 4 * cq);
-            if (row.accumulate) {
-              w.x += old[j].x; w.y += old[j].y; w.z += old[j].z; w.w += old[j].w;
+          for (int p = 0; p < CB / 2; p++) {
+            const int a = at[row_of(p)], c = c0 + col_of(p) + 2 * (lane & 3);
+            if (a < 0 || c >= row.n_out) continue;
+            float *const d = o + (size_t) a * dstT.C + col_of(p);
+            float2 x = make_float2(v[2 * p], v[2 * p + 1]);
+            if (vec) {
+              if (row.accumulate) {
+                x.x += old[p].x;
+                x.y += old[p].y;
+              }
+              *reinterpret_cast<float2 *>(d) = x;
+            } else {    // rows of an odd width: value by value
+              d[0] = row.accumulate ? d[0] + x.x : x.x;
+              if (c + 1 < row.n_out) d[1] = row.accumulate ? d[1] + x.y : x.y;
             }
-            reinterpret_cast<float4 *>(out + (size_t) a * dstT.C + c0)[cq] = w;
+          }
+        }
+      } else {
+        const bool vec = ((dstT.C | row.n_out) & 3) == 0;
+        // atom of row r of this warp's quarter of tile tt, -1: none
+        auto atom_of = [&](int tt, int r) {
+          const int at = (cur.tile0 + tt) * TM + ew * 32 + r;
+          return at < na ? at : -1;
+        };
+        // the old values of an accumulating row are fetched one block ahead of the block being written
+        float4 old[32 / RPI], oldn[32 / RPI];
+        auto load_old = [&](int b, float4 (&o)[32 / RPI]) {
+          const int tt = b / nblk, c0 = (b - tt * nblk) * CB;
+#pragma unroll
+          for (int j = 0; j < 32 / RPI; j++) {
+            const int cq = lane % LPR, a = b < nb && c0 + 4 * cq < row.n_out ? atom_of(tt, j * RPI + lane / LPR) : -1;
+            o[j] = a >= 0 ? __ldcg(reinterpret_cast<const float4 *>(out + (size_t) a * dstT.C + c0) + cq) : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+        };
+        if (row.accumulate && vec) load_old(0, oldn);
+        for (int b = 0; b < nb; b++) {
+          const int tt = b / nblk, c0 = (b - tt * nblk) * CB;
+          float v[CB];
+          const unsigned at = tmem + ((unsigned) (ew * 32) << 16) + (unsigned) ((set * TB + tt) * op.sub * N + c0);
+          tmem_ld<CB>(at, v);
+          __syncwarp();
+#pragma unroll
+          for (int q = 0; q < CB / 4; q++)
+            *reinterpret_cast<float4 *>(tr + lane * (CB + 4) + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+          __syncwarp();
+          if (!vec) {    // rows of a width that is no multiple of 4: value by value
+            const int w = min(CB, row.n_out - c0);
+            for (int e = lane; e < 32 * w; e += 32) {
+              const int r = e / w, c = e - r * w, a = atom_of(tt, r);
+              if (a < 0) continue;
+              float *o = out + (size_t) a * dstT.C + c0 + c;
+              const float x = tr[r * (CB + 4) + c];
+              *o = row.accumulate ? *o + x : x;
+            }
+            continue;
+          }
+          if (row.accumulate) {
+#pragma unroll
+            for (int j = 0; j < 32 / RPI; j++) old[j] = oldn[j];
+            load_old(b + 1, oldn);
+          }
+#pragma unroll
+          for (int j = 0; j < 32 / RPI; j++) {
+            const int r = j * RPI + lane / LPR, cq = lane % LPR, a = c0 + 4 * cq < row.n_out ? atom_of(tt, r) : -1;
+            if (a >= 0) {
+              float4 w = *reinterpret_cast<const float4 *>(tr + r * (CB + 4) + 4 * cq);
+              if (row.accumulate) {
+                w.x += old[j].x; w.y += old[j].y; w.z += old[j].z; w.w += old[j].w;
+              }
+              reinterpret_cast<float4 *>(out + (size_t) a * dstT.C + c0)[cq] = w;
+            }
           }
         }
       }
@@ -509,7 +577,7 @@ void launch_s(const MVTCDev &op, const TensorDev *T, int ntensors, int NA, int n
   }
   const char *name = ELEM ? "mv_tc_element_kernel" : "mv_tc_kernel";
   before_launch(name);
-  mv_tc_kernel<K, CB, S, ELEM><<<grid, NTHREADS, smem, dev().stream>>>(op, T, ntensors, NA, na, TB, tmem_cols, error);
+  mv_tc_kernel<K, CB, S, ELEM><<<grid, block_threads(K, ELEM), smem, dev().stream>>>(op, T, ntensors, NA, na, TB, tmem_cols, error);
   after_launch(name);
 }
 
@@ -518,12 +586,15 @@ template<int K, bool ELEM> void launch_k(const MVTCDev &op, const TensorDev *T, 
   int tmem_cols = 32;    // a power of two that holds two sets of accumulators of TB tiles
   while (tmem_cols < 2 * TB * op.sub * op.N) tmem_cols *= 2;
   const bool s4 = stages_for(K, op.N) == 4;
-  if (op.N % 32 == 0) {
-    if (s4) launch_s<K, 32, 4, ELEM>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
-    else launch_s<K, 32, 2, ELEM>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+  if constexpr (ELEM) {
+    if (s4) launch_s<K, 16, 4, true>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+    else launch_s<K, 16, 2, true>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+  } else if (op.N % 32 == 0) {
+    if (s4) launch_s<K, 32, 4, false>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+    else launch_s<K, 32, 2, false>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
   } else {
-    if (s4) launch_s<K, 16, 4, ELEM>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
-    else launch_s<K, 16, 2, ELEM>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+    if (s4) launch_s<K, 16, 4, false>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+    else launch_s<K, 16, 2, false>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
   }
 }
 
