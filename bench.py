@@ -136,15 +136,15 @@ def algorithmic_bytes(kernel, model_cfg, n_atoms, n_bonds, slots):
     c = modelgen.CONFIGS[model_cfg]
     nlm = (c["lmax"] + 1) ** 2
     C = c["c1"]
-    if kernel == "bond_fwd_kernel":       # bond record in; A[nlm][C] out; offsets, counts, element per atom
+    if kernel in ("bond_fwd_kernel", "bond_fwd_pair_kernel"):    # bond record in; A[nlm][C] out; offsets, counts, element per atom
         return 16.0 * n_bonds + (4.0 * nlm * C + 16.0) * n_atoms
-    if kernel == "bond_bwd_kernel":       # bond record and slot in, bond force out; gA in, virial out
+    if kernel in ("bond_bwd_kernel", "bond_bwd_pair_kernel"):    # bond record and slot in, bond force out; gA in, virial out
         return (16.0 + 4.0 + 12.0) * n_bonds + (4.0 * nlm * C + 48.0 + 16.0) * n_atoms
     if c["layers"] == 2:                  # the message layer: (4 message functions + the chemical one) x nlm x CR sums per atom
         CR, nq = c["cr"], 5 * nlm
-        if kernel == "bond_fwd_split_kernel":    # bond record in; every atom's message row once; Q out
+        if kernel == "bond_fwd_msg_kernel":    # bond record in; every atom's message row once; Q out
             return 16.0 * n_bonds + (4.0 * nq * CR + 4.0 * 4 * CR + 16.0) * n_atoms
-        if kernel == "bond_bwd_split_kernel":    # as bond_bwd_kernel, plus each bond's share of dE/dmsg (4 x CR floats) out
+        if kernel == "bond_bwd_msg_kernel":    # as bond_bwd_pair_kernel, plus each bond's share of dE/dmsg (4 x CR floats) out
             return (16.0 + 4.0 + 12.0 + 4.0 * 4 * CR) * n_bonds + (4.0 * nq * CR + 4.0 * 4 * CR + 48.0 + 16.0) * n_atoms
     if kernel == "nl_compact":            # list entry (j, S) and positions in, record + slot out
         return (8.0 + 16.0 + 4.0) * slots + 24.0 * n_atoms
@@ -160,11 +160,11 @@ def bond_flops(kernel, model_cfg, n_bonds, launches_per_step):
     c = modelgen.CONFIGS[model_cfg]
     nlm = (c["lmax"] + 1) ** 2
     per = [(c["c1"], 1)] + ([(c["cr"], 5)] if c["layers"] == 2 else [])
-    # message layers of at most 16 channels run as the split kernels, the others (and layer 1) as the plain ones
-    split2 = c["layers"] == 2 and c["cr"] <= 16
-    if kernel.startswith(("bond_bwd_split", "bond_fwd_split")):
+    # message layers of at most 16 channels run as kernels of their own, the others (and layer 1) as the ones for one function
+    own2 = c["layers"] == 2 and c["cr"] <= 16
+    if kernel.startswith(("bond_bwd_msg", "bond_fwd_msg")):
         per = per[1:]
-    elif split2:
+    elif own2:
         per = per[:1]
     if kernel.startswith("bond_bwd"):
         return n_bonds * sum(2.0 * nlm * C * 4 * nit for C, nit in per)

@@ -1,0 +1,77 @@
+"""The kernels that a size, a width or the number of elements chooses (csrc/bond_fwd.cu, bond_bwd.cu: two channels per lane for
+even widths, the general kernels otherwise; csrc/mv_tc.cu: atoms grouped by element; csrc/nlist.cu: a warp or a thread per atom)
+at the edges of their ranges, against the numpy fp64 oracle or against one another.
+
+Tolerance of the forces: 1e-5 in the 2-norm.  A force is a sum of about 100 bonds of fp32 terms (6e-8 each) behind a network
+of some ten fp32 sums over up to 90 inputs; two orders of summation differ by a few 1e-6."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(a, b):
+    return np.linalg.norm(np.asarray(a) - np.asarray(b)) / np.linalg.norm(b)
+
+
+def _structures(n_species):
+    from grace_runtime_b200 import structures
+    rng = np.random.default_rng(5)
+    # 110 neighbours inside 6 A: more than one round of staged bonds; and a pair, a triple and a lone atom in an open box
+    types, pos, cell, pbc = structures.crystal("fcc", 3.2, (2, 2, 2), n_species=n_species, sigma=0.1, seed=7)
+    yield types, pos, cell, pbc
+    p = np.array([[5.0, 5, 5], [7.2, 5.5, 5], [20, 20, 20], [22.1, 20, 20.4], [21, 22, 20], [35, 5, 30]])
+    yield rng.integers(1, n_species + 1, size=6).astype(np.int32), p, np.eye(3) * 45.0, np.zeros(3, dtype=np.uint8)
+
+
+@pytest.mark.parametrize("layers,lmax,c1,cr", [
+    (1, 4, 32, 0), (1, 4, 8, 0), (1, 4, 34, 0), (1, 3, 64, 0), (1, 3, 18, 0), (1, 2, 16, 0), (1, 2, 6, 0),    # channel pairs
+    (1, 4, 9, 0), (1, 3, 33, 0),                                                                             # odd: general kernels
+    (2, 3, 32, 16), (2, 3, 20, 6), (2, 2, 32, 16), (2, 2, 8, 10),                                            # four messages, pairs
+    (2, 3, 32, 7), (2, 2, 32, 18)])                                                                          # general message kernels
+def test_bond_sums_at_the_edges_of_their_widths(backend, tmp_path, layers, lmax, c1, cr):
+    from grace_runtime_b200 import modelgen
+    from oracle.grace_oracle import GraceOracle
+    els = ["Al", "Cu", "Ni"]
+    kw = dict(cr=cr, c2=32) if layers == 2 else {}
+    path = modelgen.write_model(str(tmp_path / "m.npz"), layers=layers, lmax=lmax, max_order=3, elements=tuple(els), c1=c1, seed=3, **kw)
+    system, oracle = backend.System(backend.Model(path), els), GraceOracle(path)
+    for types, pos, cell, pbc in _structures(3):
+        r = system.compute(types, pos, cell, pbc, energies=True)
+        o = oracle.compute(els, types, pos, cell, pbc)
+        assert np.abs(r["energies"] - o["energies"]).max() < 1e-5
+        assert _rel(r["forces"], o["forces"]) < 1e-5
+        assert _rel(r["virial"], o["virial"]) < 1e-5
+
+
+@pytest.mark.parametrize("cfg,reps,kinds", [("2l", (3, 6, 6), 1), ("2l", (4, 4, 9), 89), ("1l", (3, 3, 22), 40), ("2l", (12, 13, 15), 89)])
+def test_atoms_grouped_by_element(backend, tmp_path, monkeypatch, cfg, reps, kinds):
+    """one element and many (tiles that hold a few atoms each), the one-block order of the atoms and the one for more than
+    8,192 atoms, against the kernels that read every atom's weights by themselves"""
+    from grace_runtime_b200 import modelgen, structures
+    els = list(modelgen.ELEMENTS)[:kinds]
+    path = modelgen.write_config_model(str(tmp_path / "m.npz"), cfg, els, seed=4)
+    types, pos, cell, pbc = structures.crystal("fcc", 3.6, reps, n_species=kinds, sigma=0.08, seed=5)
+    out = {}
+    for mode in ("tc", "ops"):
+        monkeypatch.setenv("GRACE_B200_DENSE", mode)
+        out[mode] = backend.System(backend.Model(path), els).compute(types, pos, cell, pbc, energies=True)
+    assert np.abs(out["tc"]["energies"] - out["ops"]["energies"]).max() < 1e-5
+    assert _rel(out["tc"]["forces"], out["ops"]["forces"]) < 1e-5
+    assert _rel(out["tc"]["virial"], out["ops"]["virial"]) < 1e-5
+
+
+def test_neighbor_search_on_both_sides_of_its_line(backend, tmp_path):
+    """128,000 atoms (a warp per atom) and 160,000 (a thread per atom): copies of one cell have its forces"""
+    from grace_runtime_b200 import modelgen, structures
+    els = ["Mo", "W"]
+    path = modelgen.write_config_model(str(tmp_path / "m.npz"), "1l", els, seed=6)
+    types, pos, cell, pbc = structures.crystal("bcc", 3.2, (10, 10, 10), n_species=2, sigma=0.05, seed=8)
+    model = backend.Model(path)
+    one = backend.System(model, els).compute(types, pos, cell, pbc)
+    for reps in ((4, 4, 4), (4, 4, 5)):
+        shift = np.stack(np.meshgrid(*[np.arange(k) for k in reps], indexing="ij"), -1).reshape(-1, 3) @ cell
+        p = (pos[None] + shift[:, None]).reshape(-1, 3)
+        r = backend.System(model, els).compute(np.tile(types, len(shift)), p, cell * np.array(reps)[:, None], pbc)
+        assert abs(r["energy"] / len(shift) - one["energy"]) / len(types) < 1e-6
+        assert _rel(r["forces"], np.tile(one["forces"], (len(shift), 1))) < 1e-5
