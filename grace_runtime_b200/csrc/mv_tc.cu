@@ -225,13 +225,20 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
     if (!c.valid) return;
     c.nt = min(TB, ntiles - tile0);
     c.i0 = c.it = s_rows[row].i0;
-    c.i1 = s_rows[row].i1;
+    c.i1 = ELEM ? min(c.i0 + op.sub, s_rows[row].i1) : s_rows[row].i1;
     c.tt = 0;
+  };
+  // grouped atoms: the next items of the same row, an accumulator each
+  auto next_part = [&](Cursor &c) -> bool {
+    if (!ELEM || c.i1 == s_rows[c.row].i1) return false;
+    c.i0 = c.it = c.i1;
+    c.i1 = min(c.i0 + op.sub, s_rows[c.row].i1);
+    return true;
   };
   auto advance = [&](Cursor &c) {
     if (++c.tt < c.nt) return;
     c.tt = 0;
-    if (++c.it < c.i1) return;
+    if (++c.it < c.i1 || next_part(c)) return;
     int row = c.row + gridDim.y, tile0 = c.tile0;
     if (row >= op.nrows) {
       row = blockIdx.y;
@@ -239,7 +246,8 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
     }
     start(c, tile0, row);
   };
-  auto next_row = [&](Cursor &c) {    // first fill of the row after c's
+  auto next_row = [&](Cursor &c) {    // first fill of the row, or part of a row, after c's
+    if (next_part(c)) return;
     int row = c.row + gridDim.y, tile0 = c.tile0;
     if (row >= op.nrows) {
       row = blockIdx.y;
@@ -382,9 +390,9 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
         const unsigned b_hi = smem_u32(W_st + (size_t) (item_no % S) * 2 * W_BYTES);
         const unsigned long long dA[2] = {make_desc(a_hi, K), make_desc(a_hi + A_BYTES, K)};
         const unsigned long long dB[2] = {make_desc(b_hi, K), make_desc(b_hi + W_BYTES, K)};
-        const int sub = ELEM ? (cur.it - cur.i0) % op.sub : 0;
+        const int sub = ELEM ? cur.it - cur.i0 : 0;
         const unsigned d = tmem + (unsigned) (((set * TB + cur.tt) * op.sub + sub) * N);
-        const bool acc0 = ELEM ? cur.it - cur.i0 >= op.sub : cur.it != cur.i0;
+        const bool acc0 = !ELEM && cur.it != cur.i0;
 #pragma unroll
         for (int pass = 0; pass < 3; pass++) {    // small terms first: a_lo b_hi, a_hi b_lo, a_hi b_hi
           const unsigned long long a = dA[pass == 0 ? 1 : 0], b = dB[pass == 1 ? 1 : 0];
@@ -395,7 +403,7 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&s_empty[s])) : "memory");
         Cursor nx = cur;
         advance(nx);
-        if (!nx.valid || nx.row != cur.row || nx.tile0 != cur.tile0) {    // the row is complete once these are done
+        if (!nx.valid || nx.row != cur.row || nx.tile0 != cur.tile0 || nx.i0 != cur.i0) {    // the row is complete once these are done
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&s_accfull[set])) : "memory");
           rowc++;
         }
@@ -434,6 +442,8 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
       float *const out = dstT.p + (size_t) row.out * NA * dstT.C;
       const int nblk = N / CB, nb = cur.nt * nblk;
       if constexpr (ELEM) {    // rows of single atoms, 32-byte sectors straight from registers
+        // later parts of a row add to what this thread wrote before
+        const bool add = row.accumulate || cur.i0 > row.i0;
         const bool vec = ((dstT.C | row.n_out) & 1) == 0;
         for (int b = half; b < nb; b += NEPI / 128) {
           const int tt = b / nblk, c0 = (b - tt * nblk) * CB;
@@ -448,7 +458,7 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
           auto row_of = [](int p) { return p / (CB / 4) * 2 + (p & 1); };
           auto col_of = [](int p) { return p % (CB / 4) / 2 * 8; };
           float2 old[CB / 2];
-          if (row.accumulate && vec) {
+          if (add && vec) {
 #pragma unroll
             for (int p = 0; p < CB / 2; p++) {
               const int a = at[row_of(p)];
@@ -459,7 +469,7 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
           float v[CB];
           const unsigned from = tmem + ((unsigned) (ew * 32) << 16) + (unsigned) ((set * TB + tt) * op.sub * N + c0);
           tmem_ld_rows(from, v);
-          for (int k = 1; k < min(op.sub, row.i1 - row.i0); k++) {    // the other accumulators of the row
+          for (int k = 1; k < cur.i1 - cur.i0; k++) {    // the other accumulators of the row
             float w[CB];
             tmem_ld_rows(from + (unsigned) (k * N), w);
 #pragma unroll
@@ -472,14 +482,14 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
             float *const d = o + (size_t) a * dstT.C + col_of(p);
             float2 x = make_float2(v[2 * p], v[2 * p + 1]);
             if (vec) {
-              if (row.accumulate) {
+              if (add) {
                 x.x += old[p].x;
                 x.y += old[p].y;
               }
               *reinterpret_cast<float2 *>(d) = x;
             } else {    // rows of an odd width: value by value
-              d[0] = row.accumulate ? d[0] + x.x : x.x;
-              if (c + 1 < row.n_out) d[1] = row.accumulate ? d[1] + x.y : x.y;
+              d[0] = add ? d[0] + x.x : x.x;
+              if (c + 1 < row.n_out) d[1] = add ? d[1] + x.y : x.y;
             }
           }
         }
@@ -856,9 +866,10 @@ void MVTensorCore::launch(const TensorDev *tensors, int ntensors, int NA, int na
   }
   // one CTA per SM; two sets of accumulators share the 512 tensor-memory columns
   const int G = dev().sm_count;
-  // The rows of reduces over the element are sums of up to 89 items.  The tensor cores cut off what they add (towards zero,
-  // one bit of 2^-24 per instruction and accumulator), which over hundreds of instructions becomes a bias of 1e-5: such a row
-  // spreads its items over as many accumulators as there are columns for, and the epilogue adds them with rounding.
+  // The rows of reduces over the element are sums of up to 89 items.  The tensor cores cut off what they add (towards zero, one
+  // bit of 2^-24 per instruction and accumulator): 240 instructions in one accumulator are a bias of 8e-6, and even six items
+  // left per-atom energies of GRACE-1L of order 4 at 1.8e-6 where fp32 sums are at 2.2e-7.  So every item has an accumulator of its
+  // own, as many at a time as there are columns for, and the epilogue adds them with rounding, part of a row after part.
   op.sub = elem_ ? std::max(1, std::min(16, TMEM_COLS / 2 / N_)) : 1;
   const int tb_max = elem_ ? 1 : std::max(1, std::min(MAX_TILES, TMEM_COLS / 2 / N_));
   const int rounds = (ntiles + G * tb_max - 1) / (G * tb_max);

@@ -20,7 +20,7 @@ struct MVTCDev {
   const char *images;      // per element and matrix: [N][K] tf32 hi image, then the lo image (canonical K-major layout)
   const int *order, *tiles;    // per-element weights: ElemOrder
   int N, nrows, nitems, nmat;
-  int sub;                 // accumulators the items of a row take turns in
+  int sub;                 // accumulators, one per item, that a part of a row has (per-element weights)
 };
 
 // The atoms of a chunk grouped by element, for operations with per-element weights: tiles of 128 atoms of one element.
