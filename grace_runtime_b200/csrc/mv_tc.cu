@@ -66,14 +66,16 @@ __device__ __forceinline__ void mma_tf32_ss(unsigned tmem_d, unsigned long long 
 
 // hi + lo split of four activations for the 3 x tf32 product.  The tensor cores read the upper 19 bits of an fp32
 // operand (sign, exponent, 10 mantissa bits) and ignore the rest, so `hi` is the value itself and lo = x - trunc(x) is
-// exact in fp32; lo in turn is read truncated, which leaves a relative error of 2^-20 of x - the size of the a_lo b_lo
-// term the scheme drops anyway.  Two instructions per value and none of them a conversion.
+// exact in fp32; lo in turn is rounded to what is read by an integer addition, which leaves a relative error of 2^-22 of x - the
+// size of the a_lo b_lo term the scheme drops anyway - without a sign that it prefers.  Three instructions per value and none of
+// them a conversion.
 __device__ __forceinline__ void split4(float4 x, float sc, float4 &hi, float4 &lo)
 {
   const float v[4] = {x.x * sc, x.y * sc, x.z * sc, x.w * sc};
   float l[4];
 #pragma unroll
-  for (int q = 0; q < 4; q++) l[q] = v[q] - __uint_as_float(__float_as_uint(v[q]) & 0xffffe000u);
+  for (int q = 0; q < 4; q++)    // + half a unit of what is read: lo is rounded to nearest instead of cut off
+    l[q] = __uint_as_float(__float_as_uint(v[q] - __uint_as_float(__float_as_uint(v[q]) & 0xffffe000u)) + 0x1000u);
   hi = make_float4(v[0], v[1], v[2], v[3]);
   lo = make_float4(l[0], l[1], l[2], l[3]);
 }
@@ -153,7 +155,8 @@ constexpr int NPROD = NTH;
 __host__ __device__ constexpr int epilogue_threads(int K, bool elem) { return elem && K < 64 ? 256 : 128; }
 __host__ __device__ constexpr int block_threads(int K, bool elem) { return NTH + 32 + epilogue_threads(K, elem); }
 
-template<int K, int CB, int S, bool ELEM>
+// SEP: the two small terms of the product have accumulators of their own beside a_hi b_hi (columns N .. 2 N - 1).
+template<int K, int CB, int S, bool ELEM, bool SEP>
 __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDev op, const TensorDev *__restrict__ Tg, int ntensors, int NA,
                                                             int na, int TB, int tmem_cols, int *error)
 {
@@ -170,7 +173,7 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
   __shared__ MVItem s_items[MAX_ITEMS];
   __shared__ MVRowDev s_rows[MAX_ROWS];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const int N = op.N;
+  const int N = op.N, NC = SEP ? 2 * N : N;    // columns of an accumulator
   const int W_BYTES = N * K * 4;                         // one image of a weight matrix
   char *A_st = smem;                                     // stage s at s * 2 * A_BYTES: hi, then lo
   char *W_st = smem + (size_t) S * 2 * A_BYTES;          // buffer b at b * 2 * W_BYTES: hi, then lo
@@ -365,7 +368,7 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
   } else if (warp == NW) {
     // ---------------- matrix-instruction issuer ----------------
     if (lane == 0) {
-      const unsigned idesc = make_idesc(N);
+      const unsigned idesc = make_idesc(N), idesc2 = make_idesc(NC);
       Cursor cur;
       start(cur, blockIdx.x * TB, blockIdx.y);
       int fill = 0, item_no = -1, rowc = 0;
@@ -391,14 +394,24 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
         const unsigned long long dA[2] = {make_desc(a_hi, K), make_desc(a_hi + A_BYTES, K)};
         const unsigned long long dB[2] = {make_desc(b_hi, K), make_desc(b_hi + W_BYTES, K)};
         const int sub = ELEM ? cur.it - cur.i0 : 0;
-        const unsigned d = tmem + (unsigned) (((set * TB + cur.tt) * op.sub + sub) * N);
+        const unsigned d = tmem + (unsigned) (((set * TB + cur.tt) * op.sub + sub) * NC);
         const bool acc0 = !ELEM && cur.it != cur.i0;
-#pragma unroll
-        for (int pass = 0; pass < 3; pass++) {    // small terms first: a_lo b_hi, a_hi b_lo, a_hi b_hi
-          const unsigned long long a = dA[pass == 0 ? 1 : 0], b = dB[pass == 1 ? 1 : 0];
+        if constexpr (SEP) {
+          // the lo image of the weights lies behind the hi image like rows N .. 2 N - 1 of one matrix: a_hi meets both at once
 #pragma unroll
           for (int ks = 0; ks < K / 8; ks++)
-            mma_tf32_ss(d, a + (unsigned long long) (ks * 16), b + (unsigned long long) (ks * 16), idesc, acc0 || pass > 0 || ks > 0);
+            mma_tf32_ss(d, dA[0] + (unsigned long long) (ks * 16), dB[0] + (unsigned long long) (ks * 16), idesc2, acc0 || ks > 0);
+#pragma unroll
+          for (int ks = 0; ks < K / 8; ks++)
+            mma_tf32_ss(d + (unsigned) N, dA[1] + (unsigned long long) (ks * 16), dB[0] + (unsigned long long) (ks * 16), idesc, true);
+        } else {
+#pragma unroll
+          for (int pass = 0; pass < 3; pass++) {    // small terms first: a_lo b_hi, a_hi b_lo, a_hi b_hi
+            const unsigned long long a = dA[pass == 0 ? 1 : 0], b = dB[pass == 1 ? 1 : 0];
+#pragma unroll
+            for (int ks = 0; ks < K / 8; ks++)
+              mma_tf32_ss(d, a + (unsigned long long) (ks * 16), b + (unsigned long long) (ks * 16), idesc, acc0 || pass > 0 || ks > 0);
+          }
         }
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&s_empty[s])) : "memory");
         Cursor nx = cur;
@@ -514,8 +527,14 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
         for (int b = 0; b < nb; b++) {
           const int tt = b / nblk, c0 = (b - tt * nblk) * CB;
           float v[CB];
-          const unsigned at = tmem + ((unsigned) (ew * 32) << 16) + (unsigned) ((set * TB + tt) * op.sub * N + c0);
+          const unsigned at = tmem + ((unsigned) (ew * 32) << 16) + (unsigned) ((set * TB + tt) * op.sub * NC + c0);
           tmem_ld<CB>(at, v);
+          if constexpr (SEP) {
+            float w[CB];
+            tmem_ld<CB>(at + (unsigned) N, w);
+#pragma unroll
+            for (int q = 0; q < CB; q++) v[q] += w[q];
+          }
           __syncwarp();
 #pragma unroll
           for (int q = 0; q < CB / 4; q++)
@@ -576,29 +595,32 @@ size_t smem_bytes(int K, int N, int S)
 
 int stages_for(int K, int N) { return smem_bytes(K, N, 4) <= 200 * 1024 ? 4 : 2; }
 
-template<int K, int CB, int S, bool ELEM>
+template<int K, int CB, int S, bool ELEM, bool SEP = false>
 void launch_s(const MVTCDev &op, const TensorDev *T, int ntensors, int NA, int na, int TB, int tmem_cols, dim3 grid, int *error)
 {
   const size_t smem = smem_bytes(K, op.N, S);
   static size_t attr = 0;
   if (smem > attr) {
-    GB_CUDA(cudaFuncSetAttribute((mv_tc_kernel<K, CB, S, ELEM>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+    GB_CUDA(cudaFuncSetAttribute((mv_tc_kernel<K, CB, S, ELEM, SEP>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
     attr = smem;
   }
   const char *name = ELEM ? "mv_tc_element_kernel" : "mv_tc_kernel";
   before_launch(name);
-  mv_tc_kernel<K, CB, S, ELEM><<<grid, block_threads(K, ELEM), smem, dev().stream>>>(op, T, ntensors, NA, na, TB, tmem_cols, error);
+  mv_tc_kernel<K, CB, S, ELEM, SEP><<<grid, block_threads(K, ELEM), smem, dev().stream>>>(op, T, ntensors, NA, na, TB, tmem_cols, error);
   after_launch(name);
 }
 
 template<int K, bool ELEM> void launch_k(const MVTCDev &op, const TensorDev *T, int ntensors, int NA, int na, int TB, dim3 grid, int *error)
 {
   int tmem_cols = 32;    // a power of two that holds two sets of accumulators of TB tiles
-  while (tmem_cols < 2 * TB * op.sub * op.N) tmem_cols *= 2;
+  while (tmem_cols < 2 * TB * op.sub * op.N * (op.sep ? 2 : 1)) tmem_cols *= 2;
   const bool s4 = stages_for(K, op.N) == 4;
   if constexpr (ELEM) {
     if (s4) launch_s<K, 16, 4, true>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
     else launch_s<K, 16, 2, true>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+  } else if (op.sep) {    // (16 columns at a time: 32 of both accumulators do not fit the registers)
+    if (s4) launch_s<K, 16, 4, false, true>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+    else launch_s<K, 16, 2, false, true>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
   } else if (op.N % 32 == 0) {
     if (s4) launch_s<K, 32, 4, false>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
     else launch_s<K, 32, 2, false>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
@@ -871,7 +893,12 @@ void MVTensorCore::launch(const TensorDev *tensors, int ntensors, int NA, int na
   // left per-atom energies of GRACE-1L of order 4 at 1.8e-6 where fp32 sums are at 2.2e-7.  So every item has an accumulator of its
   // own, as many at a time as there are columns for, and the epilogue adds them with rounding, part of a row after part.
   op.sub = elem_ ? std::max(1, std::min(16, TMEM_COLS / 2 / N_)) : 1;
-  const int tb_max = elem_ ? 1 : std::max(1, std::min(MAX_TILES, TMEM_COLS / 2 / N_));
+  // Where the tiles of a CTA leave room for it, the small terms get accumulators of their own: a third of the instructions cut
+  // something off the large sum then (GRACE-3L, 54 atoms, per-atom energies against fp64: 1.4e-6 -> 7.0e-7, fp32 sums 4.8e-7).  With more
+  // atoms half as many tiles per CTA cost more than they give: 64 x 64, 1,024,000 atoms 27.8 -> 40.1 ms.
+  const int tb_sep = elem_ || 4 * N_ > TMEM_COLS ? 0 : std::min(MAX_TILES, TMEM_COLS / 4 / N_);
+  op.sep = ntiles <= G * tb_sep;
+  const int tb_max = elem_ ? 1 : op.sep ? tb_sep : std::max(1, std::min(MAX_TILES, TMEM_COLS / 2 / N_));
   const int rounds = (ntiles + G * tb_max - 1) / (G * tb_max);
   const int TB = std::max(1, std::min(tb_max, (ntiles + G * rounds - 1) / (G * rounds)));
   const int gx = std::min(G, (ntiles + TB - 1) / TB);

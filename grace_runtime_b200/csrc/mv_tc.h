@@ -20,6 +20,7 @@ struct MVTCDev {
   const char *images;      // per element and matrix: [N][K] tf32 hi image, then the lo image (canonical K-major layout)
   const int *order, *tiles;    // per-element weights: ElemOrder
   int N, nrows, nitems, nmat;
+  bool sep;                // accumulators of their own for the small terms
   int sub;                 // accumulators, one per item, that a part of a row has (per-element weights)
 };
 
