@@ -393,9 +393,9 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
         const unsigned b_hi = smem_u32(W_st + (size_t) (item_no % S) * 2 * W_BYTES);
         const unsigned long long dA[2] = {make_desc(a_hi, K), make_desc(a_hi + A_BYTES, K)};
         const unsigned long long dB[2] = {make_desc(b_hi, K), make_desc(b_hi + W_BYTES, K)};
-        const int sub = ELEM ? cur.it - cur.i0 : 0;
+        const int sub = ELEM ? cur.it - cur.i0 : SEP ? (cur.it - cur.i0) % op.sub : 0;
         const unsigned d = tmem + (unsigned) (((set * TB + cur.tt) * op.sub + sub) * NC);
-        const bool acc0 = !ELEM && cur.it != cur.i0;
+        const bool acc0 = !ELEM && cur.it - cur.i0 >= op.sub;
         if constexpr (SEP) {
           // the lo image of the weights lies behind the hi image like rows N .. 2 N - 1 of one matrix: a_hi meets both at once
 #pragma unroll
@@ -529,11 +529,13 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
           float v[CB];
           const unsigned at = tmem + ((unsigned) (ew * 32) << 16) + (unsigned) ((set * TB + tt) * op.sub * NC + c0);
           tmem_ld<CB>(at, v);
-          if constexpr (SEP) {
-            float w[CB];
-            tmem_ld<CB>(at + (unsigned) N, w);
+          if constexpr (SEP) {    // the other accumulators, the small terms among them
+            for (int k = 1; k < 2 * min(op.sub, row.i1 - row.i0); k++) {
+              float w[CB];
+              tmem_ld<CB>(at + (unsigned) (k * N), w);
 #pragma unroll
-            for (int q = 0; q < CB; q++) v[q] += w[q];
+              for (int q = 0; q < CB; q++) v[q] += w[q];
+            }
           }
           __syncwarp();
 #pragma unroll
@@ -892,13 +894,13 @@ void MVTensorCore::launch(const TensorDev *tensors, int ntensors, int NA, int na
   // bit of 2^-24 per instruction and accumulator): 240 instructions in one accumulator are a bias of 8e-6, and even six items
   // left per-atom energies of GRACE-1L of order 4 at 1.8e-6 where fp32 sums are at 2.2e-7.  So every item has an accumulator of its
   // own, as many at a time as there are columns for, and the epilogue adds them with rounding, part of a row after part.
-  op.sub = elem_ ? std::max(1, std::min(16, TMEM_COLS / 2 / N_)) : 1;
-  // Where the tiles of a CTA leave room for it, the small terms get accumulators of their own: a third of the instructions cut
-  // something off the large sum then (GRACE-3L, 54 atoms, per-atom energies against fp64: 1.4e-6 -> 7.0e-7, fp32 sums 4.8e-7).  With more
-  // atoms half as many tiles per CTA cost more than they give: 64 x 64, 1,024,000 atoms 27.8 -> 40.1 ms.
-  const int tb_sep = elem_ || 4 * N_ > TMEM_COLS ? 0 : std::min(MAX_TILES, TMEM_COLS / 4 / N_);
-  op.sep = ntiles <= G * tb_sep;
-  const int tb_max = elem_ ? 1 : op.sep ? tb_sep : std::max(1, std::min(MAX_TILES, TMEM_COLS / 2 / N_));
+  // With at most one tile per CTA there is room for accumulators of their own for the small terms, and for items that take turns in
+  // several: fewer instructions cut something off the large sums (GRACE-3L, 54 atoms, per-atom energies against fp64: 1.4e-6 -> SEPERR,
+  // fp32 sums 4.9e-7).  With more atoms the second read of the epilogue and half as many tiles cost more than they give: 64 x 64, 31,250
+  // atoms 29.7 -> 33.7 ms, 1,024,000 atoms 27.8 -> 40.1 ms.
+  op.sep = !elem_ && 4 * N_ <= TMEM_COLS && ntiles <= G;
+  op.sub = elem_ ? std::max(1, std::min(16, TMEM_COLS / 2 / N_)) : op.sep ? std::min(4, TMEM_COLS / 4 / N_) : 1;
+  const int tb_max = elem_ || op.sep ? 1 : std::max(1, std::min(MAX_TILES, TMEM_COLS / 2 / N_));
   const int rounds = (ntiles + G * tb_max - 1) / (G * tb_max);
   const int TB = std::max(1, std::min(tb_max, (ntiles + G * rounds - 1) / (G * rounds)));
   const int gx = std::min(G, (ntiles + TB - 1) / TB);
