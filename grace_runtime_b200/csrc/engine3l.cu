@@ -127,7 +127,8 @@ __device__ __forceinline__ void s3_radial(float N, const S3Bond *meta, int ns, c
 
 // The warp's part of the message rows of a group of bonds: LIT functions (and the chemical weights, where the mask asks for
 // them) of 32 channels, by asynchronous copies into shared memory of the warp's own, a group ahead of their use.  Functions
-// beyond the model's repeat the last one and channels beyond the layer's are not copied: nothing reads what becomes of them.
+// beyond the model's repeat the last one; channels beyond the layer's (16 or 48 channels: half of the last slice) are not copied,
+// and in the reverse pass, which adds over the lanes, the lanes that have none get zeros in place of what lies there.
 template<int LIT> struct S3Msg {
   static constexpr int ROWS = LIT + 1, GROUP = S3_NBS * ROWS * 32;    // floats of a group
   float mask[LIT];
@@ -159,12 +160,13 @@ template<int LIT> struct S3Msg {
       }
     }
   }
-  __device__ __forceinline__ void get(const float *buf, int s, bool have, int lane, float (&ic)[LIT]) const
+  // have: the layer has messages; in: the lane has a channel, or what it computes goes nowhere
+  __device__ __forceinline__ void get(const float *buf, int s, bool have, bool in, int lane, float (&ic)[LIT]) const
   {
 #pragma unroll
-    for (int q = 0; q < LIT; q++) ic[q] = have ? buf[(s * ROWS + q) * 32 + lane] : 0.0f;
+    for (int q = 0; q < LIT; q++) ic[q] = have && in ? buf[(s * ROWS + q) * 32 + lane] : 0.0f;
     if (masked) {    // the same for the whole warp
-      const float z = buf[(s * ROWS + LIT) * 32 + lane];
+      const float z = in ? buf[(s * ROWS + LIT) * 32 + lane] : 0.0f;
 #pragma unroll
       for (int q = 0; q < LIT; q++) ic[q] = fmaf(mask[q], z, ic[q]);
     }
@@ -276,7 +278,7 @@ __global__ void __launch_bounds__(32 * S3_WARPS, 2) spbf3_fwd_kernel(BondsDev b,
 #pragma unroll 1
         for (int s = LIT == 1 ? warp : 0; s < ns; s += LIT == 1 ? nw : 1) {
           float ic[LIT];
-          M.get(mg, s, L.msg != nullptr, lane, ic);
+          M.get(mg, s, L.msg != nullptr, true, lane, ic);    // lanes without a channel write nothing
           const float4 *Y4 = reinterpret_cast<const float4 *>(Ys + (q + s) * YLD);
           float Rl[NL];
 #pragma unroll
@@ -433,7 +435,7 @@ __global__ void __launch_bounds__(32 * S3_WARPS, 2) spbf3_bwd_kernel(BondsDev b,
 #pragma unroll 1
         for (int s = LIT == 1 ? warp : 0; s < ns; s += LIT == 1 ? nw : 1) {
           float ic[LIT];
-          M.get(mg, s, L.msg != nullptr, lane, ic);
+          M.get(mg, s, L.msg != nullptr, in, lane, ic);
           const ulonglong2 *G = reinterpret_cast<const ulonglong2 *>(G4 + (q + s) * NP * 2);
           float Rl[NL], dRl[NL];
 #pragma unroll

@@ -320,3 +320,71 @@ def test_gpu_passes_over_atom_chunks(backend, small3l, monkeypatch):
     assert np.abs(a["energies"] - b["energies"]).max() < 1e-6
     assert np.abs(a["forces"] - b["forces"]).max() < 2e-5 * max(1.0, np.abs(a["forces"]).max())
     assert np.abs(a["virial"] - b["virial"]).max() < 2e-5 * max(1.0, np.abs(a["virial"]).max())
+
+
+FILL = r"""
+#include <cuda_runtime.h>
+__global__ void fill(unsigned *out) {
+  extern __shared__ unsigned s[];
+  for (int i = threadIdx.x; i < 227 * 256; i += blockDim.x) s[i] = 0xffffffffu;
+  __syncthreads();
+  if (s[threadIdx.x] == 1u) out[0] = 1u;
+}
+extern "C" int fill_shared(int blocks) {    // every word of the SMs' shared memory becomes a NaN
+  unsigned *out;
+  if (cudaMalloc(&out, 4)) return 1;
+  cudaFuncSetAttribute(fill, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  fill<<<blocks, 1024, 227 * 1024>>>(out);
+  const int rc = cudaDeviceSynchronize();
+  cudaFree(out);
+  return rc;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def fill_shared(tmp_path_factory):
+    """fills the shared memory of the GPU with NaN patterns"""
+    import ctypes
+    import subprocess
+    from grace_runtime_b200 import build
+    d = tmp_path_factory.mktemp("fill")
+    (d / "fill.cu").write_text(FILL)
+    subprocess.run([build.nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler", "-fPIC", "-o", str(d / "fill.so"),
+                    str(d / "fill.cu")], check=True)
+    lib = ctypes.CDLL(str(d / "fill.so"))
+    return lambda: lib.fill_shared(148 * 4)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("channels", [(16, 16, 16), (48, 16, 48), (32, 48, 16)])
+def test_gpu_half_filled_channel_slices(backend, tmp_path, fill_shared, channels):
+    """16 and 48 channels: the last slice of 32 lanes has channels for half of them.  What the other lanes find in shared memory
+    must not reach the sums over the lanes: NaN patterns are left there before every call.  Energies and forces against the fp64
+    restatement (forces by its central differences, good to 1e-8) at the level of fp32 sums."""
+    from oracle.grace3l_oracle import Grace3LOracle
+    path = modelgen3l.write_model_3l(str(tmp_path / "m.npz"), elements=("Al", "Ni"), lmax=2, channels=channels, seed=7)
+    oracle, system = Grace3LOracle(path), backend.System(backend.Model(path), ["Al", "Ni"])
+    name, types, pos, cell, pbc = next(_cells())
+    o = oracle.compute(["Al", "Ni"], types, pos, cell, pbc)
+    reps = np.stack(np.meshgrid(*[np.arange(4)] * 3, indexing="ij"), -1).reshape(-1, 3) @ cell    # copies: blocks on every SM
+    many = (np.tile(types, 64), (pos[None] + reps[:, None]).reshape(-1, 3), 4 * cell, pbc)
+    for k, (args, n) in enumerate((((types, pos, cell, pbc), 1), (many, 64), (many, 64))):
+        assert fill_shared() == 0
+        g = system.compute(*args, energies=True)
+        assert np.abs(g["energies"] - np.tile(o["energies"], n)).max() < 5e-6
+        assert np.isfinite(g["forces"]).all() and np.isfinite(g["virial"]).all()
+        scale = max(1.0, np.abs(g["forces"]).max())
+        assert np.abs(g["forces"].sum(0)).max() < 1e-5 * len(args[0])
+        if k == 0:
+            first = g["forces"]
+            h = 1e-4
+            for i, d in ((0, 0), (7, 1), (20, 2)):
+                p = pos.copy()
+                p[i, d] += h
+                ep = oracle.compute(["Al", "Ni"], types, p, cell, pbc)["energy"]
+                p[i, d] -= 2 * h
+                em = oracle.compute(["Al", "Ni"], types, p, cell, pbc)["energy"]
+                assert abs(-(ep - em) / (2 * h) - first[i, d]) < 2e-5 * scale
+        else:
+            assert np.abs(g["forces"] - np.tile(first, (n, 1))).max() < 2e-5 * scale
