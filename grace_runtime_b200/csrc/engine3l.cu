@@ -628,6 +628,7 @@ __global__ void __launch_bounds__(128) rmsnorm_bwd_kernel(const float *__restric
   for (int c = lane; c < wr; c += 32) o[c] = c < n0 ? d[c] : (float) (r * d[c] * scale[c - n0] - k * xi[c]);
 }
 
+constexpr int RO_IN = 128, RO_HIDDEN = 256;    // most inputs and hidden units (build_plan refuses more)
 struct Readout3Dev {
   const double *W0, *W1, *shift;    // [nin][nh], [nh], [n_elements]
   double n0, n1, oscale;
@@ -638,8 +639,8 @@ struct Readout3Dev {
 __global__ void __launch_bounds__(128) readout3_kernel(Readout3Dev R, const float *__restrict__ sum, const int *__restrict__ mu,
                                                        double *__restrict__ e_atom, float *__restrict__ d, int want_grad, int n)
 {
-  __shared__ double s_ds[4][128];
-  __shared__ float s_h[4][128];
+  __shared__ double s_ds[4][RO_HIDDEN];
+  __shared__ float s_h[4][RO_IN];
   const int w = threadIdx.x >> 5, i = blockIdx.x * 4 + w, lane = threadIdx.x & 31;
   if (i >= n) return;
   const int wr = R.nin + 1;
@@ -765,6 +766,7 @@ void Engine::setup_3l()
   }
   S.pair_slot_host.assign((size_t) plan_.n_elements * plan_.n_elements, -1);
   S.pair_slot.upload(S.pair_slot_host);
+  if (Q.e_nin > RO_IN || Q.e_nh > RO_HIDDEN) throw Unsupported("GRACE-3L: the energy MLP is too wide");
   S.eW0.upload(Q.eW0);
   S.eW1.upload(Q.eW1);
   shift_.upload(plan_.shift);

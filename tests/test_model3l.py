@@ -388,3 +388,24 @@ def test_gpu_half_filled_channel_slices(backend, tmp_path, fill_shared, channels
                 assert abs(-(ep - em) / (2 * h) - first[i, d]) < 2e-5 * scale
         else:
             assert np.abs(g["forces"] - np.tile(first, (n, 1))).max() < 2e-5 * scale
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rho,hidden", [(16, 128), (16, 129), (32, 256), (128, 256)])
+def test_gpu_readout_widths(backend, tmp_path, rho, hidden):
+    """the energy MLP at the edges of its range: up to 127 inputs (the density has 128 channels at most) and 256 hidden units.
+    Energies against the fp64 restatement, forces by its central differences."""
+    from oracle.grace3l_oracle import Grace3LOracle
+    path = modelgen3l.write_model_3l(str(tmp_path / "m.npz"), elements=("Al", "Ni"), lmax=1, rho_width=rho, energy_hidden=hidden, seed=3)
+    oracle, system = Grace3LOracle(path), backend.System(backend.Model(path), ["Al", "Ni"])
+    name, types, pos, cell, pbc = next(_cells())
+    g, o = system.compute(types, pos, cell, pbc, energies=True), oracle.compute(["Al", "Ni"], types, pos, cell, pbc)
+    assert np.abs(g["energies"] - o["energies"]).max() < 5e-6
+    scale, h = max(1.0, np.abs(g["forces"]).max()), 1e-4
+    for i, d in ((0, 0), (7, 1), (20, 2), (31, 0)):
+        p = pos.copy()
+        p[i, d] += h
+        ep = oracle.compute(["Al", "Ni"], types, p, cell, pbc)["energy"]
+        p[i, d] -= 2 * h
+        em = oracle.compute(["Al", "Ni"], types, p, cell, pbc)["energy"]
+        assert abs(-(ep - em) / (2 * h) - g["forces"][i, d]) < 2e-5 * scale
