@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(32 * S3_WARPS, 2) spbf3_fwd_kernel(BondsDev b,
   S3Bond *meta = reinterpret_cast<S3Bond *>(Ys + S3_BB * YLD);     // [BB]
   const int nth = blockDim.x, nw = nth >> 5, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float *msg = reinterpret_cast<float *>(meta + S3_BB) + warp * 2 * S3Msg<LIT>::GROUP;    // [2] groups of the warp
-  const int ap = blockIdx.y, i = a0 + ap, c0 = blockIdx.x * 32, c = c0 + lane, C = L.C;
+  const int C = L.C, slices = (C + 31) / 32, ap = blockIdx.x / slices, i = a0 + ap, c0 = blockIdx.x % slices * 32, c = c0 + lane;
   const long long base = b.off[i];
   const int nb = b.cnt[i], mui = b.mu[i];
   const int pitch = LIT == 1 ? 1 : nw * LIT, nround = (L.nlmi + pitch - 1) / pitch;
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(32 * S3_WARPS, 2) spbf3_bwd_kernel(BondsDev b,
   __shared__ float red[2][S3_NBS * 4];
   __shared__ double vir[S3_NBS][6];
   const int nth = blockDim.x, nw = nth >> 5, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int ap = blockIdx.y, i = a0 + ap, c0 = blockIdx.x * 32, c = c0 + lane, C = L.C;
+  const int C = L.C, slices = (C + 31) / 32, ap = blockIdx.x / slices, i = a0 + ap, c0 = blockIdx.x % slices * 32, c = c0 + lane;
   const bool in = c < C;
   const long long base = b.off[i];
   const int nb = b.cnt[i], mui = b.mu[i];
@@ -840,7 +840,7 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
     d.nel = plan_.n_elements;
     return d;
   };
-  // launches of the bond kernels: a warp per 5 message functions (a layer without messages: 4 warps that share the bonds)
+  // launches of the bond kernels: a warp per S3_LIT message functions (a layer without messages: 4 warps that share the bonds)
   auto bonds_forward = [&](int k, float *A, int NC, int a0, int na) {
     const Layer3Plan &L = Q.L[k];
     const bool one = L.nlmi == 1;
@@ -848,7 +848,7 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
     const size_t group = (size_t) nw * 2 * S3_NBS * ((one ? 1 : S3_LIT) + 1) * 32;    // floats of the message buffers
     const size_t stage = sizeof(float) * (6 * (size_t) S3_NBS * nl * 32 + (size_t) S3_BB * ((np + 1) / 2 * 4) + group) + sizeof(S3Bond) * S3_BB;
     const size_t sums = sizeof(float) * 32 * (size_t) nlm * nw * (one ? 1 : S3_LIT), smem = std::max(stage, sums);
-    const dim3 grid((L.C + 31) / 32, na);
+    const unsigned grid = (unsigned) ((L.C + 31) / 32) * (unsigned) na;    // the slices of an atom side by side
     auto go = [&](auto kernel) {
       GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024));
       before_launch("spbf3_fwd_kernel");
@@ -871,7 +871,7 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
     const size_t grads = sizeof(float) * 32 * (size_t) ((np + 1) / 2 * 2) * nw * (one ? 1 : S3_LIT);
     const size_t smem = sizeof(float) * 32 * (size_t) L.nfA + std::max(stage, grads);
     if (smem > 200 * 1024) throw Unsupported("GRACE-3L: the bond sums of a layer do not fit the shared memory");
-    const dim3 grid((L.C + 31) / 32, na);
+    const unsigned grid = (unsigned) ((L.C + 31) / 32) * (unsigned) na;    // the slices of an atom side by side
     auto go = [&](auto kernel) {
       GB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
       before_launch("spbf3_bwd_kernel");

@@ -409,3 +409,21 @@ def test_gpu_readout_widths(backend, tmp_path, rho, hidden):
         p[i, d] -= 2 * h
         em = oracle.compute(["Al", "Ni"], types, p, cell, pbc)["energy"]
         assert abs(-(ep - em) / (2 * h) - g["forces"][i, d]) < 2e-5 * scale
+
+
+@pytest.mark.gpu
+def test_gpu_pass_of_more_than_65535_atoms(backend, tmp_path):
+    """70,200 atoms in one pass, copies of one cell: its energies and forces.  (The second and third dimension of a grid end at
+    65,535 blocks.)"""
+    from grace_runtime_b200 import structures
+    path = modelgen3l.write_model_3l(str(tmp_path / "m.npz"), elements=("Al", "Ni"), lmax=1, radial_hidden=16, seed=2)
+    types, pos, cell, pbc = structures.crystal("bcc", 3.2, (3, 3, 3), n_species=2, sigma=0.05, seed=4)
+    model = backend.Model(path)
+    one = backend.System(model, ["Al", "Ni"]).compute(types, pos, cell, pbc, energies=True)
+    reps = (10, 10, 13)
+    shift = np.stack(np.meshgrid(*[np.arange(k) for k in reps], indexing="ij"), -1).reshape(-1, 3) @ cell
+    p = (pos[None] + shift[:, None]).reshape(-1, 3)
+    r = backend.System(model, ["Al", "Ni"]).compute(np.tile(types, len(shift)), p, cell * np.array(reps)[:, None], pbc, energies=True)
+    assert np.abs(r["energies"] - np.tile(one["energies"], len(shift))).max() < 5e-6
+    assert np.abs(r["forces"] - np.tile(one["forces"], (len(shift), 1))).max() < 2e-5 * max(1.0, np.abs(one["forces"]).max())
+    assert np.abs(r["virial"] / len(shift) - one["virial"]).max() < 2e-5 * max(1.0, np.abs(one["virial"]).max())
