@@ -557,7 +557,7 @@ void Engine::gather_message_gradients(NeighborList &nl, const float *slots, cons
                          R.nlocal >= 0 ? nl.perm() : nullptr, R.nlocal);
 }
 
-void Engine::run(LayerEngine &E, bool forward, NeighborList &nl, const int *mu, int64_t a0, int na, int stride)
+void Engine::run(LayerEngine &E, bool forward, NeighborList &nl, NeighborList::Set set, const int *mu, int64_t a0, int na, int stride)
 {
   static const bool tag_ops = getenv("GRACE_B200_PROFILE_OPS") != nullptr;
   const auto &ts = E.plan->tensors;
@@ -573,7 +573,7 @@ void Engine::run(LayerEngine &E, bool forward, NeighborList &nl, const int *mu, 
     if (st.kind == Op::PROD) product(st.ops[0]);
     else if (tc_now_ && st.tc)
       st.tc->launch(E.tensors.get(), (int) E.tensors_host.size(), stride, na, tc_error_.get(),
-                    st.elem ? &nl.element_order(mu, a0, na, plan_.n_elements) : nullptr);
+                    st.elem ? &nl.element_order(set, mu, a0, na, plan_.n_elements) : nullptr);
     else
       for (int q : st.ops) launch_mv(E.mv[q], E.tensors.get(), mu, stride, na);
   }
@@ -894,13 +894,14 @@ void Engine::evaluate_chunked(NeighborList &nl, bool energy_only, int NA, StageT
   struct Span {
     int64_t lo, hi;
     const int *ilist, *mu;
+    NeighborList::Set set;
   };
-  Span s0{R.lo0, R.hi0, nullptr, nl.mu_sorted()}, s1{R.lo1, R.hi1, nullptr, nl.mu_sorted()};
+  Span s0{R.lo0, R.hi0, nullptr, nl.mu_sorted(), NeighborList::All}, s1{R.lo1, R.hi1, nullptr, nl.mu_sorted(), NeighborList::All};
   if (R.list0 && R.list1) {
     launch_gather_int(nl.mu_sorted(), R.list0, mu_l0_.ensure((size_t) std::max<int64_t>(R.n0, 1)), R.n0);
     launch_gather_int(nl.mu_sorted(), R.list1, mu_l1_.ensure((size_t) std::max<int64_t>(R.n1, 1)), R.n1);
-    s0 = Span{0, R.n0, R.list0, mu_l0_.get()};
-    s1 = Span{0, R.n1, R.list1, mu_l1_.get()};
+    s0 = Span{0, R.n0, R.list0, mu_l0_.get(), NeighborList::Owned};
+    s1 = Span{0, R.n1, R.list1, mu_l1_.get(), NeighborList::Inner};
   }
   // GRACE-2L with forces: layer 1 gets tensors of its own for all of its atoms in one pass when they fit, so that its
   // reverse pass finds the forward tensors where they were left instead of evaluating the layer a second time
@@ -951,14 +952,14 @@ void Engine::evaluate_chunked(NeighborList &nl, bool energy_only, int NA, StageT
       const int na = (int) std::min<int64_t>(NA, s0.hi - a0);
       if (tm) tm->begin(StageTimer::FWD);
       launch_bond_fwd(P.lmax, bonds0, L, T1(P.L1.tQ), NA, (int) a0, na);
-      run(L1_, true, nl, s0.mu + a0, a0, na, NA);
+      run(L1_, true, nl, s0.set, s0.mu + a0, a0, na, NA);
       if (uq_now_) uq_last(L1_, mu, a0, na, NA, n);
       launch_readout_1l(readout_, T1(P.t1_rho), T1(P.t1_grho), mu, e_atom_.get(), NA, na, (int) a0, !energy_only, s0.ilist);
       if (tm) tm->end(StageTimer::FWD);
       if (energy_only) continue;
       if (tm) tm->begin(StageTimer::BWD);
       zero_grads(L1_, arena_.get(), NA);
-      run(L1_, false, nl, s0.mu + a0, a0, na, NA);
+      run(L1_, false, nl, s0.set, s0.mu + a0, a0, na, NA);
       launch_bond_bwd(P.lmax, bonds0, L, T1(P.L1.tGQ), NA, (int) a0, na, fv, vir_atom_.get(), 0);
       if (tm) tm->end(StageTimer::BWD);
     }
@@ -982,7 +983,7 @@ void Engine::evaluate_chunked(NeighborList &nl, bool energy_only, int NA, StageT
     for (int64_t a0 = s1.lo; a0 < s1.hi; a0 += step1) {
       const int na = (int) std::min<int64_t>(step1, s1.hi - a0);
       { TagScope tg("layer1"); launch_bond_fwd(P.lmax, bonds1, La, T1(P.L1.tQ), S1, (int) a0, na); }
-      run(L1_, true, nl, s1.mu + a0, a0, na, S1);
+      run(L1_, true, nl, s1.set, s1.mu + a0, a0, na, S1);
       if (uq_now_) uq_layer1(mu + a0, a0, na, S1);
       launch_rows_from_chunk(T1(P.t1_I), I_rows_.get(), nI, CR, S1, na, (int) a0, s1.ilist);
       launch_rows_from_chunk(T1(P.t1_rho), rho_rows_.get(), 1, nrho, S1, na, (int) a0, s1.ilist);
@@ -994,7 +995,7 @@ void Engine::evaluate_chunked(NeighborList &nl, bool energy_only, int NA, StageT
       const int na = (int) std::min<int64_t>(NA, s0.hi - a0);
       if (tm) tm->begin(StageTimer::FWD);
       { TagScope tg("layer2"); launch_bond_fwd(P.lmax, bonds0, Lb, T2(P.L2.tQ), NA, (int) a0, na); }
-      run(L2_, true, nl, s0.mu + a0, a0, na, NA);
+      run(L2_, true, nl, s0.set, s0.mu + a0, a0, na, NA);
       if (uq_now_) uq_last(L2_, mu, a0, na, NA, n);
       launch_readout_2l(readout_, rho_rows_.get(), T2(P.t2_I2), grho_rows_.get(), T2(P.t2_gI2), mu, e_atom_.get(), NA,
                         na, (int) a0, !energy_only, s0.ilist);
@@ -1002,7 +1003,7 @@ void Engine::evaluate_chunked(NeighborList &nl, bool energy_only, int NA, StageT
       if (energy_only) continue;
       if (tm) tm->begin(StageTimer::BWD);
       zero_grads(L2_, arena_.get(), NA);
-      run(L2_, false, nl, s0.mu + a0, a0, na, NA);
+      run(L2_, false, nl, s0.set, s0.mu + a0, a0, na, NA);
       { TagScope tg("layer2"); launch_bond_bwd(P.lmax, bonds0, Lb, T2(P.L2.tGQ), NA, (int) a0, na, fv, vir_atom_.get(), 0); }
       if (tm) tm->end(StageTimer::BWD);
     }
@@ -1015,12 +1016,12 @@ void Engine::evaluate_chunked(NeighborList &nl, bool energy_only, int NA, StageT
         const int na = (int) std::min<int64_t>(step1, s1.hi - a0);
         if (!base1) {    // the tensors of layer 1 were overwritten by layer 2: evaluate it again
           launch_bond_fwd(P.lmax, bonds1, La, T1(P.L1.tQ), S1, (int) a0, na);
-          run(L1_, true, nl, s1.mu + a0, a0, na, S1);
+          run(L1_, true, nl, s1.set, s1.mu + a0, a0, na, S1);
         }
         zero_grads(L1_, abase1, S1);
         launch_chunk_from_rows(T1(P.t1_gI), gI_rows_.get(), nI, CR, S1, na, (int) a0, s1.ilist);
         launch_chunk_from_rows_f64(T1(P.t1_grho), grho_rows_.get(), 1, nrho, S1, na, (int) a0, s1.ilist);
-        run(L1_, false, nl, s1.mu + a0, a0, na, S1);
+        run(L1_, false, nl, s1.set, s1.mu + a0, a0, na, S1);
         { TagScope tg("layer1"); launch_bond_bwd(P.lmax, bonds1, La, T1(P.L1.tGQ), S1, (int) a0, na, fv, vir_atom_.get(), 1); }
       }
       if (tm) tm->end(StageTimer::BWD);
@@ -1080,6 +1081,7 @@ void Engine::evaluate(NeighborList &nl, bool energy_only, const OutputsDev &out,
                       const ActiveRanges *act, const ExchangeHooks *hooks)
 {
   hooks_ = plan_.layers == 2 ? hooks : nullptr;
+  nl.next_evaluation();
   const int64_t n = nl.n();
   const int nsys = nl.nsys();
   ActiveRanges R;

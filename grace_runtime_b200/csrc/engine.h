@@ -178,9 +178,9 @@ class Engine {
   void evaluate_chunked(NeighborList &nl, bool energy_only, int NA, StageTimer *tm, const ActiveRanges &R);
   void run_fused(LayerEngine &E, int mode, int NA, int a0, int na, const int *mu, const int *ilist, float *saved = nullptr);
   void bind_arena(LayerEngine &E, float *base, int NA);
-  // operations of one direction for `na` atoms with elements mu, chunk tensors of atom stride `stride`; list position a0 of
+  // operations of one direction for `na` atoms with elements mu, chunk tensors of atom stride `stride`; set and position in it of
   // the first atom (the grouping by element is kept with the list)
-  void run(LayerEngine &E, bool forward, NeighborList &nl, const int *mu, int64_t a0, int na, int stride);
+  void run(LayerEngine &E, bool forward, NeighborList &nl, NeighborList::Set set, const int *mu, int64_t a0, int na, int stride);
   void setup_steps(LayerEngine &E, const LayerPlan &P);
   DBuf<float> arena1_;               // chunk tensors of layer 1 for all of its atoms (GRACE-2L on the per-operation path)
   const float *arena1_bound_ = nullptr;

@@ -930,7 +930,7 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
     LayerEngine &E = S.E[k];
     const std::vector<TensorDev> &T = E.tensors_host;
     bonds_forward(k, T[L.tA].p, NC, a0, na);
-    run(E, true, nl, mu + a0, a0, na, NC);
+    run(E, true, nl, NeighborList::All, mu + a0, a0, na, NC);
     if (!outputs) return;
     if (k < 2) {
       const EqNormDev e{S.eq_dw[k].get(), S.eq_mask[k].get(), S.eq_aff[k].get(), S.eq_e[k].get(), L.nfEQ, L.cEQ, L.eq_center, L.eq_eps};
@@ -950,7 +950,7 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
       const EqNormDev e{S.eq_dw[k].get(), S.eq_mask[k].get(), S.eq_aff[k].get(), S.eq_e[k].get(), L.nfEQ, L.cEQ, L.eq_center, L.eq_eps};
       GB_LAUNCH(eqnorm_bwd_kernel, na, 32 * EQ_WARPS, 0, e, T[L.tEQ].p, S.gmsg[k].get(), T[L.tGEQ].p, NC, a0);
     }
-    run(E, false, nl, mu + a0, a0, na, NC);
+    run(E, false, nl, NeighborList::All, mu + a0, a0, na, NC);
     bonds_reverse(k, T[L.tGA].p, NC, a0, na);
   };
   for (int k = 0; k < 2; k++) S.msg[k].ensure((size_t) n * Q.L[k].nfEQ * Q.L[k].cEQ);

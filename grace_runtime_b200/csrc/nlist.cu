@@ -842,11 +842,15 @@ void NeighborList::export_host(std::vector<int> &bi, std::vector<int> &bj, std::
     }
 }
 
-const ElemOrder &NeighborList::element_order(const int *mu, int64_t a0, int na, int nel)
+const ElemOrder &NeighborList::element_order(Set set, const int *mu, int64_t a0, int na, int nel)
 {
-  for (const OrderOf &o : orders_)
-    if (o.mu == mu && o.a0 == a0 && o.na == na) return *o.order;
-  orders_.push_back(OrderOf{mu, a0, na, std::make_unique<ElemOrder>()});
+  for (OrderOf &o : orders_)
+    if (o.set == set && o.a0 == a0 && o.na == na) {
+      o.used = evaluation_;
+      return *o.order;
+    }
+  orders_.erase(std::remove_if(orders_.begin(), orders_.end(), [&](const OrderOf &o) { return o.used + 1 < evaluation_; }), orders_.end());
+  orders_.push_back(OrderOf{set, a0, na, evaluation_, std::make_unique<ElemOrder>()});
   orders_.back().order->make(mu, na, nel, std::min(kinds_, nel));
   return *orders_.back().order;
 }

@@ -55,8 +55,13 @@ class NeighborList {
   const double *build_positions() const { return xbuild_.get(); }    // device: the caller's positions of the last build
   // most different elements among the atoms (the species of the System or Batch)
   void set_kinds(int kinds) { kinds_ = kinds; }
-  // the atoms [0, na) of a chunk with elements mu (device), grouped by element; made once per list and chunk
-  const ElemOrder &element_order(const int *mu, int64_t a0, int na, int nel);
+  // The atoms [a0, a0 + na) of a set with elements mu (device, of the first of them), grouped by element.  Made once per list,
+  // set and chunk: the sets are the whole list and, for domain-decomposed callers, the two sets of active atoms that belong to
+  // the list.  next_evaluation() is called once per evaluation; what neither it nor the one before asked for is dropped when
+  // another grouping is made.
+  enum Set { All, Owned, Inner };
+  const ElemOrder &element_order(Set set, const int *mu, int64_t a0, int na, int nel);
+  void next_evaluation() { evaluation_++; }
   void release();
   size_t bytes() const;
   // diagnostics: the list of the last build (radius cutoff + skin) on the host, in the caller's atom order and frame:
@@ -65,12 +70,14 @@ class NeighborList {
 
  private:
   struct OrderOf {
-    const int *mu;
+    Set set;
     int64_t a0;
     int na;
+    uint64_t used;    // the last evaluation that asked for it
     std::unique_ptr<ElemOrder> order;
   };
   std::vector<OrderOf> orders_;    // of the present list
+  uint64_t evaluation_ = 0;
   int kinds_ = 1 << 30;
   int64_t n_ = 0, nslots_ = 0;
   int nsys_ = 0;

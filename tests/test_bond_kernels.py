@@ -91,3 +91,39 @@ def test_neighbor_search_on_both_sides_of_its_line(backend, tmp_path):
         r = backend.System(model, els).compute(np.tile(types, len(shift)), p, cell * np.array(reps)[:, None], pbc)
         assert abs(r["energy"] / len(shift) - one["energy"]) / len(types) < 1e-6
         assert _rel(r["forces"], np.tile(one["forces"], (len(shift), 1))) < 1e-5
+
+
+def test_groupings_stand_for_sets_of_atoms(backend, tmp_path):
+    """Domain-decomposed Systems of a model take turns.  Their element arrays live in buffers of the model that grow and move: when
+    the array of one set of a System's atoms comes to lie where the other set's was, its groupings by element must not be taken
+    for each other.  Blocks return through the pool of freed device memory; the sizes below make the move happen (a block is taken
+    by the first request that is not larger)."""
+    from grace_runtime_b200 import modelgen, structures
+    els = ["Al", "Cu", "Ni"]
+    path = modelgen.write_config_model(str(tmp_path / "m.npz"), "2l", els, seed=4)
+    c = structures.crystal("fcc", 3.6, (10, 10, 10), n_species=3, sigma=0.08, seed=5)
+
+    def system(model, n0, n1):
+        s = backend.System(model, els, chunksize=600)
+        s.set_owned(n0, n1)
+        return s
+
+    def energies(s):
+        return s.compute(*c, energy_only=True, energies=True)["energies"]
+    want = {sizes: energies(system(backend.Model(path), *sizes)) for sizes in ((650, 1400), (1200, 2500))}
+    model = backend.Model(path)
+    b = system(model, 610, 700)
+    energies(b)
+    spare = [system(model, 610, 700) for _ in range(6)]    # small blocks for the small requests below
+    for s in spare:
+        energies(s)
+    a = system(model, 650, 1400)
+    assert np.abs(energies(a) - want[650, 1400]).max() < 1e-6
+    e = system(model, 610, 1250)
+    energies(e)
+    del s, spare, e             # small blocks, and one for the list of owned atoms that b gets below
+    b.set_owned(650, 2500)      # the inner atoms' array grows: the block of a's inner atoms becomes free
+    energies(b)
+    b.set_owned(1200, 2500)     # the owned atoms' array grows, into that block
+    assert np.abs(energies(b) - want[1200, 2500]).max() < 1e-6
+    assert np.abs(energies(a) - want[650, 1400]).max() < 1e-6
