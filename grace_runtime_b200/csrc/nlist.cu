@@ -86,31 +86,32 @@ __global__ void __launch_bounds__(SCAN_T) scan_tile_final(const int *__restrict_
 __global__ void __launch_bounds__(1024) scan_small(const int *__restrict__ in, long long *out, int n)
 {
   constexpr int PER = SCAN_SMALL / 1024;
-  __shared__ int warp_sum[32];
+  __shared__ long long warp_sum[32];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5, t0 = t * PER;
-  int v[PER], s = 0;
+  int v[PER];
+  long long s = 0;
 #pragma unroll
   for (int k = 0; k < PER; k++) {
     v[k] = t0 + k < n ? in[t0 + k] : 0;
     s += v[k];
   }
-  int inc = s;    // inclusive scan of the thread sums
+  long long inc = s;    // inclusive scan of the thread sums
   for (int d = 1; d < 32; d <<= 1) {
-    const int o = __shfl_up_sync(0xffffffffu, inc, d);
+    const long long o = __shfl_up_sync(0xffffffffu, inc, d);
     if (lane >= d) inc += o;
   }
   if (lane == 31) warp_sum[warp] = inc;
   __syncthreads();
   if (warp == 0) {
-    int w = warp_sum[lane];
+    long long w = warp_sum[lane];
     for (int d = 1; d < 32; d <<= 1) {
-      const int o = __shfl_up_sync(0xffffffffu, w, d);
+      const long long o = __shfl_up_sync(0xffffffffu, w, d);
       if (lane >= d) w += o;
     }
     warp_sum[lane] = w;
   }
   __syncthreads();
-  int run = inc - s + (warp > 0 ? warp_sum[warp - 1] : 0);
+  long long run = inc - s + (warp > 0 ? warp_sum[warp - 1] : 0);
 #pragma unroll
   for (int k = 0; k < PER; k++) {
     if (t0 + k < n) out[t0 + k] = run;
@@ -123,7 +124,6 @@ __global__ void __launch_bounds__(1024) scan_small(const int *__restrict__ in, l
 
 void launch_scan(const int *in, long long *out, long long *tmp, int64_t n)
 {
-  // (a count is below 2^31 / SCAN_SMALL here: a bin holds at most n atoms, an atom far fewer than 2^17 neighbours)
   if (n <= SCAN_SMALL) {
     GB_LAUNCH(scan_small, 1, 1024, 0, in, out, (int) n);
     return;

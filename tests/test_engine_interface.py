@@ -115,3 +115,21 @@ def test_engine_run_rejects_bad_tables(backend, cells):
     tab = torch.full((n, 2), n + 5, dtype=torch.int32, device=dev)
     with pytest.raises(ValueError):
         eng.run(n, n, d_t, d_x, nn, tab, 2, d_f)                       # an index outside the atoms
+
+
+def test_engine_run_refuses_tables_past_the_index_range(backend):
+    """8,192 atoms (the scan of one block) with more than 2^31 table entries in all: refused before the table is looked at.  Sums
+    in 32 bits would wrap to a small number."""
+    import torch
+    n, width = 8192, (1 << 18) + 1
+    eng = backend.Engine(backend.Model(model_path("grace_1l_order3")), ["W"])
+    dev = torch.device("cuda", 0)
+    table = torch.empty((n, width), dtype=torch.int32, device=dev)     # 8.6 GB, never read
+    try:
+        with pytest.raises(RuntimeError, match="2\\^31"):
+            eng.run(n, n, torch.ones(n, dtype=torch.int32, device=dev), torch.rand((n, 3), dtype=torch.float64, device=dev),
+                    torch.full((n,), width, dtype=torch.int32, device=dev), table, width,
+                    torch.zeros((n, 3), dtype=torch.float64, device=dev))
+    finally:
+        del table
+        torch.cuda.empty_cache()
