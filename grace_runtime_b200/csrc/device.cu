@@ -167,6 +167,14 @@ void device_pool_trim()
   g_pool_bytes = 0;
 }
 
+size_t device_free_bytes()
+{
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = (size_t) 8 << 30;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  return free_b + g_pool_bytes;
+}
+
 void *device_alloc(size_t bytes, const char *label)
 {
   require_initialized();

@@ -75,6 +75,8 @@ std::string profile_report();
 void *device_alloc(size_t bytes, const char *label);
 void device_free(void *p);
 void device_pool_trim();
+// memory a request of the library can get: what the driver has free and what lies in the pool
+size_t device_free_bytes();
 
 // a device array that grows on demand (contents are not kept across a grow)
 template<class T> class DBuf {

@@ -478,9 +478,7 @@ int Engine::auto_chunk(int64_t n) const
   // what the work buffer already holds, or is small on this GPU, needs no look at the free memory (a driver call of 10 us, at
   // times of 10 ms; should it not fit all the same, the call is repeated with smaller passes)
   if ((double) most * per <= std::max(held, SMALL_WORK)) return (int) most;
-  size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = (size_t) 8 << 30;
-  const int64_t c = (int64_t) ((0.35 * (double) free_b + held) / per);
+  const int64_t c = (int64_t) ((0.35 * (double) device_free_bytes() + held) / per);
   return (int) std::min<int64_t>(std::max<int64_t>(n, 1), std::max<int64_t>(std::min(c, most), 512));
 }
 
@@ -909,11 +907,10 @@ void Engine::evaluate_chunked(NeighborList &nl, bool energy_only, int NA, StageT
   int NA1 = 0;
   if (P.layers == 2 && !energy_only && keep_l1_ && s1.hi > s1.lo) {
     const int64_t w1 = (s1.hi - s1.lo + 3) / 4 * 4;
-    size_t free_b = 0, total_b = 0;
     const size_t need = (size_t) L1_.per_atom * (size_t) w1 * sizeof(float);
     const size_t held = arena1_.capacity() * sizeof(float);
     if (w1 < ((int64_t) 1 << 30) &&
-        (need <= std::max(held, (size_t) SMALL_WORK) || (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && need <= (size_t) (0.45 * (double) free_b) + held))) {
+        (need <= std::max(held, (size_t) SMALL_WORK) || need <= (size_t) (0.45 * (double) device_free_bytes()) + held)) {
       try {
         base1 = arena1_.ensure((size_t) L1_.per_atom * (size_t) w1);
         NA1 = (int) w1;

@@ -898,11 +898,7 @@ void Engine::evaluate_3l(NeighborList &nl, bool energy_only, StageTimer *tm)
   for (int k = 0; k < 3; k++) held = held && (double) S.E[k].per_atom * NA <= (double) S.arena[k].capacity();
   double budget = 0.0;
   for (int k = 0; k < 3; k++) budget += 4.0 * (double) S.arena[k].capacity();
-  if (!held) {
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = (size_t) 8 << 30;
-    budget += 0.7 * (double) free_b;
-  }
+  if (!held) budget += 0.7 * (double) device_free_bytes();
   if (const char *env = getenv("GRACE_B200_3L_CHUNK")) budget = std::min(budget, 4.0 * per_all * std::max(4, atoi(env)) - 1.0);
   const bool keep = 4.0 * (double) per_all * NA <= budget;
   int NC = NA;    // atoms per pass (a multiple of 4: the atom stride of the arena)

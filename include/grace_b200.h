@@ -56,7 +56,11 @@ const char *grace_arch(void);                  /* arch(): "sm100" */
 const char *grace_platform(void);              /* platform(): "cuda" */
 const char *grace_blas(void);                  /* blas(): "" (no GEMM library on the path) */
 int grace_abi(void);                           /* the module attribute ABI */
-int grace_memory_info(size_t *free_bytes, size_t *total_bytes);   /* memory_info() */
+/* memory_info(): the driver's numbers.  Device blocks that the library has freed stay with it for later calls, blocks of up to
+ * 1 GiB, at most 4 GiB together: they are not free here.  grace_system_release_buffers, grace_batch_release_buffers,
+ * grace_model_free and grace_finalize give them back to the driver, and so does an allocation of the library that fails; a host
+ * that shares the GPU with another allocator calls one of the first two before it hands the memory on. */
+int grace_memory_info(size_t *free_bytes, size_t *total_bytes);
 /* tests: the nth device allocation from now on whose label contains `label` fails as out of memory (nth <= 0: off) */
 int grace_debug_fail_alloc(const char *label, int nth);           /* debug_fail_alloc(label, nth) */
 /* tests: the nth kernel launch check from now on reports an out-of-memory launch (0: off) */

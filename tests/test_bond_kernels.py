@@ -127,3 +127,33 @@ def test_groupings_stand_for_sets_of_atoms(backend, tmp_path):
     b.set_owned(1200, 2500)     # the owned atoms' array grows, into that block
     assert np.abs(energies(b) - want[1200, 2500]).max() < 1e-6
     assert np.abs(energies(a) - want[650, 1400]).max() < 1e-6
+
+
+def test_freed_blocks_count_as_free_memory(backend, tmp_path):
+    """Work buffers that a Batch has given back stay in the library's pool.  The automatic pass size of a later call is the one that
+    it gets after the pool was returned to the driver (3 %: what else the first call left on the GPU)."""
+    import torch
+    from grace_runtime_b200 import modelgen, structures
+    path = modelgen.write_config_model(str(tmp_path / "m.npz"), "1l", ["W"], seed=6)
+    model = backend.Model(path)
+    big = structures.crystal("bcc", 3.2, (50, 50, 48), seed=1)
+    backend.System(model, ["W"]).release_buffers()
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (10 << 30), dtype=torch.uint8, device="cuda")
+    try:
+        for reps in ((10, 10, 100), (10, 10, 130), (10, 10, 155)):
+            types, pos, cell, pbc = structures.crystal("bcc", 3.2, reps, seed=1)
+            backend.Batch(model, ["W"]).compute(np.array([len(types)], dtype=np.int32), types, pos, cell[None], pbc[None], energy_only=True)
+        before = torch.cuda.mem_get_info()[0]
+        chunks = []
+        for _ in range(2):
+            system = backend.System(model, ["W"])
+            system.compute(*big, energy_only=True)
+            chunks.append(system.chunksize)
+            system.release_buffers()
+            del system
+        assert before < 9 << 30      # the pool held more than a GB
+        assert 0 < chunks[1] < len(big[0]) and abs(chunks[0] - chunks[1]) < 0.03 * chunks[1], chunks
+    finally:
+        del fill
+        torch.cuda.empty_cache()
