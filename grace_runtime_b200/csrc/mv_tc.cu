@@ -26,7 +26,6 @@
 #include "mv_tc.h"
 
 #include <algorithm>
-#include <cstdio>
 #include <cstring>
 #include <map>
 
@@ -300,15 +299,8 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
     if (nxt.valid) load_tile(nxt, regsB);
     int fill = 0, item_no = -1;
     bool ok = true;
-#ifdef GB_TC_TIMING
-    long long tp_[4] = {0, 0, 0, 0}, tq_ = clock64();
-#define GB_TICK(a, i) do { const long long now_ = clock64(); a[i] += now_ - tq_; tq_ = now_; } while (0)
-#else
-#define GB_TICK(a, i) do {} while (0)
-#endif
     // one fill: `mine` holds the tile at `cur`; after its conversion it receives the tile two fills ahead
     auto step = [&](TR &mine) {
-      GB_TICK(tp_, 3);
       nxt2 = nxt;
       if (nxt.valid) advance(nxt2);
       const int s = fill % S;
@@ -317,7 +309,6 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
         ok = wait(&s_empty[s], (unsigned) ((fill / S - 1) & 1));
         if (!ok) return;
       }
-      GB_TICK(tp_, 0);
       const MVItem item = s_items[cur.it];
       if (ELEM || cur.tt == 0) {    // first tile of an item (every tile of its own element): its weight image (hi + lo)
         item_no++;
@@ -346,11 +337,9 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
           }
         }
       }
-      GB_TICK(tp_, 1);
       if (nxt2.valid) load_tile(nxt2, mine);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&s_full[s])) : "memory");
-      GB_TICK(tp_, 2);
       fill++;
       cur = nxt;
       nxt = nxt2;
@@ -360,11 +349,6 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
       if (!cur.valid || !ok) break;
       step(regsB);
     }
-#ifdef GB_TC_TIMING
-    if (t == 0 && blockIdx.x == 1 && blockIdx.y == 0)
-      printf("mv_tc K %d N %d S %d TB %d fills %d producer: wait-empty %lld W+convert %lld loads+arrive %lld other %lld\n", K, N, S, TB, fill,
-             tp_[0], tp_[1], tp_[2], tp_[3]);
-#endif
   } else if (warp == NW) {
     // ---------------- matrix-instruction issuer ----------------
     if (lane == 0) {
@@ -373,21 +357,15 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
       start(cur, blockIdx.x * TB, blockIdx.y);
       int fill = 0, item_no = -1, rowc = 0;
       bool ok = true;
-#ifdef GB_TC_TIMING
-      long long tm_[4] = {0, 0, 0, 0}, tq_ = clock64();
-#endif
       while (cur.valid && ok) {
-        GB_TICK(tm_, 3);
         const int s = fill % S, set = rowc & 1;
         if (ELEM || cur.tt == 0) item_no++;
         if (cur.it == cur.i0 && cur.tt == 0 && rowc >= 2) {    // first fill of a row: its accumulators were read out
           ok = wait(&s_accempty[set], (unsigned) ((rowc / 2 - 1) & 1));
           if (!ok) break;
         }
-        GB_TICK(tm_, 0);
         ok = wait(&s_full[s], (unsigned) ((fill / S) & 1));
         if (!ok) break;
-        GB_TICK(tm_, 1);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const unsigned a_hi = smem_u32(A_st + (size_t) s * 2 * A_BYTES);
         const unsigned b_hi = smem_u32(W_st + (size_t) (item_no % S) * 2 * W_BYTES);
@@ -422,12 +400,7 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
         }
         fill++;
         cur = nx;
-        GB_TICK(tm_, 2);
       }
-#ifdef GB_TC_TIMING
-      if (blockIdx.x == 1 && blockIdx.y == 0)
-        printf("mv_tc K %d N %d issuer: wait-accempty %lld wait-full %lld issue %lld other %lld\n", K, N, tm_[0], tm_[1], tm_[2], tm_[3]);
-#endif
     }
   } else {
     // ---------------- epilogue: tensor memory -> global, once per output row ----------------
@@ -441,14 +414,10 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
     start(cur, blockIdx.x * TB, blockIdx.y);
     int rowc = 0;
     bool ok = true;
-#ifdef GB_TC_TIMING
-    long long te_[2] = {0, 0}, tq_ = clock64();
-#endif
     while (cur.valid && ok) {
       const int set = rowc & 1;
       ok = wait(&s_accfull[set], (unsigned) ((rowc / 2) & 1));
       if (!ok) break;
-      GB_TICK(te_, 0);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const MVRowDev row = s_rows[cur.row];
       const TensorDev dstT = s_T[row.dst];
@@ -575,12 +544,7 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&s_accempty[set])) : "memory");
       rowc++;
       next_row(cur);
-      GB_TICK(te_, 1);
     }
-#ifdef GB_TC_TIMING
-    if (warp == NW + 1 && lane == 0 && blockIdx.x == 1 && blockIdx.y == 0)
-      printf("mv_tc K %d N %d epilogue: wait-accfull %lld work %lld rows %d\n", K, N, te_[0], te_[1], rowc);
-#endif
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
