@@ -5,19 +5,32 @@
 //     D[128 atoms][n_out] = sum_items X_item[128 atoms][K] . W_item[K][n_out],
 // with X_item a contiguous block of the source tensor.  A CTA owns up to 256 / n_out atom tiles at a time and keeps two
 // sets of fp32 accumulators for them in tensor memory; for every item of the row its producer warps write the tile's
-// activations as hi + lo operand images into a ring of shared-memory stages (canonical K-major layout, 8-row x 16-byte
-// core matrices), the item's weight image (split once when the model is loaded) arrives by one bulk asynchronous copy, and
-// one thread issues tcgen05.mma kind::tf32 M = 128, N = n_out: a b ~ a_lo b_hi + a_hi b_lo + a_hi b_hi keeps fp32-level
-// accuracy.  The global loads of the next two tiles are in flight in registers while a tile is written, all items of a
+// activations as three bf16 operand images into a ring of shared-memory stages (canonical K-major layout, 8-row x 16-byte
+// core matrices), the item's weight images (split once when the model is loaded) arrive by one bulk asynchronous copy, and
+// one thread issues tcgen05.mma kind::f16 M = 128, N = n_out, K = 16.
+// Accuracy.  x = x1 + x2 + x3, each part the bf16 nearest to what the ones before leave, is all 24 bits of an fp32 number, and
+//     a b ~ a3 b1 + a1 b3 + a2 b2 + a2 b1 + a1 b2 + a1 b1
+// leaves out 2^-26 of a b.  The accumulators cut off what does not fit their 24 bits, with a bias towards zero that a sum over
+// many atoms keeps; the products a1 b1 have 16 bits, so that adding them among themselves cuts off little, and where fp32 sums are
+// the measure the five small products go to an accumulator of their own (SEP), which the epilogue adds with rounding.
+// Two tf32 parts take as many instructions (half as wide in K) and more shared memory, but are 22 bits of an operand with products of
+// 22.  Errors against fp64 (2-norm, several structures; fp32 FMA kernels / two tf32 parts / this): per-atom energies of GRACE-1L of
+// order 4, 588 atoms 3.9e-7 / 3.0e-7 / 2.6e-7, GRACE-2L, 600 atoms 3.8e-7 / 3.8e-7 / 3.5e-7, GRACE-3L, 54 atoms 2.9e-7 / 4.7e-7 /
+// 2.4e-7, forces along random directions 7.0e-7 / 1.4e-6 / 6.5e-7; extrapolation grade of GRACE-2L, 600 atoms 3.0e-8 / 4.7e-7 / 2.6e-8;
+// virial of GRACE-2L, 600 atoms 5.8e-7 / 2.0e-6 / 5.4e-7.  Above 18,944 atoms (no SEP): GRACE-2L energies 2.5e-7 / 2.7e-7 / 2.0e-7, forces
+// 6.2e-7 / 6.1e-7 / 5.3e-7; GRACE-3L energies 1.22e-6 / 1.23e-6 / 1.17e-6 (the first figure with two tf32 parts in all but the
+// per-element sums).  Times are those of two tf32 parts within 0.3 %; SEP at all sizes would bring the last figure to 3.0e-7 and costs 2 % (GRACE-2L,
+// 1,024,000 atoms 222.6 -> 227.5 ms) to 5 % (GRACE-1L, 128,000 atoms).
+// The global loads of the next two tiles are in flight in registers while a tile is written, all items of a
 // row accumulate in tensor memory, and the epilogue warps write each output row once while the next row's matrix
 // instructions run.
 // Widths are padded with zeros to K = 16, 32 or 64 and N a multiple of 16, so every operation of up to 64 inputs runs here.
 // Operations whose weights depend on the central atom's element (the reduces to densities and messages, their adjoints) take
 // tiles of atoms of ONE element: the atoms are gathered through an index (ElemOrder) that groups them by element, a row of
-// 9 - 64 channels each, and the weight image is chosen per tile.  With the elements mixed in a tile the weights of every
+// 9 - 64 channels each, and the weight images are chosen per tile.  With the elements mixed in a tile the weights of every
 // element present passed through shared memory: 557,000 atoms of 89 elements 82 ms, 1,024,000 atoms of 3 elements 20.7 ms per
-// evaluation of GRACE-2L; grouped 11.0 and 17.7 ms.
-// Independent operations of the same shape are one launch (plan.h MVGroup): rows carry their tensor and whether they add.
+// evaluation of GRACE-2L; grouped 9.3 and 16.2 ms.
+// Independent operations of the same shape are one launch (Engine::setup_steps): rows carry their tensor and whether they add.
 // Same mathematics as mv_kernel (chain.cu); reference: fc_fwd / mv_batch, libgrace/include/grace/fused_cpu.h:294-356,
 // GPU fc_fwd4 libgrace/include/grace/kk/fused_dense.h:441-495.
 //
@@ -42,41 +55,47 @@ constexpr int MAX_TENSORS = 64;
 constexpr int MAX_ITEMS = MVTensorCore::MAX_ITEMS, MAX_ROWS = MVTensorCore::MAX_ROWS;    // tables of an operation staged in shared memory
 constexpr long long WAIT_CYCLES = 40000000LL;    // ~20 ms: far beyond any tile, far below a watchdog
 
-// byte offset of element (r, k) of a K-major operand tile with K columns (canonical layout, no swizzle)
-__host__ __device__ inline int tile_off(int r, int k, int K) { return (r >> 3) * (K >> 2) * 128 + (k >> 2) * 128 + (r & 7) * 16 + (k & 3) * 4; }
+constexpr int LONG_ROW = 16;    // items of a row from which on it goes in parts while fp32 sums are the measure
+constexpr int PARTS = 3;        // bf16 numbers an fp32 operand is split into
+// the products of parts (activation, weight) that are formed, small ones first
+__device__ constexpr int PRODUCTS[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};
+
+// byte offset of element (r, k) of a K-major bf16 operand tile with K columns (canonical layout, no swizzle)
+__host__ __device__ inline int tile_off(int r, int k, int K) { return (r >> 3) * (K >> 3) * 128 + (k >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2; }
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned) __cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ unsigned long long make_desc(unsigned addr, int K)
 {
-  const unsigned long long lbo = 128 >> 4, sbo = ((K >> 2) * 128) >> 4;
+  const unsigned long long lbo = 128 >> 4, sbo = ((K >> 3) * 128) >> 4;
   return (unsigned long long) ((addr & 0x3ffff) >> 4) | (lbo << 16) | (sbo << 32) | (1ull << 46);
 }
 
-// fp32 accumulate, tf32 x tf32, both operands K-major, M = 128, N = n
-__device__ __forceinline__ unsigned make_idesc(int n) { return (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned) (n >> 3) << 17) | ((unsigned) (TM >> 4) << 24); }
+// fp32 accumulate, bf16 x bf16, both operands K-major, M = 128, N = n
+__device__ __forceinline__ unsigned make_idesc(int n) { return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned) (n >> 3) << 17) | ((unsigned) (TM >> 4) << 24); }
 
-__device__ __forceinline__ void mma_tf32_ss(unsigned tmem_d, unsigned long long da, unsigned long long db, unsigned idesc, bool accumulate)
+__device__ __forceinline__ void mma_bf16_ss(unsigned tmem_d, unsigned long long da, unsigned long long db, unsigned idesc, bool accumulate)
 {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-               "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
                ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"((unsigned) accumulate) : "memory");
 }
 
-// hi + lo split of four activations for the 3 x tf32 product.  The tensor cores read the upper 19 bits of an fp32
-// operand (sign, exponent, 10 mantissa bits) and ignore the rest, so `hi` is the value itself and lo = x - trunc(x) is
-// exact in fp32; lo in turn is rounded to what is read by an integer addition, which leaves a relative error of 2^-22 of x - the
-// size of the a_lo b_lo term the scheme drops anyway - without a sign that it prefers.  Three instructions per value and none of
-// them a conversion.
-__device__ __forceinline__ void split4(float4 x, float sc, float4 &hi, float4 &lo)
+// four activations in their bf16 parts, 8 bytes per part; the differences are exact in fp32
+__device__ __forceinline__ void split4(float4 x, float sc, uint2 (&part)[PARTS])
 {
-  const float v[4] = {x.x * sc, x.y * sc, x.z * sc, x.w * sc};
-  float l[4];
+  float v[4] = {x.x * sc, x.y * sc, x.z * sc, x.w * sc};
 #pragma unroll
-  for (int q = 0; q < 4; q++)    // + half a unit of what is read: lo is rounded to nearest instead of cut off
-    l[q] = __uint_as_float(__float_as_uint(v[q] - __uint_as_float(__float_as_uint(v[q]) & 0xffffe000u)) + 0x1000u);
-  hi = make_float4(v[0], v[1], v[2], v[3]);
-  lo = make_float4(l[0], l[1], l[2], l[3]);
+  for (int p = 0; p < PARTS; p++) {
+    unsigned r[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r[q]) : "f"(v[2 * q + 1]), "f"(v[2 * q]));    // the second operand to the lower half
+      v[2 * q] -= __uint_as_float(r[q] << 16);
+      v[2 * q + 1] -= __uint_as_float(r[q] & 0xffff0000u);
+    }
+    part[p] = make_uint2(r[0], r[1]);
+  }
 }
 
 template<int NC> __device__ __forceinline__ void tmem_ld(unsigned taddr, float (&v)[NC]);
@@ -140,8 +159,8 @@ template<int K> struct TileRegs {
   float4 v[PER];
 };
 
-// Warp-specialised: warps 0-7 produce (global loads two tiles ahead in registers, tf32 hi / lo operand images of a tile
-// into one of S shared-memory stages, the weight image of an item into a ring of S buffers), warp 8 issues the matrix
+// Warp-specialised: warps 0-7 produce (global loads two tiles ahead in registers, the operand images of a tile
+// into one of S shared-memory stages, the weight images of an item into a ring of S buffers), warp 8 issues the matrix
 // instructions (one thread; nothing else runs on its critical path), the warps from 9 on move finished accumulators from tensor
 // memory to global memory.  Two sets of accumulators (TB tiles x n_out columns each) take turns, so the epilogue of a
 // row overlaps the matrix instructions of the next.  Hand-offs are mbarriers: full[s] (256 producer arrivals) / empty[s]
@@ -149,12 +168,12 @@ template<int K> struct TileRegs {
 // epilogue thread).  A wait that runs out raises `abort`, which every other wait sees, and all roles leave together.
 constexpr int NPROD = NTH;
 // grouped atoms: two epilogue warps per quarter of the lanes (the sums over several accumulators and the scattered rows take longer
-// than the matrix instructions of a row: 1,024,000 atoms, 16 inputs, 9.4 -> 6.3 ms).  17 warps leave 96 registers per thread, not
+// than the matrix instructions of a row: 1,024,000 atoms, 16 inputs, 9.4 -> 6.3 ms; 7.1 with the accumulator of the small products).  17 warps leave 96 registers per thread, not
 // enough for producers that hold two tiles of 64 channels (1.87 -> 2.13 ms) or for the other epilogue
 __host__ __device__ constexpr int epilogue_threads(int K, bool elem) { return elem && K < 64 ? 256 : 128; }
 __host__ __device__ constexpr int block_threads(int K, bool elem) { return NTH + 32 + epilogue_threads(K, elem); }
 
-// SEP: the two small terms of the product have accumulators of their own beside a_hi b_hi (columns N .. 2 N - 1).
+// SEP: the small products have an accumulator of their own behind the op.sub accumulators of a1 b1.
 template<int K, int CB, int S, bool ELEM, bool SEP>
 __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDev op, const TensorDev *__restrict__ Tg, int ntensors, int NA,
                                                             int na, int TB, int tmem_cols, int *error)
@@ -162,7 +181,7 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
   using TR = TileRegs<K>;
   constexpr int K4 = TR::K4, UNITS = TR::UNITS, PER = TR::PER;
   constexpr int NEPI = epilogue_threads(K, ELEM), NTHREADS = block_threads(K, ELEM);
-  constexpr int A_BYTES = TM * K * 4;    // one image (hi or lo) of an activation tile
+  constexpr int A_BYTES = TM * K * 2;    // one image (part) of an activation tile
   extern __shared__ __align__(1024) char smem[];
   __shared__ unsigned long long s_full[S], s_empty[S], s_accfull[2], s_accempty[2];
   __shared__ unsigned s_tmem;
@@ -172,11 +191,11 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
   __shared__ MVItem s_items[MAX_ITEMS];
   __shared__ MVRowDev s_rows[MAX_ROWS];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const int N = op.N, NC = SEP ? 2 * N : N;    // columns of an accumulator
-  const int W_BYTES = N * K * 4;                         // one image of a weight matrix
-  char *A_st = smem;                                     // stage s at s * 2 * A_BYTES: hi, then lo
-  char *W_st = smem + (size_t) S * 2 * A_BYTES;          // buffer b at b * 2 * W_BYTES: hi, then lo
-  float *tr_all = reinterpret_cast<float *>(W_st + (size_t) S * 2 * W_BYTES);    // transpose buffers of the epilogue warps
+  const int N = op.N;
+  const int W_BYTES = N * K * 2;                         // one image of a weight matrix
+  char *A_st = smem;                                     // stage s at s * PARTS * A_BYTES
+  char *W_st = smem + (size_t) S * PARTS * A_BYTES;      // buffer b at b * PARTS * W_BYTES
+  float *tr_all = reinterpret_cast<float *>(W_st + (size_t) S * PARTS * W_BYTES);    // transpose buffers of the epilogue warps
   for (int q = t; q < ntensors; q += NTHREADS) s_T[q] = Tg[q];
   for (int q = t; q < op.nrows; q += NTHREADS) s_rows[q] = op.rows[q];
   for (int q = t; q < op.nitems; q += NTHREADS) s_items[q] = op.items[q];
@@ -227,12 +246,12 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
     if (!c.valid) return;
     c.nt = min(TB, ntiles - tile0);
     c.i0 = c.it = s_rows[row].i0;
-    c.i1 = ELEM ? min(c.i0 + op.sub, s_rows[row].i1) : s_rows[row].i1;
+    c.i1 = op.parts ? min(c.i0 + op.sub, s_rows[row].i1) : s_rows[row].i1;
     c.tt = 0;
   };
-  // grouped atoms: the next items of the same row, an accumulator each
+  // rows in parts: the next items of the same row, an accumulator each
   auto next_part = [&](Cursor &c) -> bool {
-    if (!ELEM || c.i1 == s_rows[c.row].i1) return false;
+    if (c.i1 == s_rows[c.row].i1) return false;
     c.i0 = c.it = c.i1;
     c.i1 = min(c.i0 + op.sub, s_rows[c.row].i1);
     return true;
@@ -310,30 +329,30 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
         if (!ok) return;
       }
       const MVItem item = s_items[cur.it];
-      if (ELEM || cur.tt == 0) {    // first tile of an item (every tile of its own element): its weight image (hi + lo)
+      if (ELEM || cur.tt == 0) {    // first tile of an item (every tile of its own element): its weight images
         item_no++;
         if (t == 0) {
           // one bulk asynchronous copy; its bytes are counted by this stage's `full` barrier, so the matrix instructions
           // of the fill start when the image and the 256 arrivals are there, and no producer waits for the copy
-          const unsigned bar = smem_u32(&s_full[s]), dst = smem_u32(W_st + (size_t) (item_no % S) * 2 * W_BYTES);
+          const unsigned bar = smem_u32(&s_full[s]), dst = smem_u32(W_st + (size_t) (item_no % S) * PARTS * W_BYTES);
           const int e = ELEM ? __ldg(op.tiles + 1 + cur.tile0 + cur.tt) : 0;
-          const char *src = op.images + ((size_t) e * op.nmat + item.mat) * 2 * W_BYTES;
-          asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"((unsigned) (2 * W_BYTES)) : "memory");
+          const char *src = op.images + ((size_t) e * op.nmat + item.mat) * PARTS * W_BYTES;
+          asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"((unsigned) (PARTS * W_BYTES)) : "memory");
           asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                       ::"r"(dst), "l"(src), "r"((unsigned) (2 * W_BYTES)), "r"(bar) : "memory");
+                       ::"r"(dst), "l"(src), "r"((unsigned) (PARTS * W_BYTES)), "r"(bar) : "memory");
         }
       }
-      {    // registers -> tf32 hi / lo operand images of stage s
-        char *hi = A_st + (size_t) s * 2 * A_BYTES, *lo = hi + A_BYTES;
+      {    // registers -> operand images of stage s
+        char *img = A_st + (size_t) s * PARTS * A_BYTES;
 #pragma unroll
         for (int j = 0; j < PER; j++) {
           const int u = warp + NW * j, c4 = (u / 16) * 4 + (lane >> 3);
           if (u < UNITS && c4 < K4) {
-            const int off = ((u % 16) * K4 + c4) * 128 + (lane & 7) * 16;
-            float4 h, l;
-            split4(mine.v[j], item.scale, h, l);
-            *reinterpret_cast<float4 *>(hi + off) = h;
-            *reinterpret_cast<float4 *>(lo + off) = l;
+            const int off = ((u % 16) * (K4 / 2) + (c4 >> 1)) * 128 + (lane & 7) * 16 + (c4 & 1) * 8;
+            uint2 part[PARTS];
+            split4(mine.v[j], item.scale, part);
+#pragma unroll
+            for (int p = 0; p < PARTS; p++) *reinterpret_cast<uint2 *>(img + p * A_BYTES + off) = part[p];
           }
         }
       }
@@ -352,7 +371,7 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
   } else if (warp == NW) {
     // ---------------- matrix-instruction issuer ----------------
     if (lane == 0) {
-      const unsigned idesc = make_idesc(N), idesc2 = make_idesc(NC);
+      const unsigned idesc = make_idesc(N);
       Cursor cur;
       start(cur, blockIdx.x * TB, blockIdx.y);
       int fill = 0, item_no = -1, rowc = 0;
@@ -367,29 +386,21 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
         ok = wait(&s_full[s], (unsigned) ((fill / S) & 1));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const unsigned a_hi = smem_u32(A_st + (size_t) s * 2 * A_BYTES);
-        const unsigned b_hi = smem_u32(W_st + (size_t) (item_no % S) * 2 * W_BYTES);
-        const unsigned long long dA[2] = {make_desc(a_hi, K), make_desc(a_hi + A_BYTES, K)};
-        const unsigned long long dB[2] = {make_desc(b_hi, K), make_desc(b_hi + W_BYTES, K)};
-        const int sub = ELEM ? cur.it - cur.i0 : SEP ? (cur.it - cur.i0) % op.sub : 0;
-        const unsigned d = tmem + (unsigned) (((set * TB + cur.tt) * op.sub + sub) * NC);
-        const bool acc0 = !ELEM && cur.it - cur.i0 >= op.sub;
-        if constexpr (SEP) {
-          // the lo image of the weights lies behind the hi image like rows N .. 2 N - 1 of one matrix: a_hi meets both at once
+        const unsigned long long dA = make_desc(smem_u32(A_st + (size_t) s * PARTS * A_BYTES), K);
+        const unsigned long long dB = make_desc(smem_u32(W_st + (size_t) (item_no % S) * PARTS * W_BYTES), K);
+        const int at = cur.it - cur.i0;    // items take the accumulators of a1 b1 in turn
+        const unsigned base = tmem + (unsigned) ((set * TB + cur.tt) * op.cols), d1 = base + (unsigned) (at % op.sub * N);
+        const unsigned ds = SEP ? base + (unsigned) (op.sub * N) : d1;
+        const bool acc1 = at >= op.sub, accs = SEP ? at > 0 : acc1;
 #pragma unroll
-          for (int ks = 0; ks < K / 8; ks++)
-            mma_tf32_ss(d, dA[0] + (unsigned long long) (ks * 16), dB[0] + (unsigned long long) (ks * 16), idesc2, acc0 || ks > 0);
+        for (int q = 0; q < 6; q++) {
+          const bool big = SEP && q == 5;
+          const unsigned long long a = dA + (unsigned long long) (PRODUCTS[q][0] * (A_BYTES >> 4));
+          const unsigned long long b = dB + (unsigned long long) (unsigned) (PRODUCTS[q][1] * (W_BYTES >> 4));
 #pragma unroll
-          for (int ks = 0; ks < K / 8; ks++)
-            mma_tf32_ss(d + (unsigned) N, dA[1] + (unsigned long long) (ks * 16), dB[0] + (unsigned long long) (ks * 16), idesc, true);
-        } else {
-#pragma unroll
-          for (int pass = 0; pass < 3; pass++) {    // small terms first: a_lo b_hi, a_hi b_lo, a_hi b_hi
-            const unsigned long long a = dA[pass == 0 ? 1 : 0], b = dB[pass == 1 ? 1 : 0];
-#pragma unroll
-            for (int ks = 0; ks < K / 8; ks++)
-              mma_tf32_ss(d, a + (unsigned long long) (ks * 16), b + (unsigned long long) (ks * 16), idesc, acc0 || pass > 0 || ks > 0);
-          }
+          for (int ks = 0; ks < K / 16; ks++)
+            mma_bf16_ss(big ? d1 : ds, a + (unsigned long long) (ks * 16), b + (unsigned long long) (ks * 16), idesc,
+                        big ? acc1 || ks > 0 : accs || q > 0 || ks > 0);
         }
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&s_empty[s])) : "memory");
         Cursor nx = cur;
@@ -449,11 +460,12 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
             }
           }
           float v[CB];
-          const unsigned from = tmem + ((unsigned) (ew * 32) << 16) + (unsigned) ((set * TB + tt) * op.sub * N + c0);
+          const unsigned from = tmem + ((unsigned) (ew * 32) << 16) + (unsigned) ((set * TB + tt) * op.cols + c0);
           tmem_ld_rows(from, v);
-          for (int k = 1; k < cur.i1 - cur.i0; k++) {    // the other accumulators of the row
+          const int nacc = cur.i1 - cur.i0;
+          for (int k = 1; k < nacc + (SEP ? 1 : 0); k++) {    // the other accumulators of the row, the one of the small products last
             float w[CB];
-            tmem_ld_rows(from + (unsigned) (k * N), w);
+            tmem_ld_rows(from + (unsigned) ((k < nacc ? k : op.sub) * N), w);
 #pragma unroll
             for (int q = 0; q < CB; q++) v[q] += w[q];
           }
@@ -476,13 +488,14 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
           }
         }
       } else {
-        const bool vec = ((dstT.C | row.n_out) & 3) == 0;
+        const bool add = row.accumulate || cur.i0 > row.i0, vec = ((dstT.C | row.n_out) & 3) == 0;
         // atom of row r of this warp's quarter of tile tt, -1: none
         auto atom_of = [&](int tt, int r) {
           const int at = (cur.tile0 + tt) * TM + ew * 32 + r;
           return at < na ? at : -1;
         };
-        // the old values of an accumulating row are fetched one block ahead of the block being written
+        // the old values of an accumulating row are fetched one block ahead of the block being written (later parts of a row add to
+        // what this thread wrote before)
         float4 old[32 / RPI], oldn[32 / RPI];
         auto load_old = [&](int b, float4 (&o)[32 / RPI]) {
           const int tt = b / nblk, c0 = (b - tt * nblk) * CB;
@@ -492,16 +505,17 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
             o[j] = a >= 0 ? __ldcg(reinterpret_cast<const float4 *>(out + (size_t) a * dstT.C + c0) + cq) : make_float4(0.f, 0.f, 0.f, 0.f);
           }
         };
-        if (row.accumulate && vec) load_old(0, oldn);
+        if (add && vec) load_old(0, oldn);
         for (int b = 0; b < nb; b++) {
           const int tt = b / nblk, c0 = (b - tt * nblk) * CB;
           float v[CB];
-          const unsigned at = tmem + ((unsigned) (ew * 32) << 16) + (unsigned) ((set * TB + tt) * op.sub * NC + c0);
+          const unsigned at = tmem + ((unsigned) (ew * 32) << 16) + (unsigned) ((set * TB + tt) * op.cols + c0);
           tmem_ld<CB>(at, v);
-          if constexpr (SEP) {    // the other accumulators, the small terms among them
-            for (int k = 1; k < 2 * min(op.sub, row.i1 - row.i0); k++) {
+          if constexpr (SEP) {    // the other accumulators, the one of the small products last
+            const int nacc = min(op.sub, cur.i1 - cur.i0);
+            for (int k = 1; k <= nacc; k++) {
               float w[CB];
-              tmem_ld<CB>(at + (unsigned) (k * N), w);
+              tmem_ld<CB>(at + (unsigned) ((k < nacc ? k : op.sub) * N), w);
 #pragma unroll
               for (int q = 0; q < CB; q++) v[q] += w[q];
             }
@@ -518,11 +532,11 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
               if (a < 0) continue;
               float *o = out + (size_t) a * dstT.C + c0 + c;
               const float x = tr[r * (CB + 4) + c];
-              *o = row.accumulate ? *o + x : x;
+              *o = add ? *o + x : x;
             }
             continue;
           }
-          if (row.accumulate) {
+          if (add) {
 #pragma unroll
             for (int j = 0; j < 32 / RPI; j++) old[j] = oldn[j];
             load_old(b + 1, oldn);
@@ -532,7 +546,7 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
             const int r = j * RPI + lane / LPR, cq = lane % LPR, a = c0 + 4 * cq < row.n_out ? atom_of(tt, r) : -1;
             if (a >= 0) {
               float4 w = *reinterpret_cast<const float4 *>(tr + r * (CB + 4) + 4 * cq);
-              if (row.accumulate) {
+              if (add) {
                 w.x += old[j].x; w.y += old[j].y; w.z += old[j].z; w.w += old[j].w;
               }
               reinterpret_cast<float4 *>(out + (size_t) a * dstT.C + c0)[cq] = w;
@@ -556,12 +570,12 @@ __global__ void __launch_bounds__(block_threads(K, ELEM), 1) mv_tc_kernel(MVTCDe
 size_t smem_bytes(int K, int N, int S)
 {
   const size_t cb = N % 32 == 0 ? 32 : 16;
-  return (size_t) S * 2 * TM * K * 4 + (size_t) S * 2 * N * K * 4 + (size_t) 4 * 32 * (cb + 4) * 4;
+  return (size_t) S * PARTS * (TM + N) * K * 2 + (size_t) 4 * 32 * (cb + 4) * 4;
 }
 
 int stages_for(int K, int N) { return smem_bytes(K, N, 4) <= 200 * 1024 ? 4 : 2; }
 
-template<int K, int CB, int S, bool ELEM, bool SEP = false>
+template<int K, int CB, int S, bool ELEM, bool SEP>
 void launch_s(const MVTCDev &op, const TensorDev *T, int ntensors, int NA, int na, int TB, int tmem_cols, dim3 grid, int *error)
 {
   const size_t smem = smem_bytes(K, op.N, S);
@@ -579,20 +593,21 @@ void launch_s(const MVTCDev &op, const TensorDev *T, int ntensors, int NA, int n
 template<int K, bool ELEM> void launch_k(const MVTCDev &op, const TensorDev *T, int ntensors, int NA, int na, int TB, dim3 grid, int *error)
 {
   int tmem_cols = 32;    // a power of two that holds two sets of accumulators of TB tiles
-  while (tmem_cols < 2 * TB * op.sub * op.N * (op.sep ? 2 : 1)) tmem_cols *= 2;
+  while (tmem_cols < 2 * TB * op.cols) tmem_cols *= 2;
   const bool s4 = stages_for(K, op.N) == 4;
   if constexpr (ELEM) {
-    if (s4) launch_s<K, 16, 4, true>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
-    else launch_s<K, 16, 2, true>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+    if (s4 && op.sep) launch_s<K, 16, 4, true, true>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+    else if (op.sep) launch_s<K, 16, 2, true, true>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+    else launch_s<K, 16, 2, true, false>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
   } else if (op.sep) {    // (16 columns at a time: 32 of both accumulators do not fit the registers)
     if (s4) launch_s<K, 16, 4, false, true>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
     else launch_s<K, 16, 2, false, true>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
   } else if (op.N % 32 == 0) {
-    if (s4) launch_s<K, 32, 4, false>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
-    else launch_s<K, 32, 2, false>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+    if (s4) launch_s<K, 32, 4, false, false>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+    else launch_s<K, 32, 2, false, false>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
   } else {
-    if (s4) launch_s<K, 16, 4, false>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
-    else launch_s<K, 16, 2, false>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+    if (s4) launch_s<K, 16, 4, false, false>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
+    else launch_s<K, 16, 2, false, false>(op, T, ntensors, NA, na, TB, tmem_cols, grid, error);
   }
 }
 
@@ -606,22 +621,20 @@ template<bool ELEM> void launch_e(int K, const MVTCDev &op, const TensorDev *T, 
   }
 }
 
-// operand images of the matrices of an operation: B[n][k] = W[k][n], hi (rounded to tf32) then lo, zero beyond the matrix;
+// operand images of the matrices of an operation: B[n][k] = W[k][n] in its bf16 parts, zero beyond the matrix;
 // grid (matrices, elements)
 __global__ void __launch_bounds__(256) mv_images_kernel(const float *__restrict__ W, const int4 *__restrict__ mats, long long ty_stride,
                                                         int K, int N, char *images, int nmat, int first)
 {
   const int4 m = mats[blockIdx.x];    // offset, rows, row stride, columns
   const float *M = W + (long long) blockIdx.y * ty_stride + m.x;
-  char *o = images + ((size_t) blockIdx.y * nmat + first + blockIdx.x) * 2 * N * K * 4;
+  char *o = images + ((size_t) blockIdx.y * nmat + first + blockIdx.x) * PARTS * N * K * 2;
   for (int e = threadIdx.x; e < N * K; e += 256) {
     const int n = e / K, k = e - n * K;
     const float w = k < m.y && n < m.w ? M[(long long) k * m.z + n] : 0.0f;
-    const unsigned h = (__float_as_uint(w) + 0x1000u) & 0xffffe000u;    // nearest tf32 (10-bit mantissa)
-    const unsigned l = (__float_as_uint(w - __uint_as_float(h)) + 0x1000u) & 0xffffe000u;
-    const int at = tile_off(n, k, K);
-    *reinterpret_cast<unsigned *>(o + at) = h;
-    *reinterpret_cast<unsigned *>(o + (size_t) N * K * 4 + at) = l;
+    uint2 part[PARTS];
+    split4(make_float4(w, 0.f, 0.f, 0.f), 1.0f, part);
+    for (int p = 0; p < PARTS; p++) *reinterpret_cast<unsigned short *>(o + (size_t) p * N * K * 2 + tile_off(n, k, K)) = (unsigned short) part[p].x;
   }
 }
 
@@ -771,9 +784,12 @@ void MVTensorCore::setup(const std::vector<const MVOp *> &ops, const std::vector
 {
   K_ = N_ = 0;
   elem_ = ops[0]->elem;
+  odd_ = false;
   for (const MVOp *o : ops) {
     K_ = std::max(K_, padded_k(*o));
     N_ = std::max(N_, padded_n(o->n_out));
+    odd_ = odd_ || o->n_out % 16 != 0;
+    for (const MVItem &it : o->items) odd_ = odd_ || (it.n_in != 8 && it.n_in != 16 && it.n_in != 32 && it.n_in != 64);
   }
   // rows of all operations; a row that several of them write gets the items of all (the first decides whether it adds)
   std::map<std::pair<int, int>, int> index;
@@ -813,12 +829,14 @@ void MVTensorCore::setup(const std::vector<const MVOp *> &ops, const std::vector
     rows[r].i1 = (int) items.size();
   }
   nrows_ = (int) rows.size();
+  long_ = false;
+  for (const MVRowDev &r : rows) long_ = long_ || r.i1 - r.i0 > LONG_ROW;
   nitems_ = (int) items.size();
-  images_.set_label("engine:weights_tf32");
+  images_.set_label("engine:weights_bf16");
   items_.set_label("engine:tables");
   rows_.set_label("engine:tables");
   const int ne = elem_ ? n_elements : 1;
-  images_.ensure((size_t) ne * nmat_ * 2 * N_ * K_ * 4);
+  images_.ensure((size_t) ne * nmat_ * PARTS * N_ * K_ * 2);
   items_.upload(items);
   rows_.upload(rows);
   first = 0;
@@ -854,17 +872,17 @@ void MVTensorCore::launch(const TensorDev *tensors, int ntensors, int NA, int na
   }
   // one CTA per SM; two sets of accumulators share the 512 tensor-memory columns
   const int G = dev().sm_count;
-  // The rows of reduces over the element are sums of up to 89 items.  The tensor cores cut off what they add (towards zero, one
-  // bit of 2^-24 per instruction and accumulator): 240 instructions in one accumulator are a bias of 8e-6, and even six items
-  // left per-atom energies of GRACE-1L of order 4 at 1.8e-6 where fp32 sums are at 2.2e-7.  So every item has an accumulator of its
+  // Separate accumulators: operations with per-element weights and widths other than 8, 16, 32 and 64 at any size and everything while
+  // a CTA has at most one tile, where fp32 sums are the measure.  With more atoms the usual widths go without: a second read of the
+  // epilogue and half as many tiles per CTA cost more (64 x 64, 1,024,000 atoms 27.8 -> 40.1 ms).
+  // Rows of reduces over the element and of the UQ projection are sums of up to a hundred items; every item has an accumulator of its
   // own, as many at a time as there are columns for, and the epilogue adds them with rounding, part of a row after part.
-  // With at most one tile per CTA there is room for accumulators of their own for the small terms, and for items that take turns in
-  // several: fewer instructions cut something off the large sums (GRACE-3L, 54 atoms, per-atom energies against fp64: 1.4e-6 -> SEPERR,
-  // fp32 sums 4.9e-7).  With more atoms the second read of the epilogue and half as many tiles cost more than they give: 64 x 64, 31,250
-  // atoms 29.7 -> 33.7 ms, 1,024,000 atoms 27.8 -> 40.1 ms.
-  op.sep = !elem_ && 4 * N_ <= TMEM_COLS && ntiles <= G;
-  op.sub = elem_ ? std::max(1, std::min(16, TMEM_COLS / 2 / N_)) : op.sep ? std::min(4, TMEM_COLS / 4 / N_) : 1;
-  const int tb_max = elem_ || op.sep ? 1 : std::max(1, std::min(MAX_TILES, TMEM_COLS / 2 / N_));
+  op.sep = 2 * N_ <= TMEM_COLS / 2 && (elem_ || odd_ || ntiles <= G);
+  const int held = TMEM_COLS / 2 / N_ - (op.sep ? 1 : 0);
+  op.sub = elem_ ? std::max(1, std::min(15, held)) : op.sep && ntiles <= G ? std::min(4, held) : 1;
+  op.cols = (op.sub + (op.sep ? 1 : 0)) * N_;
+  op.parts = elem_ || (op.sep && ntiles <= G && long_);
+  const int tb_max = elem_ || ntiles <= G ? 1 : std::max(1, std::min(MAX_TILES, TMEM_COLS / 2 / op.cols));
   const int rounds = (ntiles + G * tb_max - 1) / (G * tb_max);
   const int TB = std::max(1, std::min(tb_max, (ntiles + G * rounds - 1) / (G * rounds)));
   const int gx = std::min(G, (ntiles + TB - 1) / TB);

@@ -17,11 +17,13 @@ struct MVRowDev {
 struct MVTCDev {
   const MVRowDev *rows;
   const MVItem *items;     // as MVDev::items with `mat` = index of the matrix's operand image
-  const char *images;      // per element and matrix: [N][K] tf32 hi image, then the lo image (canonical K-major layout)
+  const char *images;      // per element and matrix: the [N][K] images of its three bf16 parts (canonical K-major layout)
   const int *order, *tiles;    // per-element weights: ElemOrder
   int N, nrows, nitems, nmat;
-  bool sep;                // accumulators of their own for the small terms
-  int sub;                 // accumulators, one per item, that a part of a row has (per-element weights)
+  bool sep;                // an accumulator of its own for the small products
+  bool parts;              // rows in parts of `sub` items, each with an accumulator of its own
+  int sub;                 // accumulators of a1 b1 that the items of a row take in turn
+  int cols;                // columns of a tile's accumulators
 };
 
 // The atoms of a chunk grouped by element, for operations with per-element weights: tiles of 128 atoms of one element.
@@ -53,7 +55,7 @@ class MVTensorCore {
   void launch(const TensorDev *tensors, int ntensors, int NA, int na, int *error, const ElemOrder *order) const;
 
  private:
-  bool ready_ = false, elem_ = false;
+  bool ready_ = false, elem_ = false, odd_ = false, long_ = false;    // odd_: a width other than 8, 16, 32, 64 (inputs), multiples of 16 (outputs); long_: LONG_ROW
   int K_ = 0, N_ = 0, nrows_ = 0, nitems_ = 0, nmat_ = 0;
   DBuf<char> images_;
   DBuf<MVItem> items_;

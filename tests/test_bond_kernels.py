@@ -157,3 +157,55 @@ def test_freed_blocks_count_as_free_memory(backend, tmp_path):
     finally:
         del fill
         torch.cuda.empty_cache()
+
+
+def _fp64(kind, path, els, c, uq):
+    if kind == "3l":
+        from oracle.grace3l_oracle import Grace3LOracle
+        return Grace3LOracle(path).compute(els, *c)
+    from oracle.grace_oracle import GraceOracle
+    return GraceOracle(path, spline_n=1024).compute(els, *c, uq=uq)
+
+
+@pytest.mark.parametrize("kind,reps,copies", [("1l", (6, 7, 7), None), ("2l", (5, 5, 6), None), ("3l", (3, 3, 3), None), ("uq", (5, 5, 6), None),
+                                              ("2l", (3, 3, 4), (5, 6, 5)), ("odd", (3, 3, 4), (5, 6, 5))])
+def test_tensor_core_sums_are_no_further_off_than_fp32(backend, tmp_path, monkeypatch, kind, reps, copies):
+    """Errors against the fp64 oracle of the tensor-core operations and of the fp32 kernels (GRACE_B200_DENSE=ops), root mean square of
+    two structures: at few atoms, where the small products have accumulators of their own, and above 18,944 atoms (copies of a
+    cell), where the usual widths go without and others (odd: 24, 12 and 40 channels) do not.  The margins: the two errors are
+    of 2 x 50 atoms at least and hardly correlated, they scatter by 20 % (energies, forces); the grade's, of fewer and smaller sums, by
+    twice that.  With two tf32 parts per operand the ratios were 1.6 (GRACE-3L) and 16 (grade)."""
+    from grace_runtime_b200 import modelgen, modelgen3l, structures
+    els = ["Al", "Cu", "Ni", "W"]
+    path, lattice, a = str(tmp_path / "m.npz"), "fcc", 3.6
+    if kind == "3l":
+        lattice, a = "bcc", 3.2
+        modelgen3l.write_model_3l(path, elements=els, lmax=4, channels=(64, 64, 64), rho_width=32, embedding=16, radial_hidden=128,
+                                  energy_hidden=64, rcut=6.0, avg_neigh=58.0, seed=0)
+    elif kind == "uq":
+        plain = modelgen.write_model(path + ".plain.npz", elements=tuple(els), seed=0, **dict(modelgen.CONFIGS["2l"], max_order=4, lmax=2))
+        modelgen.add_uq_head(plain, path, seed=0)
+    elif kind == "odd":
+        modelgen.write_model(path, elements=tuple(els), seed=0, **dict(modelgen.CONFIGS["2l"], c1=24, cr=12, c2=40))
+    else:
+        lattice, a = ("bcc", 3.2) if kind == "1l" else (lattice, a)
+        modelgen.write_config_model(path, kind, els, seed=0)
+    err = {}
+    for seed in (1, 2):
+        types, pos, cell, pbc = structures.crystal(lattice, a, reps, n_species=4, sigma=0.06, seed=seed)
+        o = _fp64(kind, path, els, (types, pos, cell, pbc), kind == "uq")
+        m = 1
+        if copies:
+            shift = np.stack(np.meshgrid(*[np.arange(k) for k in copies], indexing="ij"), -1).reshape(-1, 3) @ cell
+            m, pos = len(shift), (pos[None] + shift[:, None]).reshape(-1, 3)
+            types, cell = np.tile(types, m), cell * np.array(copies)[:, None]
+        for mode in ("tc", "ops"):
+            monkeypatch.setenv("GRACE_B200_DENSE", mode)
+            r = backend.System(backend.Model(path), els).compute(types, pos, cell, pbc, energies=True, uq=kind == "uq")
+            for q in ("energies", "forces", "gamma"):
+                if q in o and q in r:
+                    err.setdefault((q, mode), []).append(_rel(r[q], np.tile(o[q], (m,) + (1,) * (o[q].ndim - 1))))
+    for q, mode in err:
+        if mode == "tc":
+            e = {k: np.sqrt(np.mean(np.square(err[q, k]))) for k in ("tc", "ops")}
+            assert e["tc"] < (1.4 if q == "gamma" else 1.2) * e["ops"], (q, e)
