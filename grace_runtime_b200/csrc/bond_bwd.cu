@@ -285,18 +285,34 @@ __device__ __forceinline__ void bwd_virial(double (&vred)[4][6], double (&vir)[6
   }
 }
 
-// Blocks per SM the kernels are compiled for and bonds per round, so that registers and shared memory allow the same number.
-// They wait for the table and for shared memory most of the time: warps in flight count for more than a few spilled registers.
+// Blocks per SM the kernels are compiled for, and bonds per round: as many as fit the shared memory of that many blocks, at most
+// one per thread (lmax 3: 97 and, with messages, 124; lmax 4: 65 and 115).  They wait for the table and for shared memory most of the
+// time: warps in flight count for more than a few spilled registers.  An atom that needs a second round pays two more barriers;
+// that the larger stage leaves less L1 does not show.  ns per bond at 60, 83, 94 and 104 neighbours, lmax 3: 0.300, 0.279, 0.258, 0.276
+// (with 78 bonds 0.301, 0.319, 0.303, 0.292, with 64 0.301, 0.321, 0.303, 0.292), with messages 0.470, 0.440, 0.407, 0.406 (80 bonds
+// 0.468, 0.460, 0.461, 0.447); lmax 4 at 60, 66, 73 and 81: 0.404, 0.375, 0.348, 0.381 (60 bonds 0.404, 0.407, 0.388, 0.385).
+constexpr size_t SM_SHARED = 228 * 1024, BLOCK_RESERVED = 1024;
+template<int ROW> __host__ __device__ constexpr int stage_bonds(int blocks)
+{
+  constexpr size_t fixed = sizeof(BwdStage<ROW, 1>) - (sizeof(BwdStage<ROW, 17>) - sizeof(BwdStage<ROW, 1>)) / 16;    // 16 bonds: no padding
+  constexpr size_t per = (sizeof(BwdStage<ROW, 17>) - sizeof(BwdStage<ROW, 1>)) / 16;
+  const size_t n = (SM_SHARED / blocks - BLOCK_RESERVED - fixed) / per;
+  return n < 128 ? (int) n : 128;
+}
 template<int LMAX> __host__ __device__ constexpr int pair_blocks() { return 4; }
-template<int LMAX> __host__ __device__ constexpr int pair_bonds() { return LMAX <= 3 ? 78 : 60; }
 template<int LMAX> __host__ __device__ constexpr int msg_blocks() { return LMAX <= 3 ? 3 : 2; }
-template<int LMAX> __host__ __device__ constexpr int msg_bonds() { return LMAX <= 3 ? 80 : 64; }
-template<int LMAX> using PairStage = BwdStage<2 * (LMAX + 1) * (LMAX + 1) + 1, pair_bonds<LMAX>()>;
 // The four 16-byte words a load instruction of the message kernel reads, (bond, group of harmonics), lie in different banks: the
 // groups are an odd number of words apart and the bonds three.
 template<int LMAX> __host__ __device__ constexpr int msg_half() { return 2 * LmSplit<LMAX>::NK + 1; }
 template<int LMAX> __host__ __device__ constexpr int msg_row() { return 2 * msg_half<LMAX>() + (8 + 3 - 2 * msg_half<LMAX>() % 8) % 8; }
+template<int LMAX> __host__ __device__ constexpr int pair_row() { return 2 * (LMAX + 1) * (LMAX + 1) + 1; }
+template<int LMAX> __host__ __device__ constexpr int pair_bonds() { return stage_bonds<pair_row<LMAX>()>(pair_blocks<LMAX>()); }
+template<int LMAX> __host__ __device__ constexpr int msg_bonds() { return stage_bonds<msg_row<LMAX>()>(msg_blocks<LMAX>()); }
+template<int LMAX> using PairStage = BwdStage<pair_row<LMAX>(), pair_bonds<LMAX>()>;
 template<int LMAX> using MsgStage = BwdStage<msg_row<LMAX>(), msg_bonds<LMAX>()>;
+static_assert(pair_bonds<3>() == 97 && msg_bonds<3>() == 124 && pair_bonds<4>() == 65 && msg_bonds<4>() == 115, "");
+static_assert(4 * (sizeof(PairStage<3>) + BLOCK_RESERVED) <= SM_SHARED && 3 * (sizeof(MsgStage<3>) + BLOCK_RESERVED) <= SM_SHARED, "");
+static_assert(4 * (sizeof(PairStage<4>) + BLOCK_RESERVED) <= SM_SHARED && 2 * (sizeof(MsgStage<4>) + BLOCK_RESERVED) <= SM_SHARED, "");
 
 // Layers without message functions and with an even number of channels: LPB lanes per bond, two channels per lane, 32 / LPB
 // bonds per warp at a time, with the gradients of its channels in a lane's registers.  With the chemical weight folded into

@@ -209,3 +209,25 @@ def test_tensor_core_sums_are_no_further_off_than_fp32(backend, tmp_path, monkey
         if mode == "tc":
             e = {k: np.sqrt(np.mean(np.square(err[q, k]))) for k in ("tc", "ops")}
             assert e["tc"] < (1.4 if q == "gamma" else 1.2) * e["ops"], (q, e)
+
+
+@pytest.mark.parametrize("layers,lmax", [(1, 2), (1, 3), (1, 4), (2, 2), (2, 3)])
+@pytest.mark.parametrize("neighbours", [64, 66, 97, 98, 124, 125, 129])
+def test_bond_sums_at_the_edges_of_their_rounds(backend, tmp_path, layers, lmax, neighbours):
+    """A cluster in which every atom sees all the others: as many bonds as a round of the reverse kernels holds, and one more (csrc/
+    bond_bwd.cu: 65, 97, 124 or the 128 threads; the forward kernels stage 96)."""
+    from grace_runtime_b200 import modelgen
+    from oracle.grace_oracle import GraceOracle
+    els = ["Al", "Cu", "Ni"]
+    path = modelgen.write_config_model(str(tmp_path / "m.npz"), "1l" if layers == 1 else "2l", els, seed=3) if lmax == 5 - layers else \
+        modelgen.write_model(str(tmp_path / "m.npz"), layers=layers, lmax=lmax, max_order=3, elements=tuple(els), seed=3)
+    rng = np.random.default_rng(neighbours)
+    g = np.stack(np.meshgrid(*[np.arange(-3, 4)] * 3, indexing="ij"), -1).reshape(-1, 3) * 0.9
+    g = g[np.argsort((g * g).sum(1) + 1e-3 * rng.random(len(g)))][:neighbours + 1] + 0.1 * (rng.random((neighbours + 1, 3)) - 0.5)
+    assert np.linalg.norm(g[:, None] - g[None], axis=2).max() < 6.0
+    types = rng.integers(1, 4, size=len(g)).astype(np.int32)
+    args = (types, g + 20.0, np.eye(3) * 40.0, np.zeros(3, dtype=np.uint8))
+    r, o = backend.System(backend.Model(path), els).compute(*args, energies=True), GraceOracle(path, spline_n=1024).compute(els, *args)
+    assert _rel(r["energies"], o["energies"]) < 1e-5
+    assert _rel(r["forces"], o["forces"]) < 1e-5
+    assert _rel(r["virial"], o["virial"]) < 1e-5
