@@ -589,10 +589,10 @@ def run_ours(args, rank, world, local_rank):
             ach = fl_atom * n_own / (step_ms * 1e-3) / 1e12
             peak_tf = peaks_here["tf32_tensor_tflops"] / 3.0
             roof = {"bound": "tensor", "kernel": top, "peak": peak_tf,
-                    "peak_source": "tf32 tcgen05 microbenchmark of this run (M 128, N 256) / 3: three tf32 instructions per fp32-accurate product",
+                    "peak_source": "tf32 tcgen05 microbenchmark of this run (M 128, N 256) / 3: an fp32-accurate product is six bf16 ones, which take the time of three tf32 ones",
                     "unit": "TFLOP/s", "achieved": ach, "frac": ach / peak_tf, "traffic": traffic_of(top, lps),
                     "hbm_achieved_GBs": gbs, "hbm_frac_of_measured": gbs / hbm_peak,
-                    "note": "FC layers and adjoints as 3 x tf32 grouped GEMMs with N = 32 / 64; the tf32 rate of an N = 32 (64) "
+                    "note": "FC layers and adjoints as grouped GEMMs of three bf16 parts per operand with N = 32 / 64; the rate of an N = 32 (64) "
                             "instruction is 0.29 (0.57) of the N = 256 one (grace_measure_peak), and the kernel streams its "
                             "operands from HBM: hbm_frac_of_measured is the tighter bound"}
         else:
@@ -606,12 +606,9 @@ def run_ours(args, rank, world, local_rank):
         lps = top_n / args.steps
         flop = model.dense_flops * n_own / lps
         ach = flop / (per_launch_ms * 1e-3) / 1e12
-        tensor = top.startswith("chain_tc")
-        # a 3 x tf32 product issues three tensor-core instructions per useful multiply-add
-        peak_tf = peaks_here["tf32_tensor_tflops"] / 3.0 if tensor else peaks_here["fp32_simt_tflops"]
-        roof = {"bound": "tensor" if tensor else "fp32", "kernel": top, "peak": peak_tf,
-                "peak_source": ("tf32 tcgen05 microbenchmark of this run / 3 (three tf32 instructions per fp32-accurate product)"
-                                if tensor else "fp32 FFMA microbenchmark of this run (measured in this run)"),
+        peak_tf = peaks_here["fp32_simt_tflops"]
+        roof = {"bound": "fp32", "kernel": top, "peak": peak_tf,
+                "peak_source": "fp32 FFMA microbenchmark of this run (measured in this run)",
                 "unit": "TFLOP/s", "achieved": ach, "frac": ach / peak_tf, "traffic": traffic_of(top, lps),
                 "algorithmic_bytes_per_launch": 2.0 * 4.0 * (modelgen.CONFIGS[wl["cfg"]]["lmax"] + 1) ** 2 * modelgen.CONFIGS[wl["cfg"]]["c1"] * n_own / lps,
                 "flop_per_launch": flop, "flop_per_atom": model.dense_flops, "avg_launch_ms": per_launch_ms,
@@ -631,7 +628,7 @@ def run_ours(args, rank, world, local_rank):
                 "unit": "TFLOP/s", "achieved": ach, "frac": ach / peak_tf, "traffic": None, "flop_per_step": flop,
                 "ms_per_step": top_ms / args.steps, "launches_per_step": lps,
                 "note": "useful flops of the coupled bond sums of layers 2 and 3 (lmax 4, 25 message functions, 64 channels) x "
-                        "bonds inside the cutoff / time of the kernel's launches of a step; first, untuned form of the kernel"}
+                        "bonds inside the cutoff / time of the kernel's launches of a step"}
     elif top.startswith("bond_"):
         # bond kernels: table look-ups from L1 / L2 and fp32 arithmetic per bond and channel - issue-bound, not HBM-bound
         # (their HBM fraction is in hbm_kernels); all launches of a step together (GRACE-2L: both layers)

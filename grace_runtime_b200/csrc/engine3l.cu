@@ -4,7 +4,7 @@
 // projections, couples, reduces, FCs: the same kernels as GRACE-1L / 2L), EquivariantRMSNorm of the message and RMSNorm
 // of the density; the readout on the sum of the three densities; then everything in reverse.  While they fit, the
 // tensors of the three layers of all atoms are kept for the reverse pass; larger structures run every layer in passes
-// over atom chunks and recompute a chunk's forward tensors when it is reversed.  A first form of the path, checked
+// over atom chunks and recompute a chunk's forward tensors when it is reversed.  Checked
 // against the reference's CPU engine.
 #include "engine.h"
 

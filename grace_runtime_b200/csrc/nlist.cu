@@ -379,7 +379,9 @@ __global__ void __launch_bounds__(256) nl_neigh(const double *__restrict__ xs, c
 }
 
 // The same with a thread per atom: a third of the instructions (no scan, no search for a candidate's run), and the threads
-// of a warp walk the same bins; faster once the atoms fill the GPU by themselves (557,000 atoms: 0.8 against 1.4 ms).
+// of a warp walk the same bins; faster once the atoms fill the GPU by themselves.  Both searches of a build, thread / warp, us: bcc
+// of 58 neighbours 64,000 atoms 351 / 275, 128,000 494 / 504, 195,000 763 / 732, 250,000 877 / 946; fcc of 78 131,000 657 / 644, 256,000
+// 1,123 / 1,215; fcc of 42 131,000 430 / 434, 389,000 1,008 / 1,230.
 template<bool FILL>
 __global__ void __launch_bounds__(128) nl_neigh_thread(const double *__restrict__ xs, const int *__restrict__ sid_s,
                                                        const int *__restrict__ b3_s, const NLStructHost *__restrict__ S,

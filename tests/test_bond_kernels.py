@@ -231,3 +231,19 @@ def test_bond_sums_at_the_edges_of_their_rounds(backend, tmp_path, layers, lmax,
     assert _rel(r["energies"], o["energies"]) < 1e-5
     assert _rel(r["forces"], o["forces"]) < 1e-5
     assert _rel(r["virial"], o["virial"]) < 1e-5
+
+
+@pytest.mark.parametrize("cr", [16, 6, 7])
+def test_message_gradients_by_atomics(backend, tmp_path, monkeypatch, cr):
+    """GRACE_B200_MSG_ATOMICS: what a call does whose buffer of message-gradient shares cannot be had - the reverse message kernels
+    (two channels per lane for 16 and 6, one for 7) add the shares of dE/dmsg atomically: the same forces."""
+    from grace_runtime_b200 import modelgen, structures
+    els = ["Al", "Cu", "Ni"]
+    path = modelgen.write_model(str(tmp_path / "m.npz"), layers=2, lmax=3, max_order=3, elements=tuple(els), cr=cr, c2=32, seed=3)
+    c = structures.crystal("fcc", 3.4, (3, 3, 2), n_species=3, sigma=0.1, seed=7)
+    model = backend.Model(path)
+    a = backend.System(model, els).compute(*c)
+    monkeypatch.setenv("GRACE_B200_MSG_ATOMICS", "1")
+    b = backend.System(model, els).compute(*c)
+    assert _rel(b["forces"], a["forces"]) < 1e-5
+    assert _rel(b["virial"], a["virial"]) < 1e-5

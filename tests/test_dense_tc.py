@@ -1,4 +1,4 @@
-"""The dense network on the tensor cores (csrc/mv_tc.cu: FC layers and their adjoints as tcgen05 3 x tf32 grouped GEMMs
+"""The dense network on the tensor cores (csrc/mv_tc.cu: FC layers and their adjoints as tcgen05 grouped GEMMs of bf16 parts
 over atom tiles, operation by operation on chunk tensors) against the fused fp32 kernel, the numpy oracle, the golden
 vectors and - where it travelled - the compiled reference.  The path is the default for large evaluations; here it is
 forced on small ones with GRACE_B200_DENSE=tc (read when a model's engine is built)."""

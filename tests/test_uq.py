@@ -16,7 +16,7 @@ from conftest import GOLDEN, model_path
 sys.path.insert(0, os.path.join(GOLDEN))
 from make_uq_golden import UQ_CELLS, UQ_MODELS, uq_model  # noqa: E402
 
-# gamma and sigma: the projection runs in fp32 (reference) / 3 x tf32 or fp32 (here) on an fp32 basis; everything after
+# gamma and sigma: the projection runs in fp32 (reference) / bf16 parts or fp32 (here) on an fp32 basis; everything after
 # it is fp64.  The reference documents ~1e-5 of its own fp32 projection against fp64.
 UQ_RTOL = 1e-4
 
