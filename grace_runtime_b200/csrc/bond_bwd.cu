@@ -317,7 +317,7 @@ static_assert(4 * (sizeof(PairStage<4>) + BLOCK_RESERVED) <= SM_SHARED && 2 * (s
 // Layers without message functions and with an even number of channels: LPB lanes per bond, two channels per lane, 32 / LPB
 // bonds per warp at a time, with the gradients of its channels in a lane's registers.  With the chemical weight folded into
 // the radial functions a harmonic costs four packed FMAs per lane and bond.  Bound by the shared-memory reads of the harmonics
-// and, at 16 warps per SM, by their latency.  Against one channel per lane: GRACE-2L, 1,024,000 atoms, lmax 3: 29.9 -> 23.7 ms;
+// and, at 16 warps per SM, by their latency.  Against one channel per lane: GRACE-2L, 1,024,000 atoms, lmax 3: 29.9 -> 23.0 ms;
 // GRACE-1L, 128,000 atoms, lmax 4: 3.81 -> 3.10 ms.
 template<int LMAX, int LPB>
 __global__ void __launch_bounds__(128, pair_blocks<LMAX>()) bond_bwd_pair_kernel(BondsDev b, LayerDev L, SHTable sht, const float *__restrict__ gQ, int NA, int a0,
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(128, pair_blocks<LMAX>()) bond_bwd_pair_kernel
 // everything is linear in h:
 //   dE/dx += dR_l Y_lm h,   g += R_l h grad Y_lm,   dE/dmsg_I += R_l Y_lm gQ[I][lm].
 // One channel per lane took 447 issued instructions per bond and was bound by them; this takes 228, at 12 warps per SM (168
-// registers; compiled for 16 warps it spills: 43 ms).  GRACE-2L, 1,024,000 atoms: 53.8 -> 36.8 ms.
+// registers; compiled for 16 warps it spills: 43 ms).  GRACE-2L, 1,024,000 atoms: 53.8 -> 36.7 ms.
 template<int LMAX>
 __global__ void __launch_bounds__(128, msg_blocks<LMAX>()) bond_bwd_msg_kernel(BondsDev b, LayerDev L, SHTable sht, const float *__restrict__ gQ, int NA, int a0,
                                                            float *__restrict__ fv, double *__restrict__ vir_atom, int add)
